@@ -4,9 +4,9 @@
 //
 // The host parses the chunk's page headers (Thrift compact protocol, parquet.thrift PageHeader)
 // and copies the chunk to the device once.  Then, on the device:
-//   1. Snappy pages are decompressed: a header walk per page finds where each of the
-//      compressor's independent 64 KB fragments starts, then one thread per fragment decodes it
-//      (a page that does not split that way is decoded by one thread);
+//   1. Snappy pages are decompressed: pointer doubling over the stream's bytes lists every
+//      element, then the compressor's independent 64 KB fragments resolve their copies by pointer
+//      jumping (a page that does not split that way is decoded by one thread);
 //   2. every RLE / bit-packed hybrid stream (definition levels, dictionary indices) gets a run
 //      table (one thread per stream walks the run headers, counting first, then filling);
 //   3. rows are decoded in 8,192-row tiles: definition levels give the validity bits, a block
@@ -200,35 +200,64 @@ constexpr int kPqTile = 8192;  // rows per decode tile: 256 threads x one 32-row
 // its input and no match reaches back past its fragment's start, so a page of N fragments is N
 // independent decodes once their starts in the stream are known.
 //
-// Both passes read the stream through a shared-memory window of kSnapWin bytes and first parse,
-// with all 32 lanes, the element header that WOULD start at every byte of the window (its size
-// with a literal's bytes, and its output length); following the real chain of elements through
-// the window is then one shared-memory load per element for one lane.
-//  * the walk (one 4-warp block per page) follows the chain over the whole page, one thread
-//    listing each window's element starts through next-element records (two elements per
-//    shared-memory round trip), then the block sums the listed elements' output lengths and
-//    records where each 64 KB fragment's elements start;
-//  * the decode (one warp per fragment) takes the chain 32 elements at a time, one per lane: a
-//    prefix sum gives each element's output position, literals are copied in parallel (long ones
-//    by the whole warp), and copies run in rounds of those whose source bytes are already written.
-//    The fragment is built in shared memory and written out with 16-byte stores;
-//  * a page whose elements cross a fragment boundary, or whose copies reach into an earlier
-//    fragment, is decoded again by one thread from start to end (the serial pass), which is also
-//    the pass that reports a malformed stream.
+// No pass follows the chain of elements one by one:
+//  * the maps (one block per kSnapBlk stream bytes): for every byte, the element that WOULD start
+//    there is parsed, and pointer doubling in shared memory (log2 of the elements in a block rounds)
+//    gives where the chain from that byte leaves the block, how many elements it passes and how many
+//    bytes they write;
+//  * the chain (one thread per page) steps from block to block through those maps, which gives each
+//    block the position its first element starts at;
+//  * the list (one block per kSnapBlk bytes again): doubling from that position marks the real element
+//    starts, and a scan numbers them and gives each its output position;
+//  * the decode (one block per fragment): every output byte starts as a pointer to itself (literals) or
+//    to the earlier output byte it copies, and pointer jumping in shared memory resolves all of them in
+//    log2 of the longest copy chain rounds, whatever the order of the elements;
+//  * a page whose elements cross a fragment boundary, or whose copies reach into an earlier fragment,
+//    is decoded again by one thread from start to end (the serial pass), which is also the pass that
+//    reports a malformed stream.
+//
+// Why: a page's elements are one dependent chain (a 977 KB dictionary page of doubles has ~247k of
+// them), so a thread that follows it is bound by a shared-memory round trip per element whatever the
+// chip has to offer.  Measured on such a page (125,000 prices, Snappy): one thread following the chain
+// through per-window records 6.5 ms and a warp per fragment decoding 2.3 ms; now maps 22 us, chain
+// 44 us, list 23 us and decode 58 us.
 struct SnapJob {
     const uint8_t* src;
     uint8_t* dst;
     uint32_t src_len, dst_len;
-    uint32_t plan;   // the page's plan in the plan buffer: [mode, first element, nfrag + 1 starts]
+    uint32_t plan;   // the page's plan in the plan buffer: [mode, first element, nfrag + 1 element numbers]
     uint32_t nfrag;  // 64 KB fragments of its output
+    uint32_t blk0;   // its first kSnapBlk block in the group's block array
+    uint32_t pad_;
+    uint64_t tab0;   // its first byte in the group's map table
+    uint64_t elem0;  // its first element in the group's element list
+};
+struct SnapMap {  // the chain from a stream byte to the end of its block
+    uint32_t exit;  // stream position of the first element past the block, or kSnapNone
+    uint32_t out;   // bytes the chain's elements write
+    uint32_t count; // elements
+    uint32_t pad_;
+};
+struct SnapEntry {  // a block's first element, as the page's chain reaches it
+    uint32_t pos, out, elem, valid;  // stream position, output position, number; valid == 1 or unset
 };
 constexpr uint32_t kSnapFrag = 1u << 16;  // the compressor's fragment
-constexpr uint32_t kSnapWin = 2048;       // stream bytes parsed per window
-constexpr uint32_t kSnapWinLoad = kSnapWin + 32;  // with room for the last headers' bytes
+constexpr uint32_t kSnapWin = 2048;       // the serial pass's window
+// Stream bytes per map / list block: the chain takes one dependent L2 load (~0.4 us) per block, a
+// doubling round in a block costs eight shared-memory steps per thread, and 8 KB gives a 1 MB page 122
+// blocks, one wave of the 148 SMs.
+constexpr uint32_t kSnapBlk = 8192;
+constexpr int kSnapThreads = 1024;
+constexpr uint32_t kSnapPer = kSnapBlk / kSnapThreads;
+constexpr uint32_t kSnapNone = 0xFFFFFFFFu;
 // plan modes: 0 the length varint is malformed, 1 the serial pass decodes the page, 2 its
 // fragments decode in parallel
 constexpr uint32_t kSnapSerial = 1, kSnapSplit = 2;
-constexpr size_t kSnapFragSmem = kSnapFrag + kSnapWinLoad + kSnapWin * 2 + 32 * 4;
+constexpr uint32_t kSnapPiece = 2048, kSnapPieces = 2048;  // long literals, cut into pieces for the warps
+constexpr size_t kSnapMapSmem = kSnapBlk * 8 + kSnapBlk + 32;
+constexpr size_t kSnapFragSmem = kSnapFrag * 3 + kSnapPieces * 8;
+// Stream bytes per group of pages decoded together: the maps take 16 bytes per stream byte.
+constexpr uint64_t kSnapGroupBytes = 32ull << 20;
 
 // One element header at s[0..avail): its size h (tag plus length or offset bytes), kind (0
 // literal, 1 copy), output length and copy offset; false if it does not fit in `avail`.
@@ -267,43 +296,330 @@ __device__ __forceinline__ bool snap_hdr(const uint8_t* s, uint32_t avail, uint3
     return true;
 }
 
-// The warp loads src[base, base + kSnapWinLoad) into `win`, base being the 16-byte boundary at or
-// below pos (it may lie before the stream: those bytes are not used), 16 bytes per lane-load,
-// stopping at the first boundary at or past `len` (the chunk buffer is padded past its end).
-// Returns base (as a stream offset) and the bytes loaded.
-__device__ __forceinline__ int64_t snap_load(const uint8_t* src, uint32_t len, uint32_t pos, uint8_t* win,
-                                             uint32_t& loaded) {
-    const uintptr_t a = (uintptr_t)(src + pos);
-    const uint4* v = (const uint4*)(a & ~(uintptr_t)15);
-    const int64_t base = (int64_t)pos - (int64_t)(a & 15);
-    const uint64_t need = ((uint64_t)((int64_t)len - base) + 15) / 16;
-    const uint32_t nvec = (uint32_t)(need < kSnapWinLoad / 16 ? need : kSnapWinLoad / 16);
-    const uint32_t lane = threadIdx.x & 31;
-    constexpr uint32_t kPer = (kSnapWinLoad / 16 + 31) / 32;
-    uint4 r[kPer];
-#pragma unroll
-    for (uint32_t k = 0; k < kPer; k++)
-        if (lane + 32 * k < nvec) r[k] = __ldg(v + lane + 32 * k);
-#pragma unroll
-    for (uint32_t k = 0; k < kPer; k++)
-        if (lane + 32 * k < nvec) ((uint4*)win)[lane + 32 * k] = r[k];
-    __syncwarp();
-    loaded = 16 * nvec;
-    return base;
+// The element that starts at w[0], of which `avail` stream bytes are left (w has five readable bytes):
+// its bytes in the stream (header and a literal's bytes) and in the output; false when it does not
+// fit.  Branch-free: the five bytes a header can span are read at once and every form is computed.
+__device__ __forceinline__ bool snap_elem(const uint8_t* w, uint32_t avail, uint32_t& step, uint32_t& len) {
+    const uint32_t b0 = w[0], b1 = w[1], b2 = w[2], b3 = w[3], b4 = w[4];
+    const uint32_t t = b0 & 3, l6 = b0 >> 2;
+    const uint32_t nb = l6 >= 60 ? l6 - 59 : 0;  // a literal's length bytes
+    const uint32_t ext = b1 | (nb >= 2 ? b2 << 8 : 0u) | (nb >= 3 ? b3 << 16 : 0u) | (nb >= 4 ? b4 << 24 : 0u);
+    const uint64_t lit = (uint64_t)(nb ? ext : l6) + 1;  // a literal's bytes (up to 2^32)
+    const uint64_t st = t == 0 ? 1 + nb + lit : t == 1 ? 2 : t == 2 ? 3 : 5;
+    step = (uint32_t)st;
+    len = t == 0 ? (uint32_t)lit : t == 1 ? 4 + (l6 & 7) : l6 + 1;
+    return avail > 0 && st <= (uint64_t)avail;
 }
 
-// The record of the element that would start at window offset q (stream offset base + q):
-// the step to the next element (header plus a literal's bytes) in bits 0-15 and the output
-// length in bits 16-31 (the fragment decode keeps the step); 0 = the header does not parse (or q
-// lies before `from`); a step of 0xFFFF = too long for the record: read the header again.
-__device__ __forceinline__ uint32_t snap_record(const uint8_t* win, int64_t base, uint32_t q, uint32_t from,
-                                                uint32_t end) {
-    const int64_t p = base + q;
-    if (p < (int64_t)from || p >= (int64_t)end) return 0;
-    uint32_t h, kind, len, off;
-    if (!snap_hdr(win + q, end - (uint32_t)p, h, kind, len, off)) return 0;
-    const uint64_t step = (uint64_t)h + (kind == 0 ? len : 0);
-    return step > 0xFFFE ? 0xFFFFu : (uint32_t)step | (len << 16);
+// The block loads src[b0, b0 + kSnapBlk + 5) (to the stream's end at most) into `win` with aligned
+// 16-byte loads, from the 16-byte boundary at or below (the chunk buffer is padded past its end);
+// win + the returned lead is src + b0.
+__device__ __forceinline__ uint32_t snap_window(const SnapJob& J, uint32_t b0, uint8_t* win) {
+    const uintptr_t a = (uintptr_t)(J.src + b0);
+    const uint4* v = (const uint4*)(a & ~(uintptr_t)15);
+    const uint32_t lead = (uint32_t)(a & 15);
+    const uint64_t need = ((uint64_t)(J.src_len - b0) + lead + 15) / 16;
+    const uint32_t nvec = (uint32_t)(need < kSnapBlk / 16 + 2 ? need : kSnapBlk / 16 + 2);
+    for (uint32_t i = threadIdx.x; i < nvec; i += kSnapThreads) ((uint4*)win)[i] = __ldg(v + i);
+    return lead;
+}
+
+// The maps: blocks[i] = {page, block}.  A byte's state packs the element reached (16 bits, a block
+// offset), the elements passed (16) and the bytes they write (32); an element whose successor lies
+// past the block (or that does not parse) points to itself.  States only ever move further along the
+// chain and are read and written whole, so the rounds need no second buffer: bound by shared-memory
+// round trips, log2(kSnapBlk / 2) of them.
+__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_maps(const SnapJob* jobs, const uint2* blocks, SnapMap* tab) {
+    extern __shared__ __align__(16) uint8_t snap_smem[];
+    uint64_t* st = (uint64_t*)snap_smem;
+    uint8_t* win = snap_smem + kSnapBlk * 8;
+    const uint2 f = blocks[blockIdx.x];
+    const SnapJob J = jobs[f.x];
+    const uint32_t b0 = f.y * kSnapBlk, blen = min(kSnapBlk, J.src_len - b0);
+    const uint8_t* w = win + snap_window(J, b0, win);
+    __syncthreads();
+    uint64_t v[kSnapPer];
+#pragma unroll
+    for (uint32_t e = 0; e < kSnapPer; e++) {
+        const uint32_t q = threadIdx.x + e * kSnapThreads;
+        uint32_t step, len;
+        const bool ok = q < blen && snap_elem(w + q, J.src_len - b0 - q, step, len);
+        v[e] = ok && step < blen - q ? (uint64_t)(q + step) | (1ull << 16) | ((uint64_t)len << 32) : (uint64_t)q;
+        st[q] = v[e];
+    }
+    uint32_t open = (1u << kSnapPer) - 1;  // states that may still move
+    while (__syncthreads_or(open != 0)) {
+#pragma unroll
+        for (uint32_t e = 0; e < kSnapPer; e++) {
+            if (!((open >> e) & 1)) continue;
+            const uint32_t p = (uint32_t)v[e] & 0xFFFFu;
+            const uint64_t x = *(volatile uint64_t*)(st + p);
+            if (((uint32_t)x & 0xFFFFu) == p) {
+                open &= ~(1u << e);
+            } else {
+                v[e] = (x & 0xFFFFull) | (((v[e] >> 16) + (x >> 16)) << 16);
+                *(volatile uint64_t*)(st + threadIdx.x + e * kSnapThreads) = v[e];
+            }
+        }
+    }
+#pragma unroll
+    for (uint32_t e = 0; e < kSnapPer; e++) {
+        const uint32_t q = threadIdx.x + e * kSnapThreads;
+        if (q >= blen) continue;
+        const uint32_t p = (uint32_t)v[e] & 0xFFFFu;  // the chain's last element in the block
+        uint32_t step, len;
+        SnapMap m{kSnapNone, 0, 0, 0};
+        if (snap_elem(w + p, J.src_len - b0 - p, step, len))
+            m = SnapMap{b0 + p + step, (uint32_t)(v[e] >> 32) + len, ((uint32_t)(v[e] >> 16) & 0xFFFFu) + 1u, 0};
+        *(uint4*)(tab + J.tab0 + b0 + q) = *(const uint4*)&m;
+    }
+}
+
+// The chain, one thread per page: the page's mode, each block's entry, and the number of elements.
+// Bound by one dependent L2 load per block of the page.
+__global__ void __launch_bounds__(32) k_pq_snappy_chain(const SnapJob* jobs, const SnapMap* tab, SnapEntry* entries,
+                                                        uint32_t* plan) {
+    if (threadIdx.x) return;
+    const SnapJob J = jobs[blockIdx.x];
+    uint32_t* pl = plan + J.plan;
+    uint32_t start = 0, total = 0;
+    bool ok = false;
+    for (int shift = 0; shift < 35 && start < J.src_len; shift += 7) {  // the uncompressed length
+        const uint32_t b = J.src[start++];
+        if (shift == 28 && (b & 0x70)) break;  // past 32 bits
+        total |= (b & 0x7F) << shift;
+        if (!(b & 0x80)) {
+            ok = true;
+            break;
+        }
+    }
+    pl[1] = start;
+    if (!ok || total != J.dst_len) {
+        pl[0] = 0;
+        return;
+    }
+    bool split = J.nfrag >= 1;
+    uint32_t pos = start, elem = 0;
+    uint64_t out = 0;
+    while (split && pos < J.src_len) {
+        const uint4 m = __ldg((const uint4*)(tab + J.tab0 + pos));
+        entries[J.blk0 + pos / kSnapBlk] = SnapEntry{pos, (uint32_t)out, elem, 1u};
+        out += m.y;
+        elem += m.z;
+        pos = m.x;  // past pos: an element spans at least two bytes
+        split = m.x != kSnapNone && out <= total;
+    }
+    if (split && out == total) {
+        pl[2 + J.nfrag] = elem;
+        pl[0] = kSnapSplit;
+    } else {
+        pl[0] = kSnapSerial;
+    }
+}
+
+// The list: each real element's stream and output position, in order, and the number of every
+// fragment's first element.  Marks start at the block's entry; round k marks the elements 2^k after
+// the marked ones while the jumps double, so all are marked after log2 of their number rounds (a
+// mark set early by a neighbour's write of the same round is a real element too).
+__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_list(const SnapJob* jobs, const uint2* blocks,
+                                                                 const SnapEntry* entries, uint32_t* plan, uint2* elems) {
+    __shared__ __align__(16) uint16_t jmp[kSnapBlk];
+    __shared__ __align__(16) uint8_t mark[kSnapBlk];
+    __shared__ __align__(16) uint8_t win[kSnapBlk + 32];
+    __shared__ uint64_t wsum[kSnapThreads / 32];
+    const uint2 f = blocks[blockIdx.x];
+    const SnapJob J = jobs[f.x];
+    uint32_t* pl = plan + J.plan;
+    const SnapEntry E = entries[J.blk0 + f.y];
+    if (E.valid != 1u || pl[0] == 0) return;
+    const uint32_t tid = threadIdx.x, b0 = f.y * kSnapBlk, blen = min(kSnapBlk, J.src_len - b0);
+    const uint8_t* w = win + snap_window(J, b0, win);
+    for (uint32_t i = tid; i < kSnapBlk / 16; i += kSnapThreads) ((uint4*)mark)[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+#pragma unroll
+    for (uint32_t e = 0; e < kSnapPer; e++) {
+        const uint32_t q = tid + e * kSnapThreads;
+        uint32_t step, len;
+        const bool ok = q < blen && snap_elem(w + q, J.src_len - b0 - q, step, len);
+        jmp[q] = (uint16_t)(ok && step < blen - q ? q + step : 0xFFFFu);
+    }
+    if (tid == 0) mark[E.pos - b0] = 1;
+    for (;;) {
+        __syncthreads();
+        uint32_t nj[kSnapPer / 2];  // two jumps per register
+        uint32_t all = 0xFFFFu;
+#pragma unroll
+        for (uint32_t e = 0; e < kSnapPer; e++) {
+            const uint32_t q = tid + e * kSnapThreads, j = jmp[q];
+            uint32_t x = 0xFFFFu;
+            if (j != 0xFFFFu) {
+                x = jmp[j];
+                if (*(volatile uint8_t*)(mark + q)) *(volatile uint8_t*)(mark + j) = 1;
+            }
+            all &= x;
+            nj[e / 2] = e & 1 ? nj[e / 2] | (x << 16) : x;
+        }
+        if (!__syncthreads_or(all != 0xFFFFu)) break;
+#pragma unroll
+        for (uint32_t e = 0; e < kSnapPer; e++) jmp[tid + e * kSnapThreads] = (uint16_t)(nj[e / 2] >> (16 * (e & 1)));
+    }
+    // number the marked elements and sum their output lengths: eight consecutive bytes per thread
+    const uint64_t marks = ((const uint64_t*)mark)[tid];
+    uint32_t cnt = 0, sum = 0;
+    auto length = [&](uint32_t e) {  // parses: the chain passed through it
+        const uint32_t q = tid * kSnapPer + e;
+        uint32_t step, len;
+        snap_elem(w + q, J.src_len - b0 - q, step, len);
+        return len;
+    };
+    for (uint32_t e = 0; e < kSnapPer; e++)
+        if ((marks >> (8 * e)) & 1) {
+            cnt++;
+            sum += length(e);
+        }
+    const uint64_t mine = ((uint64_t)cnt << 32) | sum;  // the block's bytes fit 32 bits (the page's do)
+    uint64_t incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t t = __shfl_up_sync(~0u, incl, d);
+        if ((int)(tid & 31) >= d) incl += t;
+    }
+    if ((tid & 31) == 31) wsum[tid >> 5] = incl;
+    __syncthreads();
+    if (tid < 32) {
+        uint64_t x = wsum[tid];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint64_t t = __shfl_up_sync(~0u, x, d);
+            if ((int)tid >= d) x += t;
+        }
+        wsum[tid] = x;
+    }
+    __syncthreads();
+    const uint64_t before = incl - mine + (tid >= 32 ? wsum[(tid >> 5) - 1] : 0ull);
+    uint32_t i = E.elem + (uint32_t)(before >> 32), o = E.out + (uint32_t)before;
+    bool bad = false;
+    for (uint32_t e = 0; e < kSnapPer; e++) {
+        if (!((marks >> (8 * e)) & 1)) continue;
+        const uint32_t l = length(e), at = o & (kSnapFrag - 1);
+        elems[J.elem0 + i] = make_uint2(b0 + tid * kSnapPer + e, o);
+        bad = bad || l > kSnapFrag - at;  // crossing a fragment's end
+        if (at == 0 && (o >> 16) < J.nfrag) pl[2 + (o >> 16)] = i;
+        i++;
+        o += l;
+    }
+    if (bad) atomicExch(pl, kSnapSerial);
+}
+
+// The decode, one block per fragment of a split page (frags[i] = {page, fragment}); a fragment that
+// does not decode as a unit hands its page to the serial pass.  `ptr` holds, per output byte, the
+// earlier output byte it equals (itself for a literal's byte, whose value is in `val`); jumping
+// ptr[i] = ptr[ptr[i]] until nothing moves ends at literal bytes.  A copy overlapping itself points
+// into the pattern it repeats.  192 KB of shared memory, so one block per SM: bound by the
+// shared-memory gathers of the rounds (64 bytes per thread and round, resolved pairs skipped).
+__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_frag(const SnapJob* jobs, const uint2* frags, const uint2* elems,
+                                                                 uint32_t* plan) {
+    extern __shared__ __align__(16) uint8_t snap_smem[];
+    uint16_t* ptr = (uint16_t*)snap_smem;
+    uint8_t* val = snap_smem + kSnapFrag * 2;
+    uint2* piece = (uint2*)(val + kSnapFrag);
+    __shared__ uint32_t npiece;
+    const uint2 f = frags[blockIdx.x];
+    const SnapJob J = jobs[f.x];
+    uint32_t* pl = plan + J.plan;
+    __shared__ uint32_t mode;  // one read: another fragment's block may hand the page over meanwhile
+    if (threadIdx.x == 0) {
+        mode = *(volatile uint32_t*)pl;
+        npiece = 0;
+    }
+    __syncthreads();
+    if (mode != kSnapSplit) return;
+    const uint32_t tid = threadIdx.x, o0 = f.y * kSnapFrag, n = min(J.dst_len - o0, kSnapFrag);
+    for (uint32_t i = tid; i < kSnapFrag / 8; i += kSnapThreads) {  // every byte its own source
+        const uint32_t b = i * 8;
+        ((uint4*)ptr)[i] = make_uint4(b | ((b + 1) << 16), (b + 2) | ((b + 3) << 16), (b + 4) | ((b + 5) << 16), (b + 6) | ((b + 7) << 16));
+    }
+    __syncthreads();
+    bool bad = false;
+    const uint2* E = elems + J.elem0;
+#pragma unroll 1
+    for (uint32_t i = pl[2 + f.y] + tid, i1 = pl[3 + f.y]; i < i1; i += kSnapThreads) {
+        const uint2 el = E[i];
+        const uint8_t* e = J.src + el.x;  // five readable bytes: the chunk buffer is padded past its end
+        const uint32_t o = el.y - o0;
+        uint32_t step, len;
+        if (!snap_elem(e, J.src_len - el.x, step, len) || o >= n || len > n - o) {
+            bad = true;
+            continue;
+        }
+        const uint32_t t = e[0] & 3;
+        const uint32_t off = t == 1 ? ((uint32_t)(e[0] >> 5) << 8) | e[1]
+                                    : e[1] | ((uint32_t)e[2] << 8) | (t == 3 ? ((uint32_t)e[3] << 16) | ((uint32_t)e[4] << 24) : 0u);
+        if (t == 0) {
+            const uint32_t s = el.x + step - len;
+            if (len <= 32) {
+#pragma unroll 4
+                for (uint32_t j = 0; j < len; j++) val[o + j] = __ldg(J.src + s + j);
+            } else {  // by the warps, in pieces (at most n / 33 + n / kSnapPiece of them)
+                const uint32_t np = (len + kSnapPiece - 1) / kSnapPiece, k0 = atomicAdd(&npiece, np);
+#pragma unroll 1
+                for (uint32_t k = 0; k < np; k++)
+                    piece[k0 + k] = make_uint2(s + k * kSnapPiece, (o + k * kSnapPiece) | (min(kSnapPiece, len - k * kSnapPiece) << 16));
+            }
+        } else if (off == 0 || off > o) {  // before the fragment
+            bad = true;
+        } else {
+            uint32_t p = o - off;
+#pragma unroll 1
+            for (uint32_t j = 0; j < len; j++) {
+                ptr[o + j] = (uint16_t)p;
+                p = p + 1 == o ? o - off : p + 1;
+            }
+        }
+    }
+    if (__syncthreads_or(bad)) {
+        if (tid == 0) atomicExch(pl, kSnapSerial);
+        return;
+    }
+    for (uint32_t k = tid >> 5; k < npiece; k += kSnapThreads / 32) {
+        const uint2 pc = piece[k];
+        const uint32_t o = pc.y & 0xFFFFu, len = pc.y >> 16;
+        for (uint32_t j = tid & 31; j < len; j += 32) val[o + j] = __ldg(J.src + pc.x + j);
+    }
+    const uint32_t words = (n + 1) / 2;  // two bytes' pointers per word
+    uint32_t open = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kSnapFrag / 2 / kSnapThreads; k++)
+        if (tid + k * kSnapThreads < words) open |= 1u << k;
+    volatile uint32_t* pw = (volatile uint32_t*)ptr;
+    const volatile uint16_t* ph = (const volatile uint16_t*)ptr;
+    while (__syncthreads_or(open != 0)) {
+#pragma unroll 2
+        for (uint32_t k = 0; k < kSnapFrag / 2 / kSnapThreads; k++) {
+            if (!((open >> k) & 1)) continue;
+            const uint32_t x = pw[tid + k * kSnapThreads];
+            const uint32_t y = (uint32_t)ph[x & 0xFFFFu] | ((uint32_t)ph[x >> 16] << 16);
+            if (x == y) open &= ~(1u << k);
+            else pw[tid + k * kSnapThreads] = y;
+        }
+    }
+    uint8_t* d = J.dst + o0;
+    if (((uintptr_t)d & 15) == 0) {
+#pragma unroll 1
+        for (uint32_t i = tid; i < n / 16; i += kSnapThreads) {
+            uint32_t r[4];
+            const uint4 pa = ((const uint4*)ptr)[2 * i], pb = ((const uint4*)ptr)[2 * i + 1];
+            const uint32_t pp[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                r[k] = val[pp[2 * k] & 0xFFFFu] | (val[pp[2 * k] >> 16] << 8) | (val[pp[2 * k + 1] & 0xFFFFu] << 16) |
+                       ((uint32_t)val[pp[2 * k + 1] >> 16] << 24);
+            ((uint4*)d)[i] = make_uint4(r[0], r[1], r[2], r[3]);
+        }
+        for (uint32_t i = (n & ~15u) + tid; i < n; i += kSnapThreads) d[i] = val[ptr[i]];
+    } else {
+        for (uint32_t i = tid; i < n; i += kSnapThreads) d[i] = val[ptr[i]];
+    }
 }
 
 // One thread's decode of the elements in [pos, end) into dst[out, out_end); copies may not reach
@@ -356,330 +672,6 @@ __device__ bool snap_decode_serial(SnapSrc& S, uint32_t pos, uint32_t end, uint8
         out += len;
     }
     return pos == end;
-}
-
-// The walk's record for window offset q (stream offset base + q): the window offset of the next
-// element if an element started at q (q + its header + a literal's bytes), or kSnapNone when no
-// element can start there (the header or the literal runs past `end`, or q lies before `from`).
-// Branch-free: the five bytes a header can span are read at once and every form is computed.
-constexpr uint32_t kSnapNone = 0xFFFFFFFFu;
-__device__ __forceinline__ uint32_t snap_next(const uint8_t* win, int64_t base, uint32_t q, uint32_t from,
-                                              uint32_t end) {
-    const int64_t p = base + q;
-    const int64_t avail = (int64_t)end - p;
-    const uint32_t b0 = win[q], b1 = win[q + 1], b2 = win[q + 2], b3 = win[q + 3], b4 = win[q + 4];
-    const uint32_t t = b0 & 3, l6 = b0 >> 2;
-    const uint32_t nb = l6 >= 60 ? l6 - 59 : 0;  // a literal's length bytes
-    const uint32_t ext = b1 | (nb >= 2 ? b2 << 8 : 0u) | (nb >= 3 ? b3 << 16 : 0u) | (nb >= 4 ? b4 << 24 : 0u);
-    const uint64_t len = (uint64_t)(nb ? ext : l6) + 1;  // a literal's bytes (up to 2^32)
-    const uint64_t step = t == 0 ? 1 + nb + len : t == 1 ? 2 : t == 2 ? 3 : 5;
-    const bool ok = p >= (int64_t)from && avail > 0 && (int64_t)step <= avail && step < (1ull << 31);
-    return ok ? q + (uint32_t)step : kSnapNone;
-}
-
-// The walk, one 4-warp block per page: the page's mode and, for a split page, where each
-// fragment's elements start (plan: [mode, first element, nfrag fragment starts, stream end]).
-// Per window: the block builds the next-element records and, from them, the element after next;
-// one thread follows the chain two elements per shared-memory round trip, listing the element
-// starts; then the block reads the listed headers' output lengths, prefix-sums them, records each
-// fragment's first element and checks that no element crosses a fragment boundary.  Every loop
-// and barrier is block-uniform: its conditions are read from shared memory after a barrier.
-constexpr uint32_t kSnapList = kSnapWin / 2 + 1;  // elements in a window (each spans >= 2 bytes)
-constexpr int kWalkThreads = 128;
-__global__ void __launch_bounds__(kWalkThreads) k_pq_snappy_walk(const SnapJob* jobs, uint32_t* plan) {
-    __shared__ __align__(16) uint8_t win[kSnapWinLoad];
-    __shared__ uint32_t nxt[kSnapWin], nxt2[kSnapWin];
-    __shared__ uint16_t list[kSnapList];
-    __shared__ uint32_t olen[kSnapList];
-    __shared__ uint32_t wsum[kWalkThreads / 32];
-    __shared__ uint32_t sh_m, sh_qe, sh_bad;
-    const SnapJob J = jobs[blockIdx.x];
-    uint32_t* pl = plan + J.plan;
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    uint32_t start = 0, total = 0;
-    bool ok = false;
-    for (int shift = 0; shift < 35 && start < J.src_len; shift += 7) {  // the uncompressed length
-        const uint32_t b = J.src[start++];
-        if (shift == 28 && (b & 0x70)) break;  // past 32 bits
-        total |= (b & 0x7F) << shift;
-        if (!(b & 0x80)) {
-            ok = true;
-            break;
-        }
-    }
-    uint32_t mode = ok && total == J.dst_len ? kSnapSerial : 0;
-    if (tid == 0) pl[1] = start;
-    if (mode && J.nfrag >= 1) {
-        bool split = true;
-        if (J.nfrag > 1) {
-            uint32_t pos = start, out = 0;  // the same in every thread
-            while (split && out < total) {
-                if (pos >= J.src_len) {
-                    split = false;
-                    break;
-                }
-                // the window: src[base, base + kSnapWinLoad) from the 16-byte boundary at or below pos
-                const uintptr_t a = (uintptr_t)(J.src + pos);
-                const uint4* v = (const uint4*)(a & ~(uintptr_t)15);
-                const int64_t base = (int64_t)pos - (int64_t)(a & 15);
-                const uint64_t need = ((uint64_t)((int64_t)J.src_len - base) + 15) / 16;
-                const uint32_t nvec = (uint32_t)(need < kSnapWinLoad / 16 ? need : kSnapWinLoad / 16);
-                for (uint32_t i = tid; i < nvec; i += kWalkThreads) ((uint4*)win)[i] = __ldg(v + i);
-                __syncthreads();
-#pragma unroll 4
-                for (uint32_t q = tid; q < kSnapWin; q += kWalkThreads) nxt[q] = snap_next(win, base, q, pos, J.src_len);
-                __syncthreads();
-#pragma unroll 4
-                for (uint32_t q = tid; q < kSnapWin; q += kWalkThreads) {
-                    const uint32_t n = nxt[q];
-                    nxt2[q] = n < kSnapWin ? nxt[n] : kSnapNone;
-                }
-                __syncthreads();
-                if (tid == 0) {  // the chain through the window, up to the stream's end
-                    const int64_t rest = (int64_t)J.src_len - base;
-                    const uint32_t qlim = rest < (int64_t)kSnapWin ? (uint32_t)rest : kSnapWin;
-                    uint32_t q = (uint32_t)(pos - base), m = 0;
-                    while (q < qlim) {
-                        const uint32_t n1 = nxt[q], n2 = nxt2[q];
-                        list[m++] = (uint16_t)q;
-                        if (n1 >= qlim) {
-                            q = n1;
-                            break;
-                        }
-                        list[m++] = (uint16_t)n1;
-                        q = n2;
-                    }
-                    sh_m = m;
-                    sh_qe = q;
-                    sh_bad = 0;
-                }
-                __syncthreads();
-                const uint32_t m = sh_m;
-                uint32_t qe = sh_qe;
-                // output lengths of the listed elements (a long literal's next position, which its
-                // record could not hold, from its header), each thread a consecutive run of them
-                const uint32_t per = (m + kWalkThreads - 1) / kWalkThreads, i0 = tid * per, i1 = min(m, i0 + per);
-                uint32_t sum = 0;
-                bool bad = false;
-                for (uint32_t i = i0; i < i1; i++) {
-                    const uint32_t q = list[i];
-                    const uint32_t p = (uint32_t)(base + q);
-                    uint32_t h, kind, len, off;
-                    if (!snap_hdr(win + q, J.src_len - p, h, kind, len, off)) {
-                        bad = true;
-                        len = 0;
-                    }
-                    olen[i] = len;
-                    sum += len;
-                    if (i == m - 1) sh_qe = qe == kSnapNone && !bad ? q + h + (kind == 0 ? len : 0) : qe;
-                }
-                // exclusive prefix of the threads' sums: within the warp, then over the warps
-                uint32_t incl = sum;
-#pragma unroll
-                for (uint32_t d = 1; d < 32; d <<= 1) {
-                    const uint32_t t = __shfl_up_sync(~0u, incl, d);
-                    if (lane >= d) incl += t;
-                }
-                if (lane == 31) wsum[warp] = incl;
-                __syncthreads();
-                uint32_t before = 0, all = 0;
-                for (uint32_t w = 0; w < kWalkThreads / 32; w++) {
-                    before += w < warp ? wsum[w] : 0;
-                    all += wsum[w];
-                }
-                uint32_t o = out + before + incl - sum;
-                for (uint32_t i = i0; i < i1 && !bad; i++) {
-                    const uint32_t l = olen[i];
-                    if (o > total || l > total - o || (o & (kSnapFrag - 1)) + l > kSnapFrag) {
-                        bad = true;  // past the end, or crossing a fragment's end
-                        break;
-                    }
-                    if ((o & (kSnapFrag - 1)) == 0 && o < total) pl[2 + (o >> 16)] = (uint32_t)(base + list[i]);
-                    o += l;
-                }
-                if (bad) atomicOr(&sh_bad, 1u);
-                __syncthreads();
-                qe = sh_qe;
-                const bool stop = sh_bad || qe == kSnapNone || all > total - out;
-                __syncthreads();  // sh_* and the window are rewritten by the next window
-                if (stop) {
-                    split = false;
-                    break;
-                }
-                out += all;
-                pos = (uint32_t)(base + qe);
-            }
-        }
-        if (tid == 0) {
-            if (J.nfrag == 1) pl[2] = start;
-            pl[2 + J.nfrag] = J.src_len;
-        }
-        if (split) mode = kSnapSplit;
-    }
-    if (tid == 0) pl[0] = mode;
-}
-
-// A literal longer than a lane's share, by the whole warp: aligned 16-byte loads from the stream,
-// bytes stored into the fragment (the loads may pass the literal's ends by 15 bytes, inside the
-// padded chunk buffer).
-__device__ __forceinline__ void snap_warp_copy(const uint8_t* src, uint32_t len, uint8_t* dst) {
-    const uintptr_t a = (uintptr_t)src;
-    const uint4* v = (const uint4*)(a & ~(uintptr_t)15);
-    const int32_t lead = (int32_t)(a & 15);
-    const uint32_t nvec = ((uint32_t)lead + len + 15) / 16;
-    const uint32_t lane = threadIdx.x & 31;
-    auto put = [&](const uint4& r, uint32_t i) {
-        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-        for (int b = 0; b < 16; b++) {
-            const int32_t idx = (int32_t)(16 * i) + b - lead;
-            if (idx >= 0 && (uint32_t)idx < len) dst[idx] = (uint8_t)(w[b >> 2] >> (8 * (b & 3)));
-        }
-    };
-    for (uint32_t i = lane; i < nvec; i += 64) {
-        const uint4 r0 = __ldg(v + i);
-        const bool two = i + 32 < nvec;
-        uint4 r1 = r0;
-        if (two) r1 = __ldg(v + i + 32);
-        put(r0, i);
-        if (two) put(r1, i + 32);
-    }
-}
-
-// One copy element by one lane: o[at, at + len) from o[at - off, ...), the source bytes read as the
-// repeating pattern o[at - off, at) (what a byte-by-byte copy of an overlapping match produces), so
-// the loads never depend on this copy's stores.
-__device__ __forceinline__ void snap_copy(uint8_t* o, uint32_t at, uint32_t off, uint32_t len) {
-    const uint8_t* s = o + at - off;
-    uint32_t j = 0;
-    for (uint32_t i = 0; i < len; i += 8) {
-        uint8_t t[8];
-#pragma unroll
-        for (uint32_t k = 0; k < 8; k++) {
-            t[k] = i + k < len ? s[j] : 0;
-            j = j + 1 == off ? 0 : j + 1;
-        }
-#pragma unroll
-        for (uint32_t k = 0; k < 8; k++)
-            if (i + k < len) o[at + i + k] = t[k];
-    }
-}
-
-// The decode, one warp per fragment of a split page (frags[i] = {page, fragment}); a fragment that
-// does not decode as a unit hands its page to the serial pass.
-__global__ void __launch_bounds__(32) k_pq_snappy_frag(const SnapJob* jobs, const uint2* frags, uint32_t* plan) {
-    extern __shared__ __align__(16) uint8_t snap_smem[];
-    uint8_t* o = snap_smem;                                    // the fragment, kSnapFrag bytes
-    uint8_t* win = o + kSnapFrag;                              // the stream window
-    uint16_t* rec = (uint16_t*)(win + kSnapWinLoad);           // steps to the next element
-    uint32_t* list = (uint32_t*)(rec + kSnapWin);              // a batch's element starts
-    const uint2 f = frags[blockIdx.x];
-    const SnapJob J = jobs[f.x];
-    uint32_t* pl = plan + J.plan;
-    if (pl[0] != kSnapSplit) return;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t o0 = f.y * kSnapFrag, n = min(J.dst_len - o0, kSnapFrag);
-    uint32_t pos = pl[2 + f.y], out = 0;
-    const uint32_t end = pl[3 + f.y];
-    bool ok = true;
-    while (ok && out < n) {
-        if (pos >= end) {
-            ok = false;
-            break;
-        }
-        uint32_t loaded;
-        const int64_t base = snap_load(J.src, end, pos, win, loaded);
-        for (uint32_t q = lane; q < kSnapWin; q += 32) rec[q] = (uint16_t)(snap_record(win, base, q, pos, end) & 0xFFFF);
-        __syncwarp();
-        uint32_t q0 = (uint32_t)(pos - base);
-        while (ok && out < n && q0 < kSnapWin && base + q0 < end) {
-            uint32_t m = 0;
-            if (lane == 0) {  // up to 32 elements of the chain
-                uint32_t q = q0;
-                while (m < 32 && q < kSnapWin && base + q < end) {
-                    const uint32_t r = rec[q];
-                    list[m++] = q;
-                    if (r == 0 || r == 0xFFFF) break;  // its lane reads the header (or finds it malformed)
-                    q += r;
-                }
-            }
-            m = __shfl_sync(~0u, m, 0);
-            __syncwarp();
-            uint32_t h = 0, kind = 0, len = 0, off = 0, q = 0;
-            bool good = true;
-            if (lane < m) {
-                q = list[lane];
-                good = snap_hdr(win + q, end - (uint32_t)(base + q), h, kind, len, off);
-            }
-            // output positions: the exclusive prefix sum of the lengths
-            const uint32_t x = lane < m && good ? len : 0;
-            uint32_t incl = x;
-#pragma unroll
-            for (uint32_t d = 1; d < 32; d <<= 1) {
-                const uint32_t t = __shfl_up_sync(~0u, incl, d);
-                if (lane >= d) incl += t;
-            }
-            const uint32_t my = out + incl - x;
-            if (lane < m && good) {
-                if (my > n || len > n - my) good = false;
-                else if (kind == 1 && (off == 0 || off > my)) good = false;  // before the fragment
-            }
-            if (__any_sync(~0u, lane < m && !good)) {
-                ok = false;
-                break;
-            }
-            // literals: short ones by their lane, long ones by the whole warp
-            const uint32_t lit = (uint32_t)(base + q) + h;  // stream offset of a literal's bytes
-            const bool is_lit = lane < m && kind == 0;
-            if (is_lit && len <= 32) {
-                if ((int64_t)lit - base + len <= (int64_t)loaded) {
-                    const uint8_t* s = win + (lit - base);
-                    for (uint32_t i = 0; i < len; i++) o[my + i] = s[i];
-                } else {
-                    for (uint32_t i = 0; i < len; i++) o[my + i] = __ldg(J.src + lit + i);
-                }
-            }
-            uint32_t longs = __ballot_sync(~0u, is_lit && len > 32);
-            while (longs) {
-                const uint32_t l = __ffs(longs) - 1;
-                longs &= longs - 1;
-                const uint32_t ls = __shfl_sync(~0u, lit, l), ll = __shfl_sync(~0u, len, l), lo = __shfl_sync(~0u, my, l);
-                snap_warp_copy(J.src + ls, ll, o + lo);
-            }
-            __syncwarp();
-            // copies in rounds: a copy runs once every byte it reads is written, i.e. its source
-            // ends at or before the output position of the earliest copy still waiting
-            uint32_t pend = __ballot_sync(~0u, lane < m && kind == 1);
-            const uint32_t need = kind == 1 ? (off >= len ? my - off + len : my) : 0;
-            while (pend) {
-                const uint32_t lim = __shfl_sync(~0u, my, __ffs(pend) - 1);
-                const uint32_t ready = pend & __ballot_sync(~0u, need <= lim);
-                if ((ready >> lane) & 1) snap_copy(o, my, off, len);
-                __syncwarp();
-                pend &= ~ready;
-            }
-            // the next batch starts after the last element
-            const uint32_t nxt = (uint32_t)(base + q) + h + (kind == 0 ? len : 0);
-            pos = __shfl_sync(~0u, nxt, m - 1);
-            out += __shfl_sync(~0u, incl, 31);
-            q0 = (uint32_t)(pos - base);
-        }
-        __syncwarp();  // the window and the records are reused
-    }
-    if (ok && pos != end) ok = false;
-    if (!ok) {
-        if (lane == 0) atomicExch(pl, kSnapSerial);
-        return;
-    }
-    __syncwarp();
-    uint8_t* d = J.dst + o0;
-    if (((uintptr_t)d & 15) == 0) {
-        const uint32_t nv = n / 16;
-        for (uint32_t i = lane; i < nv; i += 32) ((uint4*)d)[i] = ((const uint4*)o)[i];
-        for (uint32_t i = 16 * nv + lane; i < n; i += 32) d[i] = o[i];
-    } else {
-        for (uint32_t i = lane; i < n; i += 32) d[i] = o[i];
-    }
 }
 
 // The serial pass, one thread per page not decoded by fragments: it decodes the page from start
@@ -1313,8 +1305,14 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
     CK(cudaMemcpyAsync(dchunk.get(), chunk, (size_t)chunk_bytes, cudaMemcpyHostToDevice, s));
     const uint8_t* dc = dchunk.get<uint8_t>();
     uint8_t* up = upages.get<uint8_t>();
+    // the Snappy pages in groups (usually one) of at most kSnapGroupBytes stream bytes, or one page
+    struct SnapGroup {
+        int job0 = 0, njobs = 0, frag0 = 0, nfrags = 0, blk0 = 0, nblks = 0;
+        uint64_t bytes = 0, elems = 0;
+    };
     std::vector<SnapJob> jobs;
-    std::vector<uint2> frags;  // {page, fragment} per 64 KB of Snappy output
+    std::vector<SnapGroup> groups;
+    std::vector<uint2> frags, blocks;  // {page, fragment} per 64 KB of output, {page, block} per kSnapBlk of stream
     uint32_t plan_words = 0;
     for (size_t i = 0; i < pages.size(); i++) {
         const Page& pg = pages[i];
@@ -1324,11 +1322,23 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
         const bool compressed = codec == ML_PQ_CODEC_SNAPPY && (!v2 || pg.v2_compressed);
         if (compressed) {
             const uint32_t dlen = (uint32_t)(pg.uncompressed - lv);
+            const uint32_t slen = (uint32_t)(pg.compressed - lv);
             const uint32_t nfrag = (uint32_t)(((uint64_t)dlen + kSnapFrag - 1) / kSnapFrag);
-            for (uint32_t k = 0; k < nfrag; k++) frags.push_back(uint2{(uint32_t)jobs.size(), k});
-            jobs.push_back(SnapJob{dc + pg.payload + lv, up + uoff[i] + lv, (uint32_t)(pg.compressed - lv), dlen,
-                                   plan_words, nfrag});
+            const uint32_t nblk = (uint32_t)(((uint64_t)slen + kSnapBlk - 1) / kSnapBlk);
+            if (groups.empty() || groups.back().bytes + slen > kSnapGroupBytes) {
+                SnapGroup g;
+                g.job0 = (int)jobs.size(), g.frag0 = (int)frags.size(), g.blk0 = (int)blocks.size();
+                groups.push_back(g);
+            }
+            SnapGroup& g = groups.back();
+            const uint32_t id = (uint32_t)jobs.size();
+            for (uint32_t k = 0; k < nfrag; k++) frags.push_back(uint2{id, k});
+            for (uint32_t k = 0; k < nblk; k++) blocks.push_back(uint2{id, k});
+            jobs.push_back(SnapJob{dc + pg.payload + lv, up + uoff[i] + lv, slen, dlen, plan_words, nfrag,
+                                   (uint32_t)g.nblks, 0u, g.bytes, g.elems});
             plan_words += nfrag + 3;
+            g.njobs++, g.nfrags += (int)nfrag, g.nblks += (int)nblk;
+            g.bytes += slen, g.elems += slen / 2 + 1;  // an element spans at least two stream bytes
         } else {
             if (pg.compressed != pg.uncompressed) raise(ML_ERR_INVALID, "parquet: an uncompressed page changes size");
             if (pg.compressed > lv)
@@ -1338,29 +1348,44 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
     DevBuf err(ctx, 16, nullptr);
     CK(cudaMemsetAsync(err.get(), 0, 4, s));
     uint32_t* derr = err.get<uint32_t>();
-    DevBuf dj, splan;  // read by the Snappy kernels: live to the end of the call
+    DevBuf dj, splan, smap, sentry;  // the Snappy kernels': live to the end of the call
     if (!jobs.empty()) {
-        // the jobs and the fragment table in one upload
-        const size_t jb = jobs.size() * sizeof(SnapJob), fb = frags.size() * sizeof(uint2);
-        std::vector<uint8_t> hj(jb + fb);
+        // the jobs, the fragment and the block table in one upload
+        const size_t jb = jobs.size() * sizeof(SnapJob), fb = frags.size() * sizeof(uint2), bb = blocks.size() * sizeof(uint2);
+        std::vector<uint8_t> hj(jb + fb + bb);
         std::memcpy(hj.data(), jobs.data(), jb);
         if (fb) std::memcpy(hj.data() + jb, frags.data(), fb);
+        if (bb) std::memcpy(hj.data() + jb + fb, blocks.data(), bb);
         dj = DevBuf(ctx, hj.size(), nullptr);
         CK(cudaMemcpyAsync(dj.get(), hj.data(), hj.size(), cudaMemcpyHostToDevice, s));
         const SnapJob* J = dj.get<SnapJob>();
         const uint2* F = (const uint2*)(dj.get<uint8_t>() + jb);
-        const int nj = (int)jobs.size(), nf = (int)frags.size();
+        const uint2* B = (const uint2*)(dj.get<uint8_t>() + jb + fb);
         splan = DevBuf(ctx, (size_t)plan_words * 4, nullptr);
+        uint64_t most = 0, most_elems = 0;
+        int most_blks = 0;
+        for (const SnapGroup& g : groups)
+            most = std::max(most, g.bytes), most_elems = std::max(most_elems, g.elems), most_blks = std::max(most_blks, g.nblks);
+        // the maps; the element list takes their place once the chains are known
+        smap = DevBuf(ctx, std::max<size_t>(std::max(most * sizeof(SnapMap), most_elems * sizeof(uint2)), 16), nullptr);
+        sentry = DevBuf(ctx, std::max<size_t>((size_t)most_blks * sizeof(SnapEntry), 16), nullptr);
         // per call: the attribute belongs to the current device's copy of the kernel
+        CK(cudaFuncSetAttribute(k_pq_snappy_maps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSnapMapSmem));
         CK(cudaFuncSetAttribute(k_pq_snappy_frag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSnapFragSmem));
-        k_pq_snappy_walk<<<nj, kWalkThreads, 0, s>>>(J, splan.get<uint32_t>());
-        if (nf) k_pq_snappy_frag<<<nf, 32, kSnapFragSmem, s>>>(J, F, splan.get<uint32_t>());
-        k_pq_snappy_serial<<<nj, 32, 0, s>>>(J, splan.get<uint32_t>(), derr);
-        ctx->count_launch(nf ? 3 : 2);
-        // wait here: a long Snappy kernel with the decode queued behind it holds up other calls'
-        // work that shares its hardware queue (measured: 3.6 s instead of 0.9 s for 960 chunks
-        // decoded from 16 threads)
-        CK(cudaStreamSynchronize(s));
+        for (const SnapGroup& g : groups) {
+            if (g.nblks) {
+                CK(cudaMemsetAsync(sentry.get(), 0, (size_t)g.nblks * sizeof(SnapEntry), s));
+                k_pq_snappy_maps<<<g.nblks, kSnapThreads, kSnapMapSmem, s>>>(J, B + g.blk0, smap.get<SnapMap>());
+            }
+            k_pq_snappy_chain<<<g.njobs, 32, 0, s>>>(J + g.job0, smap.get<SnapMap>(), sentry.get<SnapEntry>(), splan.get<uint32_t>());
+            if (g.nblks)
+                k_pq_snappy_list<<<g.nblks, kSnapThreads, 0, s>>>(J, B + g.blk0, sentry.get<SnapEntry>(), splan.get<uint32_t>(),
+                                                                  smap.get<uint2>());
+            if (g.nfrags)
+                k_pq_snappy_frag<<<g.nfrags, kSnapThreads, kSnapFragSmem, s>>>(J, F + g.frag0, smap.get<uint2>(), splan.get<uint32_t>());
+            k_pq_snappy_serial<<<g.njobs, 32, 0, s>>>(J + g.job0, splan.get<uint32_t>(), derr);
+            ctx->count_launch(2 + (g.nblks ? 2 : 0) + (g.nfrags ? 1 : 0));
+        }
     }
     auto read_err = [&]() {
         uint32_t e = 0;
