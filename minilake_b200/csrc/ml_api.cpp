@@ -733,39 +733,119 @@ std::vector<SortWord> sort_words(Ctx* ctx, const std::vector<const DevColumn*>& 
     return words;
 }
 
-// The sorted order of n rows (perm[i] = row at position i) by `words`; nullptr-free result.
+// Above this many rows, runs of rows that share 32 key bits are common enough (half of uniform doubles
+// share their exponent, which leaves them 2^25 different keys) that sorting every piece is cheaper
+// than putting them right.
+constexpr int64_t kSortPrefixRows = 1ll << 25;
+
+// The sorted order of n rows (perm[i] = row at position i) by `words`; nullptr-free result.  The work
+// has finished when it returns (its temporaries are handed back).
 DevBuf radix_sort_rows(Ctx* ctx, const std::vector<SortWord>& words, int64_t n, cudaStream_t st, Reservation* res) {
-    DevBuf ka(ctx, std::max<size_t>((size_t)n * 8, 8), res), kb(ctx, std::max<size_t>((size_t)n * 8, 8), res);
-    DevBuf pa(ctx, std::max<size_t>((size_t)n * 4, 4), res), pb(ctx, std::max<size_t>((size_t)n * 4, 4), res);
-    DevBuf hist(ctx, 8 * 256 * 8, nullptr);
-    const int nb = radix_blocks(n);
-    DevBuf counts(ctx, std::max<size_t>((size_t)nb * 256 * 4, 4), nullptr);
-    bool have_perm = false;  // pa holds the current order (else: rows in input order)
-    std::vector<unsigned long long> h(8 * 256);
-    for (const SortWord& w : words) {
-        launch_sort_words(w, have_perm ? pa.get<uint32_t>() : nullptr, n, ka.get<uint64_t>(), st);
-        CK(cudaMemsetAsync(hist.get(), 0, 8 * 256 * 8, st));
-        launch_radix_hist8(ka.get<uint64_t>(), n, hist.get<unsigned long long>(), st);
-        ctx->count_launch(2);
-        CK(cudaMemcpyAsync(h.data(), hist.get(), 8 * 256 * 8, cudaMemcpyDeviceToHost, st));
+    DevBuf perm(ctx, std::max<size_t>((size_t)n * 4, 4), res);
+    const int nw = (int)words.size();
+    DevBuf dwords(ctx, std::max<size_t>(words.size() * sizeof(SortWord), 16), nullptr);
+    CK(cudaMemcpyAsync(dwords.get(), words.data(), words.size() * sizeof(SortWord), cudaMemcpyHostToDevice, st));
+    const SortWord* W = dwords.get<SortWord>();
+    // the key's varying bits, from the most significant word down, a batch of words at a time
+    struct Bits {
+        int word, shift, len;  // bits [shift, shift + len) of a word
+    };
+    std::vector<Bits> bits;
+    int nbits = 0, known = 0;  // words examined, from the last one down
+    constexpr int kBatch = 16;
+    DevBuf ddiff(ctx, kBatch * 8, nullptr);
+    unsigned long long diff[kBatch];
+    auto examine = [&] {
+        const int m = std::min(kBatch, nw - known), lo = nw - known - m;
+        CK(cudaMemsetAsync(ddiff.get(), 0, (size_t)m * 8, st));
+        launch_sort_bits(W + lo, m, n, ddiff.get<unsigned long long>(), st);
+        ctx->count_launch();
+        CK(cudaMemcpyAsync(diff, ddiff.get(), (size_t)m * 8, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        for (int b = 0; b < 8; b++) {
-            bool trivial = false;  // one digit for every row: the pass would not move anything
-            for (int d = 0; d < 256 && !trivial; d++) trivial = h[b * 256 + d] == (unsigned long long)n;
-            if (trivial) continue;
-            launch_radix_count(ka.get<uint64_t>(), n, 8 * b, counts.get<uint32_t>(), st);
-            DevBuf offs;
-            scan_counts(ctx, counts.get<uint32_t>(), (int64_t)nb * 256, offs, st);
-            launch_radix_scatter(ka.get<uint64_t>(), have_perm ? pa.get<uint32_t>() : nullptr, n, 8 * b,
-                                 offs.get<uint64_t>(), kb.get<uint64_t>(), pb.get<uint32_t>(), st);
-            ctx->count_launch(2);
-            std::swap(ka, kb);
-            std::swap(pa, pb);
-            have_perm = true;
+        for (int k = m - 1; k >= 0; k--)
+            for (int b = 63; b >= 0; b--) {
+                if (!((diff[k] >> b) & 1)) continue;
+                int e = b;
+                while (e > 0 && ((diff[k] >> (e - 1)) & 1)) e--;
+                bits.push_back({lo + k, e, b - e + 1});
+                nbits += b - e + 1;
+                b = e;
+            }
+        known += m;
+    };
+    while (known < nw && nbits <= 32) examine();
+    if (nbits == 0) {
+        launch_iota_u32(perm.get<uint32_t>(), n, st);
+        ctx->count_launch();
+        CK(cudaStreamSynchronize(st));
+        return perm;
+    }
+    bool prefix = nbits > 32 && n <= kSortPrefixRows;  // sort by the top 32 bits, then put runs right
+    const int64_t tiles = radix_tiles(n);
+    DevBuf ka(ctx, (size_t)n * 4, res), kb(ctx, (size_t)n * 4, res), pb(ctx, (size_t)n * 4, res);
+    // per piece: 4 x 256 digit counters, the passes' tile counters and their status words
+    const size_t hist_b = 4 * 256 * 4 + 64, stat_b = (size_t)tiles * 256 * 8;
+    DevBuf scratch(ctx, hist_b + 4 * stat_b, nullptr);
+    ErrWord ew(ctx);
+    CK(cudaMemsetAsync(ew.d.get(), 0, 4, st));
+    uint32_t* rows = nullptr;  // the current order (nullptr: 0..n), in perm or pb
+    uint32_t *keys = ka.get<uint32_t>(), *spare = kb.get<uint32_t>();
+    // one stable sort by the key bits [from, from + len) counted from the most significant varying bit
+    auto sort_piece = [&](int from, int len, bool keep_keys) {
+        SortSegs S{};
+        int at = 0, pos = len;
+        for (const Bits& b : bits) {
+            const int lo = std::max(at, from), hi = std::min(at + b.len, from + len);
+            if (lo < hi) {
+                const int take = hi - lo;
+                pos -= take;
+                auto& g = S.s[S.n++];
+                g.word = b.word;
+                g.shift = b.shift + (at + b.len - hi);
+                g.mask = take == 32 ? 0xFFFFFFFFu : (1u << take) - 1u;
+                g.pos = pos;
+            }
+            at += b.len;
+        }
+        const int digits = (len + 7) / 8;
+        uint32_t* hist = scratch.get<uint32_t>();
+        uint32_t* counters = hist + 4 * 256;
+        CK(cudaMemsetAsync(hist, 0, hist_b + (size_t)digits * stat_b, st));
+        launch_sort_keys(W, S, rows, n, keys, digits, hist, st);
+        for (int d = 0; d < digits; d++) {
+            uint32_t* out = rows == perm.get<uint32_t>() ? pb.get<uint32_t>() : perm.get<uint32_t>();
+            const bool want_keys = d + 1 < digits || keep_keys;
+            CK(launch_radix_pass(keys, rows, n, 8 * d, hist + 256 * d, (uint64_t*)(scratch.get<uint8_t>() + hist_b + d * stat_b),
+                                 counters + d, want_keys ? spare : nullptr, out, ew.d.get<uint32_t>(), st));
+            rows = out;
+            if (want_keys) std::swap(keys, spare);
+        }
+        ctx->count_launch(1 + digits);
+    };
+    if (prefix) {
+        sort_piece(0, 32, true);
+        const uint32_t cap = (uint32_t)(n / 8 + 1024);
+        DevBuf list(ctx, (size_t)cap * 8 + 16, nullptr);
+        uint32_t* state = (uint32_t*)(list.get<uint8_t>() + (size_t)cap * 8);
+        CK(cudaMemsetAsync(state, 0, 8, st));
+        launch_sort_runs(keys, rows, W, nw, n, list.get<uint2>(), cap, state, st);
+        ctx->count_launch(2);
+        uint32_t got[2] = {0, 0};
+        CK(cudaMemcpyAsync(got, state, 8, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        if (got[1]) {
+            prefix = false;
+            rows = nullptr;  // from the input order again
         }
     }
-    if (!have_perm) launch_iota_u32(pa.get<uint32_t>(), n, st);
-    return pa;
+    if (!prefix) {
+        while (known < nw) examine();
+        for (int end = nbits; end > 0; end -= 32) sort_piece(std::max(end - 32, 0), std::min(end, 32), false);
+    }
+    CK(cudaMemcpyAsync(ew.h, ew.d.get(), 4, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    check_device_error(ctx, *ew.h);
+    return rows == perm.get<uint32_t>() ? std::move(perm) : std::move(pb);
 }
 
 // ORDER BY keys [LIMIT limit] over a device batch: the first min(limit, n) rows in sorted order

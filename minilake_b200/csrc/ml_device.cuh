@@ -651,6 +651,11 @@ __device__ inline uint32_t table_upsert(const TableView& t, const uint64_t* w, u
     return kNone;
 }
 
+// The f64 total order (f64::total_cmp) as a signed integer (sort.rs:43-82).
+__device__ __forceinline__ int64_t total_key(double d) {
+    int64_t x = __double_as_longlong(d);
+    return x ^ (int64_t)(((uint64_t)(x >> 63)) >> 1);
+}
 // Order-preserving map of f64 onto u64 (for atomic MIN/MAX).
 __device__ __forceinline__ uint64_t f64_order(double d) {
     uint64_t b = f64_bits(d);

@@ -116,9 +116,7 @@ void launch_count_dense(const uint32_t* dense, uint64_t n, unsigned long long* o
 void launch_dense_bits(const uint32_t* dense, uint64_t n, uint32_t* bits, cudaStream_t s);
 void launch_topn_chunk(const SortDev& S, const uint32_t* in, int64_t n, int k, uint32_t* out, cudaStream_t s);
 
-// Full ORDER BY: one 64-bit word of the composite sort key per row (k_sort_words), the word's
-// eight byte histograms (hist8: 8 x 256 u64, zeroed), and per non-trivial byte a stable radix
-// pass: per-block digit counts (digit-major), their exclusive scan `offs`, the scatter.
+// Full ORDER BY (ml_sort.cu): a row's sort key as 64-bit words, least significant first.
 enum SortWordKind : int32_t { SW_VALUE = 0, SW_NULL_FLAG = 1, SW_CHUNK = 2, SW_LENGTH = 3, SW_RANK = 4 };
 struct SortWord {
     DCol col;
@@ -128,13 +126,30 @@ struct SortWord {
     int32_t nulls_first;
     const uint32_t* rank;  // SW_RANK: rank of each dictionary code (dict_len + 1 entries)
 };
-constexpr int kRadixRows = 1024;
-int radix_blocks(int64_t n);
-void launch_sort_words(const SortWord& w, const uint32_t* perm, int64_t n, uint64_t* out, cudaStream_t s);
-void launch_radix_hist8(const uint64_t* keys, int64_t n, unsigned long long* hist, cudaStream_t s);
-void launch_radix_count(const uint64_t* keys, int64_t n, int shift, uint32_t* counts, cudaStream_t s);
-void launch_radix_scatter(const uint64_t* keys_in, const uint32_t* perm_in, int64_t n, int shift, const uint64_t* offs,
-                          uint64_t* keys_out, uint32_t* perm_out, cudaStream_t s);
+// Bits of the key words that form a u32 sort key: ((word >> shift) & mask) << pos each; the segments
+// of one word follow each other.
+struct SortSegs {
+    int32_t n;
+    struct {
+        int32_t word, shift, pos;
+        uint32_t mask;
+    } s[32];
+};
+// diff[y] |= the bits in which word y differs between rows (zeroed), `nwords` device words.
+void launch_sort_bits(const SortWord* words, int nwords, int64_t n, unsigned long long* diff, cudaStream_t s);
+// The u32 keys of rows perm[0..n) (nullptr: 0..n) and their digit histograms (digits x 256, zeroed).
+void launch_sort_keys(const SortWord* words, const SortSegs& S, const uint32_t* perm, int64_t n, uint32_t* keys, int digits,
+                      uint32_t* hist, cudaStream_t s);
+// One stable pass by the digit at `shift` over (key, row id); rows_in nullptr: row ids 0..n; keys_out
+// nullptr: row ids only.  status: radix_tiles(n) x 256 zeroed words; next_tile: a zeroed counter.
+int64_t radix_tiles(int64_t n);
+cudaError_t launch_radix_pass(const uint32_t* keys_in, const uint32_t* rows_in, int64_t n, int shift, const uint32_t* hist,
+                              uint64_t* status, uint32_t* next_tile, uint32_t* keys_out, uint32_t* rows_out, uint32_t* err,
+                              cudaStream_t s);
+// Rows with equal keys put in the order of their whole key words, unless state[1] is set (a run too
+// long, or more runs than `cap`): then nothing has moved.  state: two zeroed words.
+void launch_sort_runs(const uint32_t* keys, uint32_t* rows, const SortWord* words, int nwords, int64_t n, uint2* list,
+                      uint32_t cap, uint32_t* state, cudaStream_t s);
 void launch_max_strlen(const uint32_t* off, int64_t n, unsigned int* out, cudaStream_t s);
 void launch_iota_u32(uint32_t* out, int64_t n, cudaStream_t s);  // out[i] = i
 // Top-k for k <= kTopNWarpMax: each CTA writes its best k rows (sorted) to out[block * k ..].
