@@ -67,6 +67,138 @@ __device__ __forceinline__ void count_global(uint64_t* w) {
     asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(w), "l"(1ull) : "memory");
 }
 
+// Warp-cooperative updates of group blocks (the generated code, emit_coop in ml_jit.cpp): the words of
+// a block that take the same reduction are updated by neighbouring lanes of one instruction, because L2
+// serves one request per 32-byte sector and instruction, whatever the number of words in it (measured on
+// 1.5M 16-byte groups: two reductions by one lane 96 G rows/s, the same two by a pair of lanes 188, one
+// reduction alone 188).  Counts join the f64 sums: a count's bits k are the subnormal k * 2^-1074, so an
+// f64 add of the subnormal with bits 1 makes them k + 1, exactly, up to 2^53 (IEEE 754 gradual
+// underflow; f64 reductions do not flush subnormals).  A NULL argument adds -0.0, which changes no sum.
+template <int OP>
+__device__ __forceinline__ void coop_red(uint64_t* w, uint64_t v) {
+    if (OP == CO_ADD_F64) asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(w), "d"(as_f64(v)) : "memory");
+    else if (OP == CO_ADD_U64) asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(w), "l"(v) : "memory");
+    else if (OP == CO_MIN_U64) asm volatile("red.relaxed.gpu.global.min.u64 [%0], %1;" ::"l"(w), "l"(v) : "memory");
+    else if (OP == CO_MAX_U64) asm volatile("red.relaxed.gpu.global.max.u64 [%0], %1;" ::"l"(w), "l"(v) : "memory");
+    else if (OP == CO_MIN_S64) asm volatile("red.relaxed.gpu.global.min.s64 [%0], %1;" ::"l"(w), "l"(v) : "memory");
+    else asm volatile("red.relaxed.gpu.global.max.s64 [%0], %1;" ::"l"(w), "l"(v) : "memory");
+}
+
+// A new group's id (kNone when the table takes no more).  The lanes that insert together take theirs
+// with one atomic: every insertion counts on the same word.
+__device__ __forceinline__ uint32_t new_group(const AggArgs& A) {
+    const unsigned m = __activemask();
+    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+    uint32_t base = 0;
+    if (lane == leader) base = atomicAdd(A.ngroups, (uint32_t)__popc(m));
+    const uint32_t id = __shfl_sync(m, base, leader) + __popc(m & ((1u << lane) - 1u));
+    return id < A.gid_cap ? id : kNone;
+}
+
+// table_upsert for a whole warp and K keys per lane: every lane calls it, need[k] set where it has a
+// key.  g[k] becomes the key's group (kNone: the table is full), bit k of the result is set where this
+// lane created it.  `full` is the warp's note that the table takes no more groups.
+//
+// Bound by the latency of its dependent accesses (slot, claim, group id), so the keys of a lane are taken
+// through them together, and the lanes step together instead of splitting into groups that issue the
+// same code one after another.  The claims of one step take their group ids with one atomic: every
+// insertion counts on the same word, which L2 serves one access after the other.
+// 4.7M rows with 1.4M new groups: 1,960 us row by row with an atomic and a release per insertion, 780 us
+// so; 14.8M rows with 0.15M new groups 2,530 us and 1,400 us (its accumulators, 8 words a group, then miss
+// L2: 2.8 GB read and 1.2 GB written).
+template <int K>
+__device__ __forceinline__ uint32_t warp_upsert(const AggArgs& A, bool (&need)[K], const uint64_t (&w)[K][2],
+                                                const uint32_t (&nm)[K], const uint64_t (&h)[K], uint32_t (&g)[K], bool& full,
+                                                uint32_t* err) {
+    const TableView& t = A.t;
+    const bool wide = t.nwords > 1;
+    const int lane = threadIdx.x & 31;
+    uint64_t i[K];
+    ulonglong2 v[K];
+    uint32_t made = 0, steps = 0, spins = 0;
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        i[k] = h[k] & t.mask;
+        g[k] = kNone;
+        any = any || need[k];
+    }
+    while (__any_sync(0xFFFFFFFFu, any)) {
+#pragma unroll
+        for (int k = 0; k < K; k++)
+            if (need[k]) v[k] = wide ? ld_slot_acquire(slot_at(t, i[k])) : ld_slot(slot_at(t, i[k]));
+        uint32_t old[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            old[k] = 1;
+            if (need[k] && (uint32_t)v[k].x == 0) {
+                if (full) need[k] = false;  // the row overflows
+                else old[k] = atomicCAS((uint32_t*)slot_at(t, i[k]), 0u, 1u);
+            }
+        }
+        unsigned m[K];
+        uint32_t total = 0;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            m[k] = __ballot_sync(0xFFFFFFFFu, old[k] == 0);
+            total += __popc(m[k]);
+        }
+        if (total) {  // the same in every lane
+            uint32_t id = 0;
+            if (lane == 0) id = atomicAdd(A.ngroups, total);
+            id = __shfl_sync(0xFFFFFFFFu, id, 0);
+            full = id + total > A.gid_cap || id + total < id;
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                if (old[k] == 0) {
+                    const uint32_t mine = id + __popc(m[k] & ((1u << lane) - 1u));
+                    uint64_t* s = slot_at(t, i[k]);
+                    const uint64_t x = (2u | (nm[k] << 8)) | ((uint64_t)mine << 32);
+                    if (mine >= A.gid_cap) {
+                        publish_state((uint32_t*)s, 0);
+                    } else {
+                        if (wide) {
+                            s[2] = w[k][1];
+                            st_slot_release(s, x, w[k][0]);
+                        } else {
+                            st_slot(s, x, w[k][0]);
+                        }
+                        g[k] = mine;
+                        made |= 1u << k;
+                    }
+                    need[k] = false;
+                }
+                id += __popc(m[k]);
+            }
+        }
+        any = false;
+        bool waiting = false;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            if (!need[k]) continue;
+            const uint32_t st = (uint32_t)v[k].x;
+            if (st > 1) {  // a published slot: this key's, or the next one's turn
+                g[k] = slot_match(t, i[k], v[k], w[k], nm[k]);
+                need[k] = g[k] == kNone;
+                i[k] = (i[k] + 1) & t.mask;
+            }
+            waiting = waiting || st <= 1;
+            any = any || need[k];
+        }
+        // a claim that is never published, or a table without an empty slot, ends the wait
+        if (waiting && ++spins >= kSpinLimit) {
+            atomicOr(err, (uint32_t)DE_TIMEOUT);
+            any = false;
+        }
+        if (++steps > t.mask + kSpinLimit) any = false;
+        if (!any) {
+#pragma unroll
+            for (int k = 0; k < K; k++) need[k] = false;
+        }
+    }
+    return made;
+}
+
 // Merge a shared-memory partial (word(s) at src) into the global block word(s) at dst.
 __device__ __forceinline__ void acc_merge(int kind, uint64_t* dst, const uint64_t* src) {
     uint64_t v = src[0];

@@ -36,6 +36,7 @@ struct ProbeDev {
 // HashJoinProbe) for one launch.
 struct PipeArgs {
     int64_t n;               // rows to visit (selection length when `sel` is set)
+    int64_t row0;            // first row to visit (a multiple of 4096; runtime-specialized aggregates only)
     const uint32_t* sel;     // optional input selection vector
     int64_t nsrc;            // rows of the source batch: every selected row id is below it
     const Instr* prog;
@@ -69,6 +70,8 @@ struct AggArgs {
     uint32_t* ovf;            // overflow row contexts
     unsigned long long* ovf_count;
     uint64_t ovf_cap;
+    const uint32_t* skip;     // optional (runtime-specialized kernels only): the launch does nothing when
+                              // *skip is set (the rows before it showed that the table is too small)
     // Direct group slots (runtime-specialized kernels only; 0 = off): when every GROUP BY key
     // takes few values in this launch (a dictionary-coded string: its string ids lie in
     // [dbase, dbase + range - 2]; a BOOL), the key's slot is sum_k term_k * dmul[k] with
@@ -90,6 +93,9 @@ constexpr int kAggSmemBudget = 74 << 10;
 
 ML_HD inline bool agg_direct_on(const AggArgs& A) { return A.smem_groups > 0 && !A.ungrouped && A.group_probe < 0; }
 ML_HD inline uint64_t agg_direct_bytes(const AggArgs& A) { return agg_direct_on(A) ? 4 * kDirectSlots : 0; }
+
+// Reductions of the warp-cooperative group updates (coop_red in ml_agg.cuh).
+enum CoopOp { CO_ADD_F64 = 0, CO_ADD_U64, CO_MIN_U64, CO_MAX_U64, CO_MIN_S64, CO_MAX_S64 };
 
 struct SortDev {
     int32_t nkeys, pad;

@@ -594,56 +594,97 @@ __device__ inline uint32_t table_insert_row1(const TableView& t, uint64_t key, u
     return kNone;
 }
 
+// A slot's first 16 bytes (state, payload, first key word) as one 128-bit access, so a reader never
+// sees a state without its payload and key.
+__device__ __forceinline__ ulonglong2 ld_slot(const uint64_t* p) {
+    ulonglong2 v;
+    asm volatile("{\n\t.reg .b128 v;\n\tld.relaxed.gpu.global.b128 v, [%2];\n\tmov.b128 {%0, %1}, v;\n\t}"
+                 : "=l"(v.x), "=l"(v.y)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ ulonglong2 ld_slot_acquire(const uint64_t* p) {
+    ulonglong2 v;
+    asm volatile("{\n\t.reg .b128 v;\n\tld.acquire.gpu.global.b128 v, [%2];\n\tmov.b128 {%0, %1}, v;\n\t}"
+                 : "=l"(v.x), "=l"(v.y)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_slot(uint64_t* p, uint64_t x, uint64_t y) {
+    asm volatile("{\n\t.reg .b128 v;\n\tmov.b128 v, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], v;\n\t}" ::"l"(p), "l"(x), "l"(y)
+                 : "memory");
+}
+__device__ __forceinline__ void st_slot_release(uint64_t* p, uint64_t x, uint64_t y) {
+    asm volatile("{\n\t.reg .b128 v;\n\tmov.b128 v, {%1, %2};\n\tst.release.gpu.global.b128 [%0], v;\n\t}" ::"l"(p), "l"(x), "l"(y)
+                 : "memory");
+}
+// The payload of a slot read by ld_slot (ld_slot_acquire for two-word keys) if it holds the key w under
+// the null mask nm, else kNone.
+__device__ __forceinline__ uint32_t slot_match(const TableView& t, uint64_t i, ulonglong2 v, const uint64_t* w, uint32_t nm) {
+    if ((uint32_t)v.x != (2u | (nm << 8)) || v.y != w[0]) return kNone;
+    if (t.nwords > 1 && *(const volatile uint64_t*)(slot_at(t, i) + 2) != w[1]) return kNone;
+    return (uint32_t)(v.x >> 32);
+}
+
 // Find or insert under concurrent insertion.  On insert, `assign` produces the payload
 // (kNone = refuse: the slot is released and kNone returned).  *inserted tells the caller
 // whether this thread created the entry.
 // With `count` set, a new key is refused without touching the slot once *count has reached
 // `limit` (a full aggregation table: the row goes to the overflow list at once).
+// A one-word key's slot is published by one 128-bit store and read by one 128-bit load, so neither side
+// needs a fence (a release store here also waited for all of the thread's group updates in flight);
+// the second word of a wider key is written before a release and read after an acquire.
 template <class Assign>
 __device__ inline uint32_t table_upsert(const TableView& t, const uint64_t* w, uint32_t nm, uint64_t h, uint32_t* err,
                                         Assign assign, bool* inserted, uint64_t* slot_out,
                                         const uint32_t* count = nullptr, uint32_t limit = 0) {
     uint64_t i = h & t.mask;
     const uint32_t full = 2u | (nm << 8);
+    const bool wide = t.nwords > 1;
     *inserted = false;
     for (uint64_t n = 0; n <= t.mask;) {
         uint64_t* s = slot_at(t, i);
         uint32_t* st_p = (uint32_t*)s;
-        uint32_t st = load_state(st_p);
-        if (st == 0) {
+        ulonglong2 v = wide ? ld_slot_acquire(s) : ld_slot(s);
+        if ((uint32_t)v.x == 0) {
             if (count && *(const volatile uint32_t*)count >= limit) return kNone;
-            uint32_t old = atomicCAS(st_p, 0u, 1u);
-            if (old == 0) {
-                uint32_t p = assign();
+            if (atomicCAS(st_p, 0u, 1u) == 0) {
+                const uint32_t p = assign();
                 if (p == kNone) {
                     publish_state(st_p, 0);
                     return kNone;
                 }
-                s[1] = w[0];
-                if (t.nwords > 1) s[2] = w[1];
-                st_p[1] = p;
-                publish_state(st_p, full);
+                const uint64_t x = full | ((uint64_t)p << 32);
+                if (wide) {
+                    s[2] = w[1];
+                    st_slot_release(s, x, w[0]);
+                } else {
+                    st_slot(s, x, w[0]);
+                }
                 *inserted = true;
                 *slot_out = i;
                 return p;
             }
-            st = old;
+            v = wide ? ld_slot_acquire(s) : ld_slot(s);
         }
-        if (st == 1) {
+        if ((uint32_t)v.x == 1) {
             uint32_t spins = 0;
             do {
                 __nanosleep(20);
-                st = load_state(st_p);
-            } while (st == 1 && ++spins < kSpinLimit);
-            if (st == 1) {
+                v = wide ? ld_slot_acquire(s) : ld_slot(s);
+            } while ((uint32_t)v.x == 1 && ++spins < kSpinLimit);
+            if ((uint32_t)v.x == 1) {
                 atomicOr(err, (uint32_t)DE_TIMEOUT);
                 return kNone;
             }
-            if (st == 0) continue;  // the claimer released the slot: retry it
         }
-        if (st == full && s[1] == w[0] && (t.nwords == 1 || s[2] == w[1])) {
+        if ((uint32_t)v.x == 0) continue;  // the claimer released the slot: retry it
+        const uint32_t p = slot_match(t, i, v, w, nm);
+        if (p != kNone) {
             *slot_out = i;
-            return st_p[1];
+            return p;
         }
         i = (i + 1) & t.mask;
         n++;

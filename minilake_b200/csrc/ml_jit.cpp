@@ -85,6 +85,8 @@ Nvrtc& nvrtc() {
     return n;
 }
 
+}  // namespace
+
 bool jit_enabled(Ctx* ctx) {
     if (ctx->flags & ML_CTX_INTERPRET) return false;
     static const bool env_off = [] {
@@ -93,6 +95,8 @@ bool jit_enabled(Ctx* ctx) {
     }();
     return !env_off && nvrtc().ok;
 }
+
+namespace {
 
 const char kStdint[] =
     "#pragma once\n"
@@ -807,14 +811,14 @@ std::string row_loop(const PipeArgs& P, bool batched, const std::string& body, i
     std::string s;
     if (!batched) {
         s += "    const int64_t stride = (int64_t)gridDim.x * blockDim.x;\n";
-        s += "    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P.n; i += stride) {\n";
+        s += "    for (int64_t i = P.row0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P.n; i += stride) {\n";
         s += "        RowCtx x;\n";
         s += P.sel ? "        bool sel_ok = true;\n        x.r = sel_row(P, i, sel_ok);\n        if (!sel_ok) continue;\n"
                    : "        x.r = (uint32_t)i;\n";
         s += "        x.b0 = x.b1 = x.b2 = x.b3 = 0;\n        x.head = 0;\n";
     } else {
         s += "    const int64_t tile = (int64_t)" + num(K) + " * blockDim.x;\n";
-        s += "    for (int64_t base = (int64_t)blockIdx.x * tile; base < P.n; base += (int64_t)gridDim.x * tile) {\n";
+        s += "    for (int64_t base = P.row0 + (int64_t)blockIdx.x * tile; base < P.n; base += (int64_t)gridDim.x * tile) {\n";
         s += tile_rows(P, K, contig, "        ");
     }
     s += body;
@@ -826,9 +830,104 @@ std::string row_loop(const PipeArgs& P, bool batched, const std::string& body, i
     return s;
 }
 
+// Whether a launch's batched rows update global group blocks by the warp together (emit_coop, and for a
+// hashed GROUP BY warp_upsert): where the groups are too many for shared memory to take a large share of
+// the rows, or are a join's build rows.  Elsewhere its registers cost more than it saves (the star join,
+// 25 groups: 189 us without, 268 us with it).
+bool coop_updates(const AggArgs& A) { return !A.ungrouped && A.dslots == 0 && (A.group_probe >= 0 || A.smem_groups == 0); }
+
+// The warp-cooperative update of the batched row `j`'s group block (coop_red): the words that take the
+// same reduction, up to eight at a time, by that many neighbouring lanes per row.  gg<j> is the row's
+// group (kNone: none, or updated already), av<j>_<k> / ak<j>_<k> aggregate k's argument.
+void emit_coop(Gen& g, const AggArgs& A, int j) {
+    struct Word {
+        int off;
+        std::string value;  // "": the constant 1 (the row counter)
+        bool flag;          // a 0 / 1 value
+        std::string when;   // condition of the update, "" when every row of the group has one
+        std::string null_value;
+    };
+    std::vector<Word> ops[6], counts{{0, "", false, "", ""}};
+    const std::string J = num(j), gg = "gg" + J;
+    for (int k = 0; k < A.nagg; k++) {
+        const AggDev& a = A.aggs[k];
+        if (a.func == ML_AGG_COUNT_STAR) continue;
+        const std::string v = a.has_arg ? "av" + J + "_" + num(k) : "0ull", ok = a.has_arg ? "ak" + J + "_" + num(k) : "";
+        const std::string order = "f64_order(as_f64(" + v + "))";
+        switch (a.kind) {
+            case A_SUM_I64: ops[CO_ADD_U64].push_back({a.off, v, false, ok, "0ull"}); break;
+            case A_SUM_F64: ops[CO_ADD_F64].push_back({a.off, v, false, ok, "0x8000000000000000ull"}); break;
+            case A_AVG:
+                ops[CO_ADD_F64].push_back({a.off, v, false, ok, "0x8000000000000000ull"});
+                counts.push_back({a.off + 1, ok, true, ok, "0ull"});
+                break;
+            case A_MIN_I64: ops[CO_MIN_S64].push_back({a.off, v, false, ok, "0x7FFFFFFFFFFFFFFFull"}); break;
+            case A_MAX_I64: ops[CO_MAX_S64].push_back({a.off, v, false, ok, "0x8000000000000000ull"}); break;
+            case A_MIN_F64: ops[CO_MIN_U64].push_back({a.off, order, false, ok, "~0ull"}); break;
+            case A_MAX_F64: ops[CO_MAX_U64].push_back({a.off, order, false, ok, "0ull"}); break;
+            default: counts.push_back({a.off, ok, true, ok, "0ull"}); break;  // COUNT(x)
+        }
+    }
+    auto& with = ops[!ops[CO_ADD_F64].empty() ? CO_ADD_F64 : CO_ADD_U64];
+    with.insert(with.begin(), counts.begin(), counts.end());
+    g.open("if (__any_sync(0xFFFFFFFFu, " + gg + " != kNone)) {  // the warp's groups of row " + J);
+    const std::string S = num(A.stride);
+    for (int op = 0; op < 6; op++)
+        for (size_t w0 = 0; w0 < ops[op].size(); w0 += 8) {
+            const std::vector<Word> ws(ops[op].begin() + w0, ops[op].begin() + std::min(w0 + 8, ops[op].size()));
+            const int m = (int)ws.size();
+            if (m == 1) {
+                const Word& x = ws[0];
+                g.line("if (" + gg + " != kNone" + (x.when.empty() ? "" : " && " + x.when) + ") coop_red<" + num(op) +
+                       ">(A.acc + (uint64_t)" + gg + " * " + S + " + " + num(x.off) + ", " +
+                       (x.value.empty() || x.flag ? "1ull" : x.value) + ");");
+                continue;
+            }
+            int L = 2;
+            while (L < m) L *= 2;
+            uint64_t offs = 0;
+            for (int i = 0; i < m; i++) offs |= (uint64_t)ws[i].off << (8 * i);
+            g.open("{");
+            for (int i = 0; i < m; i++) {  // each word's value, its identity for a NULL argument
+                const Word& x = ws[i];
+                if (x.value.empty()) continue;
+                const std::string n = "u" + num(i);
+                if (x.flag) g.line("const uint32_t " + n + " = " + x.value + " ? 1u : 0u;");
+                else if (x.when.empty()) g.line("const uint64_t " + n + " = " + x.value + ";");
+                else g.line("const uint64_t " + n + " = " + x.when + " ? " + x.value + " : " + x.null_value + ";");
+            }
+            g.line("const int lw = threadIdx.x & " + num(L - 1) + ";");
+            g.line("const uint32_t ow = (uint32_t)(" + hex(offs) + " >> (8 * lw)) & 255u;");
+            // rolled past pairs: unrolled, four rows' updates of many words no longer fit the instruction cache
+            g.line(L == 2 ? "_Pragma(\"unroll\")" : "_Pragma(\"unroll 1\")");
+            g.open("for (int h = 0; h < " + num(L) + "; h++) {");
+            g.line("const int src = (int)((threadIdx.x & 31) / " + num(L) + ") + h * " + num(32 / L) + ";");
+            g.line("const uint32_t gr = __shfl_sync(0xFFFFFFFFu, " + gg + ", src);");
+            g.line("uint64_t x = 1ull;");
+            for (int i = 0; i < m; i++) {
+                if (ws[i].value.empty()) continue;
+                const std::string n = "u" + num(i);
+                g.line("{ const uint64_t y = __shfl_sync(0xFFFFFFFFu, " + n + ", src); if (lw == " + num(i) + ") x = y; }");
+            }
+            g.line("if (gr != kNone" + std::string(m < L ? " && lw < " + num(m) : "") + ") coop_red<" + num(op) +
+                   ">(A.acc + (uint64_t)gr * " + S + " + ow, x);");
+            g.close();
+            g.close();
+        }
+    for (int k = 0; k < A.nagg; k++)
+        if (A.aggs[k].count_valid && A.aggs[k].func != ML_AGG_COUNT_STAR) {
+            const std::string ok = A.aggs[k].has_arg ? " && ak" + J + "_" + num(k) : "";
+            g.line("if (" + gg + " != kNone" + ok + ") count_global(A.aggs[" + num(k) + "].vcnt + " + gg + ");");
+        }
+    g.close();
+}
+
 // The aggregate update of one row combination (agg_update + agg_fold), in `g`'s current
-// row context; `g.fail` abandons the combination.
-void emit_aggregate(Gen& g, const AggArgs& A) {
+// row context; `g.fail` abandons the combination.  coop >= 0: the batched row's number; groups past
+// shared memory are left to emit_coop through gg<coop> and av<coop>_* / ak<coop>_*.
+// With `found` the row's key words, null mask, group (kNone: the table is full) and whether it is new
+// are in wkg[coop], nmg[coop], gf[coop] and bit coop of `made` (jit_agg_source).
+void emit_aggregate(Gen& g, const AggArgs& A, int coop = -1, bool found = false) {
     const bool smem = A.smem_groups > 0;
     const std::string S = num(A.stride);
     if (A.group_probe >= 0) {
@@ -837,28 +936,35 @@ void emit_aggregate(Gen& g, const AggArgs& A) {
         g.line("const uint32_t g = 0;");
     } else {
         const bool direct = A.dslots > 0;  // implies agg_direct_on(A)
-        g.line("uint64_t wkg[2] = {0ull, 0ull};");
-        g.line("uint32_t nmg = 0;");
-        if (direct) g.line("uint32_t dsg = 0;");
-        g.key(A.keys, "wkg", "", "nmg", direct ? "dsg" : "");
-        g.line("bool ins = false;");
-        // with direct slots, the CTA's index first: the global table only on the slot's first use
-        g.line(direct ? "uint32_t g = dsg < A.dslots ? dsl[dsg] - 1u : kNone;" : "uint32_t g = kNone;");
-        g.open("if (g == kNone) {");
-        g.line("uint64_t slot;");
-        g.line("g = table_upsert(A.t, wkg, nmg, key_hash(wkg, " + num(A.keys.nwords) +
-               ", nmg), P.err, [&]() -> uint32_t { const uint32_t id = atomicAdd(A.ngroups, 1u); "
-               "return id < A.gid_cap ? id : kNone; }, &ins, &slot, A.ngroups, A.gid_cap);");
-        if (direct) g.line("if (g != kNone && dsg < A.dslots) dsl[dsg] = g + 1u;");
-        g.close();
+        const std::string J = found ? "[" + num(coop) + "]" : "", wkg = "wkg" + J, nmg = "nmg" + J;
+        if (!found) {
+            g.line("uint64_t wkg[2] = {0ull, 0ull};");
+            g.line("uint32_t nmg = 0;");
+            if (direct) g.line("uint32_t dsg = 0;");
+            g.key(A.keys, "wkg", "", "nmg", direct ? "dsg" : "");
+        }
+        if (found) {
+            g.line("const uint32_t g = gf" + J + ";");
+            g.line("const bool ins = (made >> " + num(coop) + ") & 1u;");
+        } else {
+            g.line("bool ins = false;");
+            // with direct slots, the CTA's index first: the global table only on the slot's first use
+            g.line(direct ? "uint32_t g = dsg < A.dslots ? dsl[dsg] - 1u : kNone;" : "uint32_t g = kNone;");
+            g.open("if (g == kNone) {");
+            g.line("uint64_t slot;");
+            g.line("g = table_upsert(A.t, wkg, nmg, key_hash(wkg, " + num(A.keys.nwords) +
+                   ", nmg), P.err, [&]() -> uint32_t { return new_group(A); }, &ins, &slot, A.ngroups, A.gid_cap);");
+            if (direct) g.line("if (g != kNone && dsg < A.dslots) dsl[dsg] = g + 1u;");
+            g.close();
+        }
         g.open("if (g == kNone) {");
         g.line("record_overflow(P, A, " + g.x + ");");
         g.line(g.fail);
         g.close();
         g.open("if (ins) {");
-        g.line("A.gkeys[g] = wkg[0];");
-        if (A.keys.nwords > 1) g.line("A.gkeys[(uint64_t)A.gid_cap + g] = wkg[1];");
-        g.line("A.gnull[g] = nmg;");
+        g.line("A.gkeys[g] = " + wkg + "[0];");
+        if (A.keys.nwords > 1) g.line("A.gkeys[(uint64_t)A.gid_cap + g] = " + wkg + "[1];");
+        g.line("A.gnull[g] = " + nmg + ";");
         g.close();
     }
     // every aggregate's argument, evaluated once for whichever accumulators the group uses
@@ -902,8 +1008,21 @@ void emit_aggregate(Gen& g, const AggArgs& A) {
         g.close("} else {");
         g.open("");
     }
+    if (coop >= 0) {
+        const std::string J = num(coop);
+        for (int k = 0; k < A.nagg; k++)
+            if (A.aggs[k].func != ML_AGG_COUNT_STAR && A.aggs[k].has_arg)
+                g.line("av" + J + "_" + num(k) + " = " + args[k].v + "; ak" + J + "_" + num(k) + " = " + args[k].k + ";");
+        if (!smem) {
+            g.line("gg" + J + " = g;");
+            if (priv > 0) g.close();
+            return;
+        }
+        g.line("if ((int)g >= A.smem_groups) { gg" + J + " = g; " + g.fail + " }");
+    }
     if (smem) {
-        g.line("uint64_t* blk = (int)g < A.smem_groups ? smem + (uint64_t)g * " + S + " : A.acc + (uint64_t)g * " + S + ";");
+        g.line("uint64_t* blk = " + std::string(coop >= 0 ? "" : "(int)g >= A.smem_groups ? A.acc + (uint64_t)g * " + S + " : ") +
+               "smem + (uint64_t)g * " + S + ";");
         g.line("atomicAdd((unsigned long long*)blk, 1ull);");
     } else {
         g.line("uint64_t* blk = A.acc + (uint64_t)g * " + S + ";");
@@ -1057,11 +1176,42 @@ std::string jit_agg_source(const Pipeline& pipe, const PipeArgs& P, const AggArg
                 if (A.aggs[k].has_arg && A.aggs[k].func != ML_AGG_COUNT_STAR) g.slots_of(A.aggs[k].arg, slots);
             std::vector<std::map<int, Gen::V>> pre;
             g.preload_rows(slots, pre);
+            // a hashed GROUP BY reads the first slot of every row's key before any row is resolved
+            const bool found = A.group_probe < 0 && coop_updates(A);
+            if (found) {
+                const std::string K = num(g.rows_per_thread);
+                g.line("uint64_t wkg[" + K + "][2] = {}, hg[" + K + "] = {};");
+                g.line("uint32_t nmg[" + K + "] = {}, gf[" + K + "];");
+                g.line("bool nd[" + K + "] = {};");
+                rows([&](int j, const std::string& a) {
+                    g.cols = pre[j];
+                    const std::string J = num(j);
+                    g.open("if (" + a + ") {  // group key of row " + J);
+                    g.key(A.keys, "wkg[" + J + "]", "", "nmg[" + J + "]");
+                    g.line("hg[" + J + "] = key_hash(wkg[" + J + "], " + num(A.keys.nwords) + ", nmg[" + J + "]);");
+                    g.line("nd[" + J + "] = true;");
+                    g.close();
+                });
+                g.line("const uint32_t made = warp_upsert<" + K + ">(A, nd, wkg, nmg, hg, gf, tfull, P.err);");
+            }
             rows([&](int j, const std::string& a) {
                 g.cols = pre[j];
+                const bool coop = coop_updates(A);
+                if (coop) {
+                    g.line("uint32_t gg" + num(j) + " = kNone;");
+                    for (int k = 0; k < A.nagg; k++)
+                        if (A.aggs[k].has_arg && A.aggs[k].func != ML_AGG_COUNT_STAR) {
+                            const std::string n = num(j) + "_" + num(k);
+                            g.line("uint64_t av" + n + " = 0; bool ak" + n + " = false;");
+                        }
+                }
                 g.open("if (" + a + ") do {  // aggregate");
-                emit_aggregate(g, A);
+                emit_aggregate(g, A, coop ? j : -1, found);
                 g.close("} while (0);");
+                if (coop) {
+                    g.line("__syncwarp();");
+                    emit_coop(g, A, j);
+                }
             });
             g.cols.clear();
         });
@@ -1076,10 +1226,12 @@ std::string jit_agg_source(const Pipeline& pipe, const PipeArgs& P, const AggArg
     src += "extern \"C\" __global__ void __launch_bounds__(256) ml_pipeline_aggregate(const __grid_constant__ PipeArgs P, "
            "const __grid_constant__ AggArgs A) {\n";
     src += "    extern __shared__ __align__(16) uint64_t smem[];\n";
+    if (A.group_probe < 0 && !A.ungrouped) src += "    if (A.skip && *A.skip) return;\n";
     if (smem) src += "    smem_setup(A, smem);\n    __syncthreads();\n";
     if (A.dslots > 0) src += "    uint32_t* const dsl = direct_slots(A, smem);\n";
     if (A.priv_groups > 0) src += priv_init(A);
     src += g.pre();
+    if (batched && A.group_probe < 0 && coop_updates(A)) src += "    bool tfull = false;  // the table takes no more groups\n";
     src += row_loop(P, batched, g.body(), kRowsPerThread, g.contig);
     if (smem) src += "    __syncthreads();\n    smem_flush(A, smem);\n";
     if (A.priv_groups > 0) src += priv_flush(A);
@@ -1095,7 +1247,7 @@ namespace {
 // sizes and constants to zero): equal signatures give equal generated sources.
 std::string signature(char kind, const PipeArgs& P, const AggArgs* A, const KeyLayout* L) {
     PipeArgs p = P;
-    p.n = 0;
+    p.n = p.row0 = 0;
     p.sel = P.sel ? (const uint32_t*)1 : nullptr;
     p.prog = nullptr;
     p.arena = nullptr;
@@ -1128,6 +1280,7 @@ std::string signature(char kind, const PipeArgs& P, const AggArgs* A, const KeyL
         a.acc = nullptr;
         a.ovf = nullptr;
         a.ovf_count = nullptr;
+        a.skip = nullptr;
         a.gid_cap = 0;
         a.ovf_cap = 0;
         a.smem_groups = a.smem_groups > 0;

@@ -13,6 +13,9 @@
 
 namespace mlg {
 
+// Whether the context's pipelines run as specialized kernels.
+bool jit_enabled(Ctx* ctx);
+
 // Specialized fused filter/probe/aggregate kernel (signature of k_agg) for this launch,
 // or nullptr when runtime compilation is unavailable or disabled for the context.
 void* jit_agg_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, const AggArgs& A);

@@ -34,6 +34,10 @@ int xpart_blocks(int64_t n);
 void launch_xpart_count(const uint64_t* h, int64_t n, int nparts, uint32_t* counts, cudaStream_t s);
 void launch_xpart_scatter(const uint64_t* h, int64_t n, int nparts, const uint64_t* offs, uint32_t* perm, cudaStream_t s);
 // Initialize group blocks [from, to) to the identities of the aggregates.
+// *skip = the first rows of a batch showed that the group table is too small for the rest: some did
+// not fit, or the groups fill more than a quarter of it.
+void launch_agg_guard(const unsigned long long* ovf_count, const uint32_t* ngroups, uint32_t gid_cap, uint32_t* skip,
+                      cudaStream_t s);
 void launch_acc_init(const AggArgs& A, uint32_t from, uint32_t to, cudaStream_t s);
 // Final values: keys decoded into `key_out` (fixed-width or u32 string ids), aggregates into
 // `agg_out`; validity as u32 words (LSB first) in *_valid.
@@ -126,17 +130,19 @@ struct SortWord {
     int32_t nulls_first;
     const uint32_t* rank;  // SW_RANK: rank of each dictionary code (dict_len + 1 entries)
 };
-// Bits of the key words that form a u32 sort key: ((word >> shift) & mask) << pos each; the segments
-// of one word follow each other.
+// Bits of the key words that form a u32 sort key: (((word - sub) >> shift) & mask) << pos each; the
+// segments of one word follow each other.
 struct SortSegs {
     int32_t n;
     struct {
         int32_t word, shift, pos;
         uint32_t mask;
+        uint64_t sub;
     } s[32];
 };
-// diff[y] |= the bits in which word y differs between rows (zeroed), `nwords` device words.
-void launch_sort_bits(const SortWord* words, int nwords, int64_t n, unsigned long long* diff, cudaStream_t s);
+// stats[3 y ..]: the bits in which word y differs between rows, its smallest and its largest value
+// (`nwords` device words, at most 32).
+void launch_sort_bits(const SortWord* words, int nwords, int64_t n, unsigned long long* stats, cudaStream_t s);
 // The u32 keys of rows perm[0..n) (nullptr: 0..n) and their digit histograms (digits x 256, zeroed).
 void launch_sort_keys(const SortWord* words, const SortSegs& S, const uint32_t* perm, int64_t n, uint32_t* keys, int digits,
                       uint32_t* hist, cudaStream_t s);

@@ -3,8 +3,9 @@
 // sort_batches without a limit (sort.rs:85-132) is a stable sort by compare_rows.  Every sort key is a
 // sequence of order-preserving 64-bit words (sort_word below; SortWord lists them least significant
 // first), so a row's key is one long bit string.  Bits that are the same in every row cannot decide, so
-// only the varying ones are sorted (their order is kept): 32 of them at a time form a u32 key, sorted
-// with its row id by 8-bit digits, one kernel per digit (k_radix_pass).
+// only the varying ones are sorted (their order is kept), or a word's distance from the smallest one
+// where that is shorter (small numbers of both signs vary in every bit): 32 bits at a time form a u32
+// key, sorted with its row id by 8-bit digits, one kernel per digit (k_radix_pass).
 //
 // With more than 32 varying bits, the top 32 usually tell almost all rows apart (10M random doubles:
 // some 20k rows share theirs with another row): the rows are sorted by those, and the few runs of equal
@@ -100,14 +101,14 @@ __device__ __forceinline__ void with_word(const SortWord& w, F&& f) {
     f(AnyWord{w});
 }
 
-// diff[y] |= the bits of word y that differ from row 0's in some row (grid.y words): one pass over the
-// column, bound by reading it.
+// Per word y (grid.y words): stats[3 y] |= the bits that differ from row 0's in some row, stats[3 y + 1]
+// and [3 y + 2] = the smallest and the largest word.  One pass over the column, bound by reading it.
 constexpr int kWordRows = 8;  // rows per thread and step
-__global__ void __launch_bounds__(256) k_sort_bits(const SortWord* words, int64_t n, unsigned long long* diff) {
+__global__ void __launch_bounds__(256) k_sort_bits(const SortWord* words, int64_t n, unsigned long long* stats) {
     __shared__ SortWord w;
     if (threadIdx.x == 0) w = words[blockIdx.y];
     __syncthreads();
-    uint64_t acc = 0;
+    uint64_t acc = 0, lo = ~0ull, hi = 0;
     with_word(w, [&](auto get) {
         const uint64_t ref = get(0);
         for (int64_t base = (int64_t)blockIdx.x * (256 * kWordRows); base < n; base += (int64_t)gridDim.x * (256 * kWordRows)) {
@@ -118,13 +119,45 @@ __global__ void __launch_bounds__(256) k_sort_bits(const SortWord* words, int64_
                 x[j] = r < n ? get((uint32_t)r) : ref;
             }
 #pragma unroll
-            for (int j = 0; j < kWordRows; j++) acc |= x[j] ^ ref;
+            for (int j = 0; j < kWordRows; j++) {
+                acc |= x[j] ^ ref;
+                lo = x[j] < lo ? x[j] : lo;
+                hi = x[j] > hi ? x[j] : hi;
+            }
         }
     });
-    const uint32_t lo = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)acc), hi = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)(acc >> 32));
-    const uint64_t all = ((uint64_t)hi << 32) | lo;
-    if ((threadIdx.x & 31) == 0 && (all & ~*(volatile unsigned long long*)(diff + blockIdx.y)))
-        atomicOr(diff + blockIdx.y, (unsigned long long)all);
+    for (int o = 16; o; o >>= 1) {
+        const uint64_t l = __shfl_xor_sync(0xFFFFFFFFu, lo, o), h = __shfl_xor_sync(0xFFFFFFFFu, hi, o);
+        acc |= __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+        lo = l < lo ? l : lo;
+        hi = h > hi ? h : hi;
+    }
+    __shared__ uint64_t part[3][8];  // one update per block: they all go to the same words
+    if ((threadIdx.x & 31) == 0) {
+        part[0][threadIdx.x >> 5] = acc;
+        part[1][threadIdx.x >> 5] = lo;
+        part[2][threadIdx.x >> 5] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x) return;
+    for (int k = 1; k < 8; k++) {
+        acc |= part[0][k];
+        lo = part[1][k] < lo ? part[1][k] : lo;
+        hi = part[2][k] > hi ? part[2][k] : hi;
+    }
+    if (lo > hi) return;  // no rows
+    unsigned long long* st = stats + 3 * blockIdx.y;
+    const volatile unsigned long long* seen = st;
+    if (acc & ~seen[0]) atomicOr(st, (unsigned long long)acc);
+    if (lo < seen[1]) atomicMin(st + 1, (unsigned long long)lo);
+    if (hi > seen[2]) atomicMax(st + 2, (unsigned long long)hi);
+}
+__global__ void k_sort_stats_init(unsigned long long* stats, int nwords) {
+    if (threadIdx.x < nwords) {
+        stats[3 * threadIdx.x] = 0;
+        stats[3 * threadIdx.x + 1] = ~0ull;
+        stats[3 * threadIdx.x + 2] = 0;
+    }
 }
 
 // keys[i] = the segments' bits of row perm[i] (row i without perm), and the histograms of the key's
@@ -155,8 +188,9 @@ __global__ void __launch_bounds__(256) k_sort_keys(const SortWord* words, const 
                 for (int k = k0; k < k1; k++) {
                     const int shift = S.s[k].shift, pos = S.s[k].pos;
                     const uint32_t mask = S.s[k].mask;
+                    const uint64_t sub = S.s[k].sub;
 #pragma unroll
-                    for (int j = 0; j < kWordRows; j++) key[j] |= ((uint32_t)(x[j] >> shift) & mask) << pos;
+                    for (int j = 0; j < kWordRows; j++) key[j] |= ((uint32_t)((x[j] - sub) >> shift) & mask) << pos;
                 }
             });
         }
@@ -377,8 +411,9 @@ void launch_iota_u32(uint32_t* out, int64_t n, cudaStream_t s) {
 void launch_max_strlen(const uint32_t* off, int64_t n, unsigned int* out, cudaStream_t s) {
     if (n > 0) k_max_strlen<<<grid_rows(n, 256, 4), 256, 0, s>>>(off, n, out);
 }
-void launch_sort_bits(const SortWord* words, int nwords, int64_t n, unsigned long long* diff, cudaStream_t s) {
-    if (n > 0 && nwords > 0) k_sort_bits<<<dim3(grid_rows(n, 256 * kWordRows, 8), nwords), 256, 0, s>>>(words, n, diff);
+void launch_sort_bits(const SortWord* words, int nwords, int64_t n, unsigned long long* stats, cudaStream_t s) {
+    k_sort_stats_init<<<1, 32, 0, s>>>(stats, nwords);
+    if (n > 0 && nwords > 0) k_sort_bits<<<dim3(grid_rows(n, 256 * kWordRows, 6), nwords), 256, 0, s>>>(words, n, stats);
 }
 void launch_sort_keys(const SortWord* words, const SortSegs& S, const uint32_t* perm, int64_t n, uint32_t* keys, int digits,
                       uint32_t* hist, cudaStream_t s) {
