@@ -7,6 +7,7 @@
 // as a multiple of the 148 SMs, state that fits in L2 (126 MB) kept there, and
 // shared-memory privatization wherever many rows hit few addresses.
 #include <algorithm>
+#include <cmath>
 
 #include "ml_agg.cuh"
 #include "ml_kernels.cuh"
@@ -975,23 +976,12 @@ __device__ __forceinline__ uint64_t sort_prefix(const SortDev& S, uint32_t r) {
     return S.asc[0] ? p : ~p;
 }
 
-// One block sorts kTopNChunk rows (bitonic, ascending by compare_rows) and writes the
-// first k.  Keys are compared by their shared-memory prefix first.
-__global__ void __launch_bounds__(1024) k_topn_chunk(const __grid_constant__ SortDev S, const uint32_t* in, int64_t n,
-                                                    int k, uint32_t* out) {
-    __shared__ uint64_t pre[kTopNChunk];
-    __shared__ uint32_t idx[kTopNChunk];
-    int64_t base = (int64_t)blockIdx.x * kTopNChunk;
-    for (int j = threadIdx.x; j < kTopNChunk; j += blockDim.x) {
-        int64_t i = base + j;
-        uint32_t r = i < n ? (in ? in[i] : (uint32_t)i) : kNone;
-        idx[j] = r;
-        pre[j] = sort_prefix(S, r);
-    }
-    __syncthreads();
-    for (int size = 2; size <= kTopNChunk; size <<= 1) {
+// The block sorts `n` rows (a power of two; prefixes and row ids in shared memory), ascending by
+// compare_rows, equal keys in input order; a padding row (kNone) sorts last.
+__device__ void bitonic_rows(const SortDev& S, uint64_t* pre, uint32_t* idx, int n) {
+    for (int size = 2; size <= n; size <<= 1) {
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int t = threadIdx.x; t < kTopNChunk / 2; t += blockDim.x) {
+            for (int t = threadIdx.x; t < n / 2; t += blockDim.x) {
                 int lo = 2 * t - (t & (stride - 1));
                 int hi = lo + stride;
                 bool up = (lo & size) == 0;
@@ -1009,6 +999,23 @@ __global__ void __launch_bounds__(1024) k_topn_chunk(const __grid_constant__ Sor
             __syncthreads();
         }
     }
+}
+
+// One block sorts kTopNChunk rows (bitonic, ascending by compare_rows) and writes the
+// first k.  Keys are compared by their shared-memory prefix first.
+__global__ void __launch_bounds__(1024) k_topn_chunk(const __grid_constant__ SortDev S, const uint32_t* in, int64_t n,
+                                                    int k, uint32_t* out) {
+    __shared__ uint64_t pre[kTopNChunk];
+    __shared__ uint32_t idx[kTopNChunk];
+    int64_t base = (int64_t)blockIdx.x * kTopNChunk;
+    for (int j = threadIdx.x; j < kTopNChunk; j += blockDim.x) {
+        int64_t i = base + j;
+        uint32_t r = i < n ? (in ? in[i] : (uint32_t)i) : kNone;
+        idx[j] = r;
+        pre[j] = sort_prefix(S, r);
+    }
+    __syncthreads();
+    bitonic_rows(S, pre, idx, kTopNChunk);
     for (int j = threadIdx.x; j < k; j += blockDim.x) out[(int64_t)blockIdx.x * k + j] = idx[j];
 }
 
@@ -1350,6 +1357,232 @@ __global__ void __launch_bounds__(256, 2) k_topn_warp(const __grid_constant__ So
     }
 }
 
+
+// ---- top-N by selection: limits up to kMaxTopN over a fixed-width first key ------------------------
+// k_topn_sample takes the r-th smallest key prefix of a sample of the rows, r chosen so that more than k
+// rows lie at or below it all but surely; k_topn_take streams the key column once and lists the rows at
+// or below; k_topn_finish finds the k-th of those exactly, keeps the rows up to it and sorts them.  The
+// host checks that the list held at least k rows and not more than it has room for (else every row goes
+// through k_topn_chunk / k_topn_warp).
+// Why: the chunk sort orders all rows in shared memory, 2.0 ms for 20M rows and k = 100; the selection
+// reads the column at 5.1 to 5.9 TB/s (32 us), before it 15 us for the bound, after it 17 us for the
+// finish.
+
+// The block finds the r-th smallest (r >= 1) of n values get(i): by 8-bit digits from the highest bit in
+// which the values differ, counted in shared memory.  Returns an upper bound of it that no further value
+// lies below: all values <= the result are the m smallest, m returned in *taken.  With `slack` it may
+// stop early while at most `slack` more than r values are taken.
+// f(i, get(i)) for the block's values, eight of a thread's in flight together (one after the other, a
+// pass over 30,000 listed rows took 12 us).
+template <class Get, class F>
+__device__ __forceinline__ void block_values(Get get, uint32_t n, F f) {
+    for (uint32_t i0 = threadIdx.x; i0 < n; i0 += 8 * blockDim.x) {
+        uint64_t v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const uint32_t i = i0 + j * blockDim.x;
+            v[j] = i < n ? get(i) : 0ull;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const uint32_t i = i0 + j * blockDim.x;
+            if (i < n) f(i, v[j]);
+        }
+    }
+}
+template <class Get>
+__device__ uint64_t block_select(Get get, uint32_t n, uint32_t r, uint32_t slack, uint32_t* taken) {
+    __shared__ uint32_t hist[256];
+    __shared__ unsigned long long diff_s;
+    __shared__ uint32_t digit_s, below_s, in_s;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    const uint64_t ref = get(0);
+    uint64_t diff = 0;
+    if (tid == 0) diff_s = 0;
+    __syncthreads();
+    block_values(get, n, [&](uint32_t, uint64_t v) { diff |= v ^ ref; });
+    const uint32_t dlo = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)diff), dhi = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)(diff >> 32));
+    if (lane == 0) atomicOr(&diff_s, ((unsigned long long)dhi << 32) | dlo);
+    __syncthreads();
+    diff = diff_s;
+    if (!diff) {
+        *taken = n;
+        return ref;
+    }
+    int top = 64 - __clzll((long long)diff);           // bits [0, top) are undecided
+    uint64_t want = top < 64 ? ref >> top << top : 0;  // the decided bits
+    uint32_t before = 0;                               // values below the range of `want`
+    for (;;) {
+        const int low = top > 8 ? top - 8 : 0;
+        for (uint32_t i = tid; i < 256; i += blockDim.x) hist[i] = 0;
+        __syncthreads();
+        block_values(get, n, [&](uint32_t, uint64_t x) {
+            const uint64_t v = x ^ want;
+            if (top == 64 || (v >> top) == 0) atomicAdd(&hist[(v >> low) & ((1u << (top - low)) - 1u)], 1u);
+        });
+        __syncthreads();
+        if (tid < 32) {  // the digit in which the r-th lies: eight bins per lane
+            uint32_t c[8], sum = 0;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                c[j] = hist[lane * 8 + j];
+                sum += c[j];
+            }
+            uint32_t incl = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if ((int)lane >= o) incl += t;
+            }
+            uint32_t at = before + incl - sum;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                if (at < r && r <= at + c[j]) {
+                    digit_s = lane * 8 + j;
+                    below_s = at;
+                    in_s = c[j];
+                }
+                at += c[j];
+            }
+        }
+        __syncthreads();
+        const uint32_t below = below_s, in = in_s;
+        want |= (uint64_t)digit_s << low;
+        before = below;
+        top = low;
+        if (top == 0 || below + in <= r + slack) {
+            *taken = below + in;
+            return top ? want | ((1ull << top) - 1) : want;
+        }
+        __syncthreads();  // hist and the digit are rewritten
+    }
+}
+
+// The bound: one row of each of `samples` equal pieces of the column, the smallest prefix of every 4 or 16
+// neighbouring samples (kTopNMinima of them), and the r-th smallest of those, found by the last block to
+// finish (`done` starts at zero).  At least r samples lie at or below it.  Many blocks, because the rows
+// lie far apart: one block took 25 us for 16,384 of them.
+constexpr uint32_t kTopNMinima = 4096;
+template <int DT>
+__global__ void __launch_bounds__(256) k_topn_sample(const __grid_constant__ SortDev S, int64_t n, uint32_t samples, uint32_t r,
+                                                     uint64_t* minima, uint32_t* done, uint64_t* bound) {
+    __shared__ uint64_t mins[kTopNMinima];
+    __shared__ bool last;
+    const DCol& c = S.cols[0];
+    const uint64_t flip = S.asc[0] ? 0ull : ~0ull, nullp = S.nulls_first[0] ? 0ull : ~0ull;
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x, step = (uint32_t)((uint64_t)n / samples);  // at least 1
+    uint32_t x = i * 0x9E3779B9u;  // not always the same row of a piece: a period of the data must not matter
+    x ^= x >> 15;
+    x *= 0x85EBCA6Bu;
+    x ^= x >> 13;
+    const uint32_t row = (uint32_t)((uint64_t)i * (uint64_t)n / samples + x % step);
+    uint64_t p = fixed_prefix<DT>(load_value(c, row), valid_bit(c.valid, row), flip, nullp);
+    const uint32_t lanes = samples / kTopNMinima;
+    for (uint32_t o = lanes >> 1; o; o >>= 1) {
+        const uint64_t q = __shfl_xor_sync(0xFFFFFFFFu, p, o);
+        p = q < p ? q : p;
+    }
+    if (i % lanes == 0) minima[i / lanes] = p;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (uint32_t j = threadIdx.x; j < kTopNMinima; j += 256) mins[j] = __ldcg((const unsigned long long*)minima + j);
+    __syncthreads();
+    uint32_t taken;
+    const uint64_t b = block_select([&](uint32_t j) { return mins[j]; }, kTopNMinima, r, r, &taken);
+    if (threadIdx.x == 0) *bound = b;
+}
+
+// Rows whose prefix is at or below *bound: {prefix, row} appended to the list (*count of them, those past
+// `cap` counted only).  Bound by streaming the column: four loads of four rows each in flight per thread.
+template <int DT>
+__global__ void __launch_bounds__(256) k_topn_take(const __grid_constant__ SortDev S, int64_t n, const uint64_t* bound,
+                                                   uint64_t* list_p, uint32_t* list_r, uint32_t cap, uint32_t* count) {
+    const DCol& c = S.cols[0];
+    const bool vec = ((uintptr_t)c.data & 15) == 0;
+    const uint64_t flip = S.asc[0] ? 0ull : ~0ull, nullp = S.nulls_first[0] ? 0ull : ~0ull, b = __ldg(bound);
+    const uint32_t n32 = (uint32_t)n;
+    constexpr int kQuads = 4;
+    for (int64_t base = (int64_t)blockIdx.x * (256 * 4 * kQuads); base < n; base += (int64_t)gridDim.x * (256 * 4 * kQuads)) {
+        Quad q[kQuads];
+#pragma unroll
+        for (int j = 0; j < kQuads; j++) {
+            const int64_t r0 = base + (int64_t)(j * 256 + threadIdx.x) * 4;
+            q[j] = Quad{0, 0, 0, 0};
+            if (r0 < n) q[j] = load_quad<DT>(c, vec, n32, (uint32_t)r0);
+        }
+#pragma unroll
+        for (int j = 0; j < kQuads; j++) {
+            const int64_t r0 = base + (int64_t)(j * 256 + threadIdx.x) * 4;
+            if (r0 >= n) continue;
+            uint32_t vb = 0xFu;
+            if (c.valid) vb = (uint32_t)(__ldg(c.valid + (r0 >> 6)) >> (r0 & 63));
+            const uint64_t p[4] = {fixed_prefix<DT>(q[j].v0, vb & 1u, flip, nullp), fixed_prefix<DT>(q[j].v1, vb & 2u, flip, nullp),
+                                   fixed_prefix<DT>(q[j].v2, vb & 4u, flip, nullp), fixed_prefix<DT>(q[j].v3, vb & 8u, flip, nullp)};
+            if (p[0] > b && p[1] > b && p[2] > b && p[3] > b) continue;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (p[k] > b || r0 + k >= n) continue;
+                const uint32_t at = atomicAdd(count, 1u);
+                if (at < cap) {
+                    list_p[at] = p[k];
+                    list_r[at] = (uint32_t)r0 + k;
+                }
+            }
+        }
+    }
+}
+
+// The best k rows of the list (list_p == nullptr: of the rows 0..n themselves), sorted, into out[0..k).
+// state[0]: rows listed (in); state[1]: set when the list does not give the result.
+constexpr uint32_t kTopNSort = 4096;
+template <int DT>
+__global__ void __launch_bounds__(1024) k_topn_finish(const __grid_constant__ SortDev S, const uint64_t* list_p,
+                                                      const uint32_t* list_r, uint32_t cap, int64_t n, int k, uint32_t* state,
+                                                      uint32_t* out) {
+    extern __shared__ __align__(16) uint64_t pre[];
+    uint32_t* idx = (uint32_t*)(pre + kTopNSort);
+    __shared__ uint32_t m_s;
+    const DCol& c = S.cols[0];
+    const uint64_t flip = S.asc[0] ? 0ull : ~0ull, nullp = S.nulls_first[0] ? 0ull : ~0ull;
+    const uint32_t m = list_p ? state[0] : (uint32_t)n;
+    for (int j = threadIdx.x; j < k; j += 1024) out[j] = 0;  // rows that exist, whatever comes of it
+    if (threadIdx.x == 0) m_s = 0;
+    if (m < (uint32_t)k || (list_p && m > cap)) {
+        if (threadIdx.x == 0) state[1] = 1;
+        return;
+    }
+    auto get = [&](uint32_t i) -> uint64_t {
+        return list_p ? __ldg((const unsigned long long*)list_p + i)
+                      : fixed_prefix<DT>(load_value(c, i), valid_bit(c.valid, i), flip, nullp);
+    };
+    uint32_t taken;
+    const uint64_t bound = block_select(get, m, (uint32_t)k, max((uint32_t)k / 4, 32u), &taken);
+    if (taken > kTopNSort) {  // ties at the limit beyond what the sort holds
+        if (threadIdx.x == 0) state[1] = 1;
+        return;
+    }
+    uint32_t size = 2;
+    while (size < taken) size *= 2;
+    for (uint32_t i = threadIdx.x; i < size; i += 1024) {
+        pre[i] = ~0ull;
+        idx[i] = kNone;
+    }
+    __syncthreads();
+    block_values(get, m, [&](uint32_t i, uint64_t p) {
+        if (p > bound) return;
+        const uint32_t at = atomicAdd(&m_s, 1u);
+        pre[at] = p;
+        idx[at] = list_p ? __ldg(list_r + i) : i;
+    });
+    __syncthreads();
+    bitonic_rows(S, pre, idx, (int)size);
+    for (int j = threadIdx.x; j < k; j += 1024) out[j] = idx[j];
+}
+
 }  // namespace
 
 // Temporaries of ml_gpu_filter_static: a fixed-size device array, so that call allocates no
@@ -1533,6 +1766,52 @@ int topn_warp_blocks(int64_t n) {
     return (int)std::max<int64_t>(1, std::min(want, cap));
 }
 size_t topn_entry_bytes() { return sizeof(TopEntry); }
+
+TopNPlan topn_plan(const SortDev& S, int64_t n, int k) {
+    TopNPlan p{};
+    const DCol& c = S.cols[0];
+    if (S.nkeys < 1 || c.kind != CK_FIXED || c.src != 0 || k < 1 || k > kMaxTopN || n < k) return p;
+    if (n <= kTopNDirect) {
+        p.use = true;
+        return p;
+    }
+    // the sample's rank: k rows of n are `mean` of the sample on average; six standard deviations and
+    // six more make fewer than k rows at or below it a matter of one in 10^8
+    p.samples = n >= (4 << 20) ? 16 * kTopNMinima : 4 * kTopNMinima;
+    const double mean = (double)k * p.samples / (double)n;
+    const double r = std::ceil(mean + 6 * std::sqrt(mean) + 6);
+    const double rows = r / p.samples * (double)n;  // rows at or below, on average
+    if (r > kTopNMinima / 4 || rows > 262144.0) return p;
+    p.use = true;
+    p.rank = (uint32_t)r;
+    p.cap = (uint32_t)(8 * rows) + 4096;
+    return p;
+}
+size_t topn_minima_bytes() { return kTopNMinima * 8; }
+template <int DT>
+static cudaError_t topn_select(const SortDev& S, int64_t n, int k, const TopNPlan& p, uint64_t* bound, uint64_t* minima, uint64_t* list_p,
+                               uint32_t* list_r, uint32_t* state, uint32_t* out, cudaStream_t s) {
+    // per call: the attribute belongs to the current device's copy of the kernel
+    constexpr int sort_b = kTopNSort * 12;
+    cudaError_t e = cudaFuncSetAttribute(k_topn_finish<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_b);
+    if (e != cudaSuccess) return e;
+    if (p.rank) {
+        k_topn_sample<DT><<<p.samples / 256, 256, 0, s>>>(S, n, p.samples, p.rank, minima, state + 2, bound);
+        const int64_t want = (n + 4095) / 4096;
+        k_topn_take<DT><<<(int)std::min<int64_t>(want, (int64_t)num_sms() * 8), 256, 0, s>>>(S, n, bound, list_p, list_r, p.cap, state);
+    }
+    k_topn_finish<DT><<<1, 1024, sort_b, s>>>(S, p.rank ? list_p : nullptr, list_r, p.cap, n, k, state, out);
+    return cudaSuccess;
+}
+cudaError_t launch_topn_select(const SortDev& S, int64_t n, int k, const TopNPlan& p, uint64_t* bound, uint64_t* minima, uint64_t* list_p,
+                               uint32_t* list_r, uint32_t* state, uint32_t* out, cudaStream_t s) {
+    switch (S.cols[0].dt) {
+        case ML_TYPE_FLOAT64: return topn_select<ML_TYPE_FLOAT64>(S, n, k, p, bound, minima, list_p, list_r, state, out, s);
+        case ML_TYPE_INT64: return topn_select<ML_TYPE_INT64>(S, n, k, p, bound, minima, list_p, list_r, state, out, s);
+        case ML_TYPE_BOOL: return topn_select<ML_TYPE_BOOL>(S, n, k, p, bound, minima, list_p, list_r, state, out, s);
+        default: return topn_select<ML_TYPE_INT32>(S, n, k, p, bound, minima, list_p, list_r, state, out, s);
+    }
+}
 int launch_topn_warp(const SortDev& S, int64_t n, int k, int blocks, uint32_t* out, void* cand, unsigned int* done,
                      uint32_t* final_out, cudaStream_t s, const uint64_t* n_dev) {
     const DCol& c = S.cols[0];

@@ -158,6 +158,20 @@ void launch_sort_runs(const uint32_t* keys, uint32_t* rows, const SortWord* word
                       uint32_t cap, uint32_t* state, cudaStream_t s);
 void launch_max_strlen(const uint32_t* off, int64_t n, unsigned int* out, cudaStream_t s);
 void launch_iota_u32(uint32_t* out, int64_t n, cudaStream_t s);  // out[i] = i
+// Top-k by selection (a sampled bound, one pass that lists the rows at or below it, the exact k-th of
+// those, a sort of the rest): topn_plan says whether a call takes it.
+constexpr int64_t kTopNDirect = 65536;  // up to here the rows are the list
+struct TopNPlan {
+    bool use;
+    uint32_t samples, rank;  // sampled rows and the bound's rank among them; rank 0: no sample and no list
+    uint32_t cap;            // rows the list has room for
+};
+size_t topn_minima_bytes();
+TopNPlan topn_plan(const SortDev& S, int64_t n, int k);
+// out[0 .. k): the rows, sorted, unless state[1] is set afterwards (then they are 0).  bound: one word;
+// minima: topn_minima_bytes(); list_p / list_r: p.cap entries each; state: three zeroed words.
+cudaError_t launch_topn_select(const SortDev& S, int64_t n, int k, const TopNPlan& p, uint64_t* bound, uint64_t* minima, uint64_t* list_p,
+                               uint32_t* list_r, uint32_t* state, uint32_t* out, cudaStream_t s);
 // Top-k for k <= kTopNWarpMax: each CTA writes its best k rows (sorted) to out[block * k ..].
 constexpr int kTopNWarpMax = 32;
 int topn_warp_blocks(int64_t n);
