@@ -1395,7 +1395,15 @@ void* jit_select_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P) {
                     [&] { return (void*)get_kernel(ctx, jit_select_source(pipe, P, contig), "ml_select_flags"); });
 }
 
-std::string jit_select_source(const Pipeline& pipe, const PipeArgs& P, bool contig) {
+void* jit_probe_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P) {
+    if (!jit_enabled(ctx) || !batchable(P)) return nullptr;
+    const bool contig = contig_ok(P);
+    return memoized(pipe, signature('p', P, nullptr, nullptr) + std::string((const char*)&ctx->device, sizeof(int)) +
+                              (contig ? "c" : "s"),
+                    [&] { return (void*)get_kernel(ctx, jit_select_source(pipe, P, contig, true), "ml_probe_flags"); });
+}
+
+std::string jit_select_source(const Pipeline& pipe, const PipeArgs& P, bool contig, bool builds) {
     {
         // Pass bits and per-chunk pass counts of 2048-row chunks (the layout of the ahead-of-time
         // k_select_flags), 8 rows per thread with every chunk's loads issued together.  CTAs stride
@@ -1407,8 +1415,10 @@ std::string jit_select_source(const Pipeline& pipe, const PipeArgs& P, bool cont
         g.batched_stages([&](auto&&) {});
         const int K = g.rows_per_thread;
         std::string src = kPrelude;
-        src += "extern \"C\" __global__ void __launch_bounds__(256) ml_select_flags(const __grid_constant__ PipeArgs P, "
-               "uint32_t* bits, uint32_t* chunk_counts) {\n";
+        // `builds`: the matched build row of each row's first probe is kept too (ml_probe_flags)
+        src += std::string("extern \"C\" __global__ void __launch_bounds__(256) ") + (builds ? "ml_probe_flags" : "ml_select_flags") +
+               "(const __grid_constant__ PipeArgs P, uint32_t* bits, uint32_t* chunk_counts" +
+               (builds ? ", uint32_t* builds" : "") + ") {\n";
         src += g.pre();
         src += "    const int lane = threadIdx.x & 31;\n";
         src += "    const int64_t chunks = (P.n + 2047) / 2048;\n";
@@ -1418,6 +1428,15 @@ std::string jit_select_source(const Pipeline& pipe, const PipeArgs& P, bool cont
             // thread t's rows are base + 8t .. +7 (the per-CTA tile of the strided form, 8 x 256)
             src += tile_rows(P, K, true, "        ");
             src += g.body();
+            if (builds) {
+                src += "        if (full) {\n";
+                for (int j = 0; j < K; j += 4)
+                    src += "            *(uint4*)(builds + r0 + " + num(j) + ") = make_uint4(x" + num(j) + ".b0, x" + num(j + 1) + ".b0, x" +
+                           num(j + 2) + ".b0, x" + num(j + 3) + ".b0);\n";
+                src += "        } else {\n";
+                for (int j = 0; j < K; j++) src += "            if (a" + num(j) + ") builds[r0 + " + num(j) + "] = x" + num(j) + ".b0;\n";
+                src += "        }\n";
+            }
             src += "        uint32_t byte = 0;\n";
             for (int j = 0; j < K; j++) src += "        byte |= (a" + num(j) + " ? 1u : 0u) << " + num(j) + ";\n";
             // a 32-row word is the bytes of 4 consecutive lanes
@@ -1432,6 +1451,7 @@ std::string jit_select_source(const Pipeline& pipe, const PipeArgs& P, bool cont
             src += "        uint32_t cnt = 0;\n";
             for (int j = 0; j < K; j++) {
                 std::string J = num(j);
+                if (builds) src += "        if (a" + J + ") builds[i" + J + "] = x" + J + ".b0;\n";
                 src += "        {\n            const uint32_t b = __ballot_sync(0xFFFFFFFFu, a" + J + ");\n";
                 src += "            const int64_t w0 = base + " + J + " * 256 + (threadIdx.x & ~31);\n";
                 src += "            if (lane == 0 && w0 < P.n) bits[w0 >> 5] = b;\n";

@@ -28,13 +28,15 @@ void* jit_join_insert_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, 
 // Filter pass bits and per-CTA counts (the layout of launch_select_flags), or nullptr when the
 // pipeline has duplicate-key probes or specialization is off.  Arguments: P, bits, block_counts.
 void* jit_select_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P);
+// The same for a single probe, keeping each row's matched build row: P, bits, block_counts, builds.
+void* jit_probe_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P);
 // Cardinality features scan of the key layout L (64 KB of dynamic shared memory per CTA).
 // Arguments: P, L, cta_regs (gridDim x 4096 words), nulls, minmax.
 void* jit_hll_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, const KeyLayout& L);
 // Sources of the kernels above.
 // `contig`: consecutive rows per thread with vector loads (needs no selection vector and 16-byte
 // aligned source columns).
-std::string jit_select_source(const Pipeline& pipe, const PipeArgs& P, bool contig);
+std::string jit_select_source(const Pipeline& pipe, const PipeArgs& P, bool contig, bool builds = false);
 std::string jit_hll_source(const Pipeline& pipe, const PipeArgs& P, const KeyLayout& L, bool contig);
 
 // Rows one thread of the specialized aggregate kernel handles per iteration (its grid

@@ -67,6 +67,9 @@ int select_rows_per_block();  // rows of one select_blocks block
 void launch_select_flags(const PipeArgs& P, uint32_t* bits, uint32_t* block_counts, cudaStream_t s);
 void launch_select_write(const PipeArgs& P, const uint32_t* bits, const uint64_t* block_offsets, uint32_t* out,
                          cudaStream_t s);
+// launch_select_write for join pairs: the kept positions and their entries of `builds`.
+void launch_pairs_write(const PipeArgs& P, const uint32_t* bits, const uint64_t* block_offsets, const uint32_t* builds,
+                        uint32_t* out_p, uint32_t* out_b, cudaStream_t s);
 // Groups with at least one row (group blocks' word 0 > 0) and, with `member`, whose entry
 // there is not kNone: pass bits + per-block counts; then launch_index_write turns bits into
 // the ordered list of group ids.

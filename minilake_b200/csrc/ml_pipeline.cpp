@@ -404,40 +404,56 @@ uint64_t scan_counts(Ctx* ctx, const uint32_t* counts, int64_t n, DevBuf& offset
     return total;
 }
 
-int64_t run_select(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, DevBuf& out, cudaStream_t s, Reservation* res) {
-    int nb = select_blocks(P.n);
+// Pass bits and per-block counts of the launch's rows, by the specialized kernel or k_select_flags.
+static void select_flags(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, DevBuf& bits, DevBuf& counts, cudaStream_t s) {
+    const int nb = select_blocks(P.n);
+    void* jit = jit_select_kernel(ctx, pipe, P);
+    KernelTimer kt(ctx, s, "select");
+    if (jit) {
+        if (nb) {
+            uint32_t* b = bits.get<uint32_t>();
+            uint32_t* c = counts.get<uint32_t>();
+            CK(cudaMemsetAsync(c, 0, (size_t)nb * 4, s));
+            void* args[] = {(void*)&P, &b, &c};
+            const int grid = std::min<int64_t>(nb, (int64_t)jit_resident_blocks(jit, kPipelineThreads, 0) * num_sms());
+            jit_launch(jit, grid, kPipelineThreads, 0, s, args);
+        }
+        ctx->add_profile("jit_launch", 0);
+    } else {
+        launch_select_flags(P, bits.get<uint32_t>(), counts.get<uint32_t>(), s);
+    }
+    kt.stop();
+    ctx->count_launch();
+}
+
+int64_t run_select(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, DevBuf& out, cudaStream_t s, Reservation* res,
+                   uint32_t* direct, const uint32_t* err, uint32_t* err_host) {
+    const int nb = select_blocks(P.n);
     DevBuf bits(ctx, std::max<size_t>((size_t)(P.n + 31) / 32 * 4, 4), res);
     DevBuf counts(ctx, std::max<size_t>((size_t)nb * 4, 4), res);
-    {
-        void* jit = jit_select_kernel(ctx, pipe, P);
-        KernelTimer kt(ctx, s, "select");
-        if (jit) {
-            if (nb) {
-                uint32_t* b = bits.get<uint32_t>();
-                uint32_t* c = counts.get<uint32_t>();
-                CK(cudaMemsetAsync(c, 0, (size_t)nb * 4, s));
-                void* args[] = {(void*)&P, &b, &c};
-                const int grid = std::min<int64_t>(nb, (int64_t)jit_resident_blocks(jit, kPipelineThreads, 0) * num_sms());
-                jit_launch(jit, grid, kPipelineThreads, 0, s, args);
-            }
-            ctx->add_profile("jit_launch", 0);
-        } else {
-            launch_select_flags(P, bits.get<uint32_t>(), counts.get<uint32_t>(), s);
-        }
-        kt.stop();
+    DevBuf offs(ctx, (size_t)(nb + 1) * 8, res), scratch(ctx, scan_scratch_words(nb) * 8, res);
+    PinnedSlot total(ctx);
+    select_flags(ctx, pipe, P, bits, counts, s);
+    launch_scan_u32(counts.get<uint32_t>(), offs.get<uint64_t>(), nb, scratch.get<uint64_t>(), s);
+    ctx->count_launch(3);
+    CK(cudaMemcpyAsync(total.p, offs.get<uint64_t>() + nb, 8, cudaMemcpyDeviceToHost, s));
+    // the selection's size is needed now to allocate it, or to charge what the caller's buffer holds to a
+    // budget; else one wait at the end is enough
+    if (!direct || ctx->pool.limit != UINT64_MAX) {
+        CK(cudaStreamSynchronize(s));
+        const size_t bytes = std::max<size_t>(*total.as<uint64_t>() * 4, 4);
+        if (!direct) out = DevBuf(ctx, bytes, res);
+        else if (res) res->try_grow(bytes);
     }
-    ctx->count_launch();
-    DevBuf offs;
-    uint64_t total = scan_counts(ctx, counts.get<uint32_t>(), nb, offs, s, res);
-    out = DevBuf(ctx, std::max<size_t>(total * 4, 4), res);
     {
         KernelTimer kt(ctx, s, "select_write");
-        launch_select_write(P, bits.get<uint32_t>(), offs.get<uint64_t>(), out.get<uint32_t>(), s);
+        launch_select_write(P, bits.get<uint32_t>(), offs.get<uint64_t>(), direct ? direct : out.get<uint32_t>(), s);
         kt.stop();
     }
     ctx->count_launch();
+    if (err) CK(cudaMemcpyAsync(err_host, err, 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    return (int64_t)total;
+    return (int64_t)*total.as<uint64_t>();
 }
 
 void gather_utf8(Ctx* ctx, const uint32_t* off, const uint8_t* bytes, const uint32_t* idx, int64_t k, DevColumn& out,

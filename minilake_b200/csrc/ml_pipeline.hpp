@@ -75,10 +75,12 @@ class Pipeline {
 };
 
 // Ordered selection of the rows where all of the pipeline's stages pass (no probes).
-// Returns the number of selected rows; `out` holds them (device).  Its device buffers are
-// charged to `res` when given.
+// Returns the number of selected rows; `out` holds them (device), or `direct` when given (room for
+// P.n entries).  Its device buffers, the selection included, are charged to `res` when given.  `err`
+// (optional): a device word copied to err_host before the call's last wait.
 int64_t run_select(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, DevBuf& out, cudaStream_t s,
-                   Reservation* res = nullptr);
+                   Reservation* res = nullptr, uint32_t* direct = nullptr, const uint32_t* err = nullptr,
+                   uint32_t* err_host = nullptr);
 
 // Exclusive scan helper (device u32 counts -> u64 offsets incl. total); returns the total.
 uint64_t scan_counts(Ctx* ctx, const uint32_t* counts, int64_t n, DevBuf& offsets, cudaStream_t s,

@@ -152,6 +152,16 @@ class Ctx {
     size_t cached_bytes_ = 0;
 };
 
+// A pinned readback slot (64 bytes) for the duration of a call.
+struct PinnedSlot {
+    Ctx* ctx;
+    void* p;
+    explicit PinnedSlot(Ctx* c) : ctx(c), p(c->pinned_slot()) {}
+    ~PinnedSlot() { ctx->release_slot(p); }
+    PinnedSlot(const PinnedSlot&) = delete;
+    template <class T> T* as() const { return (T*)p; }
+};
+
 // Times one kernel launch on `s` with CUDA events when the context profiles.
 class KernelTimer {
    public:
