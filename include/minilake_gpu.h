@@ -222,6 +222,10 @@ int ml_gpu_batch_column_info(const ml_batch* b, int32_t col, int32_t* dtype, int
  * bytes); `offsets`: len+1 (UTF8 only); `validity`: ceil(len/64) words or NULL. */
 int ml_gpu_batch_fetch(const ml_batch* b, int32_t col, void* values, uint32_t* offsets,
                        uint64_t* validity);
+/* Every column at once, as ml_gpu_batch_fetch gives each: arrays of `ncols` buffers (validity[i]
+ * and, for fixed-width columns, offsets[i] may be NULL). */
+int ml_gpu_batch_fetch_all(const ml_batch* b, int32_t ncols, void* const* values, uint32_t* const* offsets,
+                           uint64_t* const* validity);
 int ml_gpu_batch_destroy(ml_batch* b);
 
 /* ---- Operator: FilterOperator (operators/filter.rs:19-25, expr/eval.rs:167-196) --- */

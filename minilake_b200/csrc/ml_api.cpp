@@ -149,6 +149,66 @@ std::unique_ptr<DevColumn> gather_column(Ctx* ctx, const DevColumn& s, const uin
     return d;
 }
 
+// Rows `idx` (device, k entries, each row at most once) of every column of a batch; the work has finished
+// when it returns.  Few rows of fixed-width and plain string columns take one launch and one wait (a
+// column at a time: two launches for a fixed-width one, seven and a wait for a string).
+std::vector<std::unique_ptr<DevColumn>> gather_rows(Ctx* ctx, const ml_batch& b, const uint32_t* idx, int64_t k,
+                                                    cudaStream_t st, Reservation* res) {
+    std::vector<std::unique_ptr<DevColumn>> out;
+    // strings get room for 64 KB before their size is known: not under a budget
+    bool small = k > 0 && k <= kSmallRows && (int)b.cols.size() <= kSmallCols && ctx->pool.limit == UINT64_MAX;
+    for (auto& c : b.cols) small = small && c->kind != CK_DICT;
+    if (small) {
+        constexpr uint32_t kRoom = 64 << 10;
+        SmallCols G{};
+        DevBuf info(ctx, kSmallCols * 4, nullptr);
+        PinnedSlot told(ctx);  // 64 bytes: a word per column
+        static_assert(kSmallCols * 4 <= 64, "a pinned slot holds the columns' sizes");
+        G.info = info.get<uint32_t>();
+        bool strings = false;
+        for (auto& c : b.cols) {
+            auto d = std::make_unique<DevColumn>();
+            d->dtype = c->dtype;
+            d->kind = c->kind;
+            d->n = k;
+            SmallCol& g = G.c[G.n++];
+            g.src = c->dptr();
+            if (c->kind == CK_UTF8) {
+                strings = true;
+                d->offsets = DevBuf(ctx, (size_t)(k + 1) * 4, res);
+                d->data = DevBuf(ctx, kRoom, res);
+                g.cap = kRoom;
+                g.src_off = c->optr();
+                g.dst_off = d->offsets.get<uint32_t>();
+            } else {
+                g.width = width_of(c->dtype);
+                d->data = DevBuf(ctx, (size_t)k * g.width, res);
+            }
+            g.dst = d->data.get();
+            if (c->vptr()) {
+                d->validity = DevBuf(ctx, (size_t)(k + 63) / 64 * 8, res);
+                g.src_valid = c->vptr();
+                g.dst_valid = d->validity.get<uint32_t>();
+            }
+            out.push_back(std::move(d));
+        }
+        launch_gather_small(G, idx, (int)k, st);
+        ctx->count_launch();
+        if (strings) CK(cudaMemcpyAsync(told.p, G.info, (size_t)G.n * 4, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        for (int i = 0; i < G.n; i++)
+            if (out[i]->kind == CK_UTF8) {
+                out[i]->str_bytes = told.as<uint32_t>()[i];
+                small = small && out[i]->str_bytes != kNone;
+            }
+        if (small) return out;
+        out.clear();  // strings past the room: a column at a time
+    }
+    for (auto& c : b.cols) out.push_back(gather_column(ctx, *c, idx, k, st, res));
+    CK(cudaStreamSynchronize(st));
+    return out;
+}
+
 // Evaluate program `p` for the rows of launch `P` into a new fixed-width column.
 std::unique_ptr<DevColumn> project_column(Ctx* ctx, const PipeArgs& P, Prog p, int type, cudaStream_t st, Reservation* res) {
     auto d = std::make_unique<DevColumn>();
@@ -603,11 +663,13 @@ std::unique_ptr<ml_batch> topn_batch(Ctx* ctx, ml_batch& b, const std::vector<So
             progs.push_back(kp.C.compile_value(key.expr, kp.out, key.type));
         }
     }
-    kp.upload();
     Staging stg(ctx);
     Pipeline::Launch L;
-    auto views = device_views(b);
-    kp.prepare(L, views.data(), (int)views.size(), n, nullptr, 0, st, stg, nullptr);
+    if (std::find(direct.begin(), direct.end(), -1) != direct.end()) {
+        kp.upload();
+        auto views = device_views(b);
+        kp.prepare(L, views.data(), (int)views.size(), n, nullptr, 0, st, stg, nullptr);
+    }
     for (size_t i = 0; i < keys.size(); i++) {
         const DevColumn* c;
         if (direct[i] >= 0) {
@@ -629,6 +691,17 @@ std::unique_ptr<ml_batch> topn_batch(Ctx* ctx, ml_batch& b, const std::vector<So
     }
     DevBuf a, bb;
     const uint32_t* in = nullptr;
+    if (n <= kTopNTiny) {
+        a = DevBuf(ctx, (size_t)k * 4, nullptr);
+        {
+            KernelTimer kt(ctx, st, "topn");
+            launch_topn_tiny(S, (int)n, (int)k, a.get<uint32_t>(), st);
+            kt.stop();
+        }
+        ctx->count_launch();
+        out->cols = gather_rows(ctx, b, a.get<uint32_t>(), k, st, res);
+        return out;
+    }
     // By selection above the per-warp lists' limit, and from 2M rows on below it too: the lists' kernel
     // runs at half the rate of one that only streams the column.  60M doubles, LIMIT 10: 149 us by lists,
     // 116 us by selection; 20M, LIMIT 100: 1,990 us by chunk sorts, 64 us by selection.
@@ -650,8 +723,7 @@ std::unique_ptr<ml_batch> topn_batch(Ctx* ctx, ml_batch& b, const std::vector<So
         // the result is gathered before the host knows that it is one (the rows exist either way)
         ErrWord told(ctx);
         CK(cudaMemcpyAsync(told.h, state + 1, 4, cudaMemcpyDeviceToHost, st));
-        for (auto& c : b.cols) out->cols.push_back(gather_column(ctx, *c, (const uint32_t*)(base + ro), k, st, res));
-        CK(cudaStreamSynchronize(st));
+        out->cols = gather_rows(ctx, b, (const uint32_t*)(base + ro), k, st, res);
         if (!*told.h) return out;
         out->cols.clear();
     }
@@ -690,8 +762,7 @@ std::unique_ptr<ml_batch> topn_batch(Ctx* ctx, ml_batch& b, const std::vector<So
             m = nb * k;
         }
     }
-    for (auto& c : b.cols) out->cols.push_back(gather_column(ctx, *c, in, k, st, res));
-    CK(cudaStreamSynchronize(st));
+    out->cols = gather_rows(ctx, b, in, k, st, res);
     return out;
 }
 
@@ -931,8 +1002,7 @@ std::unique_ptr<ml_batch> sort_batch(Ctx* ctx, ml_batch& b, const std::vector<So
     auto out = std::make_unique<ml_batch>();
     out->ctx = ctx;
     out->nrows = k;
-    for (auto& c : b.cols) out->cols.push_back(gather_column(ctx, *c, perm.get<uint32_t>(), k, st, res));
-    CK(cudaStreamSynchronize(st));
+    out->cols = gather_rows(ctx, b, perm.get<uint32_t>(), k, st, res);
     return out;
 }
 
@@ -1112,6 +1182,75 @@ int ml_gpu_batch_fetch(const ml_batch* b, int32_t col, void* values, uint32_t* o
         } else {
             for (size_t w = 0; w < words; w++) validity[w] = ~0ull;
             if (n % 64) validity[words - 1] = (1ull << (n % 64)) - 1;
+        }
+    }
+    API_END
+}
+
+// Every column as ml_gpu_batch_fetch gives it.  A small batch comes back with one kernel and one copy.
+int ml_gpu_batch_fetch_all(const ml_batch* b, int32_t ncols, void* const* values, uint32_t* const* offsets,
+                           uint64_t* const* validity) {
+    API_BEGIN
+    HostTimer host_timer_(b ? b->ctx : nullptr, "host:batch_fetch");
+    REQUIRE(b && ncols == (int32_t)b->cols.size(), "column count mismatch");
+    REQUIRE(ncols == 0 || (values && offsets && validity), "null argument");
+    Ctx* ctx = b->ctx;
+    ctx->set_current();
+    constexpr size_t kSmall = 64 << 10;
+    PackPieces P{};
+    size_t total = 0;
+    bool small = ncols <= kSmallCols && b->nrows > 0;
+    auto piece = [&](const void* src, size_t bytes) {
+        P.p[P.n++] = {src, (uint32_t)bytes, (uint32_t)total};
+        total += (bytes + 7) / 8 * 8;
+    };
+    for (int i = 0; small && i < ncols; i++) {
+        const DevColumn& c = *b->cols[i];
+        small = c.kind == CK_FIXED || (c.kind == CK_UTF8 && c.str_bytes >= 0);
+        const size_t n = (size_t)c.n, vb = c.kind == CK_FIXED ? n * width_of(c.dtype) : (size_t)std::max<int64_t>(c.str_bytes, 0);
+        small = small && total + vb + (n + 1) * 4 + n / 8 + 64 <= kSmall;
+        if (!small) break;
+        REQUIRE(c.kind == CK_FIXED || offsets[i], "UTF8 fetch needs an offsets buffer");
+        REQUIRE(vb == 0 || values[i], "null values buffer");
+        piece(c.dptr(), vb);
+        if (c.kind == CK_UTF8) piece(c.optr(), (n + 1) * 4);
+        if (validity[i] && c.vptr()) piece(c.vptr(), (n + 63) / 64 * 8);
+    }
+    if (!small) {
+        for (int i = 0; i < ncols; i++) {
+            const int st = ml_gpu_batch_fetch(b, i, values[i], offsets[i], validity[i]);
+            if (st != ML_OK) return st;
+        }
+        return ML_OK;
+    }
+    {
+        OpStream op_stream(ctx);
+        Staging st(ctx);
+        DevBuf packed(ctx, std::max<size_t>(total, 8), nullptr);
+        uint8_t* host = (uint8_t*)st.get(std::max<size_t>(total, 8));
+        launch_pack(P, packed.get(), op_stream.s);
+        ctx->count_launch();
+        CK(cudaMemcpyAsync(host, packed.get(), total, cudaMemcpyDeviceToHost, op_stream.s));
+        CK(cudaStreamSynchronize(op_stream.s));
+        int q = 0;
+        for (int i = 0; i < ncols; i++) {
+            const DevColumn& c = *b->cols[i];
+            const int64_t n = c.n;
+            const size_t words = (size_t)(n + 63) / 64;
+            if (P.p[q].bytes) memcpy(values[i], host + P.p[q].at, P.p[q].bytes);
+            q++;
+            if (c.kind == CK_UTF8) {  // known sizes: the column's own offsets, from 0
+                memcpy(offsets[i], host + P.p[q].at, P.p[q].bytes);
+                q++;
+            }
+            if (!validity[i]) continue;
+            if (c.vptr()) {
+                memcpy(validity[i], host + P.p[q].at, P.p[q].bytes);
+                q++;
+            } else {
+                for (size_t w = 0; w < words; w++) validity[i][w] = ~0ull;
+            }
+            if (n % 64) validity[i][words - 1] &= (1ull << (n % 64)) - 1;
         }
     }
     API_END
@@ -2760,8 +2899,10 @@ std::unique_ptr<ml_batch> hashagg_emit(ml_hashagg* h, cudaStream_t s) {
         ctx->count_launch(2);
         ng = (uint32_t)total;
     } else if (!h->ungrouped) {
-        CK(cudaMemcpy(&ng, h->ngroups.get(), 4, cudaMemcpyDeviceToHost));
-        ng = std::min(ng, h->gid_cap);
+        PinnedSlot told(ctx);
+        CK(cudaMemcpyAsync(told.p, h->ngroups.get(), 4, cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        ng = std::min(*told.as<uint32_t>(), h->gid_cap);
     }
     h->final_groups = ng;
     auto b = std::make_unique<ml_batch>();
@@ -2789,7 +2930,7 @@ std::unique_ptr<ml_batch> hashagg_emit(ml_hashagg* h, cudaStream_t s) {
         d->kind = CK_FIXED;
         d->n = ng;
         d->validity = DevBuf(ctx, vbytes, b->res.get());
-        CK(cudaMemsetAsync(d->validity.get(), 0, vbytes, s));
+        if (!ng) CK(cudaMemsetAsync(d->validity.get(), 0, vbytes, s));  // else k_agg_final writes every word
         if (h->dec[k].str_kind) {
             id_bufs[k] = DevBuf(ctx, std::max<size_t>((size_t)ng * 4, 4), nullptr);
             F.key_out[k] = id_bufs[k].get();
@@ -2828,57 +2969,87 @@ std::unique_ptr<ml_batch> hashagg_emit(ml_hashagg* h, cudaStream_t s) {
         d->n = ng;
         d->data = DevBuf(ctx, std::max<size_t>((size_t)ng * width_of(a.out_type), 8), b->res.get());
         d->validity = DevBuf(ctx, vbytes, b->res.get());
-        CK(cudaMemsetAsync(d->validity.get(), 0, vbytes, s));
+        if (!ng) CK(cudaMemsetAsync(d->validity.get(), 0, vbytes, s));
         F.agg_out[k] = d->data.get();
         F.agg_valid[k] = d->validity.get<uint32_t>();
         aggcols.push_back(std::move(d));
     }
     launch_agg_final(F, s);
     ctx->count_launch();
-    CK(cudaStreamSynchronize(s));
-    // global string ids (dictionary keys, string MIN/MAX) become the strings on the host
-    auto strings_of_ids = [&](DevColumn& c, const void* id_dev) {
-        std::vector<uint32_t> ids(ng);
-        if (ng) CK(cudaMemcpy(ids.data(), id_dev, (size_t)ng * 4, cudaMemcpyDeviceToHost));
-        std::vector<uint64_t> valid((ng + 63) / 64 + 1, 0);
-        if (ng) CK(cudaMemcpy(valid.data(), c.validity.get(), (size_t)(ng + 63) / 64 * 8, cudaMemcpyDeviceToHost));
-        std::vector<uint32_t> off(ng + 1, 0);
-        std::string bytes;
-        {
-            std::lock_guard<std::mutex> g(h->pipe.intern.mu);
-            for (uint32_t g2 = 0; g2 < ng; g2++) {
-                bool v = (valid[g2 / 64] >> (g2 % 64)) & 1;
-                if (v) bytes += h->pipe.intern.strs.at(ids[g2]);
-                off[g2 + 1] = (uint32_t)bytes.size();
-            }
-        }
-        c.kind = CK_UTF8;
-        c.offsets = DevBuf(ctx, (size_t)(ng + 1) * 4, b->res.get());
-        c.data = DevBuf(ctx, std::max<size_t>(bytes.size(), 1), b->res.get());
-        h2d_now(c.offsets.get(), off.data(), (size_t)(ng + 1) * 4);
-        h2d_now(c.data.get(), bytes.data(), bytes.size());
+    // global string ids (dictionary keys, string MIN/MAX) become the strings on the host: their ids and
+    // validity words come back together, and the strings go out together
+    struct Strings {
+        DevColumn* col;
+        DevBuf ids;
+        size_t at;  // of the ids in the staging buffer; the validity words follow
+    };
+    std::vector<Strings> strs;
+    size_t back = 0;
+    auto want = [&](DevColumn& c, DevBuf ids) {
+        strs.push_back({&c, std::move(ids), back});
+        back += ((size_t)ng * 4 + 7) / 8 * 8 + vbytes;
     };
     for (int k = 0; k < F.nagg; k++)
-        if (h->aggs[k].out_type == ML_TYPE_UTF8) {
-            DevBuf ids = std::move(aggcols[k]->data);
-            strings_of_ids(*aggcols[k], ids.get());
+        if (h->aggs[k].out_type == ML_TYPE_UTF8) want(*aggcols[k], std::move(aggcols[k]->data));
+    for (int k = 0; k < F.nkeys; k++)
+        if (h->dec[k].str_kind == 1) want(*keycols[k], std::move(id_bufs[k]));
+    Staging stg(ctx);
+    if (!strs.empty()) {
+        uint8_t* host = (uint8_t*)stg.get(std::max<size_t>(back, 8));
+        for (auto& x : strs) {
+            if (!ng) continue;
+            CK(cudaMemcpyAsync(host + x.at, x.ids.get(), (size_t)ng * 4, cudaMemcpyDeviceToHost, s));
+            CK(cudaMemcpyAsync(host + x.at + ((size_t)ng * 4 + 7) / 8 * 8, x.col->validity.get(), vbytes, cudaMemcpyDeviceToHost, s));
         }
-    // string keys: dictionary ids decode on the host, build-side ids gather on the device
+        CK(cudaStreamSynchronize(s));
+        std::vector<std::vector<uint32_t>> offs;
+        std::vector<std::string> bytes;
+        size_t out_b = 0;
+        for (auto& x : strs) {
+            const uint32_t* ids = (const uint32_t*)(host + x.at);
+            const uint64_t* valid = (const uint64_t*)(host + x.at + ((size_t)ng * 4 + 7) / 8 * 8);
+            std::vector<uint32_t> off(ng + 1, 0);
+            std::string by;
+            {
+                std::lock_guard<std::mutex> g(h->pipe.intern.mu);
+                for (uint32_t g2 = 0; g2 < ng; g2++) {
+                    if ((valid[g2 / 64] >> (g2 % 64)) & 1) by += h->pipe.intern.strs.at(ids[g2]);
+                    off[g2 + 1] = (uint32_t)by.size();
+                }
+            }
+            DevColumn& c = *x.col;
+            c.kind = CK_UTF8;
+            c.str_bytes = (int64_t)by.size();
+            c.offsets = DevBuf(ctx, (size_t)(ng + 1) * 4, b->res.get());
+            c.data = DevBuf(ctx, std::max<size_t>(by.size(), 1), b->res.get());
+            out_b += ((size_t)(ng + 1) * 4 + by.size() + 15) / 8 * 8;
+            offs.push_back(std::move(off));
+            bytes.push_back(std::move(by));
+        }
+        uint8_t* up = (uint8_t*)stg.get(std::max<size_t>(out_b, 8));  // the ids have been read
+        size_t at = 0;
+        for (size_t i = 0; i < strs.size(); i++) {
+            DevColumn& c = *strs[i].col;
+            const size_t ob = (size_t)(ng + 1) * 4;
+            memcpy(up + at, offs[i].data(), ob);
+            CK(cudaMemcpyAsync(c.offsets.get(), up + at, ob, cudaMemcpyHostToDevice, s));
+            memcpy(up + at + ob, bytes[i].data(), bytes[i].size());
+            if (!bytes[i].empty()) CK(cudaMemcpyAsync(c.data.get(), up + at + ob, bytes[i].size(), cudaMemcpyHostToDevice, s));
+            at += (ob + bytes[i].size() + 15) / 8 * 8;
+        }
+    }
+    // build-side string ids gather on the device
     for (int k = 0; k < F.nkeys; k++) {
         const KeyDecode& d = h->dec[k];
-        if (!d.str_kind) continue;
+        if (d.str_kind != 2) continue;
         auto& kc = keycols[k];
         kc->kind = CK_UTF8;
-        if (d.str_kind == 1) {
-            strings_of_ids(*kc, id_bufs[k].get());
-        } else {
-            const DevColumn& src = *h->pipe.probes[d.build].jt->batch.cols[d.build_col];
-            DevColumn tmp;
-            gather_utf8(ctx, src.optr(), (const uint8_t*)src.dptr(), id_bufs[k].get<uint32_t>(), ng, tmp, s, b->res.get());
-            kc->offsets = std::move(tmp.offsets);
-            kc->data = std::move(tmp.data);
-            CK(cudaStreamSynchronize(s));
-        }
+        const DevColumn& src = *h->pipe.probes[d.build].jt->batch.cols[d.build_col];
+        DevColumn tmp;
+        gather_utf8(ctx, src.optr(), (const uint8_t*)src.dptr(), id_bufs[k].get<uint32_t>(), ng, tmp, s, b->res.get());
+        kc->offsets = std::move(tmp.offsets);
+        kc->data = std::move(tmp.data);
+        kc->str_bytes = tmp.str_bytes;
     }
     for (auto& c : keycols) b->cols.push_back(std::move(c));
     for (auto& c : aggcols) b->cols.push_back(std::move(c));

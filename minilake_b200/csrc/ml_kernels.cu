@@ -357,6 +357,13 @@ __global__ void __launch_bounds__(kThreads) k_acc_init(const __grid_constant__ A
             for (uint64_t g = from + t0; g < to; g += stride) A.aggs[k].vcnt[g] = 0;
 }
 
+// Validity word w (32 rows) of ng rows; the last word's other half, when it has one, is cleared.
+__device__ __forceinline__ void put_valid(uint32_t* valid, uint32_t w, uint32_t ng, uint32_t bits) {
+    const uint32_t words = (ng + 31) / 32;
+    if (w < words) valid[w] = bits;
+    if (w + 1 == words && (words & 1)) valid[w + 1] = 0;
+}
+
 // Final values (accumulator.rs:500-526): AVG = sum / count, empty -> NULL.
 __global__ void k_agg_final(const __grid_constant__ FinalArgs F) {
     uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
@@ -380,7 +387,7 @@ __global__ void k_agg_final(const __grid_constant__ FinalArgs F) {
             else ((uint64_t*)F.key_out[k])[o] = v;
         }
         uint32_t bits = __ballot_sync(0xFFFFFFFFu, in && valid);
-        if (lane == 0 && (o >> 5) < (ng + 31) / 32) F.key_valid[k][o >> 5] = bits;
+        if (lane == 0) put_valid(F.key_valid[k], o >> 5, ng, bits);
     }
     const uint64_t* blk = F.acc + (uint64_t)g * F.stride;
     for (int k = 0; k < F.nagg; k++) {
@@ -422,7 +429,7 @@ __global__ void k_agg_final(const __grid_constant__ FinalArgs F) {
             }
         }
         uint32_t bits = __ballot_sync(0xFFFFFFFFu, in && valid);
-        if (lane == 0 && (o >> 5) < (ng + 31) / 32) F.agg_valid[k][o >> 5] = bits;
+        if (lane == 0) put_valid(F.agg_valid[k], o >> 5, ng, bits);
     }
 }
 
@@ -1367,6 +1374,71 @@ __global__ void __launch_bounds__(256, 2) k_topn_warp(const __grid_constant__ So
 }
 
 
+// ---- small results -------------------------------------------------------------------------------
+// The order of up to kTopNTiny rows in one step: a row's place is the number of rows before it.  (The
+// per-warp lists and their merges took 22 us for six groups ordered by two strings, 5 us so.)
+__global__ void __launch_bounds__(kTopNTiny) k_topn_tiny(const __grid_constant__ SortDev S, int n, int k, uint32_t* out) {
+    __shared__ uint64_t pre[kTopNTiny];
+    const int i = threadIdx.x;
+    if (i < n) pre[i] = sort_prefix(S, (uint32_t)i);
+    __syncthreads();
+    if (i >= n) return;
+    const uint64_t p = pre[i];
+    int place = 0;
+#pragma unroll 1
+    for (int j = 0; j < n; j++) {
+        const uint64_t q = pre[j];
+        int before = q < p ? 1 : 0;
+        if (q == p && j != i) {  // equal keys keep their input order
+            const int c = cmp_rows(S, (uint32_t)j, (uint32_t)i);
+            before = c < 0 || (c == 0 && j < i);
+        }
+        place += before;
+    }
+    if (place < k) out[place] = (uint32_t)i;
+}
+
+// Rows idx[0..k) of every column of a batch, a block per column (k <= 1,024): values, validity words and,
+// for strings, offsets and bytes.  info[c]: a string column's bytes, kNone when they exceed its buffer.
+__global__ void __launch_bounds__(1024) k_gather_small(const __grid_constant__ SmallCols G, const uint32_t* idx, int k) {
+    __shared__ uint64_t tmp[32];
+    const SmallCol& c = G.c[blockIdx.x];
+    const int i = threadIdx.x;
+    const uint32_t r = i < k ? idx[i] : 0u;
+    if (c.dst_valid) {
+        const uint32_t bits = __ballot_sync(0xFFFFFFFFu, i < k && valid_bit(c.src_valid, r));
+        if ((i & 31) == 0 && (i >> 5) < 2 * ((k + 63) / 64)) c.dst_valid[i >> 5] = bits;  // whole 64-bit words
+    }
+    if (c.width) {
+        if (i < k) {
+            if (c.width == 8) ((uint64_t*)c.dst)[i] = ((const uint64_t*)c.src)[r];
+            else if (c.width == 4) ((uint32_t*)c.dst)[i] = ((const uint32_t*)c.src)[r];
+            else ((uint8_t*)c.dst)[i] = ((const uint8_t*)c.src)[r];
+        }
+        return;
+    }
+    uint32_t a = 0, len = 0;
+    if (i < k) {
+        a = c.src_off[r];
+        len = c.src_off[r + 1] - a;
+    }
+    uint64_t total;
+    const uint64_t at = block_exclusive_scan(len, tmp, &total);
+    if (i < k) c.dst_off[i] = (uint32_t)at;
+    if (i == 0) {
+        c.dst_off[k] = (uint32_t)total;
+        G.info[blockIdx.x] = total <= c.cap ? (uint32_t)total : kNone;
+    }
+    if (total <= c.cap)
+        for (uint32_t j = 0; j < len; j++) ((uint8_t*)c.dst)[at + j] = ((const uint8_t*)c.src)[a + j];
+}
+
+// Pieces of memory into one buffer, a block per piece (a small batch read back with one copy).
+__global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackPieces P, uint8_t* dst) {
+    const auto& x = P.p[blockIdx.x];
+    for (uint32_t i = threadIdx.x; i < x.bytes; i += 256) dst[x.at + i] = ((const uint8_t*)x.src)[i];
+}
+
 // ---- top-N by selection: limits up to kMaxTopN over a fixed-width first key ------------------------
 // k_topn_sample takes the r-th smallest key prefix of a sample of the rows, r chosen so that more than k
 // rows lie at or below it all but surely; k_topn_take streams the key column once and lists the rows at
@@ -1780,6 +1852,15 @@ int topn_warp_blocks(int64_t n) {
     int64_t want = (n + 8191) / 8192;
     int64_t cap = (int64_t)num_sms() * resident;
     return (int)std::max<int64_t>(1, std::min(want, cap));
+}
+void launch_topn_tiny(const SortDev& S, int n, int k, uint32_t* out, cudaStream_t s) {
+    k_topn_tiny<<<1, kTopNTiny, 0, s>>>(S, n, k, out);
+}
+void launch_gather_small(const SmallCols& G, const uint32_t* idx, int k, cudaStream_t s) {
+    if (G.n) k_gather_small<<<G.n, 1024, 0, s>>>(G, idx, k);
+}
+void launch_pack(const PackPieces& P, void* dst, cudaStream_t s) {
+    if (P.n) k_pack<<<P.n, 256, 0, s>>>(P, (uint8_t*)dst);
 }
 size_t topn_entry_bytes() { return sizeof(TopEntry); }
 

@@ -161,6 +161,37 @@ void launch_sort_runs(const uint32_t* keys, uint32_t* rows, const SortWord* word
                       uint32_t cap, uint32_t* state, cudaStream_t s);
 void launch_max_strlen(const uint32_t* off, int64_t n, unsigned int* out, cudaStream_t s);
 void launch_iota_u32(uint32_t* out, int64_t n, cudaStream_t s);  // out[i] = i
+// The first k of n <= kTopNTiny rows in order.
+constexpr int kTopNTiny = 256;
+void launch_topn_tiny(const SortDev& S, int n, int k, uint32_t* out, cudaStream_t s);
+// Rows idx[0..k), k <= kSmallRows, of up to kSmallCols fixed-width and plain string columns in one launch.
+constexpr int kSmallRows = 1024, kSmallCols = 16;
+struct SmallCol {
+    int32_t width;  // 0: a string column
+    uint32_t cap;   // bytes dst has room for (strings)
+    const void* src;
+    const uint32_t* src_off;
+    const uint64_t* src_valid;
+    void* dst;
+    uint32_t* dst_off;
+    uint32_t* dst_valid;  // nullptr: no validity; else whole 64-bit words
+};
+struct SmallCols {
+    int32_t n;
+    uint32_t* info;  // per column: a string column's bytes (kNone: more than `cap`, dst not written)
+    SmallCol c[kSmallCols];
+};
+void launch_gather_small(const SmallCols& G, const uint32_t* idx, int k, cudaStream_t s);
+// Up to kPackPieces pieces of device memory into one buffer.
+constexpr int kPackPieces = 3 * kSmallCols;
+struct PackPieces {
+    int32_t n;
+    struct {
+        const void* src;
+        uint32_t bytes, at;
+    } p[kPackPieces];
+};
+void launch_pack(const PackPieces& P, void* dst, cudaStream_t s);
 // Top-k by selection (a sampled bound, one pass that lists the rows at or below it, the exact k-th of
 // those, a sort of the rest): topn_plan says whether a call takes it.
 constexpr int64_t kTopNDirect = 65536;  // up to here the rows are the list

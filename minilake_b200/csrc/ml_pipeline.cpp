@@ -466,6 +466,7 @@ void gather_utf8(Ctx* ctx, const uint32_t* off, const uint8_t* bytes, const uint
     out.kind = CK_UTF8;
     out.dtype = ML_TYPE_UTF8;
     out.n = k;
+    out.str_bytes = (int64_t)total;
     out.offsets = DevBuf(ctx, (size_t)(k + 1) * 4, res);
     launch_u64_to_u32(offs64.get<uint64_t>(), out.offsets.get<uint32_t>(), k + 1, s);
     out.data = DevBuf(ctx, std::max<size_t>(total, 1), res);

@@ -112,6 +112,7 @@ Ctx::~Ctx() {
     if (stream) cudaStreamDestroy(stream);
     for (auto& kv : free_) cudaFree(kv.second);
     for (void* p : slabs_) cudaFreeHost(p);
+    for (auto& kv : pinned_free_) cudaFreeHost(kv.second);
 }
 void* Ctx::pinned_slot() {
     std::lock_guard<std::mutex> g(mu_);
@@ -185,13 +186,40 @@ void Ctx::dfree(void* p, size_t cap) {
     cached_bytes_ += cap;
 }
 void* Ctx::halloc(size_t bytes) {
+    size_t cap = 64 << 10;
+    while (cap < bytes) cap *= 2;
+    {
+        std::lock_guard<std::mutex> g(mu_);
+        auto it = pinned_free_.find(cap);
+        if (it != pinned_free_.end()) {
+            void* p = it->second;
+            pinned_free_.erase(it);
+            pinned_cached_ -= cap;
+            return p;
+        }
+    }
     void* p = nullptr;
     auto t0 = std::chrono::steady_clock::now();
-    CK(cudaHostAlloc(&p, bytes, cudaHostAllocDefault));
+    CK(cudaHostAlloc(&p, cap, cudaHostAllocDefault));
     add_profile("pinned_alloc", std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
+    std::lock_guard<std::mutex> g(mu_);
+    pinned_[p] = cap;
     return p;
 }
-void Ctx::hfree(void* p) { cudaFreeHost(p); }
+void Ctx::hfree(void* p) {
+    {
+        std::lock_guard<std::mutex> g(mu_);
+        auto it = pinned_.find(p);
+        if (it == pinned_.end()) return;
+        if (pinned_cached_ + it->second <= kPinnedCache) {
+            pinned_free_.emplace(it->second, p);
+            pinned_cached_ += it->second;
+            return;
+        }
+        pinned_.erase(it);
+    }
+    cudaFreeHost(p);
+}
 cudaStream_t Ctx::new_stream() {  // streams are pooled: local sinks come and go per pipeline
     {
         std::lock_guard<std::mutex> g(mu_);
@@ -321,6 +349,7 @@ int width_of(int dt) {
 
 int64_t DevColumn::str_bytes_host() const {
     if (kind != CK_UTF8 || n == 0) return 0;
+    if (str_bytes >= 0) return str_bytes;
     uint32_t last = 0, first = 0;
     CK(cudaMemcpy(&last, optr() + n, 4, cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(&first, optr(), 4, cudaMemcpyDeviceToHost));

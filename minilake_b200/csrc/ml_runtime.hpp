@@ -117,8 +117,10 @@ class Ctx {
 
     void* dalloc(size_t bytes, size_t* cap);
     void dfree(void* p, size_t cap);
-    void* halloc(size_t bytes);  // pinned
+    // Pinned host blocks; up to kPinnedCache bytes of freed ones are kept for the next caller.
+    void* halloc(size_t bytes);
     void hfree(void* p);
+    static constexpr size_t kPinnedCache = 64u << 20;
     // 64-byte pinned slots for small device->host readbacks (error words, counters),
     // carved from slabs that live as long as the context.
     void* pinned_slot();
@@ -149,6 +151,9 @@ class Ctx {
     std::multimap<size_t, void*> free_;  // cached device blocks by capacity
     std::vector<cudaStream_t> streams_, idle_streams_;
     std::vector<void*> slabs_, free_slots_;
+    std::map<void*, size_t> pinned_;           // every block's size
+    std::multimap<size_t, void*> pinned_free_;  // cached blocks by size
+    size_t pinned_cached_ = 0;
     size_t cached_bytes_ = 0;
 };
 
@@ -210,6 +215,7 @@ struct DevColumn {
     const void* data_p = nullptr;
     const uint32_t* off_p = nullptr;
     const uint64_t* valid_p = nullptr;
+    int64_t str_bytes = -1;          // an owned CK_UTF8 column's bytes, when known (its offsets start at 0)
     const void* dptr() const { return data ? data.get() : data_p; }
     const uint32_t* optr() const { return offsets ? offsets.get<uint32_t>() : off_p; }
     const uint64_t* vptr() const { return validity ? validity.get<uint64_t>() : valid_p; }

@@ -80,6 +80,7 @@ def _load():
         "ml_gpu_batch_columns": ([VP, P(abi.MlColumn), I32], C.c_int),
         "ml_gpu_batch_column_info": ([VP, I32, P(I32), P(I64), P(I32)], C.c_int),
         "ml_gpu_batch_fetch": ([VP, I32, VP, VP, VP], C.c_int),
+        "ml_gpu_batch_fetch_all": ([VP, I32, P(VP), P(VP), P(VP)], C.c_int),
         "ml_gpu_batch_destroy": ([VP], C.c_int),
         "ml_gpu_filter": ([VP, P(abi.MlExpr), P(abi.MlColumn), I32, I64, VP, I64, I32, VP, P(I64)], C.c_int),
         "ml_gpu_filter_static": ([VP, P(abi.MlExpr), P(abi.MlColumn), I32, I64, VP, I64, VP, P(I64)], C.c_int),
@@ -261,25 +262,28 @@ class DeviceBatch:
         return out
 
     def fetch(self) -> List[HostColumn]:
-        n = self.num_rows
-        cols = []
+        n, nc = self.num_rows, self.num_columns
         words = (n + 63) // 64
-        for i in range(self.num_columns):
+        cols, keep = [], []
+        vals, offs, valids = ((C.c_void_p * max(nc, 1))() for _ in range(3))
+        for i in range(nc):
             t, sb, hv = C.c_int32(), C.c_int64(), C.c_int32()
             _check(LIB.ml_gpu_batch_column_info(self.h, i, C.byref(t), C.byref(sb), C.byref(hv)))
             valid = np.zeros(max(words, 1), dtype=np.uint64)
             if t.value == abi.UTF8:
                 data = np.zeros(max(sb.value, 1), dtype=np.uint8)
                 off = np.zeros(n + 1, dtype=np.uint32)
-                _check(LIB.ml_gpu_batch_fetch(self.h, i, _ptr(data), _ptr(off), _ptr(valid)))
+                offs[i] = _ptr(off)
                 col = HostColumn(abi.UTF8, data[:sb.value], offsets=off)
             else:
                 data = np.zeros(max(n, 1), dtype=abi.NP_DTYPE[t.value])
-                _check(LIB.ml_gpu_batch_fetch(self.h, i, _ptr(data), None, _ptr(valid)))
                 col = HostColumn(t.value, data[:n])
+            vals[i], valids[i] = _ptr(data), _ptr(valid)
+            keep += [data, valid]
             if hv.value:
                 col.validity = valid[:words]
             cols.append(col)
+        _check(LIB.ml_gpu_batch_fetch_all(self.h, nc, vals, offs, valids))
         return cols
 
 
