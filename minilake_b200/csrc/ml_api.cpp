@@ -1564,10 +1564,12 @@ int ml_gpu_join_build_sink(ml_join_build_local* local, const ml_column* cols, in
     const uint32_t* dsel = device_sel(ctx, sel, nsel, sel_hold, local->s);
     Pipeline::Launch L;
     j->pipe.prepare(L, cols, ncols, nrows, dsel, nsel, local->s, local->st, nullptr);
-    auto part = materialize(ctx, j->pipe, j->out_progs, L, local->s, j->res.get(), *local->ew);
-    CK(cudaMemcpyAsync(local->ew->h, local->ew->d.get(), 4, cudaMemcpyDeviceToHost, local->s));
-    CK(cudaStreamSynchronize(local->s));
-    check_device_error(ctx, j->pipe.nstages > 0 ? *local->ew->h : 0);
+    auto part = materialize(ctx, j->pipe, j->out_progs, L, local->s, j->res.get(), *local->ew);  // has finished
+    if (j->pipe.nstages > 0) {
+        CK(cudaMemcpyAsync(local->ew->h, local->ew->d.get(), 4, cudaMemcpyDeviceToHost, local->s));
+        CK(cudaStreamSynchronize(local->s));
+        check_device_error(ctx, *local->ew->h);
+    }
     std::lock_guard<std::mutex> g(j->mu);
     j->parts.push_back(std::move(part));
     API_END
@@ -1652,8 +1654,10 @@ int ml_gpu_join_build_finalize(ml_join_build* j, ml_join_table** table) {
     }
     if (kc) {
         DevBuf mm(ctx, 16, nullptr);
-        uint64_t init[2] = {~0ull, 0ull}, got[2];
-        CK(cudaMemcpyAsync(mm.get(), init, 16, cudaMemcpyHostToDevice, s));
+        PinnedSlot told(ctx);
+        uint64_t* got = told.as<uint64_t>();
+        CK(cudaMemsetAsync(mm.get(), 0xFF, 8, s));
+        CK(cudaMemsetAsync(mm.get<uint8_t>() + 8, 0, 8, s));
         launch_key_range(kc->dptr(), kc->dtype, kc->vptr(), n, mm.get<unsigned long long>(), s);
         ctx->count_launch();
         CK(cudaMemcpyAsync(got, mm.get(), 16, cudaMemcpyDeviceToHost, s));
@@ -1706,6 +1710,7 @@ int ml_gpu_join_build_finalize(ml_join_build* j, ml_join_table** table) {
         ctx->count_launch();
     }
     // canonical ids of the build side's strings (GROUP BY on a build-side string column)
+    std::vector<DevBuf> str_tables;  // read by the kernels in flight until the wait below
     for (auto& c : jt->batch.cols) {
         if (c->kind != CK_UTF8 || n == 0) continue;
         uint64_t cap = pow2_at_least(std::max<uint64_t>(16, (uint64_t)n * 2));
@@ -1715,14 +1720,13 @@ int ml_gpu_join_build_finalize(ml_join_build* j, ml_join_table** table) {
         c->strid = DevBuf(ctx, (size_t)n * 4, jt->res.get());
         launch_strid(c->optr(), (const uint8_t*)c->dptr(), c->vptr(), n, tv, c->strid.get<uint32_t>(), ew.d.get<uint32_t>(), s);
         ctx->count_launch();
-        CK(cudaStreamSynchronize(s));
+        str_tables.push_back(std::move(tslots));
     }
-    uint32_t dup = 0;
-    CK(cudaMemcpyAsync(&dup, jt->dup.get(), 4, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(ew.h + 1, jt->dup.get(), 4, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(ew.h, ew.d.get(), 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     check_device_error(ctx, *ew.h);
-    jt->has_dups = dup != 0;
+    jt->has_dups = ew.h[1] != 0;
     j->table = std::move(jt);
     *table = j->table.get();
     API_END

@@ -13,6 +13,7 @@
 #include <set>
 #include <type_traits>
 #include <sstream>
+#include <unordered_map>
 
 namespace mlg {
 
@@ -1293,6 +1294,19 @@ std::string signature(char kind, const PipeArgs& P, const AggArgs* A, const KeyL
     return key;
 }
 
+// Kernels by launch shape, for the process: a new sink of a shape that ran before finds its kernel without
+// generating the source again (100 to 300 us of string work per new sink or operator call).  The key is all
+// that the source depends on: the signature and the pipeline's instructions without their literals.
+struct ShapeCache {
+    std::mutex mu;
+    std::unordered_map<std::string, void*> fns;
+};
+ShapeCache& shapes() {
+    static ShapeCache c;
+    return c;
+}
+constexpr size_t kMaxShapes = 4096;
+
 template <class Make>
 void* memoized(const Pipeline& pipe, std::string key, Make make) {
     {
@@ -1300,7 +1314,23 @@ void* memoized(const Pipeline& pipe, std::string key, Make make) {
         for (auto& e : pipe.jit_memo)
             if (e.first == key) return e.second;
     }
-    void* fn = make();
+    std::string shape = key;
+    for (const Instr& in : pipe.C.code) {
+        const int32_t f[8] = {in.op, in.sub, in.t, in.flag, in.a, in.b, in.c, (int32_t)in.lit_valid};
+        shape.append((const char*)f, sizeof f);
+    }
+    void* fn = nullptr;
+    {
+        std::lock_guard<std::mutex> g(shapes().mu);
+        auto it = shapes().fns.find(shape);
+        if (it != shapes().fns.end()) fn = it->second;
+    }
+    if (!fn) {
+        fn = make();
+        std::lock_guard<std::mutex> g(shapes().mu);
+        if (shapes().fns.size() >= kMaxShapes) shapes().fns.clear();  // found again by their source
+        shapes().fns.emplace(std::move(shape), fn);
+    }
     std::lock_guard<std::mutex> g(pipe.jit_mu);
     if (pipe.jit_memo.size() >= 16) pipe.jit_memo.erase(pipe.jit_memo.begin());
     pipe.jit_memo.emplace_back(std::move(key), fn);
@@ -1326,6 +1356,11 @@ void* jit_agg_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, const Ag
 
 void* jit_agg_resume_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, const AggArgs& A) {
     if (!jit_enabled(ctx) || has_string_minmax(A)) return nullptr;
+    return memoized(pipe, signature('r', P, &A, nullptr) + std::string((const char*)&ctx->device, sizeof(int)),
+                    [&] { return (void*)get_kernel(ctx, jit_resume_source(pipe, P, A), "ml_pipeline_aggregate_resume"); });
+}
+
+std::string jit_resume_source(const Pipeline& pipe, const PipeArgs& P, const AggArgs& A) {
     // the rows a full table sent to the overflow list, aggregated again after the table grew
     Gen g(pipe.C.code, P);
     g.fail = "break;";
@@ -1349,11 +1384,16 @@ void* jit_agg_resume_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, c
     src += "    }\n";
     if (smem) src += "    __syncthreads();\n    smem_flush(A, smem);\n";
     src += "}\n";
-    return (void*)get_kernel(ctx, src, "ml_pipeline_aggregate_resume");
+    return src;
 }
 
 void* jit_join_insert_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, const KeyLayout& L) {
     if (!jit_enabled(ctx)) return nullptr;
+    return memoized(pipe, signature('j', P, nullptr, &L) + std::string((const char*)&ctx->device, sizeof(int)),
+                    [&] { return (void*)get_kernel(ctx, jit_join_insert_source(pipe, P, L), "ml_join_insert"); });
+}
+
+std::string jit_join_insert_source(const Pipeline& pipe, const PipeArgs& P, const KeyLayout& L) {
     // build_table (join.rs:160-203): distinct keys in the table, duplicates chained in `next`.
     // One-word keys insert with a single 128-bit CAS; wider keys use the claim protocol.
     Gen g(pipe.C.code, P);
@@ -1384,7 +1424,7 @@ void* jit_join_insert_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, 
     src += "        RowCtx x;\n        x.r = (uint32_t)i;\n        x.b0 = x.b1 = x.b2 = x.b3 = 0;\n        x.head = 0;\n";
     src += g.body();
     src += "    }\n}\n";
-    return (void*)get_kernel(ctx, src, "ml_join_insert");
+    return src;
 }
 
 void* jit_select_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P) {

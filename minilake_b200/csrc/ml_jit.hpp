@@ -36,6 +36,8 @@ void* jit_hll_kernel(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, const Ke
 // Sources of the kernels above.
 // `contig`: consecutive rows per thread with vector loads (needs no selection vector and 16-byte
 // aligned source columns).
+std::string jit_resume_source(const Pipeline& pipe, const PipeArgs& P, const AggArgs& A);
+std::string jit_join_insert_source(const Pipeline& pipe, const PipeArgs& P, const KeyLayout& L);
 std::string jit_select_source(const Pipeline& pipe, const PipeArgs& P, bool contig, bool builds = false);
 std::string jit_hll_source(const Pipeline& pipe, const PipeArgs& P, const KeyLayout& L, bool contig);
 
