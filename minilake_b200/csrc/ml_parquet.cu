@@ -8,14 +8,16 @@
 //      element, then the compressor's independent 64 KB fragments resolve their copies by pointer
 //      jumping (a page that does not split that way is decoded by one thread);
 //   2. every RLE / bit-packed hybrid stream (definition levels, dictionary indices) gets a run
-//      table (one thread per stream walks the run headers, counting first, then filling);
-//   3. rows are decoded in 8,192-row tiles: definition levels give the validity bits, a block
-//      scan of their popcounts gives each row's position among the chunk's present values, and
-//      the value comes from its page (PLAIN, or a dictionary index into the dictionary page) with
-//      the column's conversion (FLOAT -> f64, DECIMAL -> f64 / 10^scale);
-//   4. strings are materialized (NULL rows as "", as the reference does), canonicalized with a
-//      device hash table, and dictionary-encoded in order of first occurrence when there are at
-//      most clamp(rows / 8, 1, 65,536) distinct values, else kept plain (encode_strings).
+//      table (one warp per stream walks the run headers in a staged window of the stream);
+//   3. definition levels give the validity bits, 32 rows per thread, and the present values per
+//      8,192-row tile; a row's popcount rank in its tile gives its position among the chunk's
+//      present values, and the value comes from its page (PLAIN, or a dictionary index into the
+//      dictionary page) with the column's conversion (FLOAT -> f64, DECIMAL -> f64 / 10^scale);
+//   4. strings get a dictionary in order of first occurrence when there are at most
+//      clamp(rows / 8, 1, 65,536) distinct values, else are kept plain (encode_strings); NULL rows
+//      count as "", as in the reference.  A chunk whose pages all index a small dictionary page
+//      works on that page's entries; any other chunk's strings are materialized and canonicalized
+//      with a device hash table.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -24,6 +26,7 @@
 #include <vector>
 
 #include "ml_api_common.hpp"
+#include "ml_device.cuh"
 #include "ml_kernels.cuh"
 #include "ml_pipeline.hpp"
 
@@ -715,10 +718,7 @@ struct PageDev {
 
 __device__ uint32_t le32(const uint8_t* p) { return p[0] | (p[1] << 8) | (p[2] << 16) | ((uint32_t)p[3] << 24); }
 
-__global__ void k_pq_layout(PageDev* pages, int npages, int max_def, uint32_t* err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npages) return;
-    PageDev& p = pages[i];
+__device__ void page_layout(PageDev& p, int max_def, uint32_t* err) {
     uint32_t pos = 0;
     p.levels = nullptr;
     p.levels_len = 0;
@@ -765,90 +765,188 @@ __global__ void k_pq_layout(PageDev* pages, int npages, int max_def, uint32_t* e
     }
 }
 
-// Walk a hybrid stream of `n` values with bit width `bw`: count its runs (runs == nullptr) or
-// write them.  Returns the number of runs, or -1 when the stream is malformed.
-__device__ int64_t rle_walk(const uint8_t* s, uint32_t len, uint32_t n, int bw, Run* runs) {
+// A stream read by one warp through a window of shared memory: 16-byte loads from the 16-byte
+// boundary at or before the wanted byte.  Every stream lies in the uncompressed-page buffer, which
+// is 16-byte aligned at its start and padded by 64 bytes at its end.
+constexpr uint32_t kPqWindow = 8192;
+struct StreamWindow {
+    const uint8_t* s;
+    uint32_t len;
+    uint4* win;       // kPqWindow bytes and 16 more for peek8
+    uint32_t lo, hi;  // stream bytes [lo, hi) are in the window, byte lo at win + skew
+    uint32_t skew;
+
+    __device__ StreamWindow(const uint8_t* s_, uint32_t len_, uint4* w) : s(s_), len(len_), win(w), lo(0), hi(0), skew(0) {}
+    // Bytes [pos, min(pos + n, len)) readable by at(); n <= kPqWindow - 16.  The whole warp calls it.
+    __device__ void need(uint32_t pos, uint32_t n) {
+        if (pos >= lo && (hi >= len || (uint64_t)pos + n <= hi)) return;
+        if (pos >= len) return;
+        skew = (uint32_t)((uintptr_t)(s + pos) & 15);
+        lo = pos;
+        const uint32_t take = len - pos < kPqWindow - skew ? len - pos : kPqWindow - skew;
+        hi = pos + take;
+        const uint4* src = (const uint4*)(s + pos - skew);
+        __syncwarp();
+        // all loads in flight at once: four at a time made a refill 2.8 us
+        const uint32_t nvec = (skew + take + 15) / 16;
+        uint4 v[kPqWindow / 512];
+#pragma unroll
+        for (uint32_t j = 0; j < kPqWindow / 512; j++) {
+            const uint32_t i = j * 32 + (threadIdx.x & 31);
+            if (i < nvec) v[j] = src[i];
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kPqWindow / 512; j++) {
+            const uint32_t i = j * 32 + (threadIdx.x & 31);
+            if (i < nvec) win[i] = v[j];
+        }
+        __syncwarp();
+    }
+    __device__ uint32_t at(uint32_t pos) const { return ((const uint8_t*)win)[skew + (pos - lo)]; }
+    __device__ uint32_t at32(uint32_t pos) const { return (uint32_t)peek8(pos); }
+    __device__ uint64_t peek8(uint32_t pos) const {  // bytes past hi are whatever the window holds
+        const uint32_t b = skew + (pos - lo), sh = 8 * (b & 3);
+        const uint32_t* w = (const uint32_t*)win + (b >> 2);
+        const uint32_t w0 = w[0], w1 = w[1], w2 = w[2];
+        return (uint64_t)__funnelshift_r(w0, w1, sh) | ((uint64_t)__funnelshift_r(w1, w2, sh) << 32);
+    }
+};
+
+// Walk a hybrid stream of `n` values with bit width `bw` and write its runs: one warp, every lane
+// the same steps.  A writer fills bit-packed runs to one size, so after such a run each lane looks
+// where the i-th run of that size would start; the headers agree up to some lane, and the walk goes
+// on from there.  Short runs are looked up in the window, long ones (whose headers lie too far apart
+// for it) in memory.  Returns the number of runs, or -1 when the stream is malformed.
+__device__ int64_t rle_walk(const uint8_t* s, uint32_t len, uint32_t n, int bw, Run* runs, uint4* win) {
+    StreamWindow S(s, len, win);
+    const uint32_t lane = threadIdx.x & 31;
     uint32_t pos = 0, got = 0;
     int64_t k = 0;
     const uint32_t vbytes = (bw + 7) / 8;
     while (got < n) {
-        uint64_t h = 0;
-        for (int shift = 0;; shift += 7) {
-            if (pos >= len || shift > 35) return -1;
-            const uint8_t b = s[pos++];
-            h |= (uint64_t)(b & 0x7F) << shift;
-            if (!(b & 0x80)) break;
-        }
-        Run r{got, 0, 0, 0};
+        if (pos >= len) return -1;
+        S.need(pos, 16);  // a header (at most 6 bytes) and a value (at most 4)
+        const uint64_t w = S.peek8(pos);
+        const int hb = __ffsll((long long)(~w & 0x808080808080ull)) / 8;  // header bytes
+        if (hb == 0 || (uint64_t)pos + hb > len) return -1;
+        uint64_t h = w & 0x7F;
+        for (int i = 1; i < hb; i++) h |= ((w >> (8 * i)) & 0x7F) << (7 * i);
+        const uint32_t left = n - got;
         if (h & 1) {  // bit-packed: (h >> 1) groups of 8 values (none: malformed, every run holds a value)
-            const uint64_t vals = (h >> 1) * 8, bytes = (h >> 1) * (uint64_t)bw;
-            if (vals == 0 || pos + bytes > len) return -1;
-            r.count = (uint32_t)(uint32_t)(vals < (uint64_t)(n - got) ? vals : (uint64_t)(n - got));
-            r.value = pos;
-            r.packed = 1;
-            pos += (uint32_t)bytes;
+            const uint64_t vals = (h >> 1) * 8, bytes = (h >> 1) * (uint64_t)bw, stride = hb + bytes;
+            if (vals == 0 || pos + stride > len) return -1;
+            const uint64_t at = pos + lane * stride, before = lane * vals;
+            bool same = before < left && at + stride <= len;
+            const uint64_t mask = (1ull << (8 * hb)) - 1;
+            if (stride > kPqWindow / 16) {
+                for (int i = 0; i < hb && same; i++) same = s[at + i] == ((w >> (8 * i)) & 0xFF);
+            } else {
+                same = same && at + hb <= S.hi && (S.peek8((uint32_t)at) & mask) == (w & mask);
+            }
+            const uint32_t agree = __ballot_sync(0xFFFFFFFFu, same);
+            const uint32_t m = agree == 0xFFFFFFFFu ? 32u : (uint32_t)__ffs(~agree) - 1u;  // at least this lane 0's own
+            if (lane < m) {
+                const uint64_t rest = left - before;
+                runs[k + lane] = Run{got + (uint32_t)before, (uint32_t)(vals < rest ? vals : rest), (uint32_t)at + hb, 1};
+            }
+            k += m;
+            pos += (uint32_t)(m * stride);
+            got += (uint32_t)(m * vals < left ? m * vals : left);
         } else {
-            r.count = (uint32_t)((h >> 1) < (uint64_t)(n - got) ? (h >> 1) : (uint64_t)(n - got));
-            if (pos + vbytes > len || r.count == 0) return -1;
-            for (uint32_t b = 0; b < vbytes; b++) r.value |= (uint32_t)s[pos + b] << (8 * b);
+            Run r{got, (uint32_t)((h >> 1) < left ? (h >> 1) : left), 0, 0};
+            pos += hb;
+            if ((uint64_t)pos + vbytes > len || r.count == 0) return -1;
+            if (hb + vbytes <= 8) r.value = (uint32_t)((w >> (8 * hb)) & (vbytes == 4 ? 0xFFFFFFFFull : (1ull << (8 * vbytes)) - 1));
+            else for (uint32_t b = 0; b < vbytes; b++) r.value |= S.at(pos + b) << (8 * b);
             pos += vbytes;
+            if (lane == 0) runs[k] = r;
+            k++;
+            got += r.count;
         }
-        if (runs) runs[k] = r;
-        k++;
-        got += r.count;
     }
     return k;
 }
 
-// One thread per page and stream (`which` 0: definition levels, one per row; 1: dictionary
-// indices or RLE booleans, one per present value, `nvalues`).  With runs == nullptr it counts
-// the runs into the page; else it writes them from the page's run offset.
-__global__ void k_pq_runs(PageDev* pages, int npages, int which, int level_width, const uint32_t* nvalues, Run* runs,
-                          uint32_t* err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npages) return;
-    PageDev& p = pages[i];
-    const bool lv = which == 0;
-    const uint8_t* s = lv ? p.levels : p.values;
-    const uint32_t len = lv ? p.levels_len : p.values_len;
-    const int bw = lv ? level_width : p.idx_width;
-    const uint32_t n = lv ? p.nrows : nvalues[i];
-    uint32_t& nruns = lv ? p.lv_nruns : p.ix_nruns;
-    Run* out = runs ? runs + (lv ? p.lv_run0 : p.ix_run0) : nullptr;
-    if (!s || bw < 0 || n == 0) {
-        nruns = 0;
-        return;
+// The run table of one page's stream.
+__device__ void page_runs(const uint8_t* s, uint32_t len, uint32_t n, int bw, Run* out, uint32_t& nruns, uint4* win, uint32_t* err) {
+    uint32_t found = 0;
+    if (s && bw >= 0 && n > 0) {
+        if (bw == 0) {  // every value is 0: one run, no bytes
+            if (threadIdx.x == 0) out[0] = Run{0, n, 0, 0};
+            found = 1;
+        } else {
+            const int64_t k = rle_walk(s, len, n, bw, out, win);
+            if (k < 0 && threadIdx.x == 0) atomicOr(err, PQ_ERR_RUNS);
+            found = k < 0 ? 0u : (uint32_t)k;
+        }
     }
-    if (bw == 0) {  // every value is 0: one run, no bytes
-        if (out) out[0] = Run{0, n, 0, 0};
-        nruns = 1;
-        return;
-    }
-    const int64_t k = rle_walk(s, len, n, bw, out);
-    if (k < 0) {
-        atomicOr(err, PQ_ERR_RUNS);
-        nruns = 0;
-        return;
-    }
-    nruns = (uint32_t)k;
+    if (threadIdx.x == 0) nruns = found;
 }
 
-// Value k of a stream from its run table (k < the stream's value count).
-__device__ uint32_t rle_get(const Run* runs, uint32_t nruns, const uint8_t* s, int bw, uint32_t k) {
+// Layout and definition-level runs, one warp per page.  A walk is a chain: each header says where
+// the next one lies.  One thread per page and a dependent L2 load per link took 19 us per launch (seven
+// pages of 18,000 values, about 40 runs each); with the window and up to 32 headers per step 4.4 us here
+// and 7.5 us for index runs (23 us where short RLE runs break the sizes, of 38).
+__global__ void __launch_bounds__(32) k_pq_levels(PageDev* pages, int max_def, int level_width, Run* runs, uint32_t* err) {
+    __shared__ uint4 win[kPqWindow / 16 + 1];
+    PageDev& p = pages[blockIdx.x];
+    if (threadIdx.x == 0) page_layout(p, max_def, err);
+    __syncwarp();
+    page_runs(p.levels, p.levels_len, p.nrows, level_width, runs + p.lv_run0, p.lv_nruns, win, err);
+}
+
+__device__ uint32_t warp_sum(uint32_t x) { return __reduce_add_sync(0xFFFFFFFFu, x); }
+
+// Present values before each page's first row, each page's present values, and the runs of its
+// dictionary indices or RLE booleans (one per present value): one warp per page.
+__global__ void __launch_bounds__(32) k_pq_indices(PageDev* pages, const uint32_t* valid, const uint64_t* tile_offs, int64_t nrows,
+                                                   uint32_t* nvalues, Run* runs, uint32_t* err) {
+    __shared__ uint4 win[kPqWindow / 16 + 1];
+    PageDev& p = pages[blockIdx.x];
+    auto rank = [&](int64_t row) -> uint64_t {  // present values in rows [0, row)
+        if (row >= nrows) return tile_offs[(nrows + kPqTile - 1) / kPqTile];
+        const int64_t t = row / kPqTile, w0 = t * (kPqTile / 32);
+        const int words = (int)(row / 32 - w0);  // whole words before the row's, at most 255
+        uint32_t c = 0;
+#pragma unroll
+        for (int j = 0; j < kPqTile / 32 / 32; j++) {
+            const int w = j * 32 + (int)threadIdx.x;
+            if (w < words) c += __popc(valid[w0 + w]);
+        }
+        if (threadIdx.x == 0 && (row & 31)) c += __popc(valid[row / 32] & ((1u << (row & 31)) - 1u));
+        return tile_offs[t] + warp_sum(c);
+    };
+    const uint64_t v0 = rank(p.row0), v1 = rank(p.row0 + p.nrows);
+    if (threadIdx.x == 0) {
+        p.valid0 = v0;
+        nvalues[blockIdx.x] = (uint32_t)(v1 - v0);
+    }
+    page_runs(p.values, p.values_len, (uint32_t)(v1 - v0), p.idx_width, runs + p.ix_run0, p.ix_nruns, win, err);
+}
+
+// Eight bytes from any address (streams lie in the padded page buffer: the aligned words around
+// them are readable).
+__device__ uint64_t load8(const uint8_t* p) {
+    const uint64_t* b = (const uint64_t*)((uintptr_t)p & ~(uintptr_t)7);
+    const int sh = 8 * (int)((uintptr_t)p & 7);
+    const uint64_t lo = b[0];
+    return sh ? (lo >> sh) | (b[1] << (64 - sh)) : lo;
+}
+
+// The run that holds value k (k < the stream's value count).
+__device__ uint32_t run_of(const Run* runs, uint32_t nruns, uint32_t k) {
     uint32_t lo = 0, hi = nruns;
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
         if (runs[mid].first <= k) lo = mid;
         else hi = mid;
     }
-    const Run r = runs[lo];
+    return lo;
+}
+__device__ uint32_t run_value(const Run& r, const uint8_t* s, int bw, uint32_t k) {
     if (!r.packed) return r.value;
     const uint64_t bit = (uint64_t)(k - r.first) * bw;
-    const uint8_t* b = s + r.value + (bit >> 3);
-    uint64_t w = 0;
-    const int nb = (int)(((bit & 7) + bw + 7) >> 3);
-    for (int j = 0; j < nb; j++) w |= (uint64_t)b[j] << (8 * j);
-    return (uint32_t)((w >> (bit & 7)) & (bw == 32 ? 0xFFFFFFFFull : ((1ull << bw) - 1)));
+    return (uint32_t)((load8(s + r.value + (bit >> 3)) >> (bit & 7)) & (bw == 32 ? 0xFFFFFFFFull : ((1ull << bw) - 1)));
 }
 
 __device__ int page_of(const PageDev* pages, int npages, int64_t row) {
@@ -862,53 +960,93 @@ __device__ int page_of(const PageDev* pages, int npages, int64_t row) {
 }
 
 // ---- 3. validity: definition level == max_def, one thread per 32-row word ----------------------
+// A word's rows are taken run by run (an RLE run, or 32 one-bit levels, at once), not level by
+// level: 13.7 -> 4.7 us for a 125,000-row chunk.
 __global__ void k_pq_valid(const PageDev* pages, int npages, const Run* runs, int max_def, int level_width, int64_t nrows,
                            uint32_t* valid, uint32_t* tile_counts) {
     const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t bits = 0;
-    if (w * 32 < nrows) {
+    const int rows = w * 32 < nrows ? (int)(nrows - w * 32 < 32 ? nrows - w * 32 : 32) : 0;
+    if (rows && max_def == 0) bits = rows == 32 ? ~0u : (1u << rows) - 1u;
+    if (rows && max_def > 0) {
         int p = page_of(pages, npages, w * 32);
-        for (int j = 0; j < 32; j++) {
+        for (int j = 0; j < rows;) {
             const int64_t r = w * 32 + j;
-            if (r >= nrows) break;
             while (p + 1 < npages && pages[p + 1].row0 <= r) p++;
             const PageDev& pg = pages[p];
-            const uint32_t k = (uint32_t)(r - pg.row0);
-            bool v = true;
-            if (max_def > 0) {
-                v = k < pg.nrows && pg.lv_nruns &&
-                    rle_get(runs + pg.lv_run0, pg.lv_nruns, pg.levels, level_width, k) == (uint32_t)max_def;
+            uint32_t k = (uint32_t)(r - pg.row0);
+            int left = pg.nrows > k ? (int)(pg.nrows - k < (uint32_t)(rows - j) ? pg.nrows - k : (uint32_t)(rows - j)) : 0;
+            if (!left || !pg.lv_nruns) {  // no levels (malformed): absent
+                j += left ? left : 1;
+                continue;
             }
-            bits |= (uint32_t)v << j;
+            const Run* rs = runs + pg.lv_run0;
+            for (uint32_t i = run_of(rs, pg.lv_nruns, k); left > 0 && i < pg.lv_nruns; i++) {
+                const Run run = rs[i];
+                const uint32_t in_run = run.first + run.count - k;
+                const int m = in_run < (uint32_t)left ? (int)in_run : left;
+                uint32_t x = 0;
+                if (!run.packed) {
+                    x = run.value == (uint32_t)max_def ? ~0u : 0u;
+                } else if (level_width == 1) {  // max_def is 1; 32 levels and an offset of 7 fit eight bytes
+                    const uint32_t bit = k - run.first;
+                    x = (uint32_t)(load8(pg.levels + run.value + (bit >> 3)) >> (bit & 7));
+                } else {
+                    for (int q = 0; q < m; q++) x |= (uint32_t)(run_value(run, pg.levels, level_width, k + q) == (uint32_t)max_def) << q;
+                }
+                bits |= (m == 32 ? x : x & ((1u << m) - 1u)) << j;
+                j += m;
+                k += m;
+                left -= m;
+            }
+            j += left;
         }
-        valid[w] = bits;
     }
+    if (rows) valid[w] = bits;
     // present values per 8,192-row tile
-    const int c = __popc(bits);
+    const uint32_t c = warp_sum(__popc(bits));
     __shared__ uint32_t sum;
     if (threadIdx.x == 0) sum = 0;
     __syncthreads();
-    if (c) atomicAdd(&sum, (uint32_t)c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&sum, c);
     __syncthreads();
     if (threadIdx.x == 0) tile_counts[blockIdx.x] = sum;
 }
 
-// Present values before each page's first row, and each page's present values.
-__global__ void k_pq_page_valid(PageDev* pages, int npages, const uint32_t* valid, const uint64_t* tile_offs,
-                                int64_t nrows, uint32_t* nvalues) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > npages) return;
-    auto rank = [&](int64_t row) -> uint64_t {  // present values in rows [0, row)
-        if (row >= nrows) return tile_offs[(nrows + kPqTile - 1) / kPqTile];
-        const int64_t t = row / kPqTile;
-        uint64_t c = tile_offs[t];
-        for (int64_t w = t * (kPqTile / 32); w < row / 32; w++) c += __popc(valid[w]);
-        if (row & 31) c += __popc(valid[row / 32] & ((1u << (row & 31)) - 1u));
-        return c;
-    };
-    if (i < npages) {
-        pages[i].valid0 = rank(pages[i].row0);
-        nvalues[i] = (uint32_t)(rank(pages[i].row0 + pages[i].nrows) - pages[i].valid0);
+// Exclusive scan of the tiles' present values by one block, with the total in offs[n] and in
+// *present: a chunk has few tiles (262,144 at most: 256 steps), and one small launch replaces the
+// three of the general scan (3 x 3.1 us).
+__global__ void __launch_bounds__(1024) k_pq_tile_scan(const uint32_t* counts, int64_t n, uint64_t* offs, uint64_t* present) {
+    __shared__ uint64_t warps[32];
+    __shared__ uint64_t carry;
+    const int t = threadIdx.x;
+    if (t == 0) carry = 0;
+    for (int64_t i0 = 0; i0 < n; i0 += 1024) {
+        __syncthreads();
+        const uint64_t c = i0 + t < n ? counts[i0 + t] : 0u, base = carry;
+        uint64_t x = c;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint64_t y = __shfl_up_sync(~0u, x, d);
+            if ((t & 31) >= d) x += y;
+        }
+        if ((t & 31) == 31) warps[t >> 5] = x;
+        __syncthreads();
+        if (t < 32) {
+            uint64_t y = warps[t];
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint64_t z = __shfl_up_sync(~0u, y, d);
+                if (t >= d) y += z;
+            }
+            warps[t] = y;
+            if (t == 31) carry = base + y;
+        }
+        __syncthreads();
+        if (i0 + t < n) offs[i0 + t] = base + (t >= 32 ? warps[(t >> 5) - 1] : 0) + x - c;
+    }
+    __syncthreads();
+    if (t == 0) {
+        offs[n] = carry;
+        *present = carry;
     }
 }
 }  // namespace
@@ -938,8 +1076,18 @@ struct DecodeArgs {
     void* out;                // fixed-width output (the column's type)
     const uint8_t** str_ptr;  // strings (and byte-array decimals go through vptr)
     uint32_t* str_len;
+    // strings whose pages all index a dictionary of fewer than kPqSmallDict entries: each row's entry
+    // instead (dict_n for a NULL), ~(first row) of each entry (0: unused) and the strings' bytes
+    uint32_t* ent;
+    uint32_t* first;
+    uint64_t* total;
     uint32_t* err;
 };
+constexpr uint32_t kPqSmallDict = 1024;
+constexpr uint32_t kPqSmallDictBytes = 65536;
+// rows per block: a 125,000-row chunk in 16 blocks of a whole tile left most SMs idle and put 32 rows in
+// series on a thread (57 us); 245 blocks of two rows per thread take 9.8 us
+constexpr int kPqSlice = 512;
 
 // A big-endian two's complement integer of up to 16 bytes (be_i128, parquet_reader.rs:154-166)
 // as the nearest f64 (ties to even).
@@ -974,16 +1122,18 @@ __device__ double be_int_to_f64(const uint8_t* b, uint32_t n) {
     return neg ? -m : m;
 }
 
-__device__ uint64_t load_le(const uint8_t* p, int w) {
-    uint64_t v = 0;
-    for (int i = 0; i < w; i++) v |= (uint64_t)p[i] << (8 * i);
-    return v;
-}
-
 __global__ void __launch_bounds__(256) k_pq_values(const __grid_constant__ DecodeArgs D) {
     __shared__ uint32_t words[256], pre[256];
+    __shared__ uint32_t sfirst[kPqSmallDict];
+    __shared__ uint32_t stotal;
     const int t = threadIdx.x;
-    const int64_t w0 = (int64_t)blockIdx.x * 256;
+    const int64_t tile = blockIdx.x / (kPqTile / kPqSlice);
+    const int64_t w0 = tile * (kPqTile / 32);
+    const int64_t row0 = (int64_t)blockIdx.x * kPqSlice;
+    if (D.ent) {
+        for (uint32_t i = t; i <= D.dict_n; i += 256) sfirst[i] = 0;
+        if (t == 0) stotal = 0;
+    }
     const uint32_t word = (w0 + t) * 32 < D.nrows ? D.valid[w0 + t] : 0u;
     words[t] = word;
     // exclusive scan of the words' popcounts
@@ -992,24 +1142,32 @@ __global__ void __launch_bounds__(256) k_pq_values(const __grid_constant__ Decod
         const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
         if ((t & 31) >= o) x += y;
     }
-    __shared__ uint32_t warp_sum[8];
-    if ((t & 31) == 31) warp_sum[t >> 5] = x;
+    __shared__ uint32_t warp_total[8];
+    if ((t & 31) == 31) warp_total[t >> 5] = x;
     __syncthreads();
     uint32_t wbase = 0;
-    for (int i = 0; i < (t >> 5); i++) wbase += warp_sum[i];
+    for (int i = 0; i < (t >> 5); i++) wbase += warp_total[i];
     pre[t] = wbase + x - c;
     __syncthreads();
-    const uint64_t base = D.tile_offs[blockIdx.x];
+    const uint64_t base = D.tile_offs[tile];
+    uint32_t bytes = 0;  // of this thread's strings (each within a small dictionary page)
+    // the first rows of the block's entries: most rows only read the word
+    auto entry = [&](uint32_t e, int64_t r) {
+        D.ent[r] = e;
+        if (*(volatile uint32_t*)(sfirst + e) < ~(uint32_t)r) atomicMax(sfirst + e, ~(uint32_t)r);
+    };
     int p = -1;
-    for (int j = 0; j < 32; j++) {
-        const int64_t r = (int64_t)blockIdx.x * kPqTile + j * 256 + t;
+    for (int j = 0; j < kPqSlice / 256; j++) {
+        const int64_t r = row0 + j * 256 + t;
         if (r >= D.nrows) break;
         const int lw = (int)((r >> 5) - w0);
         const uint32_t bits = words[lw];
         const bool v = (bits >> (r & 31)) & 1;
         const int vw = D.conv == CV_BOOL ? 1 : (D.conv == CV_INT32 || D.conv == CV_DATE) ? 4 : 8;
         if (!v) {
-            if (D.conv == CV_UTF8) {
+            if (D.ent) {
+                entry(D.dict_n, r);
+            } else if (D.conv == CV_UTF8) {
                 D.str_ptr[r] = nullptr;
                 D.str_len[r] = 0;
             } else if (vw == 1) {
@@ -1031,13 +1189,21 @@ __global__ void __launch_bounds__(256) k_pq_values(const __grid_constant__ Decod
         if (dict || rle_bool) {
             if (!pg.ix_nruns) {
                 atomicOr(D.err, PQ_ERR_VALUES);
+                if (D.ent) entry(D.dict_n, r);  // the codes are looked up before the error is read
                 continue;
             }
-            idx = rle_get(D.runs + pg.ix_run0, pg.ix_nruns, pg.values, pg.idx_width, k);
+            const Run* rs = D.runs + pg.ix_run0;
+            idx = run_value(rs[run_of(rs, pg.ix_nruns, k)], pg.values, pg.idx_width, k);
             if (dict && idx >= D.dict_n) {
                 atomicOr(D.err, PQ_ERR_VALUES);
+                if (D.ent) entry(D.dict_n, r);
                 continue;
             }
+        }
+        if (D.ent) {
+            entry(idx, r);
+            bytes += D.dict_len[idx];
+            continue;
         }
         // the value's bytes: a byte array (pointer, length) or a fixed-width slot
         const uint8_t* src = nullptr;
@@ -1081,12 +1247,12 @@ __global__ void __launch_bounds__(256) k_pq_values(const __grid_constant__ Decod
                 break;
             }
             case CV_INT32:
-            case CV_DATE: ((uint32_t*)D.out)[r] = (uint32_t)load_le(src, 4); break;
+            case CV_DATE: ((uint32_t*)D.out)[r] = (uint32_t)load8(src); break;
             case CV_INT64:
-            case CV_DOUBLE: ((uint64_t*)D.out)[r] = load_le(src, 8); break;
-            case CV_FLOAT: ((double*)D.out)[r] = (double)__uint_as_float((uint32_t)load_le(src, 4)); break;
-            case CV_DEC_I32: ((double*)D.out)[r] = __ddiv_rn((double)(int32_t)load_le(src, 4), D.div); break;
-            case CV_DEC_I64: ((double*)D.out)[r] = __ddiv_rn(__ll2double_rn((long long)load_le(src, 8)), D.div); break;
+            case CV_DOUBLE: ((uint64_t*)D.out)[r] = load8(src); break;
+            case CV_FLOAT: ((double*)D.out)[r] = (double)__uint_as_float((uint32_t)load8(src)); break;
+            case CV_DEC_I32: ((double*)D.out)[r] = __ddiv_rn((double)(int32_t)(uint32_t)load8(src), D.div); break;
+            case CV_DEC_I64: ((double*)D.out)[r] = __ddiv_rn(__ll2double_rn((long long)load8(src)), D.div); break;
             case CV_DEC_BYTES: ((double*)D.out)[r] = __ddiv_rn(be_int_to_f64(src, slen), D.div); break;
             case CV_UTF8:
                 D.str_ptr[r] = src;
@@ -1094,15 +1260,23 @@ __global__ void __launch_bounds__(256) k_pq_values(const __grid_constant__ Decod
                 break;
         }
     }
+    if (!D.ent) return;
+    bytes = warp_sum(bytes);
+    if ((t & 31) == 0 && bytes) atomicAdd(&stotal, bytes);  // 512 rows of at most 64 KB
+    __syncthreads();
+    for (uint32_t i = t; i <= D.dict_n; i += 256)
+        if (sfirst[i]) atomicMax(D.first + i, sfirst[i]);
+    if (t == 0 && stotal) atomicAdd((unsigned long long*)D.total, (unsigned long long)stotal);
 }
 
-// PLAIN byte arrays (a 4-byte length, then the bytes) of the data pages, one thread per page:
-// pointer and length of each value by its index among the chunk's present values.  For the
-// dictionary page (dict != nullptr) the entries instead.
-__global__ void k_pq_byte_arrays(const PageDev* pages, int npages, const uint32_t* nvalues, const uint8_t** ptr,
-                                 uint32_t* len, const uint8_t* dict, uint32_t dict_len, uint32_t dict_n,
-                                 const uint8_t** dptr, uint32_t* dlen, uint32_t* err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// PLAIN byte arrays (a 4-byte length, then the bytes) of the data pages, one warp per page walking
+// the lengths in a staged window: pointer and length of each value by its index among the chunk's
+// present values.  For the dictionary page (dict != nullptr; the last block) the entries instead.
+__global__ void __launch_bounds__(32) k_pq_byte_arrays(const PageDev* pages, int npages, const uint32_t* nvalues, const uint8_t** ptr,
+                                                       uint32_t* len, const uint8_t* dict, uint32_t dict_len, uint32_t dict_n,
+                                                       const uint8_t** dptr, uint32_t* dlen, uint32_t* err) {
+    __shared__ uint4 win[kPqWindow / 16 + 1];
+    const int i = blockIdx.x, lane = threadIdx.x;
     const uint8_t* s;
     uint32_t n, slen;
     const uint8_t** op;
@@ -1115,7 +1289,7 @@ __global__ void k_pq_byte_arrays(const PageDev* pages, int npages, const uint32_
         n = nvalues[i];
         op = ptr + p.valid0;
         ol = len + p.valid0;
-    } else if (i == npages && dict) {
+    } else if (dict) {
         s = dict;
         slen = dict_len;
         n = dict_n;
@@ -1124,16 +1298,20 @@ __global__ void k_pq_byte_arrays(const PageDev* pages, int npages, const uint32_
     } else {
         return;
     }
+    StreamWindow S(s, slen, win);
     uint32_t pos = 0;
     for (uint32_t k = 0; k < n; k++) {
-        if (pos + 4 > slen || le32(s + pos) > slen - pos - 4) {
-            atomicOr(err, PQ_ERR_VALUES);
-            for (; k < n; k++) op[k] = s, ol[k] = 0;
+        S.need(pos, 4);
+        if ((uint64_t)pos + 4 > slen || S.at32(pos) > slen - pos - 4) {
+            if (lane == 0) atomicOr(err, PQ_ERR_VALUES);
+            for (k += lane; k < n; k += 32) op[k] = s, ol[k] = 0;
             return;
         }
-        const uint32_t l = le32(s + pos);
-        op[k] = s + pos + 4;
-        ol[k] = l;
+        const uint32_t l = S.at32(pos);
+        if (lane == 0) {
+            op[k] = s + pos + 4;
+            ol[k] = l;
+        }
         pos += 4 + l;
     }
 }
@@ -1150,10 +1328,13 @@ __global__ void k_pq_str_copy(const uint8_t* const* ptr, const uint32_t* len, co
         if (r == n - 1) off32[n] = (uint32_t)offs[n];
     }
 }
+// The words only fall: a row that reads a smaller one has nothing to do.
 __global__ void k_pq_first(const uint32_t* canon, int64_t n, uint32_t* first) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride)
-        atomicMin(first + canon[r], (uint32_t)r);
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
+        uint32_t* f = first + canon[r];
+        if (__ldcg(f) > (uint32_t)r) atomicMin(f, (uint32_t)r);
+    }
 }
 // bits: rows that are the first occurrence of their string; block counts for the compaction
 __global__ void k_pq_first_flags(const uint32_t* canon, const uint32_t* first, int64_t n, uint32_t* bits, uint32_t* counts,
@@ -1180,6 +1361,83 @@ __global__ void k_pq_codes(const uint32_t* list, uint32_t ndistinct, const uint3
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ndistinct; i += stride)
         code_of[canon[list[i]]] = (uint32_t)i;
+}
+// A small dictionary page's entries (and one more, the empty string of the NULL rows) in one block:
+// equal strings become one, ordered by first row; code_of[entry], and at `out` the number of
+// strings, their bytes, offsets [kPqSmallDict + 1] and the bytes themselves.  For a chunk of 125,000 rows
+// the rows' own path (copy the strings, hash every row, find first rows, compact) took 140 us of
+// kernels, two thirds of it on the few words that equal strings share; this kernel takes 4.5 us and the codes 3.3
+__global__ void __launch_bounds__(kPqSmallDict) k_pq_small_dict(const uint8_t* const* dptr, const uint32_t* dlen, uint32_t dict_n,
+                                                                const uint32_t* first, uint32_t* code_of, uint32_t* out) {
+    __shared__ uint32_t slots[2 * kPqSmallDict];  // entry + 1
+    __shared__ uint32_t sfirst[kPqSmallDict];     // ~(first row) of each kept string, 0 for the rest
+    __shared__ uint32_t order[kPqSmallDict], warps[32];
+    const uint32_t t = threadIdx.x;
+    slots[t] = slots[t + kPqSmallDict] = 0;
+    sfirst[t] = 0;
+    const uint32_t f = t <= dict_n ? first[t] : 0u;
+    const uint8_t* s = t < dict_n ? dptr[t] : nullptr;
+    const uint32_t n = t < dict_n ? dlen[t] : 0u;
+    __syncthreads();
+    uint32_t canon = t;
+    if (f) {
+        uint32_t q = (uint32_t)hash_bytes(s, n) & (2 * kPqSmallDict - 1);
+        for (uint32_t k = 0; k < 2 * kPqSmallDict; k++, q = (q + 1) & (2 * kPqSmallDict - 1)) {
+            const uint32_t c = atomicCAS(slots + q, 0u, t + 1);
+            if (c == 0) break;
+            const uint32_t o = c - 1, on = o < dict_n ? dlen[o] : 0u;
+            if (on == n && bytes_eq(o < dict_n ? dptr[o] : nullptr, s, n)) {
+                canon = o;
+                break;
+            }
+        }
+        atomicMax(sfirst + canon, f);
+    }
+    __syncthreads();
+    const bool kept = f && canon == t;
+    const uint32_t mine = sfirst[t];
+    uint32_t rank = 0;
+    if (kept)
+        for (uint32_t e = 0; e <= dict_n; e++) rank += sfirst[e] > mine;
+    const uint32_t distinct = __syncthreads_count(kept);
+    if (kept) {
+        order[rank] = t;
+        code_of[t] = rank;
+    }
+    __syncthreads();  // code_of of the kept entries is visible to the block
+    if (f && !kept) code_of[t] = code_of[canon];
+    // offsets of the strings in their order (at most 64 KB in all)
+    const uint32_t e = t < distinct ? order[t] : dict_n;
+    const uint32_t l = e < dict_n ? dlen[e] : 0u;
+    uint32_t x = l;
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(~0u, x, d);
+        if ((t & 31) >= (uint32_t)d) x += y;
+    }
+    if ((t & 31) == 31) warps[t >> 5] = x;
+    __syncthreads();
+    uint32_t base = 0;
+    for (uint32_t i = 0; i < (t >> 5); i++) base += warps[i];
+    const uint32_t o = base + x - l;
+    uint32_t* off = out + 2;
+    uint8_t* bytes = (uint8_t*)(off + kPqSmallDict + 1);
+    if (t == kPqSmallDict - 1) {
+        out[0] = distinct;
+        out[1] = off[kPqSmallDict] = base + x;
+    }
+    off[t] = o;
+    const uint8_t* src = e < dict_n ? dptr[e] : nullptr;
+    for (uint32_t i = 0; i < l; i++) bytes[o + i] = src[i];
+}
+// Each row's string from its dictionary entry.
+__global__ void k_pq_entry_strings(const uint32_t* ent, int64_t n, const uint8_t* const* dptr, const uint32_t* dlen, uint32_t dict_n,
+                                   const uint8_t** ptr, uint32_t* len) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
+        const uint32_t e = ent[r];
+        ptr[r] = e < dict_n ? dptr[e] : nullptr;
+        len[r] = e < dict_n ? dlen[e] : 0u;
+    }
 }
 __global__ void k_pq_codes2(const uint32_t* canon, int64_t n, const uint32_t* code_of, uint32_t* codes) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -1345,9 +1603,14 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
                 CK(cudaMemcpyAsync(up + uoff[i] + lv, dc + pg.payload + lv, (size_t)(pg.compressed - lv), cudaMemcpyDeviceToDevice, s));
         }
     }
-    DevBuf err(ctx, 16, nullptr);
-    CK(cudaMemsetAsync(err.get(), 0, 4, s));
+    // {error bits, -, present values, strings' bytes} and the first rows of a small dictionary's entries
+    DevBuf err(ctx, 32 + kPqSmallDict * 4, nullptr);
+    CK(cudaMemsetAsync(err.get(), 0, 32 + kPqSmallDict * 4, s));
     uint32_t* derr = err.get<uint32_t>();
+    uint64_t* dpresent = err.get<uint64_t>() + 1;
+    uint64_t* dtotal = err.get<uint64_t>() + 2;
+    uint32_t* dfirst = derr + 8;
+    PinnedSlot slot(ctx);
     DevBuf dj, splan, smap, sentry;  // the Snappy kernels': live to the end of the call
     if (!jobs.empty()) {
         // the jobs, the fragment and the block table in one upload
@@ -1387,11 +1650,10 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
             ctx->count_launch(2 + (g.nblks ? 2 : 0) + (g.nfrags ? 1 : 0));
         }
     }
-    auto read_err = [&]() {
-        uint32_t e = 0;
-        CK(cudaMemcpyAsync(&e, derr, 4, cudaMemcpyDeviceToHost, s));
+    auto read_err = [&]() {  // waits for the stream; slot: {error bits, -, present values, strings' bytes}
+        CK(cudaMemcpyAsync(slot.p, derr, 32, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        check_pq(ctx, e);
+        check_pq(ctx, *slot.as<uint32_t>());
     };
 
     // 2. data pages (the kernels are bounds-checked, so a decode error is read once, at the end;
@@ -1417,21 +1679,16 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
     PageDev* P = dpages.get<PageDev>();
     CK(cudaMemcpyAsync(P, hp.data(), hp.size() * sizeof(PageDev), cudaMemcpyHostToDevice, s));
     DevBuf lv_runs(ctx, (size_t)num_rows * sizeof(Run), nullptr), ix_runs(ctx, (size_t)num_rows * sizeof(Run), nullptr);
-    k_pq_layout<<<grid_of(np), 256, 0, s>>>(P, np, max_def, derr);
-    ctx->count_launch(2);
-    k_pq_runs<<<grid_of(np), 256, 0, s>>>(P, np, 0, level_width, nullptr, lv_runs.get<Run>(), derr);
+    k_pq_levels<<<np, 32, 0, s>>>(P, max_def, level_width, lv_runs.get<Run>(), derr);
     const int64_t ntiles = (num_rows + kPqTile - 1) / kPqTile;
     DevBuf valid(ctx, (size_t)ntiles * kPqTile / 8, b->res.get());  // u32 words; as u64 words the validity
     DevBuf tcounts(ctx, (size_t)ntiles * 4, nullptr), toffs(ctx, (size_t)(ntiles + 1) * 8, nullptr);
-    DevBuf scratch(ctx, std::max<size_t>(scan_scratch_words(ntiles) * 8, 8), nullptr);
     k_pq_valid<<<(int)ntiles, 256, 0, s>>>(P, np, lv_runs.get<Run>(), max_def, level_width, num_rows, valid.get<uint32_t>(),
                                            tcounts.get<uint32_t>());
-    launch_scan_u32(tcounts.get<uint32_t>(), toffs.get<uint64_t>(), ntiles, scratch.get<uint64_t>(), s);
+    k_pq_tile_scan<<<1, 1024, 0, s>>>(tcounts.get<uint32_t>(), ntiles, toffs.get<uint64_t>(), dpresent);
     DevBuf nvals(ctx, (size_t)np * 4 + 4, nullptr);
-    k_pq_page_valid<<<grid_of(np + 1), 256, 0, s>>>(P, np, valid.get<uint32_t>(), toffs.get<uint64_t>(), num_rows,
-                                                    nvals.get<uint32_t>());
-    k_pq_runs<<<grid_of(np), 256, 0, s>>>(P, np, 1, level_width, nvals.get<uint32_t>(), ix_runs.get<Run>(), derr);
-    ctx->count_launch(5);
+    k_pq_indices<<<np, 32, 0, s>>>(P, valid.get<uint32_t>(), toffs.get<uint64_t>(), num_rows, nvals.get<uint32_t>(), ix_runs.get<Run>(), derr);
+    ctx->count_launch(4);
 
     // 3. the dictionary page and PLAIN byte arrays
     DecodeArgs D{};
@@ -1459,7 +1716,7 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
         dlen = DevBuf(ctx, std::max<size_t>((size_t)D.dict_n * 4, 4), nullptr);
         vptr = DevBuf(ctx, (size_t)num_rows * 8, nullptr);  // present values <= rows
         vlen = DevBuf(ctx, (size_t)num_rows * 4, nullptr);
-        k_pq_byte_arrays<<<grid_of(np + 1), 256, 0, s>>>(
+        k_pq_byte_arrays<<<np + 1, 32, 0, s>>>(
             P, np, nvals.get<uint32_t>(), vptr.get<const uint8_t*>(), vlen.get<uint32_t>(), D.dict,
             dict_page >= 0 ? (uint32_t)pages[dict_page].uncompressed : 0u, D.dict_n, dptr.get<const uint8_t*>(),
             dlen.get<uint32_t>(), derr);
@@ -1471,27 +1728,74 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
     }
 
     // 4. values
-    DevBuf sptr, slen;
-    if (cv == CV_UTF8) {
+    DevBuf sptr, slen, ent;
+    // Strings whose pages all index one small dictionary page: its entries carry the work.  The bounds are
+    // what one block holds and copies; a larger dictionary has fewer rows per string, and the rows' own
+    // path spreads over the chip.
+    const bool small_dict = cv == CV_UTF8 && dict_page >= 0 && D.dict_n < kPqSmallDict &&
+                            (uint32_t)pages[dict_page].uncompressed <= kPqSmallDictBytes &&
+                            std::all_of(hp.begin(), hp.end(), [](const PageDev& d) { return d.encoding == ENC_RLE_DICTIONARY; });
+    auto string_rows = [&]() {
         sptr = DevBuf(ctx, (size_t)num_rows * 8, nullptr);
         slen = DevBuf(ctx, (size_t)num_rows * 4 + 4, nullptr);
+    };
+    if (small_dict) {
+        ent = DevBuf(ctx, (size_t)num_rows * 4, nullptr);
+        D.ent = ent.get<uint32_t>();
+        D.first = dfirst;
+        D.total = dtotal;
+    } else if (cv == CV_UTF8) {
+        string_rows();
         D.str_ptr = sptr.get<const uint8_t*>();
         D.str_len = slen.get<uint32_t>();
     } else {
         col->data = DevBuf(ctx, std::max<size_t>((size_t)num_rows * width_of(out_type), 8), b->res.get());
         D.out = col->data.get();
     }
-    k_pq_values<<<(int)ntiles, 256, 0, s>>>(D);
+    k_pq_values<<<(unsigned)((num_rows + kPqSlice - 1) / kPqSlice), 256, 0, s>>>(D);
     ctx->count_launch();
-    uint64_t present = 0;
-    CK(cudaMemcpyAsync(&present, toffs.get<uint64_t>() + ntiles, 8, cudaMemcpyDeviceToHost, s));
-    read_err();  // synchronizes: `present` is on the host
-    if (present != (uint64_t)num_rows) {  // validity only when a value is missing (read_all)
+    const uint64_t limit = std::min<uint64_t>(std::max<uint64_t>((uint64_t)num_rows / 8, 1), 65536);  // (n / 8).clamp(1, MAX_DICT)
+    bool encoded = false;
+    if (small_dict) {
+        const int64_t n = num_rows;
+        // one block's answer in one copy: {strings, bytes, offsets, the bytes (no more than the page holds)}
+        const size_t head = (2 + kPqSmallDict + 1) * 4, all = head + (size_t)pages[dict_page].uncompressed;
+        DevBuf code_of(ctx, kPqSmallDict * 4, nullptr), answer(ctx, all, nullptr);
+        DevBuf codes(ctx, (size_t)n * 4, b->res.get());
+        k_pq_small_dict<<<1, kPqSmallDict, 0, s>>>(D.dict_ptr, D.dict_len, D.dict_n, dfirst, code_of.get<uint32_t>(), answer.get<uint32_t>());
+        k_pq_codes2<<<grid_of(n), 256, 0, s>>>(ent.get<uint32_t>(), n, code_of.get<uint32_t>(), codes.get<uint32_t>());
+        ctx->count_launch(2);
+        std::vector<uint8_t> h(all);
+        CK(cudaMemcpyAsync(h.data(), answer.get(), all, cudaMemcpyDeviceToHost, s));
+        read_err();
+        uint32_t found[2];
+        std::memcpy(found, h.data(), 8);
+        if (slot.as<uint64_t>()[2] > 0xFFFFFFFFull) raise(ML_ERR_UNSUPPORTED, "parquet: a string column larger than 4 GiB");
+        if (found[0] <= limit) {
+            auto hd = std::make_shared<HostDict>();
+            hd->bytes.assign(h.begin() + head, h.begin() + head + found[1]);
+            std::vector<uint32_t> off(found[0] + 1);
+            std::memcpy(off.data(), h.data() + 8, off.size() * 4);
+            hd->off.insert(hd->off.end(), off.begin() + 1, off.end());
+            col->kind = CK_DICT;
+            col->data = std::move(codes);
+            col->dict = std::move(hd);
+            encoded = true;
+        } else {
+            string_rows();
+            k_pq_entry_strings<<<grid_of(n), 256, 0, s>>>(ent.get<uint32_t>(), n, D.dict_ptr, D.dict_len, D.dict_n,
+                                                          sptr.get<const uint8_t*>(), slen.get<uint32_t>());
+            ctx->count_launch();
+        }
+    } else {
+        read_err();
+    }
+    if (slot.as<uint64_t>()[1] != (uint64_t)num_rows) {  // validity only when a value is missing (read_all)
         col->validity = std::move(valid);
     }
 
     // 5. strings: encode_strings (parquet_reader.rs:176-212)
-    if (cv == CV_UTF8) {
+    if (cv == CV_UTF8 && !encoded) {
         const int64_t n = num_rows;
         DevBuf offs(ctx, (size_t)(n + 1) * 8, nullptr), sc(ctx, std::max<size_t>(scan_scratch_words(n) * 8, 8), nullptr);
         launch_scan_u32(slen.get<uint32_t>(), offs.get<uint64_t>(), n, sc.get<uint64_t>(), s);
@@ -1520,7 +1824,6 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
         CK(cudaMemcpyAsync(&distinct, boffs.get<uint64_t>() + nb, 8, cudaMemcpyDeviceToHost, s));
         ctx->count_launch(6);
         read_err();
-        const uint64_t limit = std::min<uint64_t>(std::max<uint64_t>((uint64_t)n / 8, 1), 65536);  // (n / 8).clamp(1, MAX_DICT)
         if (distinct <= limit) {
             // the first occurrences in row order are the dictionary; each row's code is its string's
             DevBuf list(ctx, (size_t)distinct * 4 + 4, nullptr), code_of(ctx, (size_t)n * 4, nullptr);
@@ -1530,18 +1833,23 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
             DevBuf codes(ctx, (size_t)n * 4, b->res.get());
             k_pq_codes2<<<grid_of(n), 256, 0, s>>>(canon.get<uint32_t>(), n, code_of.get<uint32_t>(), codes.get<uint32_t>());
             ctx->count_launch(3);
-            std::vector<uint32_t> hl(distinct), ho(n + 1);
-            if (distinct) CK(cudaMemcpyAsync(hl.data(), list.get(), distinct * 4, cudaMemcpyDeviceToHost, s));
-            CK(cudaMemcpyAsync(ho.data(), off32.get(), (size_t)(n + 1) * 4, cudaMemcpyDeviceToHost, s));
-            std::vector<uint8_t> hb(total);
-            if (total) CK(cudaMemcpyAsync(hb.data(), bytes.get(), total, cudaMemcpyDeviceToHost, s));
+            // the distinct strings alone to the host: {offsets, bytes}
+            const int64_t nd = (int64_t)distinct;
+            DevBuf dl(ctx, (size_t)nd * 4 + 4, nullptr), doff(ctx, (size_t)(nd + 1) * 8, nullptr);
+            DevBuf sc3(ctx, std::max<size_t>(scan_scratch_words(nd) * 8, 8), nullptr);
+            launch_utf8_lengths(off32.get<uint32_t>(), list.get<uint32_t>(), nd, dl.get<uint32_t>(), s);
+            launch_scan_u32(dl.get<uint32_t>(), doff.get<uint64_t>(), nd, sc3.get<uint64_t>(), s);
+            std::vector<uint64_t> ho(nd + 1);
+            CK(cudaMemcpyAsync(ho.data(), doff.get(), (size_t)(nd + 1) * 8, cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
             auto hd = std::make_shared<HostDict>();
-            for (uint64_t i = 0; i < distinct; i++) {
-                const uint32_t r = hl[i];
-                hd->bytes.insert(hd->bytes.end(), hb.begin() + ho[r], hb.begin() + ho[r + 1]);
-                hd->off.push_back((uint32_t)hd->bytes.size());
-            }
+            hd->bytes.resize(ho[nd]);
+            DevBuf db(ctx, std::max<size_t>(ho[nd], 1), nullptr);
+            launch_utf8_copy(off32.get<uint32_t>(), bytes.get<uint8_t>(), list.get<uint32_t>(), nd, doff.get<uint64_t>(), db.get<uint8_t>(), s);
+            if (ho[nd]) CK(cudaMemcpyAsync(hd->bytes.data(), db.get(), ho[nd], cudaMemcpyDeviceToHost, s));
+            ctx->count_launch(3);
+            CK(cudaStreamSynchronize(s));
+            for (int64_t i = 1; i <= nd; i++) hd->off.push_back((uint32_t)ho[i]);
             col->kind = CK_DICT;
             col->data = std::move(codes);
             col->dict = std::move(hd);
@@ -1551,8 +1859,7 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
             col->data = std::move(bytes);
         }
     }
-    CK(cudaStreamSynchronize(s));
-    read_err();
+    if (cv == CV_UTF8 && !encoded) read_err();
     b->cols.push_back(std::move(col));
     *out = b.release();
     API_END
