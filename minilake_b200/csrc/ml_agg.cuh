@@ -103,9 +103,9 @@ __device__ __forceinline__ uint32_t new_group(const AggArgs& A) {
 // through them together, and the lanes step together instead of splitting into groups that issue the
 // same code one after another.  The claims of one step take their group ids with one atomic: every
 // insertion counts on the same word, which L2 serves one access after the other.
-// 4.7M rows with 1.4M new groups: 1,960 us row by row with an atomic and a release per insertion, 780 us
-// so; 14.8M rows with 0.15M new groups 2,530 us and 1,400 us (its accumulators, 8 words a group, then miss
-// L2: 2.8 GB read and 1.2 GB written).
+// 4.7M rows with 1.4M new groups and eight words a group: 1,960 us row by row with an atomic and a release
+// per insertion, 780 us so (640 us with six words); 14.8M rows with 0.15M new groups 2,530 us and 1,400 us
+// (six words 990 us): the table and its accumulators miss L2, 2.1 GB read and 0.6 GB written.
 template <int K>
 __device__ __forceinline__ uint32_t warp_upsert(const AggArgs& A, bool (&need)[K], const uint64_t (&w)[K][2],
                                                 const uint32_t (&nm)[K], const uint64_t (&h)[K], uint32_t (&g)[K], bool& full,

@@ -154,7 +154,7 @@ struct AggDev {
     int32_t has_arg;
     int32_t off;          // word offset inside the group block
     int32_t count_valid;  // maintain vcnt (valid-input counter) in this launch
-    int32_t pad;
+    int32_t cnt_off;      // final values: the block's word that counts the argument's valid inputs (0: the rows)
     Prog arg;
     uint64_t* vcnt;       // valid-input counts by group (seen-tracking for SUM/MIN/MAX)
 };

@@ -395,7 +395,7 @@ __global__ void k_agg_final(const __grid_constant__ FinalArgs F) {
         bool valid = false;
         if (in) {
             uint64_t rows = blk[0];
-            uint64_t vc = a.vcnt ? a.vcnt[g] : rows;
+            uint64_t vc = a.vcnt ? a.vcnt[g] : blk[a.cnt_off];
             if (a.func == ML_AGG_COUNT_STAR) {
                 ((int64_t*)F.agg_out[k])[o] = (int64_t)rows;
                 valid = true;
