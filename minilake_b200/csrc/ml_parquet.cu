@@ -203,7 +203,8 @@ constexpr int kPqTile = 8192;  // rows per decode tile: 256 threads x one 32-row
 // its input and no match reaches back past its fragment's start, so a page of N fragments is N
 // independent decodes once their starts in the stream are known.
 //
-// No pass follows the chain of elements one by one:
+// A page of few elements is copied by one block (k_pq_snappy_flat).  For any other page no pass follows
+// the chain of elements one by one:
 //  * the maps (one block per kSnapBlk stream bytes): for every byte, the element that WOULD start
 //    there is parsed, and pointer doubling in shared memory (log2 of the elements in a block rounds)
 //    gives where the chain from that byte leaves the block, how many elements it passes and how many
@@ -254,8 +255,8 @@ constexpr int kSnapThreads = 1024;
 constexpr uint32_t kSnapPer = kSnapBlk / kSnapThreads;
 constexpr uint32_t kSnapNone = 0xFFFFFFFFu;
 // plan modes: 0 the length varint is malformed, 1 the serial pass decodes the page, 2 its
-// fragments decode in parallel
-constexpr uint32_t kSnapSerial = 1, kSnapSplit = 2;
+// fragments decode in parallel, 3 it is decoded, 4 undecided
+constexpr uint32_t kSnapSerial = 1, kSnapSplit = 2, kSnapDone = 3, kSnapOpen = 4;
 constexpr uint32_t kSnapPiece = 2048, kSnapPieces = 2048;  // long literals, cut into pieces for the warps
 constexpr size_t kSnapMapSmem = kSnapBlk * 8 + kSnapBlk + 32;
 constexpr size_t kSnapFragSmem = kSnapFrag * 3 + kSnapPieces * 8;
@@ -327,17 +328,99 @@ __device__ __forceinline__ uint32_t snap_window(const SnapJob& J, uint32_t b0, u
     return lead;
 }
 
+// Eight bytes from any address (in the padded chunk or page buffer: the aligned words around them
+// are readable).
+__device__ uint64_t load8(const uint8_t* p) {
+    const uint64_t* b = (const uint64_t*)((uintptr_t)p & ~(uintptr_t)7);
+    const int sh = 8 * (int)((uintptr_t)p & 7);
+    const uint64_t lo = b[0];
+    return sh ? (lo >> sh) | (b[1] << (64 - sh)) : lo;
+}
+
+// Pages of few elements, one block per page: pages that do not compress (bit-packed random indices,
+// random numbers) are a few long literals, perhaps with a stray copy.  One thread follows the elements as
+// long as they span kSnapFlatSpan stream bytes on average, at most kSnapFlat of them; if that is the whole page, the
+// block copies the literals, then one warp the copies in order, and the passes below leave the page alone.
+// Bound by the element headers' latency (0.6 us each): seven pages of 18,000 two-bit indices 4.8 us, and 16 us
+// for the passes below to find nothing to do; they took 55 us to decode them (maps 11, chain 3, list 12, decode 16 and launches).
+constexpr int kSnapFlat = 64;
+constexpr uint32_t kSnapFlatSpan = 256;
+__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_flat(const SnapJob* jobs, uint32_t* plan) {
+    __shared__ uint4 el[kSnapFlat];  // {stream position of a literal's bytes, output position, length, copy offset (0: literal)}
+    __shared__ int count;
+    const SnapJob J = jobs[blockIdx.x];
+    const uint32_t tid = threadIdx.x;
+    if (tid == 0) {
+        uint32_t pos = 0, total = 0;
+        bool ok = false;
+        for (int shift = 0; shift < 35 && pos < J.src_len; shift += 7) {  // the uncompressed length
+            const uint32_t b = J.src[pos++];
+            if (shift == 28 && (b & 0x70)) break;  // past 32 bits
+            total |= (b & 0x7F) << shift;
+            if (!(b & 0x80)) {
+                ok = total == J.dst_len;
+                break;
+            }
+        }
+        const uint32_t start = pos;
+        uint32_t out = 0;
+        int n = 0;
+        while (ok && pos < J.src_len) {
+            const uint8_t* e = J.src + pos;  // five readable bytes: the chunk buffer is padded past its end
+            uint32_t step, len;
+            ok = n < kSnapFlat && (n < 2 || pos - start >= n * kSnapFlatSpan) && snap_elem(e, J.src_len - pos, step, len) &&
+                 len <= J.dst_len - out;
+            if (!ok) break;
+            const uint32_t t = e[0] & 3;
+            const uint32_t off = t == 0 ? 0u
+                                 : t == 1 ? ((uint32_t)(e[0] >> 5) << 8) | e[1]
+                                          : e[1] | ((uint32_t)e[2] << 8) | (t == 3 ? ((uint32_t)e[3] << 16) | ((uint32_t)e[4] << 24) : 0u);
+            ok = t == 0 || (off != 0 && off <= out);
+            el[n++] = make_uint4(pos + step - len, out, len, off);
+            pos += step;
+            out += len;
+        }
+        ok = ok && out == J.dst_len;
+        count = ok ? n : -1;
+        plan[J.plan] = ok ? kSnapDone : kSnapOpen;
+    }
+    __syncthreads();
+    const int n = count;
+    if (n < 0) return;
+    for (int k = 0; k < n; k++) {
+        const uint4 e = el[k];
+        if (e.w) continue;
+        const uint8_t* src = J.src + e.x;
+        uint8_t* d = J.dst + e.y;
+        const uint32_t lead = min((uint32_t)((8 - ((uintptr_t)d & 7)) & 7), e.z), words = (e.z - lead) / 8;
+        for (uint32_t i = tid; i < words; i += kSnapThreads) ((uint64_t*)(d + lead))[i] = load8(src + lead + 8ull * i);
+        const uint32_t tail = lead + words * 8;
+        if (tid < lead) d[tid] = src[tid];
+        else if (tid >= 32 && tail + tid - 32 < e.z) d[tail + tid - 32] = src[tail + tid - 32];
+    }
+    __syncthreads();
+    if (tid >= 32) return;
+    for (int k = 0; k < n; k++) {
+        const uint4 e = el[k];
+        if (!e.w) continue;
+        for (uint32_t i = tid; i < e.z; i += 32) J.dst[e.y + i] = J.dst[e.y - e.w + i % e.w];  // a copy over itself repeats
+        __syncwarp();
+    }
+}
+
 // The maps: blocks[i] = {page, block}.  A byte's state packs the element reached (16 bits, a block
 // offset), the elements passed (16) and the bytes they write (32); an element whose successor lies
 // past the block (or that does not parse) points to itself.  States only ever move further along the
 // chain and are read and written whole, so the rounds need no second buffer: bound by shared-memory
 // round trips, log2(kSnapBlk / 2) of them.
-__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_maps(const SnapJob* jobs, const uint2* blocks, SnapMap* tab) {
+__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_maps(const SnapJob* jobs, const uint2* blocks, const uint32_t* plan,
+                                                                 SnapMap* tab) {
     extern __shared__ __align__(16) uint8_t snap_smem[];
     uint64_t* st = (uint64_t*)snap_smem;
     uint8_t* win = snap_smem + kSnapBlk * 8;
     const uint2 f = blocks[blockIdx.x];
     const SnapJob J = jobs[f.x];
+    if (plan[J.plan] == kSnapDone) return;
     const uint32_t b0 = f.y * kSnapBlk, blen = min(kSnapBlk, J.src_len - b0);
     const uint8_t* w = win + snap_window(J, b0, win);
     __syncthreads();
@@ -385,6 +468,7 @@ __global__ void __launch_bounds__(32) k_pq_snappy_chain(const SnapJob* jobs, con
     if (threadIdx.x) return;
     const SnapJob J = jobs[blockIdx.x];
     uint32_t* pl = plan + J.plan;
+    if (pl[0] == kSnapDone) return;
     uint32_t start = 0, total = 0;
     bool ok = false;
     for (int shift = 0; shift < 35 && start < J.src_len; shift += 7) {  // the uncompressed length
@@ -685,7 +769,7 @@ __global__ void __launch_bounds__(32) k_pq_snappy_serial(const SnapJob* jobs, co
     const SnapJob J = jobs[blockIdx.x];
     const uint32_t* pl = plan + J.plan;
     const uint32_t mode = pl[0];
-    if (mode == kSnapSplit) return;
+    if (mode == kSnapSplit || mode == kSnapDone) return;
     SnapSrc S{J.src, J.src_len, win};
     if (mode != kSnapSerial || !snap_decode_serial(S, pl[1], J.src_len, J.dst, J.dst_len)) atomicOr(err, PQ_ERR_SNAPPY);
 }
@@ -922,15 +1006,6 @@ __global__ void __launch_bounds__(32) k_pq_indices(PageDev* pages, const uint32_
         nvalues[blockIdx.x] = (uint32_t)(v1 - v0);
     }
     page_runs(p.values, p.values_len, (uint32_t)(v1 - v0), p.idx_width, runs + p.ix_run0, p.ix_nruns, win, err);
-}
-
-// Eight bytes from any address (streams lie in the padded page buffer: the aligned words around
-// them are readable).
-__device__ uint64_t load8(const uint8_t* p) {
-    const uint64_t* b = (const uint64_t*)((uintptr_t)p & ~(uintptr_t)7);
-    const int sh = 8 * (int)((uintptr_t)p & 7);
-    const uint64_t lo = b[0];
-    return sh ? (lo >> sh) | (b[1] << (64 - sh)) : lo;
 }
 
 // The run that holds value k (k < the stream's value count).
@@ -1636,9 +1711,10 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
         CK(cudaFuncSetAttribute(k_pq_snappy_maps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSnapMapSmem));
         CK(cudaFuncSetAttribute(k_pq_snappy_frag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSnapFragSmem));
         for (const SnapGroup& g : groups) {
+            k_pq_snappy_flat<<<g.njobs, kSnapThreads, 0, s>>>(J + g.job0, splan.get<uint32_t>());
             if (g.nblks) {
                 CK(cudaMemsetAsync(sentry.get(), 0, (size_t)g.nblks * sizeof(SnapEntry), s));
-                k_pq_snappy_maps<<<g.nblks, kSnapThreads, kSnapMapSmem, s>>>(J, B + g.blk0, smap.get<SnapMap>());
+                k_pq_snappy_maps<<<g.nblks, kSnapThreads, kSnapMapSmem, s>>>(J, B + g.blk0, splan.get<uint32_t>(), smap.get<SnapMap>());
             }
             k_pq_snappy_chain<<<g.njobs, 32, 0, s>>>(J + g.job0, smap.get<SnapMap>(), sentry.get<SnapEntry>(), splan.get<uint32_t>());
             if (g.nblks)
@@ -1647,7 +1723,7 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
             if (g.nfrags)
                 k_pq_snappy_frag<<<g.nfrags, kSnapThreads, kSnapFragSmem, s>>>(J, F + g.frag0, smap.get<uint2>(), splan.get<uint32_t>());
             k_pq_snappy_serial<<<g.njobs, 32, 0, s>>>(J + g.job0, splan.get<uint32_t>(), derr);
-            ctx->count_launch(2 + (g.nblks ? 2 : 0) + (g.nfrags ? 1 : 0));
+            ctx->count_launch(3 + (g.nblks ? 2 : 0) + (g.nfrags ? 1 : 0));
         }
     }
     auto read_err = [&]() {  // waits for the stream; slot: {error bits, -, present values, strings' bytes}
