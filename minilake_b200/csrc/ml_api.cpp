@@ -3462,6 +3462,9 @@ struct ml_query {
     void* jit = nullptr;
     int grid = 0, smem = 0;
     DevBuf tables, ovf, count, guard, ng, gids, bits, counts, offs, scratch, tbuf;
+    static constexpr int kBoundTopNBlocks = 32;
+    DevBuf best;  // launch_group_bound's, when the top-N's first key is an aggregate of a large group table
+    GroupKey best_key{};
     std::vector<std::unique_ptr<DevColumn>> outcols, rescols;
     FinalArgs F{};
     uint32_t* hguard = nullptr;  // pinned readbacks
@@ -3599,8 +3602,16 @@ void query_enqueue(ml_query* q) {
     if (h->group_probe >= 0) {  // GROUP BY the join key: the groups are matched build rows
         const ml_join_table* jt = h->pipe.probes[h->group_probe].jt;
         const int nb = select_blocks(q->cap);
-        launch_group_flags(h->acc.get<uint64_t>(), h->stride, q->cap, h->dense_groups ? jt->dense.get<uint32_t>() : nullptr,
-                           q->bits.get<uint32_t>(), q->counts.get<uint32_t>(), s);
+        const uint32_t* member = h->dense_groups ? jt->dense.get<uint32_t>() : nullptr;
+        const GroupKey* key = q->best ? &q->best_key : nullptr;
+        const uint64_t* bound = nullptr;
+        if (key) {
+            bound = launch_group_bound(h->acc.get<uint64_t>(), h->stride, q->cap, member, *key, (int)q->k,
+                                       group_bound_blocks(q->cap, q->k), q->best.get<uint64_t>(), s);
+            nk += 2;
+        }
+        launch_group_flags(h->acc.get<uint64_t>(), h->stride, q->cap, member, q->bits.get<uint32_t>(), q->counts.get<uint32_t>(), s,
+                           key, bound);
         launch_scan_u32(q->counts.get<uint32_t>(), q->offs.get<uint64_t>(), nb, q->scratch.get<uint64_t>(), s);
         nk += 4;
         if (!h->dense_groups)  // the key gathers read every position: past the groups, build row 0
@@ -3631,7 +3642,9 @@ void query_enqueue(ml_query* q) {
     nk++;
     // 4. the top-N (sort.rs:117-122) and the result's read-back
     if (q->topn) {
-        const int nb = topn_warp_blocks(q->cap);
+        // behind a bound few groups are left: fewer lists to merge (and a table that ties throughout still
+        // has this many blocks for it)
+        const int nb = q->best ? std::min(topn_warp_blocks(q->cap), q->kBoundTopNBlocks) : topn_warp_blocks(q->cap);
         const size_t rows_b = ((size_t)nb * q->k * 4 + 15) & ~(size_t)15, cand_b = (size_t)nb * q->k * topn_entry_bytes();
         uint8_t* base = q->tbuf.get<uint8_t>();
         uint32_t* rows = nullptr;
@@ -3806,6 +3819,16 @@ void query_capture(ml_query* q) {
             const int c = (int)kk.expr.index;
             if (c < 0 || c >= (int)q->outcols.size() || q->outcols[c]->dtype != kk.type)
                 raise(ML_ERR_INVALID, "a sort key does not name an output column of its type");
+        }
+        // Only with exactly `limit` rows in the plan: a shorter result has to be told from a longer one by
+        // the number of all groups.
+        q->best.release();
+        const int agg = (int)q->keys[0].expr.index - (int)(q->outcols.size() - F.nagg);
+        const int bnb = h->group_probe >= 0 && agg >= 0 && q->k == q->limit ? group_bound_blocks(q->cap, q->k) : 0;
+        if (bnb && F.aggs[agg].kind != A_MIN_STR && F.aggs[agg].kind != A_MAX_STR) {
+            const AggDev& a = F.aggs[agg];
+            q->best = DevBuf(ctx, (size_t)(bnb + 1) * 8, nullptr);
+            q->best_key = GroupKey{a.kind, a.func, a.off, a.cnt_off, F.out_type[agg], q->keys[0].asc, q->keys[0].nulls_first, 0, a.vcnt};
         }
         const int nb = topn_warp_blocks(q->cap);
         const size_t rows_b = ((size_t)nb * q->k * 4 + 15) & ~(size_t)15, cand_b = (size_t)nb * q->k * topn_entry_bytes();

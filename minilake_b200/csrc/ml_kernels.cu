@@ -515,14 +515,86 @@ __global__ void __launch_bounds__(kThreads) k_index_write(int64_t n, const uint3
     }
 }
 
+// The first sort key of group g (FinalArgs' value of an aggregate that is no string) as sort_prefix orders
+// it: the group with the smallest prefix comes first.
+__device__ __forceinline__ uint64_t group_prefix(const GroupKey& K, const uint64_t* blk, uint64_t g) {
+    uint64_t x;
+    bool valid = true;
+    if (K.func == ML_AGG_COUNT_STAR) {
+        x = blk[0];
+    } else if (K.func == ML_AGG_COUNT) {
+        x = blk[K.off];
+    } else if (K.kind == A_AVG) {
+        const uint64_t c = blk[K.off + 1];
+        valid = c > 0;
+        x = f64_bits(__ddiv_rn(as_f64(blk[K.off]), __ll2double_rn((long long)c)));
+    } else {
+        valid = (K.vcnt ? K.vcnt[g] : blk[K.cnt_off]) > 0;
+        x = blk[K.off];
+        if (K.kind == A_MIN_F64 || K.kind == A_MAX_F64) x = f64_bits(f64_unorder(x));
+        else if (K.dt == ML_TYPE_INT32 || K.dt == ML_TYPE_DATE) x = (uint64_t)(int64_t)(int32_t)(uint32_t)x;
+    }
+    if (!valid) return K.nulls_first ? 0ull : ~0ull;
+    const uint64_t p = (K.dt == ML_TYPE_FLOAT64 ? (uint64_t)total_key(as_f64(x)) : x) ^ 0x8000000000000000ull;
+    return K.asc ? p : ~p;
+}
+
+// A bound that at least k groups' prefixes reach, for a top-N over a group table: the k-th smallest of the
+// blocks' smallest prefixes (each belongs to another group).  With it only a few times k groups are flagged,
+// and the index, the keys, the final values and the top-N after it touch those alone.  1.5M groups, k = 10:
+// the kernels after the aggregate 118 -> 66 us, of which this pass over the table takes 13
+// and the bound 4.5.
+__global__ void __launch_bounds__(1024) k_group_best(const uint64_t* acc, int stride, int64_t n, const uint32_t* member,
+                                                         const __grid_constant__ GroupKey K, uint64_t* best) {
+    const int64_t step = (int64_t)gridDim.x * 1024;
+    uint64_t m = ~0ull;
+#pragma unroll 4
+    for (int64_t i = (int64_t)blockIdx.x * 1024 + threadIdx.x; i < n; i += step) {
+        const uint64_t* blk = acc + i * stride;
+        const uint64_t p = group_prefix(K, blk, (uint64_t)i);
+        if (blk[0] != 0 && (member == nullptr || member[i] != kNone) && p < m) m = p;
+    }
+    __shared__ uint64_t red[32];
+    auto smallest = [](uint64_t x) {
+        for (int o = 16; o; o >>= 1) {
+            const uint64_t y = __shfl_xor_sync(0xFFFFFFFFu, x, o);
+            x = y < x ? y : x;
+        }
+        return x;
+    };
+    m = smallest(m);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        m = smallest(red[threadIdx.x]);
+        if (threadIdx.x == 0) best[blockIdx.x] = m;
+    }
+}
+// best[nb] = the k-th smallest of best[0..nb) (nb <= 256)
+__global__ void __launch_bounds__(256) k_group_bound(uint64_t* best, int nb, int k) {
+    __shared__ uint64_t v[256];
+    const int i = threadIdx.x;
+    if (i < nb) v[i] = best[i];
+    __syncthreads();
+    if (i >= nb) return;
+    int place = 0;
+    for (int j = 0; j < nb; j++) place += v[j] < v[i] || (v[j] == v[i] && j < i);
+    if (place == k - 1) best[nb] = v[i];
+}
+
+// Groups with rows (and, with a bound, a prefix that reaches it): bits and block counts.
 __global__ void __launch_bounds__(kThreads) k_group_flags(const uint64_t* acc, int stride, int64_t n,
                                                           const uint32_t* member, uint32_t* bits,
-                                                          uint32_t* block_counts) {
+                                                          uint32_t* block_counts, const __grid_constant__ GroupKey K,
+                                                          const uint64_t* bound) {
     int64_t base = (int64_t)blockIdx.x * kSelRowsPerBlock;
     uint32_t cnt = 0;
+    const uint64_t limit = bound ? *bound : 0ull;
+#pragma unroll
     for (int it = 0; it < 8; it++) {
         int64_t i = base + it * kThreads + threadIdx.x;
         bool pass = i < n && acc[i * stride] != 0 && (member == nullptr || member[i] != kNone);
+        if (bound) pass = pass && group_prefix(K, acc + i * stride, (uint64_t)i) <= limit;
         uint32_t b = __ballot_sync(0xFFFFFFFFu, pass);
         if ((threadIdx.x & 31) == 0 && base + it * kThreads + (threadIdx.x & ~31) < n) bits[(base + it * kThreads + threadIdx.x) >> 5] = b;
         cnt += pass;
@@ -1285,6 +1357,27 @@ __device__ TopEntry warp_topk_fixed(const SortDev& S, int64_t n, int k, int64_t 
     return best;
 }
 
+// The block puts up to blockDim.x rows in order: out[place] = row for the first k places.
+__device__ __forceinline__ void place_rows(const SortDev& S, uint64_t* pre, int n, int k, uint32_t* out) {
+    const int i = threadIdx.x;
+    if (i < n) pre[i] = sort_prefix(S, (uint32_t)i);
+    __syncthreads();
+    if (i >= n) return;
+    const uint64_t p = pre[i];
+    int place = 0;
+#pragma unroll 1
+    for (int j = 0; j < n; j++) {
+        const uint64_t q = pre[j];
+        int before = q < p ? 1 : 0;
+        if (q == p && j != i) {  // equal keys keep their input order
+            const int c = cmp_rows(S, (uint32_t)j, (uint32_t)i);
+            before = c < 0 || (c == 0 && j < i);
+        }
+        place += before;
+    }
+    if (place < k) out[place] = (uint32_t)i;
+}
+
 // Each CTA writes its best k rows to out[block * k ..].  With `final_out`, CTAs also write
 // their (prefix, row) entries to `cand`, and the last CTA to finish (the counter `done` starts
 // at zero) merges all CTAs' entries into final_out[0 .. k): the whole top-k in one launch.
@@ -1294,6 +1387,15 @@ __global__ void __launch_bounds__(256, 2) k_topn_warp(const __grid_constant__ So
                                                    TopEntry* cand, unsigned int* done, uint32_t* final_out,
                                                    const uint64_t* n_dev) {
     if (n_dev) n = min(n, (int64_t)__ldcg(n_dev));  // a replayed plan's row count
+    if (n_dev && n <= 256) {
+        // few rows after all (groups behind a bound): one CTA places each row by the rows before it.  The
+        // lists' merges, a chain of 14 sorts, took 27 us for 20 rows; this takes 3.9.
+        if (blockIdx.x) return;
+        __shared__ uint64_t pre[256];
+        place_rows(S, pre, (int)n, k, final_out ? final_out : out);
+        if ((int)threadIdx.x >= n && (int)threadIdx.x < k) (final_out ? final_out : out)[threadIdx.x] = kNone;
+        return;
+    }
     __shared__ TopEntry lists[8][32];
     __shared__ TopEntry queue[8][kTopNQueue];
     __shared__ bool last;
@@ -1379,23 +1481,7 @@ __global__ void __launch_bounds__(256, 2) k_topn_warp(const __grid_constant__ So
 // per-warp lists and their merges took 22 us for six groups ordered by two strings, 5 us so.)
 __global__ void __launch_bounds__(kTopNTiny) k_topn_tiny(const __grid_constant__ SortDev S, int n, int k, uint32_t* out) {
     __shared__ uint64_t pre[kTopNTiny];
-    const int i = threadIdx.x;
-    if (i < n) pre[i] = sort_prefix(S, (uint32_t)i);
-    __syncthreads();
-    if (i >= n) return;
-    const uint64_t p = pre[i];
-    int place = 0;
-#pragma unroll 1
-    for (int j = 0; j < n; j++) {
-        const uint64_t q = pre[j];
-        int before = q < p ? 1 : 0;
-        if (q == p && j != i) {  // equal keys keep their input order
-            const int c = cmp_rows(S, (uint32_t)j, (uint32_t)i);
-            before = c < 0 || (c == 0 && j < i);
-        }
-        place += before;
-    }
-    if (place < k) out[place] = (uint32_t)i;
+    place_rows(S, pre, n, k, out);
 }
 
 // Rows idx[0..k) of every column of a batch, a block per column (k <= 1,024): values, validity words and,
@@ -1763,9 +1849,21 @@ void launch_dense_keys(const uint32_t* gids, int64_t n, uint64_t dmin, int dt, v
     if (n) k_dense_keys<<<grid_for(n, 8), kThreads, 0, s>>>(gids, n, n_dev, dmin, dt, out);
 }
 void launch_group_flags(const uint64_t* acc, int stride, int64_t n, const uint32_t* member, uint32_t* bits,
-                        uint32_t* block_counts, cudaStream_t s) {
+                        uint32_t* block_counts, cudaStream_t s, const GroupKey* key, const uint64_t* bound) {
     int nb = select_blocks(n);
-    if (nb) k_group_flags<<<nb, kThreads, 0, s>>>(acc, stride, n, member, bits, block_counts);
+    if (nb) k_group_flags<<<nb, kThreads, 0, s>>>(acc, stride, n, member, bits, block_counts, key ? *key : GroupKey{}, bound);
+}
+// From 256 groups per block on (38,000: below that all groups' own kernels take less than the bound's 18 us), and
+// k at most a quarter of the blocks: more, and the k-th of the blocks' best groups lies well below the k-th best.
+int group_bound_blocks(int64_t n, int64_t k) {
+    const int nb = std::min(num_sms(), 256);
+    return k >= 1 && k * 4 <= nb && n >= 256 * (int64_t)nb ? nb : 0;
+}
+const uint64_t* launch_group_bound(const uint64_t* acc, int stride, int64_t n, const uint32_t* member, const GroupKey& key, int k, int nb,
+                                   uint64_t* best, cudaStream_t s) {
+    k_group_best<<<nb, 1024, 0, s>>>(acc, stride, n, member, key, best);
+    k_group_bound<<<1, 256, 0, s>>>(best, nb, k);
+    return best + nb;
 }
 void launch_count_slots(TableView t, unsigned long long* out, cudaStream_t s) {
     k_count_slots<<<grid_for((int64_t)t.mask + 1, 8), kThreads, 0, s>>>(t, out);

@@ -59,6 +59,11 @@ struct FinalArgs {
     const uint64_t* ng64;
     const uint32_t* ng32;
 };
+// An aggregate as the first sort key of a top-N over the group table (group_prefix).
+struct GroupKey {
+    int32_t kind, func, off, cnt_off, dt, asc, nulls_first, pad;
+    const uint64_t* vcnt;
+};
 void launch_agg_final(const FinalArgs& F, cudaStream_t s);
 
 // Filter: pass bits (u32 words) + per-block counts, then ordered compaction.
@@ -74,7 +79,13 @@ void launch_pairs_write(const PipeArgs& P, const uint32_t* bits, const uint64_t*
 // there is not kNone: pass bits + per-block counts; then launch_index_write turns bits into
 // the ordered list of group ids.
 void launch_group_flags(const uint64_t* acc, int stride, int64_t n, const uint32_t* member, uint32_t* bits,
-                        uint32_t* block_counts, cudaStream_t s);
+                        uint32_t* block_counts, cudaStream_t s, const GroupKey* key = nullptr, const uint64_t* bound = nullptr);
+// A bound on the first sort key that at least k groups reach (k_group_best), in best[nb]; nb from
+// group_bound_blocks, 0 when the table is too small for it to pay, or k too large for the blocks' best groups
+// to bound it closely.
+int group_bound_blocks(int64_t n, int64_t k);
+const uint64_t* launch_group_bound(const uint64_t* acc, int stride, int64_t n, const uint32_t* member, const GroupKey& key, int k, int nb,
+                                   uint64_t* best, cudaStream_t s);
 // Key values of dense-index groups: out[i] = dmin + gids[i] as int64, or as int32 / date.
 // n_dev (optional): the device-side count of gids (at most n)
 void launch_dense_keys(const uint32_t* gids, int64_t n, uint64_t dmin, int dt, void* out, cudaStream_t s,
