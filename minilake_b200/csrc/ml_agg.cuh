@@ -101,11 +101,12 @@ __device__ __forceinline__ uint32_t new_group(const AggArgs& A) {
 //
 // Bound by the latency of its dependent accesses (slot, claim, group id), so the keys of a lane are taken
 // through them together, and the lanes step together instead of splitting into groups that issue the
-// same code one after another.  The claims of one step take their group ids with one atomic: every
-// insertion counts on the same word, which L2 serves one access after the other.
+// same code one after another.  The warp's claims take their group ids with one atomic, once every key is
+// resolved or one has to wait: every insertion counts on the same word, which L2 serves one access after
+// the other (an atomic per step: 640 and 990 us for the two cases below).
 // 4.7M rows with 1.4M new groups and eight words a group: 1,960 us row by row with an atomic and a release
-// per insertion, 780 us so (640 us with six words); 14.8M rows with 0.15M new groups 2,530 us and 1,400 us
-// (six words 990 us): the table and its accumulators miss L2, 2.1 GB read and 0.6 GB written.
+// per insertion, 780 us so (570 us with six words); 14.8M rows with 0.15M new groups 2,530 us and 1,400 us
+// (six words 940 us): the table and its accumulators miss L2, 2.1 GB read and 0.6 GB written.
 template <int K>
 __device__ __forceinline__ uint32_t warp_upsert(const AggArgs& A, bool (&need)[K], const uint64_t (&w)[K][2],
                                                 const uint32_t (&nm)[K], const uint64_t (&h)[K], uint32_t (&g)[K], bool& full,
@@ -115,7 +116,7 @@ __device__ __forceinline__ uint32_t warp_upsert(const AggArgs& A, bool (&need)[K
     const int lane = threadIdx.x & 31;
     uint64_t i[K];
     ulonglong2 v[K];
-    uint32_t made = 0, steps = 0, spins = 0;
+    uint32_t made = 0, steps = 0, spins = 0, claimed = 0;
     bool any = false;
 #pragma unroll
     for (int k = 0; k < K; k++) {
@@ -123,6 +124,42 @@ __device__ __forceinline__ uint32_t warp_upsert(const AggArgs& A, bool (&need)[K
         g[k] = kNone;
         any = any || need[k];
     }
+    // the warp's claims take their ids, with one atomic, and are published
+    auto publish = [&] {
+        unsigned m[K];
+        uint32_t total = 0;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            m[k] = __ballot_sync(0xFFFFFFFFu, (claimed >> k) & 1u);
+            total += __popc(m[k]);
+        }
+        uint32_t id = 0;
+        if (lane == 0) id = atomicAdd(A.ngroups, total);
+        id = __shfl_sync(0xFFFFFFFFu, id, 0);
+        full = id + total > A.gid_cap || id + total < id;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            if ((claimed >> k) & 1u) {
+                const uint32_t mine = id + __popc(m[k] & ((1u << lane) - 1u));
+                uint64_t* s = slot_at(t, i[k]);
+                const uint64_t x = (2u | (nm[k] << 8)) | ((uint64_t)mine << 32);
+                if (mine >= A.gid_cap) {
+                    publish_state((uint32_t*)s, 0);
+                } else {
+                    if (wide) {
+                        s[2] = w[k][1];
+                        st_slot_release(s, x, w[k][0]);
+                    } else {
+                        st_slot(s, x, w[k][0]);
+                    }
+                    g[k] = mine;
+                    made |= 1u << k;
+                }
+            }
+            id += __popc(m[k]);
+        }
+        claimed = 0;
+    };
     while (__any_sync(0xFFFFFFFFu, any)) {
 #pragma unroll
         for (int k = 0; k < K; k++)
@@ -136,41 +173,12 @@ __device__ __forceinline__ uint32_t warp_upsert(const AggArgs& A, bool (&need)[K
                 else old[k] = atomicCAS((uint32_t*)slot_at(t, i[k]), 0u, 1u);
             }
         }
-        unsigned m[K];
-        uint32_t total = 0;
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-            m[k] = __ballot_sync(0xFFFFFFFFu, old[k] == 0);
-            total += __popc(m[k]);
-        }
-        if (total) {  // the same in every lane
-            uint32_t id = 0;
-            if (lane == 0) id = atomicAdd(A.ngroups, total);
-            id = __shfl_sync(0xFFFFFFFFu, id, 0);
-            full = id + total > A.gid_cap || id + total < id;
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                if (old[k] == 0) {
-                    const uint32_t mine = id + __popc(m[k] & ((1u << lane) - 1u));
-                    uint64_t* s = slot_at(t, i[k]);
-                    const uint64_t x = (2u | (nm[k] << 8)) | ((uint64_t)mine << 32);
-                    if (mine >= A.gid_cap) {
-                        publish_state((uint32_t*)s, 0);
-                    } else {
-                        if (wide) {
-                            s[2] = w[k][1];
-                            st_slot_release(s, x, w[k][0]);
-                        } else {
-                            st_slot(s, x, w[k][0]);
-                        }
-                        g[k] = mine;
-                        made |= 1u << k;
-                    }
-                    need[k] = false;
-                }
-                id += __popc(m[k]);
+        for (int k = 0; k < K; k++)
+            if (old[k] == 0) {
+                claimed |= 1u << k;
+                need[k] = false;
             }
-        }
         any = false;
         bool waiting = false;
 #pragma unroll
@@ -185,6 +193,9 @@ __device__ __forceinline__ uint32_t warp_upsert(const AggArgs& A, bool (&need)[K
             waiting = waiting || st <= 1;
             any = any || need[k];
         }
+        // no key of the warp left to resolve, or one waits for a claim (this warp's own, or another's whose
+        // warp may wait for this one's)
+        if (__any_sync(0xFFFFFFFFu, claimed != 0) && (__any_sync(0xFFFFFFFFu, waiting) || !__any_sync(0xFFFFFFFFu, any))) publish();
         // a claim that is never published, or a table without an empty slot, ends the wait
         if (waiting && ++spins >= kSpinLimit) {
             atomicOr(err, (uint32_t)DE_TIMEOUT);
@@ -196,6 +207,7 @@ __device__ __forceinline__ uint32_t warp_upsert(const AggArgs& A, bool (&need)[K
             for (int k = 0; k < K; k++) need[k] = false;
         }
     }
+    if (__any_sync(0xFFFFFFFFu, claimed != 0)) publish();  // a lane gave up above
     return made;
 }
 

@@ -2685,7 +2685,7 @@ int ml_gpu_hashagg_sink(ml_hashagg_local* local, const ml_column* cols, int32_t 
     // range the table grows to what the groups per row so far predict (groups_ahead), so few rows
     // overflow and the table is not sized for every row being a new group.  20M rows with 2M groups:
     // one launch into a 1,024-group table, 20M rows through the overflow list and a table for 20M groups
-    // took 9.6 ms of kernels; the ranges take 1.9 ms.
+    // took 9.6 ms of kernels; the ranges take 1.8 ms.
     constexpr int64_t kFirstRows = 65536;
     const bool ranges = can_overflow && !h->hinted && !h->sized && n >= 4 * kFirstRows && (int64_t)h->gid_cap < n / 4 &&
                         jit_enabled(ctx) && !h->str_minmax;
