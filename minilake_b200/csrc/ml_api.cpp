@@ -204,7 +204,43 @@ std::vector<std::unique_ptr<DevColumn>> gather_rows(Ctx* ctx, const ml_batch& b,
         if (small) return out;
         out.clear();  // strings past the room: a column at a time
     }
-    for (auto& c : b.cols) out.push_back(gather_column(ctx, *c, idx, k, st, res));
+    GatherCols G{};
+    int64_t bytes = 0;  // of G's columns
+    // Columns share a launch while half the L2 holds them: their rows are read at random.  Three columns of 10M rows
+    // (200 MB) took 403 us together and 225 apart; eight of 2M (120 MB) 220 us with a launch for each column's
+    // values and another for its validity, 185 with one for both, 164 in two launches.
+    constexpr int64_t kTogether = 64 << 20;
+    auto flush = [&] {
+        // one column without validity: 4 bytes of 10M rows 53 us row by row, 57 in batches
+        if (G.n == 1 && !G.c[0].src_valid) launch_gather_fixed(G.c[0].src, G.c[0].width, idx, k, G.c[0].dst, st);
+        else launch_gather_cols(G, idx, k, st);
+        if (G.n) ctx->count_launch();
+        G.n = 0;
+        bytes = 0;
+    };
+    for (auto& c : b.cols) {
+        if (c->kind != CK_FIXED || k <= 0) {
+            out.push_back(gather_column(ctx, *c, idx, k, st, res));
+            continue;
+        }
+        auto d = std::make_unique<DevColumn>();
+        d->dtype = c->dtype;
+        d->kind = CK_FIXED;
+        d->n = k;
+        const int64_t size = c->n * width_of(c->dtype);
+        if (G.n == kGatherCols || (G.n && bytes + size > kTogether)) flush();
+        bytes += size;
+        GatherCol& g = G.c[G.n++];
+        g = GatherCol{c->dptr(), nullptr, c->vptr(), nullptr, width_of(c->dtype)};
+        d->data = DevBuf(ctx, (size_t)k * g.width, res);
+        g.dst = d->data.get();
+        if (g.src_valid) {
+            d->validity = DevBuf(ctx, (size_t)(k + 63) / 64 * 8, res);
+            g.dst_valid = d->validity.get<uint32_t>();
+        }
+        out.push_back(std::move(d));
+    }
+    flush();
     CK(cudaStreamSynchronize(st));
     return out;
 }

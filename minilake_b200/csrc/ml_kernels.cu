@@ -969,6 +969,49 @@ __global__ void k_gather_valid(const uint64_t* src, const uint32_t* idx, int64_t
         if ((threadIdx.x & 31) == 0 && i < k) dst[i >> 5] = b;
     }
 }
+// The rows of several columns in one launch: kGatherRows row ids per thread are read once, and a column's
+// loads for all of them are in flight together.  2M rows of an 8-byte column with validity: 27.5 us in two
+// launches with a row id and then its value per step, 23 us alone so, 20.5 with three others.
+constexpr int kGatherRows = 4;
+template <class T>
+__device__ __forceinline__ void gather_values(const GatherCol& c, const uint32_t (&r)[kGatherRows], int64_t i0, int64_t k) {
+    T v[kGatherRows];
+#pragma unroll
+    for (int j = 0; j < kGatherRows; j++) v[j] = ((const T*)c.src)[r[j]];
+#pragma unroll
+    for (int j = 0; j < kGatherRows; j++) {
+        const int64_t i = i0 + j * kThreads;
+        if (i < k) __stcs((T*)c.dst + i, v[j]);
+    }
+}
+__global__ void __launch_bounds__(kThreads) k_gather_cols(const __grid_constant__ GatherCols G, const uint32_t* idx, int64_t k) {
+    const int64_t step = (int64_t)gridDim.x * kThreads * kGatherRows;
+    for (int64_t base = (int64_t)blockIdx.x * kThreads * kGatherRows; base < k; base += step) {
+        const int64_t i0 = base + threadIdx.x;
+        uint32_t r[kGatherRows];
+#pragma unroll
+        for (int j = 0; j < kGatherRows; j++) {
+            const int64_t i = i0 + j * kThreads;
+            r[j] = ld_stream_u32(idx + (i < k ? i : k - 1));
+        }
+        for (int n = 0; n < G.n; n++) {
+            const GatherCol& c = G.c[n];
+            if (c.width == 8) gather_values<uint64_t>(c, r, i0, k);
+            else if (c.width == 4) gather_values<uint32_t>(c, r, i0, k);
+            else gather_values<uint8_t>(c, r, i0, k);
+            if (!c.dst_valid) continue;
+            bool v[kGatherRows];
+#pragma unroll
+            for (int j = 0; j < kGatherRows; j++) v[j] = valid_bit(c.src_valid, r[j]);
+#pragma unroll
+            for (int j = 0; j < kGatherRows; j++) {
+                const int64_t i = i0 + j * kThreads;
+                const uint32_t bits = __ballot_sync(0xFFFFFFFFu, i < k && v[j]);
+                if ((threadIdx.x & 31) == 0 && (i >> 5) < 2 * ((k + 63) / 64)) c.dst_valid[i >> 5] = bits;
+            }
+        }
+    }
+}
 __global__ void k_utf8_lengths(const uint32_t* off, const uint32_t* idx, int64_t k, uint32_t* len) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < k; i += stride) {
@@ -1916,6 +1959,9 @@ void launch_strid(const uint32_t* off, const uint8_t* bytes, const uint64_t* val
 }
 void launch_gather_fixed(const void* src, int width, const uint32_t* idx, int64_t k, void* dst, cudaStream_t s) {
     if (k) k_gather_fixed<<<grid_for(k, 8), kThreads, 0, s>>>((const uint8_t*)src, width, idx, k, (uint8_t*)dst);
+}
+void launch_gather_cols(const GatherCols& G, const uint32_t* idx, int64_t k, cudaStream_t s) {
+    if (k && G.n) k_gather_cols<<<grid_for((k + kGatherRows - 1) / kGatherRows, 8), kThreads, 0, s>>>(G, idx, k);
 }
 void launch_gather_valid(const uint64_t* src, const uint32_t* idx, int64_t k, uint32_t* dst, cudaStream_t s) {
     if (k) k_gather_valid<<<grid_for(k, 8), kThreads, 0, s>>>(src, idx, k, dst);

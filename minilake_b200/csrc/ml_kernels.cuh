@@ -115,6 +115,20 @@ void launch_strid(const uint32_t* off, const uint8_t* bytes, const uint64_t* val
 
 // Gathers.
 // dst row i = src row idx[i]; width is 1, 4 or a multiple of 8 bytes
+// Rows idx[0..k) of several fixed-width columns (widths 1, 4 and 8) and their validity words at once.
+constexpr int kGatherCols = 16;
+struct GatherCol {
+    const void* src;
+    void* dst;
+    const uint64_t* src_valid;  // with dst_valid
+    uint32_t* dst_valid;        // whole 64-bit words
+    int32_t width;
+};
+struct GatherCols {
+    int n;
+    GatherCol c[kGatherCols];
+};
+void launch_gather_cols(const GatherCols& G, const uint32_t* idx, int64_t k, cudaStream_t s);
 void launch_gather_fixed(const void* src, int width, const uint32_t* idx, int64_t k, void* dst, cudaStream_t s);
 void launch_gather_valid(const uint64_t* src, const uint32_t* idx, int64_t k, uint32_t* dst, cudaStream_t s);
 void launch_utf8_lengths(const uint32_t* off, const uint32_t* idx, int64_t k, uint32_t* len, cudaStream_t s);
