@@ -255,8 +255,8 @@ constexpr int kSnapThreads = 1024;
 constexpr uint32_t kSnapPer = kSnapBlk / kSnapThreads;
 constexpr uint32_t kSnapNone = 0xFFFFFFFFu;
 // plan modes: 0 the length varint is malformed, 1 the serial pass decodes the page, 2 its
-// fragments decode in parallel, 3 it is decoded, 4 undecided
-constexpr uint32_t kSnapSerial = 1, kSnapSplit = 2, kSnapDone = 3, kSnapOpen = 4;
+// fragments decode in parallel
+constexpr uint32_t kSnapSerial = 1, kSnapSplit = 2;
 constexpr uint32_t kSnapPiece = 2048, kSnapPieces = 2048;  // long literals, cut into pieces for the warps
 constexpr size_t kSnapMapSmem = kSnapBlk * 8 + kSnapBlk + 32;
 constexpr size_t kSnapFragSmem = kSnapFrag * 3 + kSnapPieces * 8;
@@ -265,7 +265,7 @@ constexpr uint64_t kSnapGroupBytes = 32ull << 20;
 
 // One element header at s[0..avail): its size h (tag plus length or offset bytes), kind (0
 // literal, 1 copy), output length and copy offset; false if it does not fit in `avail`.
-__device__ __forceinline__ bool snap_hdr(const uint8_t* s, uint32_t avail, uint32_t& h, uint32_t& kind,
+__host__ __device__ __forceinline__ bool snap_hdr(const uint8_t* s, uint32_t avail, uint32_t& h, uint32_t& kind,
                                          uint32_t& len, uint32_t& off) {
     if (avail == 0) return false;
     const uint32_t tag = s[0], t = tag & 3;
@@ -338,55 +338,79 @@ __device__ uint64_t load8(const uint8_t* p) {
 }
 
 // Pages of few elements, one block per page: pages that do not compress (bit-packed random indices,
-// random numbers) are a few long literals, perhaps with a stray copy.  One thread follows the elements as
-// long as they span kSnapFlatSpan stream bytes on average, at most kSnapFlat of them; if that is the whole page, the
-// block copies the literals, then one warp the copies in order, and the passes below leave the page alone.
-// Bound by the element headers' latency (0.6 us each): seven pages of 18,000 two-bit indices 4.8 us, and 16 us
-// for the passes below to find nothing to do; they took 55 us to decode them (maps 11, chain 3, list 12, decode 16 and launches).
+// random numbers) are a few long literals, perhaps with a stray copy.  The host, which parses the page
+// headers, follows the elements as long as they span kSnapFlatSpan stream bytes on average, at most
+// kSnapFlat of them (flat_elements: a few cache lines of the page), or kSnapFlatTiny of a page of at most
+// kSnapTiny bytes (a small dictionary page); a page that ends by then is not one of the passes' pages, and the
+// block copies its literals, then one warp its copies in order (in shared memory for a tiny page: 49 copies
+// 12 us).  Seven pages of 18,000 two-bit indices: 55 us in the six launches of the passes below, 3.6 us in one
+// here (4.8 us when the device followed the elements, and 16 for the passes to find nothing to do).
 constexpr int kSnapFlat = 64;
 constexpr uint32_t kSnapFlatSpan = 256;
-__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_flat(const SnapJob* jobs, uint32_t* plan) {
-    __shared__ uint4 el[kSnapFlat];  // {stream position of a literal's bytes, output position, length, copy offset (0: literal)}
-    __shared__ int count;
-    const SnapJob J = jobs[blockIdx.x];
-    const uint32_t tid = threadIdx.x;
-    if (tid == 0) {
-        uint32_t pos = 0, total = 0;
-        bool ok = false;
-        for (int shift = 0; shift < 35 && pos < J.src_len; shift += 7) {  // the uncompressed length
-            const uint32_t b = J.src[pos++];
-            if (shift == 28 && (b & 0x70)) break;  // past 32 bits
-            total |= (b & 0x7F) << shift;
-            if (!(b & 0x80)) {
-                ok = total == J.dst_len;
-                break;
-            }
+constexpr uint32_t kSnapTiny = 4096;
+constexpr int kSnapFlatTiny = 256;
+struct SnapFlat {
+    const uint8_t* src;
+    uint8_t* dst;
+    uint32_t dst_len, tiny;  // tiny: at most kSnapTiny bytes, and not literals alone
+    uint32_t el0, n;  // its elements: {stream position of a literal's bytes, output position, length, copy offset (0: literal)}
+};
+bool flat_elements(const uint8_t* s, uint32_t len, uint32_t out_len, std::vector<uint4>& el) {
+    uint32_t pos = 0, total = 0;
+    bool ok = false;
+    for (int shift = 0; shift < 35 && pos < len; shift += 7) {  // the uncompressed length
+        const uint32_t b = s[pos++];
+        if (shift == 28 && (b & 0x70)) break;  // past 32 bits
+        total |= (b & 0x7F) << shift;
+        if (!(b & 0x80)) {
+            ok = total == out_len;
+            break;
         }
-        const uint32_t start = pos;
-        uint32_t out = 0;
-        int n = 0;
-        while (ok && pos < J.src_len) {
-            const uint8_t* e = J.src + pos;  // five readable bytes: the chunk buffer is padded past its end
-            uint32_t step, len;
-            ok = n < kSnapFlat && (n < 2 || pos - start >= n * kSnapFlatSpan) && snap_elem(e, J.src_len - pos, step, len) &&
-                 len <= J.dst_len - out;
-            if (!ok) break;
-            const uint32_t t = e[0] & 3;
-            const uint32_t off = t == 0 ? 0u
-                                 : t == 1 ? ((uint32_t)(e[0] >> 5) << 8) | e[1]
-                                          : e[1] | ((uint32_t)e[2] << 8) | (t == 3 ? ((uint32_t)e[3] << 16) | ((uint32_t)e[4] << 24) : 0u);
-            ok = t == 0 || (off != 0 && off <= out);
-            el[n++] = make_uint4(pos + step - len, out, len, off);
-            pos += step;
-            out += len;
-        }
-        ok = ok && out == J.dst_len;
-        count = ok ? n : -1;
-        plan[J.plan] = ok ? kSnapDone : kSnapOpen;
     }
+    const size_t el0 = el.size();
+    const uint32_t start = pos;
+    uint32_t out = 0, n = 0;
+    for (; ok && pos < len; n++) {
+        uint32_t h, kind, l, off;
+        ok = (out_len <= kSnapTiny ? n < (uint32_t)kSnapFlatTiny
+                                   : n < (uint32_t)kSnapFlat && (n < 2 || pos - start >= n * kSnapFlatSpan)) &&
+             snap_hdr(s + pos, len - pos, h, kind, l, off) &&
+             l <= out_len - out && (kind == 0 || (off != 0 && off <= out));
+        if (!ok) break;
+        el.push_back(make_uint4(pos + h, out, l, off));
+        pos += h + (kind == 0 ? l : 0);
+        out += l;
+    }
+    ok = ok && out == out_len;
+    if (!ok) el.resize(el0);  // the passes decode it, or report it
+    return ok;
+}
+__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_flat(const SnapFlat* pages, const uint4* elems) {
+    __shared__ uint4 el[kSnapFlatTiny];
+    __shared__ uint8_t tiny[kSnapTiny];
+    const SnapFlat J = pages[blockIdx.x];
+    const uint32_t tid = threadIdx.x;
+    const int n = (int)J.n;
+    if ((int)tid < n) el[tid] = elems[J.el0 + tid];
     __syncthreads();
-    const int n = count;
-    if (n < 0) return;
+    if (J.tiny) {
+        for (int k = tid >> 5; k < n; k += kSnapThreads / 32) {  // a warp per literal
+            const uint4 e = el[k];
+            if (!e.w)
+                for (uint32_t i = tid & 31; i < e.z; i += 32) tiny[e.y + i] = J.src[e.x + i];
+        }
+        __syncthreads();
+        if (tid < 32)
+            for (int k = 0; k < n; k++) {
+                const uint4 e = el[k];
+                if (!e.w) continue;
+                for (uint32_t i = tid; i < e.z; i += 32) tiny[e.y + i] = tiny[e.y - e.w + (i < e.w ? i : i % e.w)];  // a copy over itself repeats
+                __syncwarp();
+            }
+        __syncthreads();
+        for (uint32_t i = tid; i < J.dst_len; i += kSnapThreads) J.dst[i] = tiny[i];
+        return;
+    }
     for (int k = 0; k < n; k++) {
         const uint4 e = el[k];
         if (e.w) continue;
@@ -403,7 +427,7 @@ __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_flat(const SnapJob* 
     for (int k = 0; k < n; k++) {
         const uint4 e = el[k];
         if (!e.w) continue;
-        for (uint32_t i = tid; i < e.z; i += 32) J.dst[e.y + i] = J.dst[e.y - e.w + i % e.w];  // a copy over itself repeats
+        for (uint32_t i = tid; i < e.z; i += 32) J.dst[e.y + i] = J.dst[e.y - e.w + (i < e.w ? i : i % e.w)];  // a copy over itself repeats
         __syncwarp();
     }
 }
@@ -413,14 +437,12 @@ __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_flat(const SnapJob* 
 // past the block (or that does not parse) points to itself.  States only ever move further along the
 // chain and are read and written whole, so the rounds need no second buffer: bound by shared-memory
 // round trips, log2(kSnapBlk / 2) of them.
-__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_maps(const SnapJob* jobs, const uint2* blocks, const uint32_t* plan,
-                                                                 SnapMap* tab) {
+__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_maps(const SnapJob* jobs, const uint2* blocks, SnapMap* tab) {
     extern __shared__ __align__(16) uint8_t snap_smem[];
     uint64_t* st = (uint64_t*)snap_smem;
     uint8_t* win = snap_smem + kSnapBlk * 8;
     const uint2 f = blocks[blockIdx.x];
     const SnapJob J = jobs[f.x];
-    if (plan[J.plan] == kSnapDone) return;
     const uint32_t b0 = f.y * kSnapBlk, blen = min(kSnapBlk, J.src_len - b0);
     const uint8_t* w = win + snap_window(J, b0, win);
     __syncthreads();
@@ -468,7 +490,6 @@ __global__ void __launch_bounds__(32) k_pq_snappy_chain(const SnapJob* jobs, con
     if (threadIdx.x) return;
     const SnapJob J = jobs[blockIdx.x];
     uint32_t* pl = plan + J.plan;
-    if (pl[0] == kSnapDone) return;
     uint32_t start = 0, total = 0;
     bool ok = false;
     for (int shift = 0; shift < 35 && start < J.src_len; shift += 7) {  // the uncompressed length
@@ -769,7 +790,7 @@ __global__ void __launch_bounds__(32) k_pq_snappy_serial(const SnapJob* jobs, co
     const SnapJob J = jobs[blockIdx.x];
     const uint32_t* pl = plan + J.plan;
     const uint32_t mode = pl[0];
-    if (mode == kSnapSplit || mode == kSnapDone) return;
+    if (mode == kSnapSplit) return;
     SnapSrc S{J.src, J.src_len, win};
     if (mode != kSnapSerial || !snap_decode_serial(S, pl[1], J.src_len, J.dst, J.dst_len)) atomicOr(err, PQ_ERR_SNAPPY);
 }
@@ -1646,6 +1667,8 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
     std::vector<SnapJob> jobs;
     std::vector<SnapGroup> groups;
     std::vector<uint2> frags, blocks;  // {page, fragment} per 64 KB of output, {page, block} per kSnapBlk of stream
+    std::vector<SnapFlat> flats;             // pages of few elements, and those
+    std::vector<uint4> elems;
     uint32_t plan_words = 0;
     for (size_t i = 0; i < pages.size(); i++) {
         const Page& pg = pages[i];
@@ -1656,6 +1679,13 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
         if (compressed) {
             const uint32_t dlen = (uint32_t)(pg.uncompressed - lv);
             const uint32_t slen = (uint32_t)(pg.compressed - lv);
+            const uint32_t el0 = (uint32_t)elems.size();
+            if (flat_elements(chunk + pg.payload + lv, slen, dlen, elems)) {
+                const bool copies = std::any_of(elems.begin() + el0, elems.end(), [](const uint4& e) { return e.w != 0; });
+                flats.push_back(SnapFlat{dc + pg.payload + lv, up + uoff[i] + lv, dlen, dlen <= kSnapTiny && copies ? 1u : 0u, el0,
+                                         (uint32_t)elems.size() - el0});
+                continue;
+            }
             const uint32_t nfrag = (uint32_t)(((uint64_t)dlen + kSnapFrag - 1) / kSnapFrag);
             const uint32_t nblk = (uint32_t)(((uint64_t)slen + kSnapBlk - 1) / kSnapBlk);
             if (groups.empty() || groups.back().bytes + slen > kSnapGroupBytes) {
@@ -1687,43 +1717,53 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
     uint32_t* dfirst = derr + 8;
     PinnedSlot slot(ctx);
     DevBuf dj, splan, smap, sentry;  // the Snappy kernels': live to the end of the call
-    if (!jobs.empty()) {
-        // the jobs, the fragment and the block table in one upload
-        const size_t jb = jobs.size() * sizeof(SnapJob), fb = frags.size() * sizeof(uint2), bb = blocks.size() * sizeof(uint2);
-        std::vector<uint8_t> hj(jb + fb + bb);
-        std::memcpy(hj.data(), jobs.data(), jb);
-        if (fb) std::memcpy(hj.data() + jb, frags.data(), fb);
-        if (bb) std::memcpy(hj.data() + jb + fb, blocks.data(), bb);
+    if (!jobs.empty() || !flats.empty()) {
+        // the elements, the jobs, the fragment and the block table in one upload
+        const size_t eb = elems.size() * sizeof(uint4), lb = flats.size() * sizeof(SnapFlat), jb = jobs.size() * sizeof(SnapJob);
+        const size_t fb = frags.size() * sizeof(uint2), bb = blocks.size() * sizeof(uint2);
+        std::vector<uint8_t> hj(eb + lb + jb + fb + bb);
+        uint8_t* at = hj.data();
+        auto put = [&](const void* p, size_t n) {
+            if (n) std::memcpy(at, p, n);
+            at += n;
+        };
+        put(elems.data(), eb), put(flats.data(), lb), put(jobs.data(), jb), put(frags.data(), fb), put(blocks.data(), bb);
         dj = DevBuf(ctx, hj.size(), nullptr);
         CK(cudaMemcpyAsync(dj.get(), hj.data(), hj.size(), cudaMemcpyHostToDevice, s));
-        const SnapJob* J = dj.get<SnapJob>();
-        const uint2* F = (const uint2*)(dj.get<uint8_t>() + jb);
-        const uint2* B = (const uint2*)(dj.get<uint8_t>() + jb + fb);
-        splan = DevBuf(ctx, (size_t)plan_words * 4, nullptr);
-        uint64_t most = 0, most_elems = 0;
-        int most_blks = 0;
-        for (const SnapGroup& g : groups)
-            most = std::max(most, g.bytes), most_elems = std::max(most_elems, g.elems), most_blks = std::max(most_blks, g.nblks);
-        // the maps; the element list takes their place once the chains are known
-        smap = DevBuf(ctx, std::max<size_t>(std::max(most * sizeof(SnapMap), most_elems * sizeof(uint2)), 16), nullptr);
-        sentry = DevBuf(ctx, std::max<size_t>((size_t)most_blks * sizeof(SnapEntry), 16), nullptr);
-        // per call: the attribute belongs to the current device's copy of the kernel
-        CK(cudaFuncSetAttribute(k_pq_snappy_maps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSnapMapSmem));
-        CK(cudaFuncSetAttribute(k_pq_snappy_frag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSnapFragSmem));
-        for (const SnapGroup& g : groups) {
-            k_pq_snappy_flat<<<g.njobs, kSnapThreads, 0, s>>>(J + g.job0, splan.get<uint32_t>());
-            if (g.nblks) {
-                CK(cudaMemsetAsync(sentry.get(), 0, (size_t)g.nblks * sizeof(SnapEntry), s));
-                k_pq_snappy_maps<<<g.nblks, kSnapThreads, kSnapMapSmem, s>>>(J, B + g.blk0, splan.get<uint32_t>(), smap.get<SnapMap>());
+        const uint8_t* D0 = dj.get<uint8_t>();
+        if (!flats.empty()) {
+            k_pq_snappy_flat<<<(unsigned)flats.size(), kSnapThreads, 0, s>>>((const SnapFlat*)(D0 + eb), (const uint4*)D0);
+            ctx->count_launch();
+        }
+        const SnapJob* J = (const SnapJob*)(D0 + eb + lb);
+        const uint2* F = (const uint2*)(D0 + eb + lb + jb);
+        const uint2* B = (const uint2*)(D0 + eb + lb + jb + fb);
+        if (!jobs.empty()) {
+            splan = DevBuf(ctx, (size_t)plan_words * 4, nullptr);
+            uint64_t most = 0, most_elems = 0;
+            int most_blks = 0;
+            for (const SnapGroup& g : groups)
+                most = std::max(most, g.bytes), most_elems = std::max(most_elems, g.elems), most_blks = std::max(most_blks, g.nblks);
+            // the maps; the element list takes their place once the chains are known
+            smap = DevBuf(ctx, std::max<size_t>(std::max(most * sizeof(SnapMap), most_elems * sizeof(uint2)), 16), nullptr);
+            sentry = DevBuf(ctx, std::max<size_t>((size_t)most_blks * sizeof(SnapEntry), 16), nullptr);
+            // per call: the attribute belongs to the current device's copy of the kernel
+            CK(cudaFuncSetAttribute(k_pq_snappy_maps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSnapMapSmem));
+            CK(cudaFuncSetAttribute(k_pq_snappy_frag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSnapFragSmem));
+            for (const SnapGroup& g : groups) {
+                if (g.nblks) {
+                    CK(cudaMemsetAsync(sentry.get(), 0, (size_t)g.nblks * sizeof(SnapEntry), s));
+                    k_pq_snappy_maps<<<g.nblks, kSnapThreads, kSnapMapSmem, s>>>(J, B + g.blk0, smap.get<SnapMap>());
+                }
+                k_pq_snappy_chain<<<g.njobs, 32, 0, s>>>(J + g.job0, smap.get<SnapMap>(), sentry.get<SnapEntry>(), splan.get<uint32_t>());
+                if (g.nblks)
+                    k_pq_snappy_list<<<g.nblks, kSnapThreads, 0, s>>>(J, B + g.blk0, sentry.get<SnapEntry>(), splan.get<uint32_t>(),
+                                                                      smap.get<uint2>());
+                if (g.nfrags)
+                    k_pq_snappy_frag<<<g.nfrags, kSnapThreads, kSnapFragSmem, s>>>(J, F + g.frag0, smap.get<uint2>(), splan.get<uint32_t>());
+                k_pq_snappy_serial<<<g.njobs, 32, 0, s>>>(J + g.job0, splan.get<uint32_t>(), derr);
+                ctx->count_launch(2 + (g.nblks ? 2 : 0) + (g.nfrags ? 1 : 0));
             }
-            k_pq_snappy_chain<<<g.njobs, 32, 0, s>>>(J + g.job0, smap.get<SnapMap>(), sentry.get<SnapEntry>(), splan.get<uint32_t>());
-            if (g.nblks)
-                k_pq_snappy_list<<<g.nblks, kSnapThreads, 0, s>>>(J, B + g.blk0, sentry.get<SnapEntry>(), splan.get<uint32_t>(),
-                                                                  smap.get<uint2>());
-            if (g.nfrags)
-                k_pq_snappy_frag<<<g.nfrags, kSnapThreads, kSnapFragSmem, s>>>(J, F + g.frag0, smap.get<uint2>(), splan.get<uint32_t>());
-            k_pq_snappy_serial<<<g.njobs, 32, 0, s>>>(J + g.job0, splan.get<uint32_t>(), derr);
-            ctx->count_launch(3 + (g.nblks ? 2 : 0) + (g.nfrags ? 1 : 0));
         }
     }
     auto read_err = [&]() {  // waits for the stream; slot: {error bits, -, present values, strings' bytes}

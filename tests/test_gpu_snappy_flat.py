@@ -43,6 +43,11 @@ CASES = {
     "sparse": [3000] + [(5, 4)] * 11,
     "dense": [256, 254, 250] + [10] * 200,
     "big": [(1 << 20) + 3],
+    "tiny": [3, (1, 5), 6, (6, 7), (2, 64), 1, (80, 30), 2],
+    "tiny_256": [8] + [(8, 8), 7] * 127 + [(3, 15)],
+    "tiny_257": [8] + [(8, 8), 7] * 128,
+    "tiny_4096": [4000, (4000, 64), 32],
+    "above_4096": [4000, (4000, 64), 40],
 }
 
 
