@@ -209,7 +209,7 @@ constexpr int kPqTile = 8192;  // rows per decode tile: 256 threads x one 32-row
 //    there is parsed, and pointer doubling in shared memory (log2 of the elements in a block rounds)
 //    gives where the chain from that byte leaves the block, how many elements it passes and how many
 //    bytes they write;
-//  * the chain (one thread per page) steps from block to block through those maps, which gives each
+//  * the chain (one warp per page) steps from block to block through those maps, which gives each
 //    block the position its first element starts at;
 //  * the list (one block per kSnapBlk bytes again): doubling from that position marks the real element
 //    starts, and a scan numbers them and gives each its output position;
@@ -224,7 +224,7 @@ constexpr int kPqTile = 8192;  // rows per decode tile: 256 threads x one 32-row
 // them), so a thread that follows it is bound by a shared-memory round trip per element whatever the
 // chip has to offer.  Measured on such a page (125,000 prices, Snappy): one thread following the chain
 // through per-window records 6.5 ms and a warp per fragment decoding 2.3 ms; now maps 22 us, chain
-// 44 us, list 23 us and decode 58 us.
+// 16 us, list 23 us and decode 58 us.
 struct SnapJob {
     const uint8_t* src;
     uint8_t* dst;
@@ -247,7 +247,8 @@ struct SnapEntry {  // a block's first element, as the page's chain reaches it
 };
 constexpr uint32_t kSnapFrag = 1u << 16;  // the compressor's fragment
 constexpr uint32_t kSnapWin = 2048;       // the serial pass's window
-// Stream bytes per map / list block: the chain takes one dependent L2 load (~0.4 us) per block, a
+// Stream bytes per map / list block: the chain takes a step (0.1 us, or a dependent L2 load where
+// its guess is wrong) per block, a
 // doubling round in a block costs eight shared-memory steps per thread, and 8 KB gives a 1 MB page 122
 // blocks, one wave of the 148 SMs.
 constexpr uint32_t kSnapBlk = 8192;
@@ -483,11 +484,14 @@ __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_maps(const SnapJob* 
     }
 }
 
-// The chain, one thread per page: the page's mode, each block's entry, and the number of elements.
-// Bound by one dependent L2 load per block of the page.
+// The chain, one warp per page: the page's mode, each block's entry, and the number of elements.
+// A block's entry is known when the chain has left the block before it: one dependent L2 load per block (42 us
+// for the 89 blocks of a 721 KB stream).  But chains that start at different bytes soon meet, so where the chain
+// from a block's first byte leaves it is mostly where the real one does: the lanes load the next 32 blocks' maps at
+// those places together, and the walk takes a lane's map where its guess is right (15.5 us), else loads it.
 __global__ void __launch_bounds__(32) k_pq_snappy_chain(const SnapJob* jobs, const SnapMap* tab, SnapEntry* entries,
                                                         uint32_t* plan) {
-    if (threadIdx.x) return;
+    const uint32_t lane = threadIdx.x;
     const SnapJob J = jobs[blockIdx.x];
     uint32_t* pl = plan + J.plan;
     uint32_t start = 0, total = 0;
@@ -501,22 +505,41 @@ __global__ void __launch_bounds__(32) k_pq_snappy_chain(const SnapJob* jobs, con
             break;
         }
     }
-    pl[1] = start;
+    if (lane == 0) pl[1] = start;
     if (!ok || total != J.dst_len) {
-        pl[0] = 0;
+        if (lane == 0) pl[0] = 0;
         return;
     }
+    const SnapMap* maps = tab + J.tab0;
     bool split = J.nfrag >= 1;
     uint32_t pos = start, elem = 0;
     uint64_t out = 0;
-    while (split && pos < J.src_len) {
-        const uint4 m = __ldg((const uint4*)(tab + J.tab0 + pos));
-        entries[J.blk0 + pos / kSnapBlk] = SnapEntry{pos, (uint32_t)out, elem, 1u};
+    uint32_t g0 = 0, guess = kSnapNone;  // lane l holds block g0 + l's guessed entry and the map there
+    uint4 gm = make_uint4(kSnapNone, 0, 0, 0);
+    bool held = false;
+    while (split && pos < J.src_len) {  // the same in every lane
+        const uint32_t blk = pos / kSnapBlk;
+        if (!held || blk - g0 >= 32) {
+            g0 = blk;
+            held = true;
+            const uint64_t mine = (uint64_t)g0 + lane;
+            guess = lane == 0 ? pos : mine * kSnapBlk < J.src_len ? maps[(mine - 1) * kSnapBlk].exit : kSnapNone;
+            if (guess >= J.src_len || guess / kSnapBlk != mine) guess = kSnapNone;
+            if (guess != kSnapNone) gm = __ldg((const uint4*)(maps + guess));
+        }
+        const int from = (int)(blk - g0);
+        uint4 m;
+        m.x = __shfl_sync(0xFFFFFFFFu, gm.x, from);
+        m.y = __shfl_sync(0xFFFFFFFFu, gm.y, from);
+        m.z = __shfl_sync(0xFFFFFFFFu, gm.z, from);
+        if (__shfl_sync(0xFFFFFFFFu, guess, from) != pos) m = __ldg((const uint4*)(maps + pos));
+        if (lane == 0) entries[J.blk0 + blk] = SnapEntry{pos, (uint32_t)out, elem, 1u};
         out += m.y;
         elem += m.z;
         pos = m.x;  // past pos: an element spans at least two bytes
         split = m.x != kSnapNone && out <= total;
     }
+    if (lane) return;
     if (split && out == total) {
         pl[2 + J.nfrag] = elem;
         pl[0] = kSnapSplit;
