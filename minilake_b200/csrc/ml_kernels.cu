@@ -1575,8 +1575,8 @@ __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackPieces
 // host checks that the list held at least k rows and not more than it has room for (else every row goes
 // through k_topn_chunk / k_topn_warp).
 // Why: the chunk sort orders all rows in shared memory, 2.0 ms for 20M rows and k = 100; the selection
-// reads the column at 5.1 to 5.9 TB/s (32 us), before it 15 us for the bound, after it 17 us for the
-// finish.
+// reads the column at 5.1 to 5.9 TB/s (32 us), before it 13 us for the bound, after it 11 us for the
+// finish (a bound from 16,384 samples, eight times the rows in the list and a sort of them: 17 and 19 us).
 
 // The block finds the r-th smallest (r >= 1) of n values get(i): by 8-bit digits from the highest bit in
 // which the values differ, counted in shared memory.  Returns an upper bound of it that no further value
@@ -1668,19 +1668,20 @@ __device__ uint64_t block_select(Get get, uint32_t n, uint32_t r, uint32_t slack
     }
 }
 
-// The bound: one row of each of `samples` equal pieces of the column, the smallest prefix of every 4 or 16
+// The bound: one row of each of `samples` equal pieces of the column, the smallest prefix of every 4 or 32
 // neighbouring samples (kTopNMinima of them), and the r-th smallest of those, found by the last block to
 // finish (`done` starts at zero).  At least r samples lie at or below it.  Many blocks, because the rows
-// lie far apart: one block took 25 us for 16,384 of them.
+// lie far apart (one block took 25 us for 16,384 of them), and large ones, because the last selects alone (256
+// threads 17 us, 1,024 13).
 constexpr uint32_t kTopNMinima = 4096;
 template <int DT>
-__global__ void __launch_bounds__(256) k_topn_sample(const __grid_constant__ SortDev S, int64_t n, uint32_t samples, uint32_t r,
+__global__ void __launch_bounds__(1024) k_topn_sample(const __grid_constant__ SortDev S, int64_t n, uint32_t samples, uint32_t r,
                                                      uint64_t* minima, uint32_t* done, uint64_t* bound) {
     __shared__ uint64_t mins[kTopNMinima];
     __shared__ bool last;
     const DCol& c = S.cols[0];
     const uint64_t flip = S.asc[0] ? 0ull : ~0ull, nullp = S.nulls_first[0] ? 0ull : ~0ull;
-    const uint32_t i = blockIdx.x * 256 + threadIdx.x, step = (uint32_t)((uint64_t)n / samples);  // at least 1
+    const uint32_t i = blockIdx.x * 1024 + threadIdx.x, step = (uint32_t)((uint64_t)n / samples);  // at least 1
     uint32_t x = i * 0x9E3779B9u;  // not always the same row of a piece: a period of the data must not matter
     x ^= x >> 15;
     x *= 0x85EBCA6Bu;
@@ -1699,7 +1700,7 @@ __global__ void __launch_bounds__(256) k_topn_sample(const __grid_constant__ Sor
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (uint32_t j = threadIdx.x; j < kTopNMinima; j += 256) mins[j] = __ldcg((const unsigned long long*)minima + j);
+    for (uint32_t j = threadIdx.x; j < kTopNMinima; j += 1024) mins[j] = __ldcg((const unsigned long long*)minima + j);
     __syncthreads();
     uint32_t taken;
     const uint64_t b = block_select([&](uint32_t j) { return mins[j]; }, kTopNMinima, r, r, &taken);
@@ -1777,7 +1778,8 @@ __global__ void __launch_bounds__(1024) k_topn_finish(const __grid_constant__ So
     }
     uint32_t size = 2;
     while (size < taken) size *= 2;
-    for (uint32_t i = threadIdx.x; i < size; i += 1024) {
+    const bool few = taken <= 512;  // placed by counting: no steps to wait for
+    for (uint32_t i = threadIdx.x; i < size && !few; i += 1024) {
         pre[i] = ~0ull;
         idx[i] = kNone;
     }
@@ -1789,6 +1791,26 @@ __global__ void __launch_bounds__(1024) k_topn_finish(const __grid_constant__ So
         idx[at] = list_p ? __ldg(list_r + i) : i;
     });
     __syncthreads();
+    if (few) {
+        // two threads per row count the rows before it, half of them each
+        const uint32_t i = threadIdx.x >> 1, half = threadIdx.x & 1;
+        uint32_t place = 0;
+        if (i < taken) {
+            const uint64_t p = pre[i];
+            for (uint32_t j = half; j < taken; j += 2) {
+                const uint64_t q = pre[j];
+                bool before = q < p;
+                if (q == p && j != i) {  // equal keys keep their input order
+                    const int o = cmp_rows(S, idx[j], idx[i]);
+                    before = o < 0 || (o == 0 && idx[j] < idx[i]);
+                }
+                place += before;
+            }
+        }
+        place += __shfl_xor_sync(0xFFFFFFFFu, place, 1);
+        if (i < taken && half == 0 && place < (uint32_t)k) out[place] = idx[i];
+        return;
+    }
     bitonic_rows(S, pre, idx, (int)size);
     for (int j = threadIdx.x; j < k; j += 1024) out[j] = idx[j];
 }
@@ -2018,7 +2040,9 @@ TopNPlan topn_plan(const SortDev& S, int64_t n, int k) {
     }
     // the sample's rank: k rows of n are `mean` of the sample on average; six standard deviations and
     // six more make fewer than k rows at or below it a matter of one in 10^8
-    p.samples = n >= (4 << 20) ? 16 * kTopNMinima : 4 * kTopNMinima;
+    // 131,072 samples leave some 3,000 rows of 60M in the list for k = 10 (16,384: 25,000, and 6 us more in the
+    // finish); with fewer rows than 4M as many samples would be the scan itself
+    p.samples = n >= (4 << 20) ? 32 * kTopNMinima : 4 * kTopNMinima;
     const double mean = (double)k * p.samples / (double)n;
     const double r = std::ceil(mean + 6 * std::sqrt(mean) + 6);
     const double rows = r / p.samples * (double)n;  // rows at or below, on average
@@ -2037,7 +2061,7 @@ static cudaError_t topn_select(const SortDev& S, int64_t n, int k, const TopNPla
     cudaError_t e = cudaFuncSetAttribute(k_topn_finish<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_b);
     if (e != cudaSuccess) return e;
     if (p.rank) {
-        k_topn_sample<DT><<<p.samples / 256, 256, 0, s>>>(S, n, p.samples, p.rank, minima, state + 2, bound);
+        k_topn_sample<DT><<<p.samples / 1024, 1024, 0, s>>>(S, n, p.samples, p.rank, minima, state + 2, bound);
         const int64_t want = (n + 4095) / 4096;
         k_topn_take<DT><<<(int)std::min<int64_t>(want, (int64_t)num_sms() * 8), 256, 0, s>>>(S, n, bound, list_p, list_r, p.cap, state);
     }
