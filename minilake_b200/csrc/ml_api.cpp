@@ -1415,9 +1415,9 @@ int ml_gpu_filter_static(ml_ctx* ctx, const ml_expr* pred, const ml_column* cols
     uint64_t* offs = (uint64_t*)(base + kStaticOffsetsOff);
     const int nb = select_blocks(n);
     launch_select_flags(L.P, bits, counts, s);
-    launch_scan_u32(counts, offs, nb, (uint64_t*)(base + kStaticScanOff), s);
+    const int scans = launch_scan_u32(counts, offs, nb, (uint64_t*)(base + kStaticScanOff), s);
     launch_select_write(L.P, bits, offs, sel_out, s);
-    ctx->count_launch(5);
+    ctx->count_launch(2 + scans);
     uint64_t total = 0;
     uint32_t errw = 0;
     CK(cudaMemcpyAsync(&total, offs + nb, 8, cudaMemcpyDeviceToHost, s));
@@ -3648,8 +3648,7 @@ void query_enqueue(ml_query* q) {
         }
         launch_group_flags(h->acc.get<uint64_t>(), h->stride, q->cap, member, q->bits.get<uint32_t>(), q->counts.get<uint32_t>(), s,
                            key, bound);
-        launch_scan_u32(q->counts.get<uint32_t>(), q->offs.get<uint64_t>(), nb, q->scratch.get<uint64_t>(), s);
-        nk += 4;
+        nk += 1 + launch_scan_u32(q->counts.get<uint32_t>(), q->offs.get<uint64_t>(), nb, q->scratch.get<uint64_t>(), s);
         if (!h->dense_groups)  // the key gathers read every position: past the groups, build row 0
             CK(cudaMemsetAsync(q->gids.get(), 0, (size_t)q->cap * 4, s));
         launch_index_write(q->cap, q->bits.get<uint32_t>(), q->offs.get<uint64_t>(), q->gids.get<uint32_t>(), s);

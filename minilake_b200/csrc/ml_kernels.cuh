@@ -92,7 +92,7 @@ void launch_dense_keys(const uint32_t* gids, int64_t n, uint64_t dmin, int dt, v
                        const uint64_t* n_dev = nullptr);
 void launch_index_write(int64_t n, const uint32_t* bits, const uint64_t* block_offsets, uint32_t* out, cudaStream_t s);
 // Exclusive scan of u32 counts into u64 offsets (offsets[n] = total).
-void launch_scan_u32(const uint32_t* in, uint64_t* out, int64_t n, uint64_t* scratch, cudaStream_t s);
+int launch_scan_u32(const uint32_t* in, uint64_t* out, int64_t n, uint64_t* scratch, cudaStream_t s);  // -> kernels launched
 size_t scan_scratch_words(int64_t n);
 
 // Projection: evaluate program `prog` for output row i = row idx[i] (or i) of the source.

@@ -1937,7 +1937,7 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
     if (cv == CV_UTF8 && !encoded) {
         const int64_t n = num_rows;
         DevBuf offs(ctx, (size_t)(n + 1) * 8, nullptr), sc(ctx, std::max<size_t>(scan_scratch_words(n) * 8, 8), nullptr);
-        launch_scan_u32(slen.get<uint32_t>(), offs.get<uint64_t>(), n, sc.get<uint64_t>(), s);
+        ctx->count_launch(launch_scan_u32(slen.get<uint32_t>(), offs.get<uint64_t>(), n, sc.get<uint64_t>(), s));
         uint64_t total = 0;
         CK(cudaMemcpyAsync(&total, offs.get<uint64_t>() + n, 8, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -1958,10 +1958,10 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
         DevBuf sc2(ctx, std::max<size_t>(scan_scratch_words(nb) * 8, 8), nullptr);
         k_pq_first_flags<<<nb, 256, 0, s>>>(canon.get<uint32_t>(), first.get<uint32_t>(), n, bits.get<uint32_t>(),
                                             counts.get<uint32_t>(), rpb);
-        launch_scan_u32(counts.get<uint32_t>(), boffs.get<uint64_t>(), nb, sc2.get<uint64_t>(), s);
+        ctx->count_launch(launch_scan_u32(counts.get<uint32_t>(), boffs.get<uint64_t>(), nb, sc2.get<uint64_t>(), s));
         uint64_t distinct = 0;
         CK(cudaMemcpyAsync(&distinct, boffs.get<uint64_t>() + nb, 8, cudaMemcpyDeviceToHost, s));
-        ctx->count_launch(6);
+        ctx->count_launch(4);  // the copy, the ids, the first rows and their flags
         read_err();
         if (distinct <= limit) {
             // the first occurrences in row order are the dictionary; each row's code is its string's
@@ -1977,7 +1977,7 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
             DevBuf dl(ctx, (size_t)nd * 4 + 4, nullptr), doff(ctx, (size_t)(nd + 1) * 8, nullptr);
             DevBuf sc3(ctx, std::max<size_t>(scan_scratch_words(nd) * 8, 8), nullptr);
             launch_utf8_lengths(off32.get<uint32_t>(), list.get<uint32_t>(), nd, dl.get<uint32_t>(), s);
-            launch_scan_u32(dl.get<uint32_t>(), doff.get<uint64_t>(), nd, sc3.get<uint64_t>(), s);
+            ctx->count_launch(launch_scan_u32(dl.get<uint32_t>(), doff.get<uint64_t>(), nd, sc3.get<uint64_t>(), s));
             std::vector<uint64_t> ho(nd + 1);
             CK(cudaMemcpyAsync(ho.data(), doff.get(), (size_t)(nd + 1) * 8, cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
@@ -1986,7 +1986,7 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
             DevBuf db(ctx, std::max<size_t>(ho[nd], 1), nullptr);
             launch_utf8_copy(off32.get<uint32_t>(), bytes.get<uint8_t>(), list.get<uint32_t>(), nd, doff.get<uint64_t>(), db.get<uint8_t>(), s);
             if (ho[nd]) CK(cudaMemcpyAsync(hd->bytes.data(), db.get(), ho[nd], cudaMemcpyDeviceToHost, s));
-            ctx->count_launch(3);
+            ctx->count_launch(2);
             CK(cudaStreamSynchronize(s));
             for (int64_t i = 1; i <= nd; i++) hd->off.push_back((uint32_t)ho[i]);
             col->kind = CK_DICT;

@@ -396,8 +396,7 @@ bool Pipeline::reads_nullable(const Prog& p, const Launch& L) const {
 uint64_t scan_counts(Ctx* ctx, const uint32_t* counts, int64_t n, DevBuf& offsets, cudaStream_t s, Reservation* res) {
     offsets = DevBuf(ctx, (size_t)(n + 1) * 8, res);
     DevBuf scratch(ctx, scan_scratch_words(n) * 8, res);
-    launch_scan_u32(counts, offsets.get<uint64_t>(), n, scratch.get<uint64_t>(), s);
-    ctx->count_launch(3);
+    ctx->count_launch(launch_scan_u32(counts, offsets.get<uint64_t>(), n, scratch.get<uint64_t>(), s));
     uint64_t total = 0;
     CK(cudaMemcpyAsync(&total, offsets.get<uint64_t>() + n, 8, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -434,8 +433,7 @@ int64_t run_select(Ctx* ctx, const Pipeline& pipe, const PipeArgs& P, DevBuf& ou
     DevBuf offs(ctx, (size_t)(nb + 1) * 8, res), scratch(ctx, scan_scratch_words(nb) * 8, res);
     PinnedSlot total(ctx);
     select_flags(ctx, pipe, P, bits, counts, s);
-    launch_scan_u32(counts.get<uint32_t>(), offs.get<uint64_t>(), nb, scratch.get<uint64_t>(), s);
-    ctx->count_launch(3);
+    ctx->count_launch(launch_scan_u32(counts.get<uint32_t>(), offs.get<uint64_t>(), nb, scratch.get<uint64_t>(), s));
     CK(cudaMemcpyAsync(total.p, offs.get<uint64_t>() + nb, 8, cudaMemcpyDeviceToHost, s));
     // the selection's size is needed now to allocate it, or to charge what the caller's buffer holds to a
     // budget; else one wait at the end is enough
