@@ -1731,29 +1731,55 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
                 CK(cudaMemcpyAsync(up + uoff[i] + lv, dc + pg.payload + lv, (size_t)(pg.compressed - lv), cudaMemcpyDeviceToDevice, s));
         }
     }
-    // {error bits, -, present values, strings' bytes} and the first rows of a small dictionary's entries
-    DevBuf err(ctx, 32 + kPqSmallDict * 4, nullptr);
-    CK(cudaMemsetAsync(err.get(), 0, 32 + kPqSmallDict * 4, s));
-    uint32_t* derr = err.get<uint32_t>();
-    uint64_t* dpresent = err.get<uint64_t>() + 1;
-    uint64_t* dtotal = err.get<uint64_t>() + 2;
-    uint32_t* dfirst = derr + 8;
-    PinnedSlot slot(ctx);
-    DevBuf dj, splan, smap, sentry;  // the Snappy kernels': live to the end of the call
-    if (!jobs.empty() || !flats.empty()) {
-        // the elements, the jobs, the fragment and the block table in one upload
-        const size_t eb = elems.size() * sizeof(uint4), lb = flats.size() * sizeof(SnapFlat), jb = jobs.size() * sizeof(SnapJob);
-        const size_t fb = frags.size() * sizeof(uint2), bb = blocks.size() * sizeof(uint2);
-        std::vector<uint8_t> hj(eb + lb + jb + fb + bb);
+    std::vector<PageDev> hp(np);
+    int64_t row0 = 0;
+    for (int j = 0; j < np; j++) {
+        const Page& pg = pages[data[j]];
+        PageDev& d = hp[j];
+        d = PageDev{};
+        d.data = up + uoff[data[j]];
+        d.len = (uint32_t)pg.uncompressed;
+        d.v2 = pg.type == PAGE_DATA_V2;
+        d.def_bytes = pg.def_bytes;
+        d.rep_bytes = pg.rep_bytes;
+        d.encoding = pg.encoding == ENC_PLAIN_DICTIONARY ? ENC_RLE_DICTIONARY : pg.encoding;
+        d.row0 = row0;
+        d.nrows = (uint32_t)pg.num_values;
+        d.lv_run0 = d.ix_run0 = (uint64_t)row0;
+        row0 += pg.num_values;
+    }
+    // One upload: the elements, the flat pages, the Snappy jobs, their fragment and block tables, the data pages, and
+    // zeros for the first rows of a small dictionary's entries and for {error bits, -, present values, strings'
+    // bytes}; behind those lies the small dictionary's answer, so one copy brings both back.
+    const size_t eb = elems.size() * sizeof(uint4), lb = flats.size() * sizeof(SnapFlat), jb = jobs.size() * sizeof(SnapJob);
+    const size_t fb = frags.size() * sizeof(uint2), bb = blocks.size() * sizeof(uint2), pb = hp.size() * sizeof(PageDev);
+    const size_t zb = (cv == CV_UTF8 ? kPqSmallDict * 4 : 0) + 32;
+    // {strings, bytes, offsets, the bytes (no more than the page holds)}
+    const size_t answer_head = (2 + kPqSmallDict + 1) * 4;
+    const size_t answer_b = cv == CV_UTF8 && dict_page >= 0 && (uint32_t)pages[dict_page].uncompressed <= kPqSmallDictBytes
+                                ? answer_head + (size_t)pages[dict_page].uncompressed : 0;
+    std::vector<uint8_t> hj(eb + lb + jb + fb + bb + pb + zb);
+    {
         uint8_t* at = hj.data();
         auto put = [&](const void* p, size_t n) {
             if (n) std::memcpy(at, p, n);
             at += n;
         };
         put(elems.data(), eb), put(flats.data(), lb), put(jobs.data(), jb), put(frags.data(), fb), put(blocks.data(), bb);
-        dj = DevBuf(ctx, hj.size(), nullptr);
-        CK(cudaMemcpyAsync(dj.get(), hj.data(), hj.size(), cudaMemcpyHostToDevice, s));
-        const uint8_t* D0 = dj.get<uint8_t>();
+        put(hp.data(), pb);
+    }
+    DevBuf dj(ctx, hj.size() + answer_b, nullptr);
+    CK(cudaMemcpyAsync(dj.get(), hj.data(), hj.size(), cudaMemcpyHostToDevice, s));
+    uint8_t* const D0 = dj.get<uint8_t>();
+    PageDev* P = (PageDev*)(D0 + eb + lb + jb + fb + bb);
+    uint32_t* derr = (uint32_t*)(D0 + hj.size() - 32);
+    uint64_t* dpresent = (uint64_t*)derr + 1;
+    uint64_t* dtotal = (uint64_t*)derr + 2;
+    uint32_t* dfirst = derr - kPqSmallDict;  // strings only
+    uint32_t* danswer = derr + 8;
+    PinnedSlot slot(ctx);
+    DevBuf splan, smap, sentry;  // the Snappy kernels': live to the end of the call
+    if (!jobs.empty() || !flats.empty()) {
         if (!flats.empty()) {
             k_pq_snappy_flat<<<(unsigned)flats.size(), kSnapThreads, 0, s>>>((const SnapFlat*)(D0 + eb), (const uint4*)D0);
             ctx->count_launch();
@@ -1797,26 +1823,6 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
 
     // 2. data pages (the kernels are bounds-checked, so a decode error is read once, at the end;
     //    a page's run table starts at its first row: a stream has at most one run per value): layout, level runs, validity, present values, index runs
-    std::vector<PageDev> hp(np);
-    int64_t row0 = 0;
-    for (int j = 0; j < np; j++) {
-        const Page& pg = pages[data[j]];
-        PageDev& d = hp[j];
-        d = PageDev{};
-        d.data = up + uoff[data[j]];
-        d.len = (uint32_t)pg.uncompressed;
-        d.v2 = pg.type == PAGE_DATA_V2;
-        d.def_bytes = pg.def_bytes;
-        d.rep_bytes = pg.rep_bytes;
-        d.encoding = pg.encoding == ENC_PLAIN_DICTIONARY ? ENC_RLE_DICTIONARY : pg.encoding;
-        d.row0 = row0;
-        d.nrows = (uint32_t)pg.num_values;
-        d.lv_run0 = d.ix_run0 = (uint64_t)row0;
-        row0 += pg.num_values;
-    }
-    DevBuf dpages(ctx, hp.size() * sizeof(PageDev), nullptr);
-    PageDev* P = dpages.get<PageDev>();
-    CK(cudaMemcpyAsync(P, hp.data(), hp.size() * sizeof(PageDev), cudaMemcpyHostToDevice, s));
     DevBuf lv_runs(ctx, (size_t)num_rows * sizeof(Run), nullptr), ix_runs(ctx, (size_t)num_rows * sizeof(Run), nullptr);
     k_pq_levels<<<np, 32, 0, s>>>(P, max_def, level_width, lv_runs.get<Run>(), derr);
     const int64_t ntiles = (num_rows + kPqTile - 1) / kPqTile;
@@ -1897,24 +1903,25 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
     bool encoded = false;
     if (small_dict) {
         const int64_t n = num_rows;
-        // one block's answer in one copy: {strings, bytes, offsets, the bytes (no more than the page holds)}
-        const size_t head = (2 + kPqSmallDict + 1) * 4, all = head + (size_t)pages[dict_page].uncompressed;
-        DevBuf code_of(ctx, kPqSmallDict * 4, nullptr), answer(ctx, all, nullptr);
+        DevBuf code_of(ctx, kPqSmallDict * 4, nullptr);
         DevBuf codes(ctx, (size_t)n * 4, b->res.get());
-        k_pq_small_dict<<<1, kPqSmallDict, 0, s>>>(D.dict_ptr, D.dict_len, D.dict_n, dfirst, code_of.get<uint32_t>(), answer.get<uint32_t>());
+        k_pq_small_dict<<<1, kPqSmallDict, 0, s>>>(D.dict_ptr, D.dict_len, D.dict_n, dfirst, code_of.get<uint32_t>(), danswer);
         k_pq_codes2<<<grid_of(n), 256, 0, s>>>(ent.get<uint32_t>(), n, code_of.get<uint32_t>(), codes.get<uint32_t>());
         ctx->count_launch(2);
-        std::vector<uint8_t> h(all);
-        CK(cudaMemcpyAsync(h.data(), answer.get(), all, cudaMemcpyDeviceToHost, s));
-        read_err();
+        std::vector<uint8_t> told(32 + answer_b);  // the status words, then the answer
+        CK(cudaMemcpyAsync(told.data(), derr, told.size(), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        std::memcpy(slot.p, told.data(), 32);
+        check_pq(ctx, *slot.as<uint32_t>());
+        const uint8_t* h = told.data() + 32;
         uint32_t found[2];
-        std::memcpy(found, h.data(), 8);
+        std::memcpy(found, h, 8);
         if (slot.as<uint64_t>()[2] > 0xFFFFFFFFull) raise(ML_ERR_UNSUPPORTED, "parquet: a string column larger than 4 GiB");
         if (found[0] <= limit) {
             auto hd = std::make_shared<HostDict>();
-            hd->bytes.assign(h.begin() + head, h.begin() + head + found[1]);
+            hd->bytes.assign(h + answer_head, h + answer_head + found[1]);
             std::vector<uint32_t> off(found[0] + 1);
-            std::memcpy(off.data(), h.data() + 8, off.size() * 4);
+            std::memcpy(off.data(), h + 8, off.size() * 4);
             hd->off.insert(hd->off.end(), off.begin() + 1, off.end());
             col->kind = CK_DICT;
             col->data = std::move(codes);
