@@ -1676,7 +1676,7 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
     }
 
     // 1. the chunk to the device, then every page uncompressed
-    // 64 bytes of padding: warp_copy reads up to 8 bytes past a copy's source
+    // 64 bytes of padding: the aligned 8- and 16-byte loads read past the last byte
     DevBuf dchunk(ctx, (size_t)chunk_bytes + 64, nullptr), upages(ctx, (size_t)ubytes + 64, nullptr);
     // from the caller's (pageable) buffer: a pinned staging buffer per call costs more than it saves
     CK(cudaMemcpyAsync(dchunk.get(), chunk, (size_t)chunk_bytes, cudaMemcpyHostToDevice, s));
