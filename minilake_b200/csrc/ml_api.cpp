@@ -1263,7 +1263,7 @@ int ml_gpu_batch_fetch_all(const ml_batch* b, int32_t ncols, void* const* values
         OpStream op_stream(ctx);
         Staging st(ctx);
         DevBuf packed(ctx, std::max<size_t>(total, 8), nullptr);
-        uint8_t* host = (uint8_t*)st.get(std::max<size_t>(total, 8));
+        uint8_t* host = (uint8_t*)st.get(std::max<size_t>(total, 8), op_stream.s);
         launch_pack(P, packed.get(), op_stream.s);
         ctx->count_launch();
         CK(cudaMemcpyAsync(host, packed.get(), total, cudaMemcpyDeviceToHost, op_stream.s));
@@ -1551,6 +1551,7 @@ struct ml_join_build_local {
         sink->streams.add(s);
     }
     ~ml_join_build_local() {
+        st.release();
         sink->streams.remove(s);
         sink->ctx->free_stream(s);
     }
@@ -1722,10 +1723,10 @@ int ml_gpu_join_build_finalize(ml_join_build* j, ml_join_table** table) {
     CK(cudaMemsetAsync(jt->slots.get(), 0, slot_bytes, s));
     ErrWord ew(ctx);
     CK(cudaMemsetAsync(ew.d.get(), 0, 4, s));
+    Pipeline::Launch LA;  // the insert kernel's tables and the copy that brings them: live until the wait below
+    Staging st(ctx);
     if (nh) {  // the key programs run only here (a dense index reads the key column directly)
         kp.upload();
-        Staging st(ctx);
-        Pipeline::Launch LA;
         auto views = device_views(jt->batch);
         kp.prepare(LA, views.data(), (int)views.size(), nh, nullptr, 0, s, st, nullptr);
         LA.P.err = ew.d.get<uint32_t>();
@@ -2569,6 +2570,7 @@ struct ml_hashagg_local {
         sink->streams.add(s);
     }
     ~ml_hashagg_local() {
+        st.release();
         sink->streams.remove(s);
         sink->ctx->release_slot(h_count);
         sink->ctx->free_stream(s);
@@ -3122,7 +3124,7 @@ std::unique_ptr<ml_batch> hashagg_emit(ml_hashagg* h, cudaStream_t s) {
         if (h->dec[k].str_kind == 1) want(*keycols[k], std::move(id_bufs[k]));
     Staging stg(ctx);
     if (!strs.empty()) {
-        uint8_t* host = (uint8_t*)stg.get(std::max<size_t>(back, 8));
+        uint8_t* host = (uint8_t*)stg.get(std::max<size_t>(back, 8), s);
         for (auto& x : strs) {
             if (!ng) continue;
             CK(cudaMemcpyAsync(host + x.at, x.ids.get(), (size_t)ng * 4, cudaMemcpyDeviceToHost, s));
@@ -3153,7 +3155,7 @@ std::unique_ptr<ml_batch> hashagg_emit(ml_hashagg* h, cudaStream_t s) {
             offs.push_back(std::move(off));
             bytes.push_back(std::move(by));
         }
-        uint8_t* up = (uint8_t*)stg.get(std::max<size_t>(out_b, 8));  // the ids have been read
+        uint8_t* up = (uint8_t*)stg.get(std::max<size_t>(out_b, 8), s);  // the ids have been read
         size_t at = 0;
         for (size_t i = 0; i < strs.size(); i++) {
             DevColumn& c = *strs[i].col;
@@ -3310,6 +3312,7 @@ struct ml_topn_local {
         sink->streams.add(s);
     }
     ~ml_topn_local() {
+        st.release();
         sink->streams.remove(s);
         sink->ctx->free_stream(s);
     }
@@ -3515,6 +3518,7 @@ struct ml_query {
         if (e1) cudaEventDestroy(e1);
         if (hguard) ctx->release_slot(hguard);
         if (hng) ctx->release_slot(hng);
+        if (st) st->release();
         if (s) {
             cudaStreamSynchronize(s);
             ctx->free_stream(s);

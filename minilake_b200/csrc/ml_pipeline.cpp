@@ -371,8 +371,7 @@ void Pipeline::prepare(Launch& L, const ml_column* cols, int ncols, int64_t nrow
             base = tables_dst;
         } else {
             L.scratch = DevBuf(ctx, scratch.size(), nullptr);
-            void* h = st.get(scratch.size());
-            CK(cudaStreamSynchronize(s));  // the staging buffer may still feed an earlier copy
+            void* h = st.get(scratch.size(), s);
             memcpy(h, scratch.data(), scratch.size());
             CK(cudaMemcpyAsync(L.scratch.get(), h, scratch.size(), cudaMemcpyHostToDevice, s));
             base = L.scratch.get<uint8_t>();

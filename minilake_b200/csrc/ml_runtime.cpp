@@ -320,14 +320,21 @@ void Ctx::drain_timings(size_t keep) {  // collect all but the newest `keep` tim
     timings_.erase(timings_.begin(), timings_.begin() + n);
 }
 
-Staging::~Staging() {
-    if (p_) ctx_->hfree(p_);
+void Staging::release() {
+    if (!p_) return;
+    cudaStreamSynchronize(s_);
+    ctx_->hfree(p_);
+    p_ = nullptr;
+    cap_ = 0;
 }
-void* Staging::get(size_t bytes) {
+void* Staging::get(size_t bytes, cudaStream_t s) {
+    if (p_) CK(cudaStreamSynchronize(s_));
+    s_ = s;
     if (bytes > cap_) {
-        if (p_) ctx_->hfree(p_);
-        cap_ = std::max(bytes, cap_ * 2);
-        p_ = ctx_->halloc(cap_);
+        const size_t cap = std::max(bytes, cap_ * 2);
+        release();
+        p_ = ctx_->halloc(cap);
+        cap_ = cap;
     }
     return p_;
 }
@@ -371,13 +378,12 @@ static void h2d(void* dst, const void* src, size_t bytes, cudaStream_t s, Stagin
         CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
         return;
     }
-    // pageable: copy through the pinned staging buffer in chunks (the stream is
-    // synchronized before the staging buffer is refilled)
+    // pageable: copy through the pinned staging buffer in chunks (get waits for the stream before
+    // the buffer is refilled)
     const size_t chunk = 64ull << 20;
     for (size_t o = 0; o < bytes; o += chunk) {
         size_t k = std::min(chunk, bytes - o);
-        void* p = st.get(chunk < bytes ? chunk : bytes);
-        CK(cudaStreamSynchronize(s));
+        void* p = st.get(chunk < bytes ? chunk : bytes, s);
         memcpy(p, (const uint8_t*)src + o, k);
         CK(cudaMemcpyAsync((uint8_t*)dst + o, p, k, cudaMemcpyHostToDevice, s));
     }

@@ -181,15 +181,21 @@ class KernelTimer {
     cudaEvent_t a_ = nullptr, b_ = nullptr;
 };
 
-// Pinned staging buffer owned by one stream user.
+// Pinned staging buffer owned by one stream user.  Its block comes from a pool that every thread of the
+// context shares, so it goes back only when the copies on the stream that use it are done.
 class Staging {
    public:
     explicit Staging(Ctx* ctx) : ctx_(ctx) {}
-    ~Staging();
-    void* get(size_t bytes);
+    ~Staging() { release(); }
+    Staging(const Staging&) = delete;
+    // `bytes` for a copy on stream s, once the copies from earlier calls are done (one wait of that stream).
+    void* get(size_t bytes, cudaStream_t s);
+    // The block back to the pool; call it before the stream goes back to its own.
+    void release();
 
    private:
     Ctx* ctx_;
+    cudaStream_t s_ = nullptr;  // of the last get
     void* p_ = nullptr;
     size_t cap_ = 0;
 };
