@@ -756,12 +756,18 @@ std::unique_ptr<ml_batch> topn_batch(Ctx* ctx, ml_batch& b, const std::vector<So
             kt.stop();
         }
         ctx->count_launch(sel.rank ? 3 : 1);
-        // the result is gathered before the host knows that it is one (the rows exist either way)
+        // fixed-width columns are gathered before the host knows that the rows are the result (k rows exist
+        // either way); what a string column needs depends on the rows, and a budget counts what is asked for
+        bool wait = ctx->pool.limit != UINT64_MAX;
+        for (auto& c : b.cols) wait = wait || c->kind != CK_FIXED;
         ErrWord told(ctx);
         CK(cudaMemcpyAsync(told.h, state + 1, 4, cudaMemcpyDeviceToHost, st));
-        out->cols = gather_rows(ctx, b, (const uint32_t*)(base + ro), k, st, res);
-        if (!*told.h) return out;
-        out->cols.clear();
+        if (wait) CK(cudaStreamSynchronize(st));
+        if (!wait || !*told.h) {
+            out->cols = gather_rows(ctx, b, (const uint32_t*)(base + ro), k, st, res);
+            if (!*told.h) return out;
+            out->cols.clear();
+        }
     }
     if (k <= kTopNWarpMax) {  // small limits: one sorted list per warp, one launch
         const int nb = topn_warp_blocks(n);

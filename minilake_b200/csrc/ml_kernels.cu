@@ -1798,7 +1798,7 @@ __global__ void __launch_bounds__(1024) k_topn_finish(const __grid_constant__ So
     const DCol& c = S.cols[0];
     const uint64_t flip = S.asc[0] ? 0ull : ~0ull, nullp = S.nulls_first[0] ? 0ull : ~0ull;
     const uint32_t m = list_p ? state[0] : (uint32_t)n;
-    for (int j = threadIdx.x; j < k; j += 1024) out[j] = 0;  // rows that exist, whatever comes of it
+    for (int j = threadIdx.x; j < k; j += 1024) out[j] = j;  // rows that exist, whatever comes of it
     if (threadIdx.x == 0) m_s = 0;
     if (m < (uint32_t)k || (list_p && m > cap)) {
         if (threadIdx.x == 0) state[1] = 1;

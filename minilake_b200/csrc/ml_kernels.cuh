@@ -227,7 +227,7 @@ struct TopNPlan {
 };
 size_t topn_minima_bytes();
 TopNPlan topn_plan(const SortDev& S, int64_t n, int k);
-// out[0 .. k): the rows, sorted, unless state[1] is set afterwards (then they are 0).  bound: one word;
+// out[0 .. k): the rows, sorted, unless state[1] is set afterwards (then they are the rows 0 .. k - 1).  bound: one word;
 // minima: topn_minima_bytes(); list_p / list_r: p.cap entries each; state: three zeroed words.
 cudaError_t launch_topn_select(const SortDev& S, int64_t n, int k, const TopNPlan& p, uint64_t* bound, uint64_t* minima, uint64_t* list_p,
                                uint32_t* list_r, uint32_t* state, uint32_t* out, cudaStream_t s);
