@@ -1707,10 +1707,12 @@ __device__ uint64_t block_select(Get get, uint32_t n, uint32_t r, uint32_t slack
 }
 
 // The bound: one row of each of `samples` equal pieces of the column, the smallest prefix of every 4 or 32
-// neighbouring samples (kTopNMinima of them), and the r-th smallest of those, found by the last block to
-// finish (`done` starts at zero).  At least r samples lie at or below it.  Many blocks, because the rows
-// lie far apart (one block took 25 us for 16,384 of them), and large ones, because the last selects alone (256
-// threads 17 us, 1,024 13).
+// samples (kTopNMinima of them), and the r-th smallest of those, found by the last block to finish (`done`
+// starts at zero).  At least r samples lie at or below it.  The samples of one minimum come from pieces all
+// over the column, in no pattern: of neighbouring pieces of a sorted column one would be the smallest and
+// hide 31 almost as small, and the list would hold 32 times the rows that it has room for.  Many blocks,
+// because the rows lie far apart (one block took 25 us for 16,384 of them), and large ones, because the last
+// selects alone (256 threads 17 us, 1,024 13).
 constexpr uint32_t kTopNMinima = 4096;
 template <int DT>
 __global__ void __launch_bounds__(1024) k_topn_sample(const __grid_constant__ SortDev S, int64_t n, uint32_t samples, uint32_t r,
@@ -1720,11 +1722,17 @@ __global__ void __launch_bounds__(1024) k_topn_sample(const __grid_constant__ So
     const DCol& c = S.cols[0];
     const uint64_t flip = S.asc[0] ? 0ull : ~0ull, nullp = S.nulls_first[0] ? 0ull : ~0ull;
     const uint32_t i = blockIdx.x * 1024 + threadIdx.x, step = (uint32_t)((uint64_t)n / samples);  // at least 1
+    // thread i's piece: a permutation of 0 .. samples - 1 (a power of two: odd factors and shifted xors undo)
+    const int half = (31 - __clz((int)samples)) / 2;
+    uint32_t piece = (i * 0x9E3779B1u) & (samples - 1);
+    piece ^= piece >> half;
+    piece = (piece * 0x85EBCA6Bu) & (samples - 1);
+    piece ^= piece >> half;
     uint32_t x = i * 0x9E3779B9u;  // not always the same row of a piece: a period of the data must not matter
     x ^= x >> 15;
     x *= 0x85EBCA6Bu;
     x ^= x >> 13;
-    const uint32_t row = (uint32_t)((uint64_t)i * (uint64_t)n / samples + x % step);
+    const uint32_t row = (uint32_t)((uint64_t)piece * (uint64_t)n / samples + x % step);
     uint64_t p = fixed_prefix<DT>(load_value(c, row), valid_bit(c.valid, row), flip, nullp);
     const uint32_t lanes = samples / kTopNMinima;
     for (uint32_t o = lanes >> 1; o; o >>= 1) {
