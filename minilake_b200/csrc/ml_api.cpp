@@ -959,7 +959,7 @@ DevBuf radix_sort_rows(Ctx* ctx, const std::vector<SortWord>& words, int64_t n, 
         uint32_t* hist = scratch.get<uint32_t>();
         uint32_t* counters = hist + 4 * 256;
         CK(cudaMemsetAsync(hist, 0, hist_b + (size_t)digits * stat_b, st));
-        launch_sort_keys(W, S, rows, n, keys, digits, hist, st);
+        launch_sort_keys(W, S, rows, n, keys, digits, hist, ew.d.get<uint32_t>(), st);
         for (int d = 0; d < digits; d++) {
             uint32_t* out = rows == perm.get<uint32_t>() ? pb.get<uint32_t>() : perm.get<uint32_t>();
             const bool want_keys = d + 1 < digits || keep_keys;
@@ -976,7 +976,7 @@ DevBuf radix_sort_rows(Ctx* ctx, const std::vector<SortWord>& words, int64_t n, 
         DevBuf list(ctx, (size_t)cap * 8 + 16, nullptr);
         uint32_t* state = (uint32_t*)(list.get<uint8_t>() + (size_t)cap * 8);
         CK(cudaMemsetAsync(state, 0, 8, st));
-        launch_sort_runs(keys, rows, W, nw, n, list.get<uint2>(), cap, state, st);
+        launch_sort_runs(keys, rows, W, nw, n, list.get<uint2>(), cap, state, ew.d.get<uint32_t>(), st);
         ctx->count_launch(2);
         uint32_t got[2] = {0, 0};
         CK(cudaMemcpyAsync(got, state, 8, cudaMemcpyDeviceToHost, st));

@@ -171,9 +171,10 @@ struct SortSegs {
 // stats[3 y ..]: the bits in which word y differs between rows, its smallest and its largest value
 // (`nwords` device words, at most 32).
 void launch_sort_bits(const SortWord* words, int nwords, int64_t n, unsigned long long* stats, cudaStream_t s);
-// The u32 keys of rows perm[0..n) (nullptr: 0..n) and their digit histograms (digits x 256, zeroed).
+// The u32 keys of rows perm[0..n) (nullptr: 0..n) and their digit histograms (digits x 256, zeroed).  The next
+// three do nothing once *err is set: a pass that gave up has left row ids unwritten.
 void launch_sort_keys(const SortWord* words, const SortSegs& S, const uint32_t* perm, int64_t n, uint32_t* keys, int digits,
-                      uint32_t* hist, cudaStream_t s);
+                      uint32_t* hist, const uint32_t* err, cudaStream_t s);
 // One stable pass by the digit at `shift` over (key, row id); rows_in nullptr: row ids 0..n; keys_out
 // nullptr: row ids only.  status: radix_tiles(n) x 256 zeroed words; next_tile: a zeroed counter.
 int64_t radix_tiles(int64_t n);
@@ -183,7 +184,7 @@ cudaError_t launch_radix_pass(const uint32_t* keys_in, const uint32_t* rows_in, 
 // Rows with equal keys put in the order of their whole key words, unless state[1] is set (a run too
 // long, or more runs than `cap`): then nothing has moved.  state: two zeroed words.
 void launch_sort_runs(const uint32_t* keys, uint32_t* rows, const SortWord* words, int nwords, int64_t n, uint2* list,
-                      uint32_t cap, uint32_t* state, cudaStream_t s);
+                      uint32_t cap, uint32_t* state, const uint32_t* err, cudaStream_t s);
 void launch_max_strlen(const uint32_t* off, int64_t n, unsigned int* out, cudaStream_t s);
 void launch_iota_u32(uint32_t* out, int64_t n, cudaStream_t s);  // out[i] = i
 // The first k of n <= kTopNTiny rows in order.

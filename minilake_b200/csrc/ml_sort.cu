@@ -165,7 +165,8 @@ __global__ void k_sort_stats_init(unsigned long long* stats, int nwords) {
 // same digit serialize eight at a time, not 32.
 __global__ void __launch_bounds__(256) k_sort_keys(const SortWord* words, const __grid_constant__ SortSegs S,
                                                    const uint32_t* perm, int64_t n, uint32_t* keys, int digits,
-                                                   uint32_t* hist) {
+                                                   uint32_t* hist, const uint32_t* err) {
+    if (*err) return;  // perm was not written
     __shared__ uint32_t h[4 * 256 * 4];
     for (int i = threadIdx.x; i < digits * 1024; i += blockDim.x) h[i] = 0;
     __syncthreads();
@@ -223,6 +224,8 @@ constexpr int kPassThreads = 512, kPassItems = 16, kPassTile = kPassThreads * kP
 constexpr size_t kPassSmem = (size_t)kPassTile * 8 + (size_t)kPassWarps * 256 * 8 + 2 * 256 * 4;
 constexpr uint64_t kStatCount = 1ull << 62, kStatPrefix = 2ull << 62, kStatPoison = 3ull << 62, kStatValue = (1ull << 62) - 1;
 constexpr uint32_t kPassSpins = 1u << 21;  // polls of a predecessor's word (about a second)
+// A pass that gives up sets *err and leaves row ids unwritten; the kernels queued behind it read *err first
+// and touch no row.
 
 __global__ void __launch_bounds__(kPassThreads, 2)
     k_radix_pass(const uint32_t* keys_in, const uint32_t* rows_in, uint32_t n, int shift, const uint32_t* hist,
@@ -238,11 +241,15 @@ __global__ void __launch_bounds__(kPassThreads, 2)
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     if (tid == 0) {
         tile_s = atomicAdd(next_tile, 1u);
-        bad_s = 0;
+        bad_s = *(const volatile uint32_t*)err != 0;
     }
     for (uint32_t i = tid; i < kPassWarps * 256; i += kPassThreads) wdig[i] = make_uint2(0u, 0u);
     __syncthreads();
     const uint32_t tile = tile_s;
+    if (bad_s) {  // rows_in was not written, or this pass gave up: tiles behind this one need not wait
+        if (tid < 256) *(volatile uint64_t*)(status + (uint64_t)tile * 256 + tid) = kStatPoison;
+        return;
+    }
     const uint64_t base = (uint64_t)tile * kPassTile;
     const uint32_t rows = (uint32_t)min((uint64_t)kPassTile, (uint64_t)n - base);
     // a warp's rows are consecutive (512 of them), 32 per step: input order is warp, step, lane
@@ -353,7 +360,9 @@ __global__ void __launch_bounds__(kPassThreads, 2)
 // 41 us for 10M rows, eight in two 16-byte loads 26 us.
 constexpr uint32_t kSortRunMax = 64;
 __global__ void __launch_bounds__(256) k_sort_runs(const uint32_t* keys, const uint32_t* rows, const SortWord* words,
-                                                   int nwords, uint32_t n, uint2* list, uint32_t cap, uint32_t* state) {
+                                                   int nwords, uint32_t n, uint2* list, uint32_t cap, uint32_t* state,
+                                                   const uint32_t* err) {
+    if (*err) return;
     // an equal neighbour: whether this is its run's first inversion, and the run's ends
     auto check = [&](uint32_t i, uint32_t k) {
         if (!sort_less(words, nwords, rows[i], rows[i - 1])) return;
@@ -394,7 +403,8 @@ __global__ void __launch_bounds__(256) k_sort_runs(const uint32_t* keys, const u
 }
 // Each reported run put in order in place (an insertion sort, which keeps equal rows' order).
 __global__ void __launch_bounds__(256) k_sort_fix(uint32_t* rows, const SortWord* words, int nwords, const uint2* list,
-                                                  uint32_t cap, const uint32_t* state) {
+                                                  uint32_t cap, const uint32_t* state, const uint32_t* err) {
+    if (*err) return;
     const uint32_t m = min(state[0], cap);
     if (state[1]) return;  // every piece will be sorted instead
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
@@ -437,8 +447,8 @@ void launch_sort_bits(const SortWord* words, int nwords, int64_t n, unsigned lon
     if (n > 0 && nwords > 0) k_sort_bits<<<dim3(grid_rows(n, 256 * kWordRows, 6), nwords), 256, 0, s>>>(words, n, stats);
 }
 void launch_sort_keys(const SortWord* words, const SortSegs& S, const uint32_t* perm, int64_t n, uint32_t* keys, int digits,
-                      uint32_t* hist, cudaStream_t s) {
-    if (n > 0) k_sort_keys<<<grid_rows(n, 256 * kWordRows, 8), 256, 0, s>>>(words, S, perm, n, keys, digits, hist);
+                      uint32_t* hist, const uint32_t* err, cudaStream_t s) {
+    if (n > 0) k_sort_keys<<<grid_rows(n, 256 * kWordRows, 8), 256, 0, s>>>(words, S, perm, n, keys, digits, hist, err);
 }
 int64_t radix_tiles(int64_t n) { return (n + kPassTile - 1) / kPassTile; }
 cudaError_t launch_radix_pass(const uint32_t* keys_in, const uint32_t* rows_in, int64_t n, int shift, const uint32_t* hist,
@@ -453,10 +463,10 @@ cudaError_t launch_radix_pass(const uint32_t* keys_in, const uint32_t* rows_in, 
     return cudaSuccess;
 }
 void launch_sort_runs(const uint32_t* keys, uint32_t* rows, const SortWord* words, int nwords, int64_t n, uint2* list,
-                      uint32_t cap, uint32_t* state, cudaStream_t s) {
+                      uint32_t cap, uint32_t* state, const uint32_t* err, cudaStream_t s) {
     if (n < 2) return;
-    k_sort_runs<<<grid_rows(n, 256 * 8, 8), 256, 0, s>>>(keys, rows, words, nwords, (uint32_t)n, list, cap, state);
-    k_sort_fix<<<grid_rows(cap, 256, 4), 256, 0, s>>>(rows, words, nwords, list, cap, state);
+    k_sort_runs<<<grid_rows(n, 256 * 8, 8), 256, 0, s>>>(keys, rows, words, nwords, (uint32_t)n, list, cap, state, err);
+    k_sort_fix<<<grid_rows(cap, 256, 4), 256, 0, s>>>(rows, words, nwords, list, cap, state, err);
 }
 
 }  // namespace mlg
