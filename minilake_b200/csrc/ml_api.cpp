@@ -744,29 +744,32 @@ std::unique_ptr<ml_batch> topn_batch(Ctx* ctx, ml_batch& b, const std::vector<So
     const TopNPlan sel = k > kTopNWarpMax || n >= (1 << 21) ? topn_plan(S, n, (int)k) : TopNPlan{};
     DevBuf sb;
     if (sel.use) {
-        const size_t mn = 32, lp = mn + (sel.rank ? topn_minima_bytes() : 0), lr = lp + (size_t)sel.cap * 8, ro = lr + (((size_t)sel.cap * 4 + 15) & ~(size_t)15);
+        const size_t mn = 16 + sizeof(TopNBound), lp = mn + (sel.rank ? topn_minima_bytes() : 0), lr = lp + (size_t)sel.cap * 8;
+        const size_t ro = lr + (((size_t)sel.cap * 4 + 15) & ~(size_t)15);
         sb = DevBuf(ctx, ro + (size_t)k * 4, nullptr);
         uint8_t* base = sb.get<uint8_t>();
         uint32_t* state = (uint32_t*)base;
+        const uint32_t* rows = (const uint32_t*)(base + ro);
+        const TopNScratch t{state, (TopNBound*)(base + 16), (uint64_t*)(base + mn), (uint64_t*)(base + lp), (uint32_t*)(base + lr)};
         CK(cudaMemsetAsync(state, 0, 16, st));
-        {
-            KernelTimer kt(ctx, st, "topn");
-            CK(launch_topn_select(S, n, (int)k, sel, (uint64_t*)(base + 16), (uint64_t*)(base + mn), (uint64_t*)(base + lp), (uint32_t*)(base + lr),
-                                  state, (uint32_t*)(base + ro), st));
-            kt.stop();
-        }
-        ctx->count_launch(sel.rank ? 3 : 1);
         // fixed-width columns are gathered before the host knows that the rows are the result (k rows exist
         // either way); what a string column needs depends on the rows, and a budget counts what is asked for
         bool wait = ctx->pool.limit != UINT64_MAX;
         for (auto& c : b.cols) wait = wait || c->kind != CK_FIXED;
         ErrWord told(ctx);
-        CK(cudaMemcpyAsync(told.h, state + 1, 4, cudaMemcpyDeviceToHost, st));
-        if (wait) CK(cudaStreamSynchronize(st));
-        if (!wait || !*told.h) {
-            out->cols = gather_rows(ctx, b, (const uint32_t*)(base + ro), k, st, res);
-            if (!*told.h) return out;
-            out->cols.clear();
+        for (bool tied = false;; tied = true) {
+            KernelTimer kt(ctx, st, tied ? "topn_ties" : "topn");
+            CK(launch_topn_select(S, n, (int)k, sel, t, tied, (uint32_t*)rows, st));
+            kt.stop();
+            ctx->count_launch(sel.rank && !tied ? 3 : 1);
+            CK(cudaMemcpyAsync(told.h, state + 1, 4, cudaMemcpyDeviceToHost, st));
+            if (wait) CK(cudaStreamSynchronize(st));
+            if (!wait || !*told.h) {
+                out->cols = gather_rows(ctx, b, rows, k, st, res);
+                if (!*told.h) return out;
+                out->cols.clear();
+            }
+            if (tied || *told.h != kTopNTied) break;
         }
     }
     if (k <= kTopNWarpMax) {  // small limits: one sorted list per warp, one launch

@@ -1607,56 +1607,63 @@ __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackPieces
 }
 
 // ---- top-N by selection: limits up to kMaxTopN over a fixed-width first key ------------------------
-// k_topn_sample takes the r-th smallest key prefix of a sample of the rows, r chosen so that more than k
-// rows lie at or below it all but surely; k_topn_take streams the key column once and lists the rows at
-// or below; k_topn_finish finds the k-th of those exactly, keeps the rows up to it and sorts them.  The
-// host checks that the list held at least k rows and not more than it has room for (else every row goes
-// through k_topn_chunk / k_topn_warp).
+// k_topn_sample takes the r-th smallest row of a sample, r chosen so that more than k rows lie at or below
+// it all but surely; k_topn_take streams the key column once and lists the rows at or below; k_topn_finish
+// finds the k-th of those exactly, keeps the rows up to it and sorts them.  The host checks that the list
+// held at least k rows and not more than it has room for (else every row goes through k_topn_chunk /
+// k_topn_warp).
 // Why: the chunk sort orders all rows in shared memory, 2.0 ms for 20M rows and k = 100; the selection
 // reads the column at 5.1 to 5.9 TB/s (32 us), before it 13 us for the bound, after it 11 us for the
 // finish (a bound from 16,384 samples, eight times the rows in the list and a sort of them: 17 and 19 us).
+//
+// Rows whose first keys are equal (few distinct values, NULLs in front) are told apart as the whole sort
+// does, word by word (TopNLevel), only as far as it takes to leave few of them: in the bound, in the list
+// and in the k-th row alike.  A bound on the first key alone listed every tied row and gave up: 60M rows of
+// four values, LIMIT 10, took 2.5 ms a call (the per-warp lists alone 1.3), now 0.31; LIMIT 100 22.6 and 0.35 ms.
 
-// The block finds the r-th smallest (r >= 1) of n values get(i): by 8-bit digits from the highest bit in
-// which the values differ, counted in shared memory.  Returns an upper bound of it that no further value
-// lies below: all values <= the result are the m smallest, m returned in *taken.  With `slack` it may
-// stop early while at most `slack` more than r values are taken.
-// f(i, get(i)) for the block's values, eight of a thread's in flight together (one after the other, a
-// pass over 30,000 listed rows took 12 us).
-template <class Get, class F>
-__device__ __forceinline__ void block_values(Get get, uint32_t n, F f) {
+// f(i, get(i)) for the block's values with in(i), eight of a thread's in flight together (one after the
+// other, a pass over 30,000 listed rows took 12 us).  A value belongs to the thread i % blockDim.x.
+template <class Get, class In, class F>
+__device__ __forceinline__ void block_values(Get get, In in, uint32_t n, F f) {
     for (uint32_t i0 = threadIdx.x; i0 < n; i0 += 8 * blockDim.x) {
         uint64_t v[8];
+        bool a[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const uint32_t i = i0 + j * blockDim.x;
-            v[j] = i < n ? get(i) : 0ull;
+            a[j] = i < n && in(i);
+            v[j] = a[j] ? get(i) : 0ull;
         }
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const uint32_t i = i0 + j * blockDim.x;
-            if (i < n) f(i, v[j]);
-        }
+        for (int j = 0; j < 8; j++)
+            if (a[j]) f(i0 + j * blockDim.x, v[j]);
     }
 }
-template <class Get>
-__device__ uint64_t block_select(Get get, uint32_t n, uint32_t r, uint32_t slack, uint32_t* taken) {
+// The block finds the r-th smallest (r >= 1) of the `count` values get(i) with in(i), i < n, `ref` one of
+// them: by 8-bit digits from the highest bit in which the values differ, counted in shared memory.  Returns
+// an upper bound of it that no further value lies below: the values <= `bound` are the `below` + `last`
+// smallest.  It stops early where at most `slack` more than r values are taken, else the bound is the r-th
+// itself, `below` values lie below it and `last` are equal to it.
+struct BlockPick {
+    uint64_t bound;
+    uint32_t below, last;
+};
+template <class Get, class In>
+__device__ BlockPick block_select(Get get, In in, uint32_t n, uint32_t count, uint64_t ref, uint32_t r, uint32_t slack) {
     __shared__ uint32_t hist[256];
     __shared__ unsigned long long diff_s;
     __shared__ uint32_t digit_s, below_s, in_s;
     const uint32_t tid = threadIdx.x, lane = tid & 31;
-    const uint64_t ref = get(0);
     uint64_t diff = 0;
+    __syncthreads();
     if (tid == 0) diff_s = 0;
     __syncthreads();
-    block_values(get, n, [&](uint32_t, uint64_t v) { diff |= v ^ ref; });
+    block_values(get, in, n, [&](uint32_t, uint64_t v) { diff |= v ^ ref; });
     const uint32_t dlo = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)diff), dhi = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)(diff >> 32));
     if (lane == 0) atomicOr(&diff_s, ((unsigned long long)dhi << 32) | dlo);
     __syncthreads();
     diff = diff_s;
-    if (!diff) {
-        *taken = n;
-        return ref;
-    }
+    if (!diff) return BlockPick{ref, 0, count};
     int top = 64 - __clzll((long long)diff);           // bits [0, top) are undecided
     uint64_t want = top < 64 ? ref >> top << top : 0;  // the decided bits
     uint32_t before = 0;                               // values below the range of `want`
@@ -1664,7 +1671,7 @@ __device__ uint64_t block_select(Get get, uint32_t n, uint32_t r, uint32_t slack
         const int low = top > 8 ? top - 8 : 0;
         for (uint32_t i = tid; i < 256; i += blockDim.x) hist[i] = 0;
         __syncthreads();
-        block_values(get, n, [&](uint32_t, uint64_t x) {
+        block_values(get, in, n, [&](uint32_t, uint64_t x) {
             const uint64_t v = x ^ want;
             if (top == 64 || (v >> top) == 0) atomicAdd(&hist[(v >> low) & ((1u << (top - low)) - 1u)], 1u);
         });
@@ -1694,21 +1701,105 @@ __device__ uint64_t block_select(Get get, uint32_t n, uint32_t r, uint32_t slack
             }
         }
         __syncthreads();
-        const uint32_t below = below_s, in = in_s;
+        const uint32_t below = below_s, last = in_s;
         want |= (uint64_t)digit_s << low;
         before = below;
         top = low;
-        if (top == 0 || below + in <= r + slack) {
-            *taken = below + in;
-            return top ? want | ((1ull << top) - 1) : want;
-        }
+        if (top == 0 || below + last <= r + slack) return BlockPick{top ? want | ((1ull << top) - 1) : want, below, last};
         __syncthreads();  // hist and the digit are rewritten
     }
 }
 
-// The bound: one row of each of `samples` equal pieces of the column, the smallest prefix of every 4 or 32
-// samples (kTopNMinima of them), and the r-th smallest of those, found by the last block to finish (`done`
-// starts at zero).  At least r samples lie at or below it.  The samples of one minimum come from pieces all
+// A row's word at a level past the first (the first is the first key's prefix): smaller sorts first.
+__device__ __forceinline__ uint64_t level_value(const SortDev& S, int key, int what, uint32_t r) {
+    if (what == TL_ROW) return r;
+    const DCol& c = S.cols[key];
+    const bool valid = valid_bit(c.valid, r);
+    if (what == TL_NULL) return (valid == (S.nulls_first[key] != 0)) ? 1ull : 0ull;
+    if (!valid) return 0ull;
+    uint64_t x;
+    if (c.kind == CK_UTF8) {
+        const Str s = col_str(c, r);
+        x = s.n;
+        if (what != TL_LENGTH) {
+            x = 0;
+            for (uint32_t j = 0, b0 = 8u * (uint32_t)what; j < 8; j++)
+                if (b0 + j < s.n) x |= (uint64_t)__ldg(s.p + b0 + j) << (56 - 8 * j);
+        }
+    } else {
+        x = load_value(c, r);
+        if (c.dt == ML_TYPE_FLOAT64) x = (uint64_t)total_key(as_f64(x)) ^ 0x8000000000000000ull;
+        else if (c.dt != ML_TYPE_BOOL) x ^= 0x8000000000000000ull;
+    }
+    return S.asc[key] ? x : ~x;
+}
+// The level after {key, what}: per key its NULL flag, where it has any, and its value, or the eight-byte
+// pieces of a string (`more`: some rows' strings go on after the last one) and then its length; at last the
+// row id, so that no two rows are equal.  The first key has only its NULL flag left (kind TL_NULL).
+__device__ __forceinline__ void next_level(const SortDev& S, bool first, bool more, int& key, int& what) {
+    if (first && S.cols[0].valid) {
+        what = TL_NULL;
+    } else if (what == TL_NULL && key > 0) {
+        what = 0;
+    } else if (key > 0 && what >= 0 && S.cols[key].kind == CK_UTF8) {
+        what = more ? what + 1 : TL_LENGTH;
+    } else if (++key == S.nkeys) {
+        what = TL_ROW;
+    } else {
+        what = S.cols[key].valid ? TL_NULL : 0;
+    }
+}
+// Whether a row with the bound's first prefix lies at or below the bound.
+__device__ __noinline__ bool tie_within(const SortDev& S, const TopNBound* B, uint32_t r) {
+    for (int l = 1; l < B->n; l++) {
+        const TopNLevel& L = B->lv[l];
+        const uint64_t x = level_value(S, L.key, L.what, r);
+        if (x != L.v) return x < L.v;
+    }
+    return true;
+}
+// The block tells n rows {p[i], row[i]} apart, of which `pick` (block_select on p) leaves too many: level by
+// level, until at most `slack` more than the r wanted are left, or the levels are used up.  below(row) for
+// each row below a level's bound; the rows at the last one have row[i] != kNone and p[i] <= the bound
+// returned (p[i] then being that level's word).  The levels' bounds are added to *B (optional; one thread
+// writes).  p and row are overwritten.
+template <class Below>
+__device__ BlockPick block_refine(const SortDev& S, uint64_t* p, uint32_t* row, uint32_t n, BlockPick pick, uint32_t r, uint32_t slack,
+                                  TopNBound* B, Below below) {
+    __shared__ uint64_t ref_s;
+    auto row_at = [&](uint32_t i) -> uint32_t { return *(const volatile uint32_t*)(row + i); };  // from L2: another block's, or rewritten here
+    auto alive = [&](uint32_t i) { return row_at(i) != kNone; };
+    int key = 0, what = 0;
+    for (int l = 1; l < kTopNLevels; l++) {
+        if (pick.below + pick.last <= r + slack || what == TL_ROW) break;
+        r -= pick.below;
+        bool more = false;
+        block_values([&](uint32_t i) { return p[i]; }, alive, n, [&](uint32_t i, uint64_t x) {
+            const uint32_t t = row_at(i);
+            if (x < pick.bound) below(t);
+            if (x != pick.bound) row[i] = kNone;
+            else if (key > 0 && what >= 0 && S.cols[key].kind == CK_UTF8 && valid_bit(S.cols[key].valid, t))
+                more = more || col_str(S.cols[key], t).n > 8u * (uint32_t)(what + 1);
+        });
+        more = __syncthreads_or(more);
+        next_level(S, l == 1, more, key, what);
+        block_values([&](uint32_t i) { return level_value(S, key, what, row_at(i)); }, alive, n, [&](uint32_t i, uint64_t x) {
+            p[i] = x;
+            ref_s = x;  // any of them
+        });
+        __syncthreads();
+        pick = block_select([&](uint32_t i) { return p[i]; }, alive, n, pick.last, ref_s, r, slack);
+        if (B && threadIdx.x == 0) {
+            B->lv[l] = TopNLevel{key, what, pick.bound};
+            B->n = l + 1;
+        }
+    }
+    return pick;
+}
+
+// The bound: one row of each of `samples` equal pieces of the column, the first in the sort's order of every 4
+// or 32 samples (kTopNMinima of them), and the r-th of those, found by the last block to finish (`done` starts
+// at zero).  At least r samples lie at or below it.  The samples of one minimum come from pieces all
 // over the column, in no pattern: of neighbouring pieces of a sorted column one would be the smallest and
 // hide 31 almost as small, and the list would hold 32 times the rows that it has room for.  Many blocks,
 // because the rows lie far apart (one block took 25 us for 16,384 of them), and large ones, because the last
@@ -1716,7 +1807,7 @@ __device__ uint64_t block_select(Get get, uint32_t n, uint32_t r, uint32_t slack
 constexpr uint32_t kTopNMinima = 4096;
 template <int DT>
 __global__ void __launch_bounds__(1024) k_topn_sample(const __grid_constant__ SortDev S, int64_t n, uint32_t samples, uint32_t r,
-                                                     uint64_t* minima, uint32_t* done, uint64_t* bound) {
+                                                     uint64_t* minima, uint32_t* min_rows, uint32_t* done, TopNBound* bound) {
     __shared__ uint64_t mins[kTopNMinima];
     __shared__ bool last;
     const DCol& c = S.cols[0];
@@ -1732,14 +1823,24 @@ __global__ void __launch_bounds__(1024) k_topn_sample(const __grid_constant__ So
     x ^= x >> 15;
     x *= 0x85EBCA6Bu;
     x ^= x >> 13;
-    const uint32_t row = (uint32_t)((uint64_t)piece * (uint64_t)n / samples + x % step);
+    uint32_t row = (uint32_t)((uint64_t)piece * (uint64_t)n / samples + x % step);
     uint64_t p = fixed_prefix<DT>(load_value(c, row), valid_bit(c.valid, row), flip, nullp);
     const uint32_t lanes = samples / kTopNMinima;
+    const bool only = S.nkeys == 1 && !c.valid;  // equal prefixes are equal keys
     for (uint32_t o = lanes >> 1; o; o >>= 1) {
         const uint64_t q = __shfl_xor_sync(0xFFFFFFFFu, p, o);
-        p = q < p ? q : p;
+        const uint32_t t = __shfl_xor_sync(0xFFFFFFFFu, row, o);
+        int before = q < p ? -1 : q > p;
+        if (before == 0 && !only) before = cmp_rows(S, t, row);
+        if (before < 0 || (before == 0 && t < row)) {
+            p = q;
+            row = t;
+        }
     }
-    if (i % lanes == 0) minima[i / lanes] = p;
+    if (i % lanes == 0) {
+        minima[i / lanes] = p;
+        min_rows[i / lanes] = row;
+    }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
@@ -1748,20 +1849,31 @@ __global__ void __launch_bounds__(1024) k_topn_sample(const __grid_constant__ So
     __threadfence();
     for (uint32_t j = threadIdx.x; j < kTopNMinima; j += 1024) mins[j] = __ldcg((const unsigned long long*)minima + j);
     __syncthreads();
-    uint32_t taken;
-    const uint64_t b = block_select([&](uint32_t j) { return mins[j]; }, kTopNMinima, r, r, &taken);
-    if (threadIdx.x == 0) *bound = b;
+    const BlockPick pick = block_select([&](uint32_t j) { return mins[j]; }, [](uint32_t) { return true; }, kTopNMinima, kTopNMinima,
+                                        mins[0], r, r);
+    if (threadIdx.x == 0) {
+        bound->lv[0] = TopNLevel{0, 0, pick.bound};
+        bound->n = 1;
+    }
+    if (pick.below + pick.last > 2 * r) block_refine(S, mins, min_rows, kTopNMinima, pick, r, r, bound, [](uint32_t) {});
 }
 
-// Rows whose prefix is at or below *bound: {prefix, row} appended to the list (*count of them, those past
-// `cap` counted only).  Bound by streaming the column: four loads of four rows each in flight per thread.
+// Rows at or below the bound: {prefix, row} appended to the list (*count of them, those past `cap` counted
+// only, and a warp stops at its next).  Bound by streaming the column: four loads of four rows each in flight
+// per thread; a warp's rows of a step take their places with one addition.  (A read of the count in every step,
+// to stop at once, puts all warps on one L2 sector: 60M doubles 108 us for 82.)
 template <int DT>
-__global__ void __launch_bounds__(256) k_topn_take(const __grid_constant__ SortDev S, int64_t n, const uint64_t* bound,
+__global__ void __launch_bounds__(256) k_topn_take(const __grid_constant__ SortDev S, int64_t n, const TopNBound* bound,
                                                    uint64_t* list_p, uint32_t* list_r, uint32_t cap, uint32_t* count) {
     const DCol& c = S.cols[0];
     const bool vec = ((uintptr_t)c.data & 15) == 0;
-    const uint64_t flip = S.asc[0] ? 0ull : ~0ull, nullp = S.nulls_first[0] ? 0ull : ~0ull, b = __ldg(bound);
-    const uint32_t n32 = (uint32_t)n;
+    const uint64_t flip = S.asc[0] ? 0ull : ~0ull, nullp = S.nulls_first[0] ? 0ull : ~0ull, b = bound->lv[0].v;
+    const int levels = bound->n, what1 = bound->lv[1].what;
+    const uint64_t v1 = bound->lv[1].v;
+    // equal prefixes: every row (no further level), the rows up to one, or by their levels
+    const bool by_row = levels == 2 && what1 == TL_ROW, by_levels = levels > 1 && !by_row;
+    const uint32_t row_max = by_row ? (uint32_t)v1 : ~0u;
+    const uint32_t n32 = (uint32_t)n, lane = threadIdx.x & 31;
     constexpr int kQuads = 4;
     for (int64_t base = (int64_t)blockIdx.x * (256 * 4 * kQuads); base < n; base += (int64_t)gridDim.x * (256 * 4 * kQuads)) {
         Quad q[kQuads];
@@ -1771,6 +1883,7 @@ __global__ void __launch_bounds__(256) k_topn_take(const __grid_constant__ SortD
             q[j] = Quad{0, 0, 0, 0};
             if (r0 < n) q[j] = load_quad<DT>(c, vec, n32, (uint32_t)r0);
         }
+        uint32_t hit = 0, tied = 0;  // of the thread's 16 rows: below the bound's prefix, at it
 #pragma unroll
         for (int j = 0; j < kQuads; j++) {
             const int64_t r0 = base + (int64_t)(j * 256 + threadIdx.x) * 4;
@@ -1782,60 +1895,51 @@ __global__ void __launch_bounds__(256) k_topn_take(const __grid_constant__ SortD
             if (p[0] > b && p[1] > b && p[2] > b && p[3] > b) continue;
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                if (p[k] > b || r0 + k >= n) continue;
-                const uint32_t at = atomicAdd(count, 1u);
-                if (at < cap) {
-                    list_p[at] = p[k];
-                    list_r[at] = (uint32_t)r0 + k;
-                }
+                if (r0 + k >= n) continue;
+                if (p[k] < b) hit |= 1u << (4 * j + k);
+                else if (p[k] == b && (uint32_t)r0 + k <= row_max) tied |= 1u << (4 * j + k);
             }
+        }
+        const uint32_t r0 = (uint32_t)base + threadIdx.x * 4;
+        auto row_of = [&](int x) { return r0 + (uint32_t)(x >> 2) * 1024u + (uint32_t)(x & 3); };
+        if (by_levels) {
+#pragma unroll 1
+            for (; tied; tied &= tied - 1)
+                if (tie_within(S, bound, row_of(__ffs(tied) - 1))) hit |= tied & (0u - tied);
+        }
+        hit |= tied;
+        if (!__any_sync(0xFFFFFFFFu, hit != 0)) continue;
+        uint32_t at = __popc(hit);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, at, o);
+            if ((int)lane >= o) at += t;
+        }
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, at, 31);
+        uint32_t start = 0;
+        if (lane == 0) start = atomicAdd(count, total);
+        start = __shfl_sync(0xFFFFFFFFu, start, 0);
+        if (start > cap) return;
+        at += start - __popc(hit);
+#pragma unroll 1
+        for (; hit && at < cap; hit &= hit - 1, at++) {
+            const uint32_t r = row_of(__ffs(hit) - 1);
+            list_p[at] = fixed_prefix<DT>(load_value(c, r), valid_bit(c.valid, r), flip, nullp);
+            list_r[at] = r;
         }
     }
 }
 
-// The best k rows of the list (list_p == nullptr: of the rows 0..n themselves), sorted, into out[0..k).
-// state[0]: rows listed (in); state[1]: set when the list does not give the result.
+// Rows in the sort's order, the best k of the m in {pre, idx} (room for kTopNSort; pre is the first key's prefix).
 constexpr uint32_t kTopNSort = 4096;
-template <int DT>
-__global__ void __launch_bounds__(1024) k_topn_finish(const __grid_constant__ SortDev S, const uint64_t* list_p,
-                                                      const uint32_t* list_r, uint32_t cap, int64_t n, int k, uint32_t* state,
-                                                      uint32_t* out) {
-    extern __shared__ __align__(16) uint64_t pre[];
-    uint32_t* idx = (uint32_t*)(pre + kTopNSort);
-    __shared__ uint32_t m_s;
-    const DCol& c = S.cols[0];
-    const uint64_t flip = S.asc[0] ? 0ull : ~0ull, nullp = S.nulls_first[0] ? 0ull : ~0ull;
-    const uint32_t m = list_p ? state[0] : (uint32_t)n;
-    for (int j = threadIdx.x; j < k; j += 1024) out[j] = j;  // rows that exist, whatever comes of it
-    if (threadIdx.x == 0) m_s = 0;
-    if (m < (uint32_t)k || (list_p && m > cap)) {
-        if (threadIdx.x == 0) state[1] = 1;
-        return;
-    }
-    auto get = [&](uint32_t i) -> uint64_t {
-        return list_p ? __ldg((const unsigned long long*)list_p + i)
-                      : fixed_prefix<DT>(load_value(c, i), valid_bit(c.valid, i), flip, nullp);
-    };
-    uint32_t taken;
-    const uint64_t bound = block_select(get, m, (uint32_t)k, max((uint32_t)k / 4, 32u), &taken);
-    if (taken > kTopNSort) {  // ties at the limit beyond what the sort holds
-        if (threadIdx.x == 0) state[1] = 1;
-        return;
-    }
+__device__ __forceinline__ void put_rows(const SortDev& S, uint64_t* pre, uint32_t* idx, uint32_t taken, int k, uint32_t* out) {
     uint32_t size = 2;
     while (size < taken) size *= 2;
     const bool few = taken <= 512;  // placed by counting: no steps to wait for
-    for (uint32_t i = threadIdx.x; i < size && !few; i += 1024) {
+    for (uint32_t i = taken + threadIdx.x; i < size && !few; i += 1024) {
         pre[i] = ~0ull;
         idx[i] = kNone;
     }
-    __syncthreads();
-    block_values(get, m, [&](uint32_t i, uint64_t p) {
-        if (p > bound) return;
-        const uint32_t at = atomicAdd(&m_s, 1u);
-        pre[at] = p;
-        idx[at] = list_p ? __ldg(list_r + i) : i;
-    });
     __syncthreads();
     if (few) {
         // two threads per row count the rows before it, half of them each
@@ -1859,6 +1963,85 @@ __global__ void __launch_bounds__(1024) k_topn_finish(const __grid_constant__ So
     }
     bitonic_rows(S, pre, idx, (int)size);
     for (int j = threadIdx.x; j < k; j += 1024) out[j] = idx[j];
+}
+
+// The best k rows of the list (list_p == nullptr: of the rows 0..n themselves), sorted, into out[0..k).
+// state[0]: rows listed (in); state[1]: set when the list does not give the result, to kTopNTied when that
+// takes telling apart many rows with the k-th row's first key: k_topn_ties does that, in a kernel of its own
+// (its code in here made this one 9.2 -> 10.6 us).
+template <int DT>
+__global__ void __launch_bounds__(1024) k_topn_finish(const __grid_constant__ SortDev S, const uint64_t* list_p,
+                                                      const uint32_t* list_r, uint32_t cap, int64_t n, int k, uint32_t* state,
+                                                      uint32_t* out) {
+    extern __shared__ __align__(16) uint64_t pre[];
+    uint32_t* idx = (uint32_t*)(pre + kTopNSort);
+    __shared__ uint32_t m_s;
+    const DCol& c = S.cols[0];
+    const uint64_t flip = S.asc[0] ? 0ull : ~0ull, nullp = S.nulls_first[0] ? 0ull : ~0ull;
+    const uint32_t m = list_p ? state[0] : (uint32_t)n;
+    for (int j = threadIdx.x; j < k; j += 1024) out[j] = j;  // rows that exist, whatever comes of it
+    if (threadIdx.x == 0) m_s = 0;
+    if (m < (uint32_t)k || (list_p && m > cap)) {
+        if (threadIdx.x == 0) state[1] = 1;
+        return;
+    }
+    auto get = [&](uint32_t i) -> uint64_t {
+        return list_p ? __ldg((const unsigned long long*)list_p + i)
+                      : fixed_prefix<DT>(load_value(c, i), valid_bit(c.valid, i), flip, nullp);
+    };
+    auto all = [](uint32_t) { return true; };
+    const uint32_t slack = max((uint32_t)k / 4, 32u);
+    const BlockPick pick = block_select(get, all, m, m, get(0), (uint32_t)k, slack);
+    const uint32_t taken = pick.below + pick.last;
+    if (taken > (uint32_t)k + slack) {
+        if (threadIdx.x == 0) state[1] = kTopNTied;
+        return;
+    }
+    block_values(get, all, m, [&](uint32_t i, uint64_t p) {
+        if (p > pick.bound) return;
+        const uint32_t at = atomicAdd(&m_s, 1u);
+        pre[at] = p;
+        idx[at] = list_p ? __ldg(list_r + i) : i;
+    });
+    put_rows(S, pre, idx, taken, k, out);
+}
+// The same where many of the m rows have the k-th row's first key; `direct`: of the rows 0..m themselves, the
+// list being room for as many.  state[1]: 0, or 1 when the levels do not tell them apart.
+template <int DT>
+__global__ void __launch_bounds__(1024) k_topn_ties(const __grid_constant__ SortDev S, uint64_t* list_p, uint32_t* list_r, bool direct,
+                                                    int64_t n, int k, uint32_t* state, uint32_t* out) {
+    extern __shared__ __align__(16) uint64_t pre[];
+    uint32_t* idx = (uint32_t*)(pre + kTopNSort);
+    __shared__ uint32_t m_s;
+    const DCol& c = S.cols[0];
+    const uint64_t flip = S.asc[0] ? 0ull : ~0ull, nullp = S.nulls_first[0] ? 0ull : ~0ull;
+    const uint32_t m = direct ? (uint32_t)n : state[0], slack = max((uint32_t)k / 4, 32u);
+    auto prefix = [&](uint32_t r) { return fixed_prefix<DT>(load_value(c, r), valid_bit(c.valid, r), flip, nullp); };
+    auto all = [](uint32_t) { return true; };
+    auto row_at = [&](uint32_t i) -> uint32_t { return *(const volatile uint32_t*)(list_r + i); };
+    auto get = [&](uint32_t i) { return list_p[i]; };
+    auto keep = [&](uint32_t r) { idx[atomicAdd(&m_s, 1u)] = r; };
+    if (threadIdx.x == 0) m_s = 0;
+    if (direct)
+        block_values(prefix, all, m, [&](uint32_t i, uint64_t p) {
+            list_p[i] = p;
+            list_r[i] = i;
+        });
+    __syncthreads();
+    const uint64_t ref = list_p[0];
+    BlockPick pick = block_select(get, all, m, m, ref, (uint32_t)k, slack);
+    pick = block_refine(S, list_p, list_r, m, pick, (uint32_t)k, slack, nullptr, keep);  // keeps fewer than k
+    __syncthreads();
+    const uint32_t taken = m_s + pick.below + pick.last;
+    __syncthreads();  // m_s grows again
+    if (threadIdx.x == 0) state[1] = taken > kTopNSort;
+    if (taken > kTopNSort) return;
+    block_values(get, [&](uint32_t i) { return row_at(i) != kNone; }, m, [&](uint32_t i, uint64_t p) {
+        if (p <= pick.bound) keep(row_at(i));
+    });
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < taken; i += 1024) pre[i] = prefix(idx[i]);
+    put_rows(S, pre, idx, taken, k, out);
 }
 
 }  // namespace
@@ -2087,6 +2270,7 @@ TopNPlan topn_plan(const SortDev& S, int64_t n, int k) {
     if (S.nkeys < 1 || c.kind != CK_FIXED || c.src != 0 || k < 1 || k > kMaxTopN || n < k) return p;
     if (n <= kTopNDirect) {
         p.use = true;
+        p.cap = (uint32_t)n;
         return p;
     }
     // the sample's rank: k rows of n are `mean` of the sample on average; six standard deviations and
@@ -2103,29 +2287,37 @@ TopNPlan topn_plan(const SortDev& S, int64_t n, int k) {
     p.cap = (uint32_t)(8 * rows) + 4096;
     return p;
 }
-size_t topn_minima_bytes() { return kTopNMinima * 8; }
+size_t topn_minima_bytes() { return kTopNMinima * 12; }
 template <int DT>
-static cudaError_t topn_select(const SortDev& S, int64_t n, int k, const TopNPlan& p, uint64_t* bound, uint64_t* minima, uint64_t* list_p,
-                               uint32_t* list_r, uint32_t* state, uint32_t* out, cudaStream_t s) {
+static cudaError_t topn_select(const SortDev& S, int64_t n, int k, const TopNPlan& p, const TopNScratch& t, bool tied, uint32_t* out,
+                               cudaStream_t s) {
     // per call: the attribute belongs to the current device's copy of the kernel
     constexpr int sort_b = kTopNSort * 12;
-    cudaError_t e = cudaFuncSetAttribute(k_topn_finish<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_b);
+    const cudaError_t e = tied ? cudaFuncSetAttribute(k_topn_ties<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_b)
+                               : cudaFuncSetAttribute(k_topn_finish<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_b);
     if (e != cudaSuccess) return e;
-    if (p.rank) {
-        k_topn_sample<DT><<<p.samples / 1024, 1024, 0, s>>>(S, n, p.samples, p.rank, minima, state + 2, bound);
-        const int64_t want = (n + 4095) / 4096;
-        k_topn_take<DT><<<(int)std::min<int64_t>(want, (int64_t)num_sms() * 8), 256, 0, s>>>(S, n, bound, list_p, list_r, p.cap, state);
+    if (tied) {
+        k_topn_ties<DT><<<1, 1024, sort_b, s>>>(S, t.list_p, t.list_r, p.rank == 0, n, k, t.state, out);
+        return cudaSuccess;
     }
-    k_topn_finish<DT><<<1, 1024, sort_b, s>>>(S, p.rank ? list_p : nullptr, list_r, p.cap, n, k, state, out);
+    if (p.rank) {
+        k_topn_sample<DT><<<p.samples / 1024, 1024, 0, s>>>(S, n, p.samples, p.rank, t.minima, (uint32_t*)(t.minima + kTopNMinima),
+                                                           t.state + 2, t.bound);
+        const int64_t want = (n + 4095) / 4096;
+        // two rounds of the five blocks that fit an SM (60M doubles 82 us; eight per SM 85, one round 87)
+        k_topn_take<DT><<<(int)std::min<int64_t>(want, (int64_t)num_sms() * 10), 256, 0, s>>>(S, n, t.bound, t.list_p, t.list_r, p.cap,
+                                                                                              t.state);
+    }
+    k_topn_finish<DT><<<1, 1024, sort_b, s>>>(S, p.rank ? t.list_p : nullptr, t.list_r, p.cap, n, k, t.state, out);
     return cudaSuccess;
 }
-cudaError_t launch_topn_select(const SortDev& S, int64_t n, int k, const TopNPlan& p, uint64_t* bound, uint64_t* minima, uint64_t* list_p,
-                               uint32_t* list_r, uint32_t* state, uint32_t* out, cudaStream_t s) {
+cudaError_t launch_topn_select(const SortDev& S, int64_t n, int k, const TopNPlan& p, const TopNScratch& t, bool tied, uint32_t* out,
+                               cudaStream_t s) {
     switch (S.cols[0].dt) {
-        case ML_TYPE_FLOAT64: return topn_select<ML_TYPE_FLOAT64>(S, n, k, p, bound, minima, list_p, list_r, state, out, s);
-        case ML_TYPE_INT64: return topn_select<ML_TYPE_INT64>(S, n, k, p, bound, minima, list_p, list_r, state, out, s);
-        case ML_TYPE_BOOL: return topn_select<ML_TYPE_BOOL>(S, n, k, p, bound, minima, list_p, list_r, state, out, s);
-        default: return topn_select<ML_TYPE_INT32>(S, n, k, p, bound, minima, list_p, list_r, state, out, s);
+        case ML_TYPE_FLOAT64: return topn_select<ML_TYPE_FLOAT64>(S, n, k, p, t, tied, out, s);
+        case ML_TYPE_INT64: return topn_select<ML_TYPE_INT64>(S, n, k, p, t, tied, out, s);
+        case ML_TYPE_BOOL: return topn_select<ML_TYPE_BOOL>(S, n, k, p, t, tied, out, s);
+        default: return topn_select<ML_TYPE_INT32>(S, n, k, p, t, tied, out, s);
     }
 }
 int launch_topn_warp(const SortDev& S, int64_t n, int k, int blocks, uint32_t* out, void* cand, unsigned int* done,

@@ -224,14 +224,34 @@ constexpr int64_t kTopNDirect = 65536;  // up to here the rows are the list
 struct TopNPlan {
     bool use;
     uint32_t samples, rank;  // sampled rows and the bound's rank among them; rank 0: no sample and no list
-    uint32_t cap;            // rows the list has room for
+    uint32_t cap;            // rows the list has room for (rank 0: all rows, should they tie)
+};
+// The sort key of a row as words, the most significant first: the first key's prefix (fixed-width), then
+// where that is not enough its NULL flag, the other keys' words (next_level) and the row id.
+enum TopNWord : int32_t { TL_ROW = -3, TL_LENGTH = -2, TL_NULL = -1 };  // >= 0: the value, or a string's eight-byte piece
+struct TopNLevel {
+    int32_t key, what;
+    uint64_t v;
+};
+constexpr int kTopNLevels = 32;
+struct TopNBound {  // rows at or below: the first n levels' words, compared in order
+    int32_t n, pad;
+    TopNLevel lv[kTopNLevels];
 };
 size_t topn_minima_bytes();
 TopNPlan topn_plan(const SortDev& S, int64_t n, int k);
-// out[0 .. k): the rows, sorted, unless state[1] is set afterwards (then they are the rows 0 .. k - 1).  bound: one word;
-// minima: topn_minima_bytes(); list_p / list_r: p.cap entries each; state: three zeroed words.
-cudaError_t launch_topn_select(const SortDev& S, int64_t n, int k, const TopNPlan& p, uint64_t* bound, uint64_t* minima, uint64_t* list_p,
-                               uint32_t* list_r, uint32_t* state, uint32_t* out, cudaStream_t s);
+struct TopNScratch {
+    uint32_t* state;   // three zeroed words
+    TopNBound* bound;
+    uint64_t* minima;  // topn_minima_bytes()
+    uint64_t* list_p;  // the plan's cap entries each
+    uint32_t* list_r;
+};
+// out[0 .. k): the rows, sorted, unless state[1] is set afterwards (then they are the rows 0 .. k - 1).  When it
+// is kTopNTied, many rows have the k-th row's first key: a second call with `tied` finishes the selection.
+constexpr uint32_t kTopNTied = 2;
+cudaError_t launch_topn_select(const SortDev& S, int64_t n, int k, const TopNPlan& p, const TopNScratch& t, bool tied, uint32_t* out,
+                               cudaStream_t s);
 // Top-k for k <= kTopNWarpMax: each CTA writes its best k rows (sorted) to out[block * k ..].
 constexpr int kTopNWarpMax = 32;
 int topn_warp_blocks(int64_t n);
