@@ -1277,6 +1277,7 @@ int ml_gpu_batch_fetch_all(const ml_batch* b, int32_t ncols, void* const* values
         ctx->count_launch();
         CK(cudaMemcpyAsync(host, packed.get(), total, cudaMemcpyDeviceToHost, op_stream.s));
         CK(cudaStreamSynchronize(op_stream.s));
+        st.waited();
         int q = 0;
         for (int i = 0; i < ncols; i++) {
             const DevColumn& c = *b->cols[i];
@@ -3140,6 +3141,7 @@ std::unique_ptr<ml_batch> hashagg_emit(ml_hashagg* h, cudaStream_t s) {
             CK(cudaMemcpyAsync(host + x.at + ((size_t)ng * 4 + 7) / 8 * 8, x.col->validity.get(), vbytes, cudaMemcpyDeviceToHost, s));
         }
         CK(cudaStreamSynchronize(s));
+        stg.waited();
         std::vector<std::vector<uint32_t>> offs;
         std::vector<std::string> bytes;
         size_t out_b = 0;

@@ -322,20 +322,23 @@ void Ctx::drain_timings(size_t keep) {  // collect all but the newest `keep` tim
 
 void Staging::release() {
     if (!p_) return;
-    cudaStreamSynchronize(s_);
+    if (busy_) cudaStreamSynchronize(s_);
+    busy_ = false;
     ctx_->hfree(p_);
     p_ = nullptr;
     cap_ = 0;
 }
 void* Staging::get(size_t bytes, cudaStream_t s) {
-    if (p_) CK(cudaStreamSynchronize(s_));
-    s_ = s;
+    if (busy_) CK(cudaStreamSynchronize(s_));
+    busy_ = false;
     if (bytes > cap_) {
         const size_t cap = std::max(bytes, cap_ * 2);
         release();
         p_ = ctx_->halloc(cap);
         cap_ = cap;
     }
+    s_ = s;
+    busy_ = true;
     return p_;
 }
 

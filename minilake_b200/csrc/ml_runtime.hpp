@@ -190,12 +190,15 @@ class Staging {
     Staging(const Staging&) = delete;
     // `bytes` for a copy on stream s, once the copies from earlier calls are done (one wait of that stream).
     void* get(size_t bytes, cudaStream_t s);
+    // The caller has waited for its copies: they need no other wait.
+    void waited() { busy_ = false; }
     // The block back to the pool; call it before the stream goes back to its own.
     void release();
 
    private:
     Ctx* ctx_;
     cudaStream_t s_ = nullptr;  // of the last get
+    bool busy_ = false;         // copies on it may be in flight
     void* p_ = nullptr;
     size_t cap_ = 0;
 };
