@@ -2049,6 +2049,7 @@ struct ml_hashagg {
     double max_load = 0.5;
     bool hinted = false;               // the caller gave the number of groups: the table is sized by it
     std::atomic<bool> sized{false};    // a batch has shown how many groups to expect (sink_ranges)
+    std::atomic<bool> fed{false};      // rows were aggregated: there may be groups
     int stride = 1;        // u64 words per group block
     std::shared_mutex rw;  // shared: a launch in flight; exclusive: table growth
     uint64_t cap = 0;
@@ -2737,6 +2738,7 @@ int ml_gpu_hashagg_sink(ml_hashagg_local* local, const ml_column* cols, int32_t 
     constexpr int64_t kFirstRows = 65536;
     const bool ranges = can_overflow && !h->hinted && !h->sized && n >= 4 * kFirstRows && (int64_t)h->gid_cap < n / 4 &&
                         jit_enabled(ctx) && !h->str_minmax;
+    const bool fresh = n > 0 && !h->fed.exchange(true);
     if (!ranges) {
         room(n);
         uint64_t count;
@@ -2757,9 +2759,11 @@ int ml_gpu_hashagg_sink(ml_hashagg_local* local, const ml_column* cols, int32_t 
     };
     uint64_t count;
     bool skipped;
+    double base = 0;  // groups before this batch: earlier batches' and other threads', which tell nothing of its rows
     room(n);
     {
         std::shared_lock<std::shared_mutex> lk(h->rw);
+        if (!fresh) base = (double)groups();
         begin();
         launch(0, kFirstRows, nullptr);
         launch_agg_guard(d_count, h->ngroups.get<uint32_t>(), h->gid_cap, d_skip, s);
@@ -2770,7 +2774,7 @@ int ml_gpu_hashagg_sink(ml_hashagg_local* local, const ml_column* cols, int32_t 
     }
     resume(count);
     if (skipped) {
-        double g0 = 0, rate0 = 0, rate = 0;  // groups before the last range; new groups per row, first and last
+        double g0 = 0, rate0 = 0, rate = 0;  // new groups before the last range; new groups per row, first and last
         int64_t done = kFirstRows, last = kFirstRows;
         while (done < n) {
             int64_t next = std::min(n - done, 8 * done);
@@ -2780,16 +2784,20 @@ int ml_gpu_hashagg_sink(ml_hashagg_local* local, const ml_column* cols, int32_t 
                 std::unique_lock<std::shared_mutex> lk(h->rw);
                 h->streams.sync();
                 if (h->run.s) CK(cudaStreamSynchronize(h->run.s));
-                g = (double)groups();
-                rate = std::max(0.0, (g - g0) / (double)last);
+                const double now = (double)groups();
+                base = std::min(base, now);  // spilled meanwhile
+                g = now - base;
+                // other threads' groups count too, but a row brings one at most
+                rate = std::min(1.0, std::max(0.0, (g - g0) / (double)last));
                 if (done == kFirstRows) rate0 = rate;
-                const uint64_t want = (uint64_t)groups_ahead(g0, g, rate0, rate, (double)next) + 1024;
+                const uint64_t want = (uint64_t)(base + groups_ahead(g0, g, rate0, rate, (double)next)) + 1024;
                 if (want > h->gid_cap) {
                     try {
                         h->grow(std::min<uint64_t>(want, 0x7FFFFFFFull), s, local->ew);
                         h->resizes++;
                     } catch (const MlError& e) {
-                        if (e.code != ML_ERR_BUDGET) throw;  // rows that do not fit will overflow, and may spill
+                        // no room for a forecast (the budget, or the device): rows that do not fit will overflow, and may spill
+                        if (e.code != ML_ERR_BUDGET && e.code != ML_ERR_CUDA) throw;
                     }
                 }
             }
@@ -2903,6 +2911,7 @@ int ml_gpu_hashagg_run_resident(ml_hashagg* h, const ml_column* cols, int32_t nc
     for (auto& a : h->aggs)
         if (a.has_arg && !a.vcnt_on && !a.null_seen && a.kind != A_COUNT && (a.arg.maybe_null || h->pipe.reads_nullable(a.arg, L)))
             raise(ML_ERR_UNSUPPORTED, "ml_gpu_hashagg_run_resident: an aggregate input can be NULL; use a local sink");
+    h->fed = true;
     const int w = 1 + (int)h->pipe.probes.size();
     const bool can_overflow = !h->ungrouped && h->group_probe < 0;
     const uint64_t ovf_cap = can_overflow ? std::max<uint64_t>((uint64_t)L.P.n, 1024) : 0;
