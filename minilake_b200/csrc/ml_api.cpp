@@ -2217,7 +2217,6 @@ struct ml_hashagg {
         DevBuf nslots, ngk, ngn;
         if (hashed) {
             nslots = DevBuf(ctx, ncap * 8 * sw, res.get());
-            CK(cudaMemsetAsync(nslots.get(), 0, ncap * 8 * sw, s));
             ngk = DevBuf(ctx, (size_t)ngid * 8 * nw, res.get());
             ngn = DevBuf(ctx, (size_t)ngid * 4, res.get());
         }
@@ -2225,6 +2224,8 @@ struct ml_hashagg {
         std::vector<DevBuf> nvc(aggs.size());
         for (size_t k = 0; k < aggs.size(); k++)
             if (aggs[k].vcnt_on && aggs[k].kind != A_AVG) nvc[k] = DevBuf(ctx, (size_t)ngid * 8, res.get());
+        // enqueued only now: a refused allocation gives the others back to a pool that all threads share
+        if (hashed) CK(cudaMemsetAsync(nslots.get(), 0, ncap * 8 * sw, s));
         if (old_cap) {  // keep the existing groups
             if (hashed) {
                 for (int w = 0; w < nw; w++)
