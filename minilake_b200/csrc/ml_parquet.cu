@@ -229,13 +229,19 @@ struct SnapJob {
     const uint8_t* src;
     uint8_t* dst;
     uint32_t src_len, dst_len;
-    uint32_t plan;   // the page's plan in the plan buffer: [mode, first element, nfrag + 1 element numbers]
+    uint32_t plan;   // the page's plan in the plan buffer (SnapPlan)
     uint32_t nfrag;  // 64 KB fragments of its output
     uint32_t blk0;   // its first kSnapBlk block in the group's block array
     uint32_t pad_;
     uint64_t tab0;   // its first byte in the group's map table
     uint64_t elem0;  // its first element in the group's element list
 };
+// The plan of a page with n fragments: its mode, the first element's stream position, the number of every
+// fragment's first element and of all elements, the stream positions of the former, and where the chain
+// stopped ({stream position, output position, element}) when the page is taken in parts.
+__host__ __device__ constexpr uint32_t snap_plan_words(uint32_t n) { return 2 * n + 6; }
+__device__ __forceinline__ uint32_t snap_plan_pos(uint32_t n) { return n + 3; }
+__device__ __forceinline__ uint32_t snap_plan_state(uint32_t n) { return 2 * n + 3; }
 struct SnapMap {  // the chain from a stream byte to the end of its block
     uint32_t exit;  // stream position of the first element past the block, or kSnapNone
     uint32_t out;   // bytes the chain's elements write
@@ -256,13 +262,21 @@ constexpr int kSnapThreads = 1024;
 constexpr uint32_t kSnapPer = kSnapBlk / kSnapThreads;
 constexpr uint32_t kSnapNone = 0xFFFFFFFFu;
 // plan modes: 0 the length varint is malformed, 1 the serial pass decodes the page, 2 its
-// fragments decode in parallel
-constexpr uint32_t kSnapSerial = 1, kSnapSplit = 2;
+// fragments decode in parallel, 3 the chain goes on in the page's next part
+constexpr uint32_t kSnapSerial = 1, kSnapSplit = 2, kSnapChain = 3;
 constexpr uint32_t kSnapPiece = 2048, kSnapPieces = 2048;  // long literals, cut into pieces for the warps
 constexpr size_t kSnapMapSmem = kSnapBlk * 8 + kSnapBlk + 32;
 constexpr size_t kSnapFragSmem = kSnapFrag * 3 + kSnapPieces * 8;
-// Stream bytes per group of pages decoded together: the maps take 16 bytes per stream byte.
+// Stream bytes per group of pages decoded together: the maps take 16 bytes per stream byte, the element list
+// four.  A larger page is a group of its own, taken in parts: the maps and the chain in parts of kSnapGroupBytes, then
+// the list and the decode of the fragments that start in kSnapPart bytes.  The list of a part goes on for the
+// stream of one fragment (an output byte takes six bytes at most: a literal with a four-byte length), and holds an
+// element at its number modulo kSnapRing.
 constexpr uint64_t kSnapGroupBytes = 32ull << 20;
+constexpr uint32_t kSnapPart = (uint32_t)kSnapGroupBytes - (1u << 20), kSnapPast = 6 * kSnapFrag / kSnapBlk + 1;
+constexpr uint32_t kSnapRing = 1u << 24;
+static_assert(kSnapPart % kSnapBlk == 0 && (kSnapPart + kSnapPast * kSnapBlk) / 2 + 1 <= kSnapRing, "a part's elements");
+static_assert((uint64_t)kSnapRing * 8 <= kSnapGroupBytes * 16, "the list takes the maps' place");
 
 // One element header at s[0..avail): its size h (tag plus length or offset bytes), kind (0
 // literal, 1 copy), output length and copy offset; false if it does not fit in `avail`.
@@ -438,7 +452,8 @@ __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_flat(const SnapFlat*
 // past the block (or that does not parse) points to itself.  States only ever move further along the
 // chain and are read and written whole, so the rounds need no second buffer: bound by shared-memory
 // round trips, log2(kSnapBlk / 2) of them.
-__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_maps(const SnapJob* jobs, const uint2* blocks, SnapMap* tab) {
+// `lo`: the stream byte that the table starts at (0, or a part's first).
+__global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_maps(const SnapJob* jobs, const uint2* blocks, SnapMap* tab, uint32_t lo) {
     extern __shared__ __align__(16) uint8_t snap_smem[];
     uint64_t* st = (uint64_t*)snap_smem;
     uint8_t* win = snap_smem + kSnapBlk * 8;
@@ -480,7 +495,7 @@ __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_maps(const SnapJob* 
         SnapMap m{kSnapNone, 0, 0, 0};
         if (snap_elem(w + p, J.src_len - b0 - p, step, len))
             m = SnapMap{b0 + p + step, (uint32_t)(v[e] >> 32) + len, ((uint32_t)(v[e] >> 16) & 0xFFFFu) + 1u, 0};
-        *(uint4*)(tab + J.tab0 + b0 + q) = *(const uint4*)&m;
+        *(uint4*)(tab + J.tab0 + (b0 - lo) + q) = *(const uint4*)&m;
     }
 }
 
@@ -489,13 +504,18 @@ __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_maps(const SnapJob* 
 // for the 89 blocks of a 721 KB stream).  But chains that start at different bytes soon meet, so where the chain
 // from a block's first byte leaves it is mostly where the real one does: the lanes load the next 32 blocks' maps at
 // those places together, and the walk takes a lane's map where its guess is right (15.5 us), else loads it.
+// The maps are those of the stream bytes [lo, hi) (a page's part; all of it otherwise): the chain goes on where
+// it left the part before.
 __global__ void __launch_bounds__(32) k_pq_snappy_chain(const SnapJob* jobs, const SnapMap* tab, SnapEntry* entries,
-                                                        uint32_t* plan) {
+                                                        uint32_t* plan, uint32_t lo, uint32_t hi) {
     const uint32_t lane = threadIdx.x;
     const SnapJob J = jobs[blockIdx.x];
     uint32_t* pl = plan + J.plan;
+    uint32_t* const state = pl + snap_plan_state(J.nfrag);
+    const uint32_t end = min(J.src_len, hi);
     uint32_t start = 0, total = 0;
     bool ok = false;
+    if (lo && pl[0] != kSnapChain) return;
     for (int shift = 0; shift < 35 && start < J.src_len; shift += 7) {  // the uncompressed length
         const uint32_t b = J.src[start++];
         if (shift == 28 && (b & 0x70)) break;  // past 32 bits
@@ -512,27 +532,28 @@ __global__ void __launch_bounds__(32) k_pq_snappy_chain(const SnapJob* jobs, con
     }
     const SnapMap* maps = tab + J.tab0;
     bool split = J.nfrag >= 1;
-    uint32_t pos = start, elem = 0;
-    uint64_t out = 0;
+    uint32_t pos = lo ? state[0] : start, elem = lo ? state[2] : 0;
+    uint64_t out = lo ? state[1] : 0;
+    __syncwarp();  // before lane 0 writes them
     uint32_t g0 = 0, guess = kSnapNone;  // lane l holds block g0 + l's guessed entry and the map there
     uint4 gm = make_uint4(kSnapNone, 0, 0, 0);
     bool held = false;
-    while (split && pos < J.src_len) {  // the same in every lane
+    while (split && pos < end) {  // the same in every lane
         const uint32_t blk = pos / kSnapBlk;
         if (!held || blk - g0 >= 32) {
             g0 = blk;
             held = true;
             const uint64_t mine = (uint64_t)g0 + lane;
-            guess = lane == 0 ? pos : mine * kSnapBlk < J.src_len ? maps[(mine - 1) * kSnapBlk].exit : kSnapNone;
-            if (guess >= J.src_len || guess / kSnapBlk != mine) guess = kSnapNone;
-            if (guess != kSnapNone) gm = __ldg((const uint4*)(maps + guess));
+            guess = lane == 0 ? pos : mine * kSnapBlk < end ? maps[(mine - 1) * kSnapBlk - lo].exit : kSnapNone;
+            if (guess >= end || guess / kSnapBlk != mine) guess = kSnapNone;
+            if (guess != kSnapNone) gm = __ldg((const uint4*)(maps + (guess - lo)));
         }
         const int from = (int)(blk - g0);
         uint4 m;
         m.x = __shfl_sync(0xFFFFFFFFu, gm.x, from);
         m.y = __shfl_sync(0xFFFFFFFFu, gm.y, from);
         m.z = __shfl_sync(0xFFFFFFFFu, gm.z, from);
-        if (__shfl_sync(0xFFFFFFFFu, guess, from) != pos) m = __ldg((const uint4*)(maps + pos));
+        if (__shfl_sync(0xFFFFFFFFu, guess, from) != pos) m = __ldg((const uint4*)(maps + (pos - lo)));
         if (lane == 0) entries[J.blk0 + blk] = SnapEntry{pos, (uint32_t)out, elem, 1u};
         out += m.y;
         elem += m.z;
@@ -540,7 +561,10 @@ __global__ void __launch_bounds__(32) k_pq_snappy_chain(const SnapJob* jobs, con
         split = m.x != kSnapNone && out <= total;
     }
     if (lane) return;
-    if (split && out == total) {
+    if (split && pos < J.src_len) {
+        state[0] = pos, state[1] = (uint32_t)out, state[2] = elem;
+        pl[0] = kSnapChain;
+    } else if (split && out == total) {
         pl[2 + J.nfrag] = elem;
         pl[0] = kSnapSplit;
     } else {
@@ -553,7 +577,8 @@ __global__ void __launch_bounds__(32) k_pq_snappy_chain(const SnapJob* jobs, con
 // the marked ones while the jumps double, so all are marked after log2 of their number rounds (a
 // mark set early by a neighbour's write of the same round is a real element too).
 __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_list(const SnapJob* jobs, const uint2* blocks,
-                                                                 const SnapEntry* entries, uint32_t* plan, uint2* elems) {
+                                                                 const SnapEntry* entries, uint32_t* plan, uint2* elems,
+                                                                 uint32_t elem_mask) {
     __shared__ __align__(16) uint16_t jmp[kSnapBlk];
     __shared__ __align__(16) uint8_t mark[kSnapBlk];
     __shared__ __align__(16) uint8_t win[kSnapBlk + 32];
@@ -633,9 +658,12 @@ __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_list(const SnapJob* 
     for (uint32_t e = 0; e < kSnapPer; e++) {
         if (!((marks >> (8 * e)) & 1)) continue;
         const uint32_t l = length(e), at = o & (kSnapFrag - 1);
-        elems[J.elem0 + i] = make_uint2(b0 + tid * kSnapPer + e, o);
+        elems[J.elem0 + (i & elem_mask)] = make_uint2(b0 + tid * kSnapPer + e, o);
         bad = bad || l > kSnapFrag - at;  // crossing a fragment's end
-        if (at == 0 && (o >> 16) < J.nfrag) pl[2 + (o >> 16)] = i;
+        if (at == 0 && (o >> 16) < J.nfrag) {
+            pl[2 + (o >> 16)] = i;
+            pl[snap_plan_pos(J.nfrag) + (o >> 16)] = b0 + tid * kSnapPer + e;
+        }
         i++;
         o += l;
     }
@@ -648,8 +676,9 @@ __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_list(const SnapJob* 
 // ptr[i] = ptr[ptr[i]] until nothing moves ends at literal bytes.  A copy overlapping itself points
 // into the pattern it repeats.  192 KB of shared memory, so one block per SM: bound by the
 // shared-memory gathers of the rounds (64 bytes per thread and round, resolved pairs skipped).
+// Of a page in parts, the fragments that start in the stream bytes [lo, hi); all of them otherwise.
 __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_frag(const SnapJob* jobs, const uint2* frags, const uint2* elems,
-                                                                 uint32_t* plan) {
+                                                                 uint32_t* plan, uint32_t elem_mask, uint32_t lo, uint32_t hi) {
     extern __shared__ __align__(16) uint8_t snap_smem[];
     uint16_t* ptr = (uint16_t*)snap_smem;
     uint8_t* val = snap_smem + kSnapFrag * 2;
@@ -662,6 +691,8 @@ __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_frag(const SnapJob* 
     if (threadIdx.x == 0) {
         mode = *(volatile uint32_t*)pl;
         npiece = 0;
+        const uint32_t pos = pl[snap_plan_pos(J.nfrag) + f.y];
+        if (pos < lo || pos >= hi) mode = 0;
     }
     __syncthreads();
     if (mode != kSnapSplit) return;
@@ -675,7 +706,7 @@ __global__ void __launch_bounds__(kSnapThreads) k_pq_snappy_frag(const SnapJob* 
     const uint2* E = elems + J.elem0;
 #pragma unroll 1
     for (uint32_t i = pl[2 + f.y] + tid, i1 = pl[3 + f.y]; i < i1; i += kSnapThreads) {
-        const uint2 el = E[i];
+        const uint2 el = E[i & elem_mask];
         const uint8_t* e = J.src + el.x;  // five readable bytes: the chunk buffer is padded past its end
         const uint32_t o = el.y - o0;
         uint32_t step, len;
@@ -1722,7 +1753,7 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
             for (uint32_t k = 0; k < nblk; k++) blocks.push_back(uint2{id, k});
             jobs.push_back(SnapJob{dc + pg.payload + lv, up + uoff[i] + lv, slen, dlen, plan_words, nfrag,
                                    (uint32_t)g.nblks, 0u, g.bytes, g.elems});
-            plan_words += nfrag + 3;
+            plan_words += snap_plan_words(nfrag);
             g.njobs++, g.nfrags += (int)nfrag, g.nblks += (int)nblk;
             g.bytes += slen, g.elems += slen / 2 + 1;  // an element spans at least two stream bytes
         } else {
@@ -1791,27 +1822,46 @@ extern "C" int ml_gpu_parquet_decode(ml_ctx* ctx, const uint8_t* chunk, int64_t 
             splan = DevBuf(ctx, (size_t)plan_words * 4, nullptr);
             uint64_t most = 0, most_elems = 0;
             int most_blks = 0;
-            for (const SnapGroup& g : groups)
-                most = std::max(most, g.bytes), most_elems = std::max(most_elems, g.elems), most_blks = std::max(most_blks, g.nblks);
+            for (const SnapGroup& g : groups) {
+                const bool parts = g.bytes > kSnapGroupBytes;
+                most = std::max(most, parts ? kSnapGroupBytes : g.bytes);
+                most_elems = std::max(most_elems, parts ? (uint64_t)kSnapRing : g.elems);
+                most_blks = std::max(most_blks, g.nblks);
+            }
             // the maps; the element list takes their place once the chains are known
             smap = DevBuf(ctx, std::max<size_t>(std::max(most * sizeof(SnapMap), most_elems * sizeof(uint2)), 16), nullptr);
             sentry = DevBuf(ctx, std::max<size_t>((size_t)most_blks * sizeof(SnapEntry), 16), nullptr);
             // per call: the attribute belongs to the current device's copy of the kernel
             CK(cudaFuncSetAttribute(k_pq_snappy_maps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSnapMapSmem));
             CK(cudaFuncSetAttribute(k_pq_snappy_frag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSnapFragSmem));
+            uint32_t* const plan = splan.get<uint32_t>();
+            SnapMap* const tab = smap.get<SnapMap>();
+            SnapEntry* const entries = sentry.get<SnapEntry>();
+            uint2* const elist = smap.get<uint2>();
             for (const SnapGroup& g : groups) {
-                if (g.nblks) {
-                    CK(cudaMemsetAsync(sentry.get(), 0, (size_t)g.nblks * sizeof(SnapEntry), s));
-                    k_pq_snappy_maps<<<g.nblks, kSnapThreads, kSnapMapSmem, s>>>(J, B + g.blk0, smap.get<SnapMap>());
+                // a page in parts, or all pages of the group at once
+                const bool parts = g.bytes > kSnapGroupBytes;
+                const uint32_t mask = parts ? kSnapRing - 1 : ~0u;
+                const uint32_t blks = (uint32_t)g.nblks, group = (uint32_t)(kSnapGroupBytes / kSnapBlk), part = kSnapPart / kSnapBlk;
+                if (blks) CK(cudaMemsetAsync(entries, 0, (size_t)blks * sizeof(SnapEntry), s));
+                if (parts)  // no fragment starts anywhere yet
+                    CK(cudaMemsetAsync(plan + jobs[g.job0].plan, 0xFF, (size_t)snap_plan_words(jobs[g.job0].nfrag) * 4, s));
+                for (uint32_t b = 0; b == 0 || b < blks; b += parts ? group : std::max(blks, 1u)) {
+                    const uint32_t m = parts ? std::min(group, blks - b) : blks, lo = b * kSnapBlk;
+                    if (m) k_pq_snappy_maps<<<m, kSnapThreads, kSnapMapSmem, s>>>(J, B + g.blk0 + b, tab, lo);
+                    k_pq_snappy_chain<<<g.njobs, 32, 0, s>>>(J + g.job0, tab, entries, plan, lo, parts ? lo + m * kSnapBlk : ~0u);
+                    ctx->count_launch(m ? 2 : 1);
                 }
-                k_pq_snappy_chain<<<g.njobs, 32, 0, s>>>(J + g.job0, smap.get<SnapMap>(), sentry.get<SnapEntry>(), splan.get<uint32_t>());
-                if (g.nblks)
-                    k_pq_snappy_list<<<g.nblks, kSnapThreads, 0, s>>>(J, B + g.blk0, sentry.get<SnapEntry>(), splan.get<uint32_t>(),
-                                                                      smap.get<uint2>());
-                if (g.nfrags)
-                    k_pq_snappy_frag<<<g.nfrags, kSnapThreads, kSnapFragSmem, s>>>(J, F + g.frag0, smap.get<uint2>(), splan.get<uint32_t>());
-                k_pq_snappy_serial<<<g.njobs, 32, 0, s>>>(J + g.job0, splan.get<uint32_t>(), derr);
-                ctx->count_launch(2 + (g.nblks ? 2 : 0) + (g.nfrags ? 1 : 0));
+                for (uint32_t b = 0; b < blks; b += parts ? part : blks) {
+                    const uint32_t m = parts ? std::min(part + kSnapPast, blks - b) : blks, lo = b * kSnapBlk;
+                    k_pq_snappy_list<<<m, kSnapThreads, 0, s>>>(J, B + g.blk0 + b, entries, plan, elist, mask);
+                    if (g.nfrags)
+                        k_pq_snappy_frag<<<g.nfrags, kSnapThreads, kSnapFragSmem, s>>>(J, F + g.frag0, elist, plan, mask, lo,
+                                                                                       parts ? lo + kSnapPart : ~0u);
+                    ctx->count_launch(g.nfrags ? 2 : 1);
+                }
+                k_pq_snappy_serial<<<g.njobs, 32, 0, s>>>(J + g.job0, plan, derr);
+                ctx->count_launch();
             }
         }
     }
