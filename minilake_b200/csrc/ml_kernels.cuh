@@ -33,11 +33,11 @@ constexpr int kMaxExchangeParts = 64;
 int xpart_blocks(int64_t n);
 void launch_xpart_count(const uint64_t* h, int64_t n, int nparts, uint32_t* counts, cudaStream_t s);
 void launch_xpart_scatter(const uint64_t* h, int64_t n, int nparts, const uint64_t* offs, uint32_t* perm, cudaStream_t s);
-// Initialize group blocks [from, to) to the identities of the aggregates.
 // *skip = the first rows of a batch showed that the group table is too small for the rest: some did
 // not fit, or the groups fill more than a quarter of it.
 void launch_agg_guard(const unsigned long long* ovf_count, const uint32_t* ngroups, uint32_t gid_cap, uint32_t* skip,
                       cudaStream_t s);
+// Initialize group blocks [from, to) to the identities of the aggregates.
 void launch_acc_init(const AggArgs& A, uint32_t from, uint32_t to, cudaStream_t s);
 // Final values: keys decoded into `key_out` (fixed-width or u32 string ids), aggregates into
 // `agg_out`; validity as u32 words (LSB first) in *_valid.
@@ -114,7 +114,6 @@ void launch_strid(const uint32_t* off, const uint8_t* bytes, const uint64_t* val
                   uint32_t* canon, uint32_t* err, cudaStream_t s);
 
 // Gathers.
-// dst row i = src row idx[i]; width is 1, 4 or a multiple of 8 bytes
 // Rows idx[0..k) of several fixed-width columns (widths 1, 4 and 8) and their validity words at once.
 constexpr int kGatherCols = 16;
 struct GatherCol {
@@ -129,6 +128,7 @@ struct GatherCols {
     GatherCol c[kGatherCols];
 };
 void launch_gather_cols(const GatherCols& G, const uint32_t* idx, int64_t k, cudaStream_t s);
+// dst row i = src row idx[i]; width is 1, 4 or a multiple of 8 bytes
 void launch_gather_fixed(const void* src, int width, const uint32_t* idx, int64_t k, void* dst, cudaStream_t s);
 void launch_gather_valid(const uint64_t* src, const uint32_t* idx, int64_t k, uint32_t* dst, cudaStream_t s);
 void launch_utf8_lengths(const uint32_t* off, const uint32_t* idx, int64_t k, uint32_t* len, cudaStream_t s);

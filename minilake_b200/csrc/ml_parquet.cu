@@ -863,16 +863,16 @@ struct PageDev {
     int32_t encoding;
     int64_t row0;
     uint32_t nrows;
-    // filled by k_pq_layout
+    // filled by k_pq_levels
     const uint8_t* levels;
     uint32_t levels_len;
     const uint8_t* values;
     uint32_t values_len;
     int32_t idx_width;  // dictionary-index (or RLE boolean) bit width; -1: PLAIN values
-    // run tables (levels, then indices), filled by k_pq_runs
+    // run tables from the page's first row on: of the levels (k_pq_levels) and of the indices (k_pq_indices)
     uint64_t lv_run0, ix_run0;
     uint32_t lv_nruns, ix_nruns;
-    uint64_t valid0;  // present values of the chunk before this page's first row
+    uint64_t valid0;  // present values of the chunk before this page's first row (k_pq_indices)
 };
 
 __device__ uint32_t le32(const uint8_t* p) { return p[0] | (p[1] << 8) | (p[2] << 16) | ((uint32_t)p[3] << 24); }
