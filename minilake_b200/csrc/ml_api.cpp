@@ -1606,6 +1606,7 @@ int ml_gpu_join_build_sink(ml_join_build_local* local, const ml_column* cols, in
     REQUIRE(!j->table, "join build sink already finalized");
     Ctx* ctx = j->ctx;
     ctx->set_current();
+    const StreamScope scope(local->s);
     check_sel_bounds(sel, nsel, nrows);
     DevBuf sel_hold;
     const uint32_t* dsel = device_sel(ctx, sel, nsel, sel_hold, local->s);
@@ -1645,6 +1646,7 @@ int ml_gpu_join_build_finalize(ml_join_build* j, ml_join_table** table) {
     }
     j->streams.sync();
     cudaStream_t s = j->streams.own();
+    const StreamScope scope(s);
     auto jt = std::make_unique<ml_join_table>();
     jt->ctx = ctx;
     jt->res = std::make_unique<Reservation>(ctx, "HashJoinBuild(table)");
@@ -2613,6 +2615,7 @@ int ml_gpu_hashagg_create(ml_ctx* ctx, const ml_pipe_op* prologue, int32_t nprol
     else if (h->group_probe >= 0) want = (uint64_t)std::max<int64_t>(h->pipe.probes[h->group_probe].jt->batch.nrows, 1);
     else want = (uint64_t)std::min<int64_t>(std::max<int64_t>(size_hint > 0 ? size_hint : 1024, 16), 0x7FFFFFFF);
     h->hinted = size_hint > 0;
+    const StreamScope scope(ctx->stream);
     h->grow(want, ctx->stream, ew);
     *out = h.release();
     API_END
@@ -2635,6 +2638,7 @@ int ml_gpu_hashagg_sink(ml_hashagg_local* local, const ml_column* cols, int32_t 
     Ctx* ctx = h->ctx;
     ctx->set_current();
     cudaStream_t s = local->s;
+    const StreamScope scope(s);
     check_sel_bounds(sel, nsel, nrows);
     DevBuf sel_hold;
     const uint32_t* dsel = device_sel(ctx, sel, nsel, sel_hold, s);
@@ -2857,6 +2861,7 @@ int ml_gpu_hashagg_rebind(ml_hashagg* h, const ml_pipe_op* prologue, int32_t npr
     for (size_t p = 0; p < h->pipe.probes.size(); p++) h->pipe.probes[p].jt = fresh.pipe.probes[p].jt;
     for (size_t k = 0; k < h->aggs.size(); k++) h->aggs[k].arg = fresh.aggs[k].arg;
     cudaStream_t s = h->streams.own();
+    const StreamScope scope(s);
     if (!b.code.empty())
         CK(cudaMemcpyAsync(h->pipe.d_prog, b.code.data(), b.code.size() * sizeof(Instr), cudaMemcpyHostToDevice, s));
     if (!b.arena.empty()) CK(cudaMemcpyAsync(h->pipe.d_arena, b.arena.data(), b.arena.size(), cudaMemcpyHostToDevice, s));
@@ -2873,6 +2878,7 @@ int ml_gpu_hashagg_reset(ml_hashagg* h) {
     h->streams.sync();
     if (h->run.s) CK(cudaStreamSynchronize(h->run.s));
     cudaStream_t s = h->streams.own();
+    const StreamScope scope(s);
     CK(cudaMemsetAsync(h->ngroups.get(), 0, 16, s));
     if (h->cap) CK(cudaMemsetAsync(h->slots.get(), 0, h->cap * 8 * (h->keys.nwords == 1 ? 2 : 4), s));
     launch_acc_init(h->args(nullptr, nullptr, 0), 0, h->gid_cap, s);
@@ -2902,6 +2908,7 @@ int ml_gpu_hashagg_run_resident(ml_hashagg* h, const ml_column* cols, int32_t nc
         R.tables = DevBuf(ctx, 64 << 10, nullptr);
     }
     cudaStream_t s = R.s;
+    const StreamScope scope(s);
     Staging st(ctx);
     Pipeline::Launch L;
     h->pipe.prepare(L, cols, ncols, nrows, nullptr, 0, s, st, nullptr, R.tables.get<uint8_t>(), R.tables.bytes());
@@ -3219,6 +3226,7 @@ int ml_gpu_hashagg_finalize(ml_hashagg* h, ml_batch** out) {
     h->streams.sync();
     if (h->run.s) CK(cudaStreamSynchronize(h->run.s));
     cudaStream_t s = h->streams.own();
+    const StreamScope scope(s);
     if (!h->spill_events) {
         *out = hashagg_emit(h, s).release();
         return ML_OK;
@@ -3378,6 +3386,7 @@ int ml_gpu_topn_sink(ml_topn_local* local, const ml_column* cols, int32_t ncols,
     ml_topn* t = local->sink;
     Ctx* ctx = t->ctx;
     ctx->set_current();
+    const StreamScope scope(local->s);
     check_sel_bounds(sel, nsel, nrows);
     DevBuf sel_hold;
     const uint32_t* dsel = device_sel(ctx, sel, nsel, sel_hold, local->s);
@@ -3424,6 +3433,7 @@ int ml_gpu_topn_finalize(ml_topn* t, ml_batch** out) {
         cands = std::move(t->cands);
     }
     cudaStream_t s = t->streams.own();
+    const StreamScope scope(s);
     if (cands.size() == 1 && !t->full_sort()) {  // one local sink: its candidates are the sorted top N already
         *out = cands[0].release();
         return ML_OK;
@@ -3770,6 +3780,7 @@ void query_capture(ml_query* q) {
     Ctx* ctx = q->ctx;
     ml_hashagg* h = q->agg;
     cudaStream_t s = q->s;
+    const StreamScope scope(s);
     // hash-table builds: the key programs over the build batch (as ml_gpu_join_build_finalize)
     for (auto& bp : q->builds) {
         ml_query::Build& b = *bp;
@@ -3943,6 +3954,7 @@ std::unique_ptr<ml_batch> query_plan_run(ml_query* q) {
     std::unique_ptr<ml_batch> groups(raw);
     if (!q->topn) return groups;
     auto res = std::make_unique<Reservation>(ctx, "Query(output)");
+    const StreamScope scope(q->s);
     auto best = topn_batch(ctx, *groups, q->keys, q->limit, q->s, res.get());
     best->res = std::move(res);
     q->k = best->nrows;
@@ -3981,6 +3993,7 @@ void query_finish(ml_query* q) {
 std::unique_ptr<ml_batch> query_replay(ml_query* q) {
     Ctx* ctx = q->ctx;
     cudaStream_t s = q->s;
+    const StreamScope scope(s);
     query_launch(q);
     auto out = std::make_unique<ml_batch>();
     out->ctx = ctx;

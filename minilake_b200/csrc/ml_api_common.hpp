@@ -16,7 +16,8 @@ struct ml_ctx : mlg::Ctx {
 struct OpStream {
     mlg::Ctx* ctx;
     cudaStream_t s;
-    explicit OpStream(mlg::Ctx* c) : ctx(c), s(c->new_stream()) {}
+    mlg::StreamScope scope;
+    explicit OpStream(mlg::Ctx* c) : ctx(c), s(c->new_stream()), scope(s) {}
     ~OpStream() {
         cudaStreamSynchronize(s);
         ctx->free_stream(s);

@@ -18,7 +18,16 @@ void set_last_error(const std::string& m) { t_err = m; }
 void set_budget_error(const BudgetInfo& b) { t_budget = b; }
 const char* last_error() { return t_err.c_str(); }
 const BudgetInfo& last_budget() { return t_budget; }
-[[noreturn]] void raise(int code, const std::string& msg) { throw MlError(code, msg); }
+static thread_local StreamScope* t_scope = nullptr;
+StreamScope::StreamScope(cudaStream_t s) : s_(s), outer_(t_scope) { t_scope = this; }
+StreamScope::~StreamScope() { t_scope = outer_; }
+[[noreturn]] void raise(int code, const std::string& msg) {
+    for (const StreamScope* k = t_scope; k; k = k->outer_) {
+        cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;  // a stream being captured has nothing in flight
+        if (cudaStreamIsCapturing(k->s_, &c) == cudaSuccess && c == cudaStreamCaptureStatusNone) cudaStreamSynchronize(k->s_);
+    }
+    throw MlError(code, msg);
+}
 void check_cuda(cudaError_t e, const char* what) {
     if (e != cudaSuccess) raise(ML_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }

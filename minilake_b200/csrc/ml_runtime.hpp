@@ -25,7 +25,22 @@ struct MlError : std::runtime_error {
     int code;
     MlError(int c, const std::string& m) : std::runtime_error(m), code(c) {}
 };
+// Waits for the streams of the calling thread's StreamScopes, then throws.
 [[noreturn]] void raise(int code, const std::string& msg);
+
+// The stream that the calling thread enqueues on from here to the end of the scope.  An error unwinds device
+// and pinned buffers into pools that all threads share, so raise() first waits for the work that uses them.
+class StreamScope {
+   public:
+    explicit StreamScope(cudaStream_t s);
+    ~StreamScope();
+    StreamScope(const StreamScope&) = delete;
+
+   private:
+    friend void raise(int, const std::string&);
+    cudaStream_t s_;
+    StreamScope* outer_;
+};
 void check_cuda(cudaError_t e, const char* what);
 #define CK(x) ::mlg::check_cuda((x), #x)
 

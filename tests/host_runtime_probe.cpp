@@ -53,6 +53,7 @@ cudaError_t cudaStreamSynchronize(cudaStream_t s) {
     run(s);
     return cudaSuccess;
 }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* c) { return *c = cudaStreamCaptureStatusNone, cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() {
     for (auto& q : g_queue) run(q.first);
     return cudaSuccess;
@@ -126,10 +127,34 @@ void staging_dies() {
     cudaDeviceSynchronize();
     check("a block that a copy reads is not handed out when its owner goes", all(*mine, 1) && all(*other, 2));
 }
+
+// An allocation that the budget refuses while work on buffers that the error gives back is still in flight.
+void errors_wait() {
+    Ctx ctx(0, 64 << 20, 0);
+    const cudaStream_t a = ctx.new_stream(), b = ctx.new_stream();
+    bool refused = false;
+    try {
+        const StreamScope outer(a);
+        const StreamScope scope(b);
+        DevBuf mine(&ctx, 1 << 20, nullptr);
+        cudaMemsetAsync(mine.get(), 1, 1 << 20, a);
+        Reservation res(&ctx, "Test");
+        DevBuf large(&ctx, 128 << 20, &res);
+    } catch (const MlError& e) {
+        refused = e.code == ML_ERR_BUDGET;
+    }
+    DevBuf other(&ctx, 1 << 20, nullptr);  // the next caller's, perhaps the same memory
+    memset(other.get(), 2, 1 << 20);
+    cudaDeviceSynchronize();
+    bool kept = true;
+    for (size_t i = 0; i < 1 << 20; i++) kept = kept && other.get<uint8_t>()[i] == 2;
+    check("an error waits for the work on the buffers it gives back", refused && kept);
+}
 }  // namespace
 
 int main() {
     staging_grows();
     staging_dies();
+    errors_wait();
     return g_failed ? 1 : 0;
 }
