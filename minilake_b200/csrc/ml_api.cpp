@@ -149,15 +149,21 @@ std::unique_ptr<DevColumn> gather_column(Ctx* ctx, const DevColumn& s, const uin
     return d;
 }
 
-// Rows `idx` (device, k entries, each row at most once) of every column of a batch; the work has finished
-// when it returns.  Few rows of fixed-width and plain string columns take one launch and one wait (a
-// column at a time: two launches for a fixed-width one, seven and a wait for a string).
-std::vector<std::unique_ptr<DevColumn>> gather_rows(Ctx* ctx, const ml_batch& b, const uint32_t* idx, int64_t k,
-                                                    cudaStream_t st, Reservation* res) {
-    std::vector<std::unique_ptr<DevColumn>> out;
-    // strings get room for 64 KB before their size is known: not under a budget
+// Whether rows of the batch are gathered in one launch with room for their strings: few rows of fixed-width
+// and plain string columns.  Strings get 64 KB before their size is known: not under a budget.
+bool small_gather(const Ctx* ctx, const ml_batch& b, int64_t k) {
     bool small = k > 0 && k <= kSmallRows && (int)b.cols.size() <= kSmallCols && ctx->pool.limit == UINT64_MAX;
     for (auto& c : b.cols) small = small && c->kind != CK_DICT;
+    return small;
+}
+// Rows `idx` (device, k entries, each row at most once) of every column of a batch; the work has finished
+// when it returns.  The small form takes one launch and one wait (a column at a time: two launches for a
+// fixed-width one, seven and a wait for a string).  `voided` (optional): a host word that is set, once the
+// stream was waited for, when the rows are not wanted; the small form then returns no columns.
+std::vector<std::unique_ptr<DevColumn>> gather_rows(Ctx* ctx, const ml_batch& b, const uint32_t* idx, int64_t k,
+                                                    cudaStream_t st, Reservation* res, const uint32_t* voided = nullptr) {
+    std::vector<std::unique_ptr<DevColumn>> out;
+    bool small = small_gather(ctx, b, k);
     if (small) {
         constexpr uint32_t kRoom = 64 << 10;
         SmallCols G{};
@@ -196,6 +202,7 @@ std::vector<std::unique_ptr<DevColumn>> gather_rows(Ctx* ctx, const ml_batch& b,
         ctx->count_launch();
         if (strings) CK(cudaMemcpyAsync(told.p, G.info, (size_t)G.n * 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        if (voided && *voided) return {};
         for (int i = 0; i < G.n; i++)
             if (out[i]->kind == CK_UTF8) {
                 out[i]->str_bytes = told.as<uint32_t>()[i];
@@ -752,10 +759,12 @@ std::unique_ptr<ml_batch> topn_batch(Ctx* ctx, ml_batch& b, const std::vector<So
         const uint32_t* rows = (const uint32_t*)(base + ro);
         const TopNScratch t{state, (TopNBound*)(base + 16), (uint64_t*)(base + mn), (uint64_t*)(base + lp), (uint32_t*)(base + lr)};
         CK(cudaMemsetAsync(state, 0, 16, st));
-        // fixed-width columns are gathered before the host knows that the rows are the result (k rows exist
-        // either way); what a string column needs depends on the rows, and a budget counts what is asked for
+        // fixed-width columns, and the small form's string columns, are gathered before the host knows that the
+        // rows are the result (k rows exist either way); what a string column of the other form needs depends on
+        // the rows, and a budget counts what is asked for
         bool wait = ctx->pool.limit != UINT64_MAX;
-        for (auto& c : b.cols) wait = wait || c->kind != CK_FIXED;
+        if (!small_gather(ctx, b, k))
+            for (auto& c : b.cols) wait = wait || c->kind != CK_FIXED;
         ErrWord told(ctx);
         for (bool tied = false;; tied = true) {
             KernelTimer kt(ctx, st, tied ? "topn_ties" : "topn");
@@ -765,7 +774,7 @@ std::unique_ptr<ml_batch> topn_batch(Ctx* ctx, ml_batch& b, const std::vector<So
             CK(cudaMemcpyAsync(told.h, state + 1, 4, cudaMemcpyDeviceToHost, st));
             if (wait) CK(cudaStreamSynchronize(st));
             if (!wait || !*told.h) {
-                out->cols = gather_rows(ctx, b, rows, k, st, res);
+                out->cols = gather_rows(ctx, b, rows, k, st, res, told.h);
                 if (!*told.h) return out;
                 out->cols.clear();
             }
